@@ -130,40 +130,82 @@ extern "C" __global__ void rope_kernel(
 
 // ---------------------------------------------------------------------------
 // flash_attention_split_kv_partial_kernel, reference geometry:
-// grid (B, Hq, C), block (D, 1, 1) with D a multiple of 32 and at most 256.
-// Replaces flash_attention_split_kv_partial.hip.template:31-120.  Each warp
-// walks every (D/32)-th position of the split with vector loads and a shuffle
-// reduction, keeps its own running (m, l, o), and the warps are merged at the
-// end.  This is the compatibility kernel; the fast path is further down.
+// grid (B, Hq, C), block (D, 1, 1) with D 64, 128 or 256.
+// Replaces flash_attention_split_kv_partial.hip.template:31-120.  The warps of a
+// block take runs of P positions in turn, each keeps its own running (m, l, o),
+// and the warps are merged at the end.  This is the compatibility kernel; the
+// fast path is further down.
+//
+// What bounds it is issue slots and the latency of a warp's chain (K and V come through L2 once per query
+// head).  So a warp takes P = U * 256 / D positions per turn: U = 8 or 16 16-byte loads of K and as many of V
+// per lane are in flight while the previous turn is computed, a row's D / 8 lanes reduce their scores together
+// (one shuffle a score where one score took five), fp32 FMAs go two at a time, one exponential per position, and
+// the maximum moves only when a score passes it by kCompatLazyMax.  Eight sequences of 700 to 3,960 positions,
+// 32 query heads on 2 KV heads of 128, 8 splits, append and reduce included: 88 us a layer with one position
+// per warp and turn, 42 us so (U = 8, 128 registers, four blocks of 128 threads per SM; U = 16 needs 255
+// registers: 56 us).  Unsplit, four sequences of 103 to 1,383 positions, 12 heads of 128: 178 us against 21 us
+// (U = 16; 27 us with 8: there a block has an SM to itself).
+// kUnsplit: ONE split covering every position, together with the cache append and the normalisation:
+// flash_attention_kernel below.
 // ---------------------------------------------------------------------------
-// kUnsplit: the same walk with ONE split covering every position, preceded by the cache append and
-// followed by the normalisation: flash_attention_kernel below.
-template <int EPL, bool kUnsplit>   // EPL = elements per lane = head_dim / 32
+constexpr int kCompatSharedFloats = 24 + 8 * 256;    // m, l, largest score and o of up to eight warps
+constexpr float kCompatLazyMax = 8.f;    // log2 units: probabilities reach 256 at most
+
+// Eight halves at `p`; kVec: p is 16-byte aligned.
+template <bool kVec>
+__device__ __forceinline__ uint4 load_8_halves(const __half* p) {
+    if constexpr (kVec) return *reinterpret_cast<const uint4*>(p);
+    const unsigned short* h = reinterpret_cast<const unsigned short*>(p);
+    uint4 r;
+    r.x = h[0] | ((uint32_t)h[1] << 16); r.y = h[2] | ((uint32_t)h[3] << 16);
+    r.z = h[4] | ((uint32_t)h[5] << 16); r.w = h[6] | ((uint32_t)h[7] << 16);
+    return r;
+}
+
+struct F32x2 { unsigned long long v; };
+__device__ __forceinline__ F32x2 pack_f32x2(float x, float y) {
+    F32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(x), "f"(y));
+    return r;
+}
+__device__ __forceinline__ float2 unpack_f32x2(F32x2 a) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a.v));
+    return r;
+}
+__device__ __forceinline__ F32x2 fma_f32x2(F32x2 a, F32x2 b, F32x2 c) {
+    F32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+__device__ __forceinline__ F32x2 widen_half2(uint32_t w) {
+    const float2 f = unpack_half2(w);
+    return pack_f32x2(f.x, f.y);
+}
+
+template <int D, bool kUnsplit, bool kVec>
 __device__ __forceinline__ void compat_partial_body(
-    const __half* __restrict__ q, const __half* k_cache, const __half* v_cache,
+    float* sh, const __half* __restrict__ q, const __half* k_cache, const __half* v_cache,
     float* __restrict__ partial_m, float* __restrict__ partial_l, float* __restrict__ partial_o,
     int num_q_heads, int num_kv_heads, float scale,
     const int* __restrict__ kv_cache_offset_ptr, int kv_batch_stride, int max_chunks,
     const __half* __restrict__ k_new = nullptr, const __half* __restrict__ v_new = nullptr,
     __half* __restrict__ output = nullptr)
 {
-    constexpr int D = EPL * 32;
-    __shared__ float sh_m[8], sh_l[8];
-    __shared__ float sh_o[8][D];
+    constexpr int LPR = D / 8;         // lanes per cache row, 16 bytes each
+    constexpr int RPI = 32 / LPR;      // rows per load instruction of a warp
+    // load instructions per turn and tensor (at most LPR): more where a block has an SM to itself, few enough
+    // for four blocks of 128 threads per SM where it has not
+    constexpr int U = (kUnsplit && D > 64) ? 16 : 8;
+    constexpr int P = U * RPI;         // positions per turn of a warp
+    float* sh_m = sh; float* sh_l = sh + 8; float* sh_t = sh + 16; float* sh_o = sh + 24;
 
     const int b = blockIdx.x, h = blockIdx.y, c = kUnsplit ? 0 : blockIdx.z;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    const int sub = lane / LPR, col = (lane % LPR) * 8;
     const int total = kv_cache_offset_ptr[b] + 1;
     const int kv_head = h / (num_q_heads / num_kv_heads);
-    if constexpr (kUnsplit) {
-        // every block writes its KV head's new row (the blocks of a group write identical bytes) and
-        // reads it back only after its own barrier
-        __half* kc = const_cast<__half*>(k_cache) + (long long)b * kv_batch_stride + ((long long)(total - 1) * num_kv_heads + kv_head) * D;
-        __half* vc = const_cast<__half*>(v_cache) + (long long)b * kv_batch_stride + ((long long)(total - 1) * num_kv_heads + kv_head) * D;
-        const long long src = ((long long)b * num_kv_heads + kv_head) * D;
-        for (int d = threadIdx.x; d < D; d += blockDim.x) { kc[d] = k_new[src + d]; vc[d] = v_new[src + d]; }
-        __syncthreads();
-    }
+    const long long row_stride = (long long)num_kv_heads * D;
     const int chunk = kUnsplit ? total : split_chunk_len(total, max_chunks, SPLIT_KV_CHUNK_SIZE, 0);
     const long long stat = ((long long)b * num_q_heads + h) * max_chunks + c;
     const int start = c * chunk;
@@ -173,58 +215,133 @@ __device__ __forceinline__ void compat_partial_body(
         return;
     }
     const int end = min(start + chunk, total);
-
-    float qf[EPL];
-    {
-        const __half* qp = q + ((long long)b * num_q_heads + h) * D + lane * EPL;
-#pragma unroll
-        for (int i = 0; i < EPL; ++i) qf[i] = __half2float(qp[i]) * (scale * kLog2e);
-    }
-    float m = kNeutralM, l = 0.f, o[EPL];
-#pragma unroll
-    for (int i = 0; i < EPL; ++i) o[i] = 0.f;
-
-    const long long row_stride = (long long)num_kv_heads * D;
-    const __half* kbase = k_cache + (long long)b * kv_batch_stride + (long long)kv_head * D + lane * EPL;
-    const __half* vbase = v_cache + (long long)b * kv_batch_stride + (long long)kv_head * D + lane * EPL;
-    for (int j = start + warp; j < end; j += nwarps) {
-        __half kr[EPL], vr[EPL];
-        const __half* kp = kbase + (long long)j * row_stride;
-        const __half* vp = vbase + (long long)j * row_stride;
-        if constexpr (EPL == 8) {
-            *reinterpret_cast<uint4*>(kr) = *reinterpret_cast<const uint4*>(kp);
-            *reinterpret_cast<uint4*>(vr) = *reinterpret_cast<const uint4*>(vp);
-        } else if constexpr (EPL == 4) {
-            *reinterpret_cast<uint2*>(kr) = *reinterpret_cast<const uint2*>(kp);
-            *reinterpret_cast<uint2*>(vr) = *reinterpret_cast<const uint2*>(vp);
-        } else {
-            *reinterpret_cast<uint32_t*>(kr) = *reinterpret_cast<const uint32_t*>(kp);
-            *reinterpret_cast<uint32_t*>(vr) = *reinterpret_cast<const uint32_t*>(vp);
+    const long long head_base = (long long)b * kv_batch_stride + (long long)kv_head * D;
+    const __half* kbase = k_cache + head_base + col;
+    const __half* vbase = v_cache + head_base + col;
+    // the new row's place among this step's projections (unsplit only): the block reads it from there
+    const long long new_base = ((long long)b * num_kv_heads + kv_head) * D;
+    if constexpr (kUnsplit) {
+        // every block writes its KV head's new row (the blocks of a group write identical bytes)
+        const long long dst = head_base + (long long)(total - 1) * row_stride;
+        for (int d = threadIdx.x; d < D; d += blockDim.x) {
+            const_cast<__half*>(k_cache)[dst + d] = k_new[new_base + d];
+            const_cast<__half*>(v_cache)[dst + d] = v_new[new_base + d];
         }
-        float s = 0.f;
-#pragma unroll
-        for (int i = 0; i < EPL; ++i) s = fmaf(qf[i], __half2float(kr[i]), s);
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-        const float m_new = fmaxf(m, s);
-        const float corr = fast_exp2(m - m_new);
-        const float p = fast_exp2(s - m_new);
-        l = l * corr + p;
-#pragma unroll
-        for (int i = 0; i < EPL; ++i) o[i] = fmaf(p, __half2float(vr[i]), o[i] * corr);
-        m = m_new;
     }
-    if (lane == 0) { sh_m[warp] = m; sh_l[warp] = l; }
+
+    // rows j0, j0 + 1, ... of this warp's turn; rows past the end repeat the last one (their weight is zero)
+    auto load_turn = [&](uint4 (&r)[U], const __half* base, const __half* fresh, int j0) {
+        if (j0 + P < end) {
 #pragma unroll
-    for (int i = 0; i < EPL; ++i) sh_o[warp][lane * EPL + i] = o[i];
+            for (int i = 0; i < U; ++i) r[i] = load_8_halves<kVec>(base + (long long)(j0 + i * RPI + sub) * row_stride);
+        } else {
+#pragma unroll
+            for (int i = 0; i < U; ++i) {
+                const int j = min(j0 + i * RPI + sub, end - 1);
+                const __half* p = base + (long long)j * row_stride;
+                if (kUnsplit && j == total - 1) p = fresh + new_base + col;
+                r[i] = load_8_halves<kVec>(p);
+            }
+        }
+    };
+
+    uint4 kr[U], vr[U];
+    int j0 = start + warp * P;
+    if (j0 < end) { load_turn(kr, kbase, k_new, j0); load_turn(vr, vbase, v_new, j0); }
+    F32x2 qf[4];
+    {
+        const __half* qp = q + ((long long)b * num_q_heads + h) * D + col;
+        const float f = scale * kLog2e;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) qf[i] = pack_f32x2(__half2float(qp[2 * i]) * f, __half2float(qp[2 * i + 1]) * f);
+    }
+    float m = kNeutralM, mt = kNeutralM, l = 0.f;    // reference maximum (warp), largest score seen and sum of weights (lane)
+    F32x2 o[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) o[i] = pack_f32x2(0.f, 0.f);
+
+    for (; j0 < end; j0 += nwarps * P) {
+        const int next = j0 + nwarps * P;
+        float s[U];
+#pragma unroll
+        for (int i = 0; i < U; ++i) {
+            F32x2 a = pack_f32x2(0.f, 0.f);
+            a = fma_f32x2(qf[0], widen_half2(kr[i].x), a);
+            a = fma_f32x2(qf[1], widen_half2(kr[i].y), a);
+            a = fma_f32x2(qf[2], widen_half2(kr[i].z), a);
+            a = fma_f32x2(qf[3], widen_half2(kr[i].w), a);
+            const float2 t = unpack_f32x2(a);
+            s[i] = t.x + t.y;
+        }
+        if (next < end) load_turn(kr, kbase, k_new, next);
+        // U sums over the LPR lanes of a row at once: each exchange halves the number of scores a lane
+        // carries; lane (i * LPR / U) of a row's lanes ends with score i (its neighbours with copies of it).
+#pragma unroll
+        for (int w = U / 2, mask = LPR / 2; w >= 1; w >>= 1, mask >>= 1) {
+            const bool up = (lane & mask) != 0;
+#pragma unroll
+            for (int i = 0; i < U / 2; ++i)
+                if (i < w) {
+                    const float give = up ? s[i] : s[i + w], keep = up ? s[i + w] : s[i];
+                    s[i] = keep + __shfl_xor_sync(0xffffffffu, give, mask);
+                }
+        }
+#pragma unroll
+        for (int mask = LPR / U / 2; mask >= 1; mask >>= 1) s[0] += __shfl_xor_sync(0xffffffffu, s[0], mask);
+        const bool valid = j0 + ((lane % LPR) / (LPR / U)) * RPI + sub < end;
+        const float score = valid ? s[0] : kNeutralM;
+        mt = fmaxf(mt, score);
+        if (__any_sync(0xffffffffu, score > m + kCompatLazyMax)) {
+            float up = score;
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1) up = fmaxf(up, __shfl_xor_sync(0xffffffffu, up, off));
+            up = fmaxf(m, up);
+            const float corr = fast_exp2(m - up);
+            const F32x2 cc = pack_f32x2(corr, corr), zero = pack_f32x2(0.f, 0.f);
+            l *= corr;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) o[i] = fma_f32x2(o[i], cc, zero);
+            m = up;
+        }
+        const float p = valid ? fast_exp2(score - m) : 0.f;
+        l += p;
+#pragma unroll
+        for (int i = 0; i < U; ++i) {
+            const float pi = __shfl_sync(0xffffffffu, p, sub * LPR + i * (LPR / U));
+            const F32x2 pp = pack_f32x2(pi, pi);
+            o[0] = fma_f32x2(pp, widen_half2(vr[i].x), o[0]);
+            o[1] = fma_f32x2(pp, widen_half2(vr[i].y), o[1]);
+            o[2] = fma_f32x2(pp, widen_half2(vr[i].z), o[2]);
+            o[3] = fma_f32x2(pp, widen_half2(vr[i].w), o[3]);
+        }
+        if (next < end) load_turn(vr, vbase, v_new, next);
+    }
+    // ---- merge: the row groups of a warp, then the warps
+    float of[8];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { const float2 t = unpack_f32x2(o[i]); of[2 * i] = t.x; of[2 * i + 1] = t.y; }
+#pragma unroll
+    for (int off = LPR; off < 32; off <<= 1)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) of[i] += __shfl_xor_sync(0xffffffffu, of[i], off);
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        l += __shfl_xor_sync(0xffffffffu, l, off);
+        mt = fmaxf(mt, __shfl_xor_sync(0xffffffffu, mt, off));
+    }
+    if (lane == 0) { sh_m[warp] = m; sh_l[warp] = l * ((float)U / LPR); sh_t[warp] = mt; }   // LPR / U lanes carried every weight
+    if (sub == 0) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) sh_o[warp * D + col + i] = of[i];
+    }
     __syncthreads();
     float mm = kNeutralM;
-    for (int w = 0; w < nwarps; ++w) mm = fmaxf(mm, sh_m[w]);
+    for (int w = 0; w < nwarps; ++w) mm = fmaxf(mm, sh_t[w]);
     float ll = 0.f;
     for (int w = 0; w < nwarps; ++w) ll += sh_l[w] * fast_exp2(sh_m[w] - mm);
     for (int d = threadIdx.x; d < D; d += blockDim.x) {
         float acc = 0.f;
-        for (int w = 0; w < nwarps; ++w) acc += sh_o[w][d] * fast_exp2(sh_m[w] - mm);
+        for (int w = 0; w < nwarps; ++w) acc += sh_o[w * D + d] * fast_exp2(sh_m[w] - mm);
         if constexpr (kUnsplit) output[((long long)b * num_q_heads + h) * D + d] = __float2half(acc / fmaxf(ll, 1e-20f));
         else partial_o[stat * D + d] = acc;
     }
@@ -234,30 +351,35 @@ __device__ __forceinline__ void compat_partial_body(
     }
 }
 
-extern "C" __global__ void flash_attention_split_kv_partial_kernel(
+template <int D>
+__device__ __forceinline__ void compat_partial_dispatch(
+    float* sh, const __half* q, const __half* k_cache, const __half* v_cache, float* partial_m, float* partial_l, float* partial_o,
+    int num_q_heads, int num_kv_heads, float scale, const int* kv_cache_offset_ptr, int kv_batch_stride, int max_chunks)
+{
+    if ((((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)v_cache) & 15) == 0 && (kv_batch_stride & 7) == 0)
+        compat_partial_body<D, false, true>(sh, q, k_cache, v_cache, partial_m, partial_l, partial_o, num_q_heads, num_kv_heads,
+                                            scale, kv_cache_offset_ptr, kv_batch_stride, max_chunks);
+    else
+        compat_partial_body<D, false, false>(sh, q, k_cache, v_cache, partial_m, partial_l, partial_o, num_q_heads, num_kv_heads,
+                                             scale, kv_cache_offset_ptr, kv_batch_stride, max_chunks);
+}
+
+extern "C" __global__ void __launch_bounds__(256) flash_attention_split_kv_partial_kernel(
     const __half* __restrict__ q, const __half* __restrict__ k_cache, const __half* __restrict__ v_cache,
     float* __restrict__ partial_m, float* __restrict__ partial_l, float* __restrict__ partial_o,
     int num_q_heads, int num_kv_heads, int head_dim, float scale,
     const int* __restrict__ kv_cache_offset_ptr, int kv_batch_stride, int max_chunks)
 {
+    __shared__ float sh[kCompatSharedFloats];
     grid_launch_dependents();
     grid_dependency_wait();
-    switch (head_dim) {
-    case 64:
-        compat_partial_body<2, false>(q, k_cache, v_cache, partial_m, partial_l, partial_o, num_q_heads,
-                                      num_kv_heads, scale, kv_cache_offset_ptr, kv_batch_stride, max_chunks);
-        break;
-    case 128:
-        compat_partial_body<4, false>(q, k_cache, v_cache, partial_m, partial_l, partial_o, num_q_heads,
-                                      num_kv_heads, scale, kv_cache_offset_ptr, kv_batch_stride, max_chunks);
-        break;
-    case 256:
-        compat_partial_body<8, false>(q, k_cache, v_cache, partial_m, partial_l, partial_o, num_q_heads,
-                                      num_kv_heads, scale, kv_cache_offset_ptr, kv_batch_stride, max_chunks);
-        break;
-    default:
-        break;   // the host refuses other head sizes before launching
-    }
+#define VTEB_ARGS sh, q, k_cache, v_cache, partial_m, partial_l, partial_o, num_q_heads, num_kv_heads, scale, \
+                  kv_cache_offset_ptr, kv_batch_stride, max_chunks
+    if (head_dim == 64) compat_partial_dispatch<64>(VTEB_ARGS);
+    else if (head_dim == 128) compat_partial_dispatch<128>(VTEB_ARGS);
+    else if (head_dim == 256) compat_partial_dispatch<256>(VTEB_ARGS);
+    // the host refuses other head sizes before launching
+#undef VTEB_ARGS
 }
 
 // ---------------------------------------------------------------------------
@@ -271,31 +393,30 @@ extern "C" __global__ void flash_attention_split_kv_partial_kernel(
 // are read once per query head (through L2); the dispatcher's own one-launch path for short
 // contexts is the split kernel with one split, which reads them once per KV head.
 // ---------------------------------------------------------------------------
-extern "C" __global__ void flash_attention_kernel(
+extern "C" __global__ void __launch_bounds__(256) flash_attention_kernel(
     const __half* __restrict__ q, const __half* __restrict__ k, const __half* __restrict__ v,
     __half* __restrict__ k_cache, __half* __restrict__ v_cache, __half* __restrict__ output,
     int seq_len, int num_q_heads, int num_kv_heads, int head_dim, float scale,
     const int* __restrict__ kv_cache_offset_ptr, int kv_batch_stride)
 {
+    __shared__ float sh[kCompatSharedFloats];
     grid_launch_dependents();
     grid_dependency_wait();
     (void)seq_len;
-    switch (head_dim) {
-    case 64:
-        compat_partial_body<2, true>(q, k_cache, v_cache, nullptr, nullptr, nullptr, num_q_heads, num_kv_heads, scale,
-                                     kv_cache_offset_ptr, kv_batch_stride, 1, k, v, output);
-        break;
-    case 128:
-        compat_partial_body<4, true>(q, k_cache, v_cache, nullptr, nullptr, nullptr, num_q_heads, num_kv_heads, scale,
-                                     kv_cache_offset_ptr, kv_batch_stride, 1, k, v, output);
-        break;
-    case 256:
-        compat_partial_body<8, true>(q, k_cache, v_cache, nullptr, nullptr, nullptr, num_q_heads, num_kv_heads, scale,
-                                     kv_cache_offset_ptr, kv_batch_stride, 1, k, v, output);
-        break;
-    default:
-        break;   // the host refuses other head sizes before launching
+    const bool vec = (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)k_cache | (uintptr_t)v_cache) & 15) == 0 && (kv_batch_stride & 7) == 0;
+#define VTEB_ARGS sh, q, k_cache, v_cache, nullptr, nullptr, nullptr, num_q_heads, num_kv_heads, scale, \
+                  kv_cache_offset_ptr, kv_batch_stride, 1, k, v, output
+    if (vec) {
+        if (head_dim == 64) compat_partial_body<64, true, true>(VTEB_ARGS);
+        else if (head_dim == 128) compat_partial_body<128, true, true>(VTEB_ARGS);
+        else if (head_dim == 256) compat_partial_body<256, true, true>(VTEB_ARGS);
+    } else {
+        if (head_dim == 64) compat_partial_body<64, true, false>(VTEB_ARGS);
+        else if (head_dim == 128) compat_partial_body<128, true, false>(VTEB_ARGS);
+        else if (head_dim == 256) compat_partial_body<256, true, false>(VTEB_ARGS);
     }
+    // the host refuses other head sizes before launching
+#undef VTEB_ARGS
 }
 
 // ---------------------------------------------------------------------------

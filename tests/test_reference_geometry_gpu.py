@@ -72,3 +72,35 @@ def test_unsplit_and_split_walks_at_turn_boundaries(cuda_runtime, codegen, heads
     finally:
         for p in bufs:
             rt.safe_free(p, "walk test cleanup")
+
+
+@pytest.mark.parametrize("D", [64, 128, 256])
+def test_an_infinite_value_in_the_newest_row_stays_infinite(cuda_runtime, codegen, D):
+    """The newest row's weight is positive, so an infinite value in it gives an infinite output in that channel and
+    leaves the others finite, also where the rows past the end fill up a turn."""
+    rt = cuda_runtime
+    Hq, Hkv, S, lengths = 2, 1, 160, [1, 5, 33, 129]
+    B = len(lengths)
+    rng = np.random.default_rng(D)
+    f16 = lambda *s: rng.standard_normal(s, dtype=np.float32).astype(np.float16)
+    q, k, v, kn, vn = f16(B, Hq, D), f16(B, S, Hkv, D), f16(B, S, Hkv, D), f16(B, Hkv, D), f16(B, Hkv, D)
+    vn[:, :, 3] = np.inf
+    off, bufs = np.array(lengths, dtype=np.int32) - 1, []
+
+    def dev(arr):
+        bufs.append(rt.safe_malloc(arr.nbytes, "infinite row test output"))
+        rt.safe_memcpy_host_to_device(bufs[-1], np.ascontiguousarray(arr), "infinite row test output")
+        return bufs[-1]
+    try:
+        dq, dk, dv, dkn, dvn, doff, dout = (dev(x) for x in (q, k, v, kn, vn, off, np.zeros((B, Hq, D), np.float16)))
+        ci, cf = ctypes.c_int, ctypes.c_float
+        _, unsplit = codegen.load_kernel_safe(rt, 'flash_attention', rt.get_gpu_architecture(), 'flash_attention_kernel')
+        rt.launch_kernel(unsplit, (B, Hq, 1), (D, 1, 1), [dq, dkn, dvn, dk, dv, dout, ci(1), ci(Hq), ci(Hkv), ci(D),
+                                                          cf(1.0 / np.sqrt(D)), doff, ci(S * Hkv * D)], 2 * D * 4)
+        rt.synchronize()
+        out = np.zeros((B, Hq, D), np.float16)
+        rt.safe_memcpy_device_to_host(out, dout, "infinite row test output")
+        assert np.all(out[:, :, 3] == np.inf) and np.all(np.isfinite(np.delete(out, 3, axis=2)))
+    finally:
+        for p in bufs:
+            rt.safe_free(p, "infinite row test cleanup")

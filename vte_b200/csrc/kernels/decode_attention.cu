@@ -229,7 +229,8 @@ __device__ __forceinline__ void compat_partial_body(
         }
     }
 
-    // rows j0, j0 + 1, ... of this warp's turn; rows past the end repeat the last one (their weight is zero)
+    // rows j0, j0 + 1, ... of this warp's turn; rows past the end are zeros (an infinite row repeated there with
+    // weight zero would make the sum NaN)
     auto load_turn = [&](uint4 (&r)[U], const __half* base, const __half* fresh, int j0) {
         if (j0 + P < end) {
 #pragma unroll
@@ -237,10 +238,11 @@ __device__ __forceinline__ void compat_partial_body(
         } else {
 #pragma unroll
             for (int i = 0; i < U; ++i) {
-                const int j = min(j0 + i * RPI + sub, end - 1);
+                const int j = j0 + i * RPI + sub;
                 const __half* p = base + (long long)j * row_stride;
                 if (kUnsplit && j == total - 1) p = fresh + new_base + col;
-                r[i] = load_8_halves<kVec>(p);
+                r[i] = make_uint4(0u, 0u, 0u, 0u);
+                if (j < end) r[i] = load_8_halves<kVec>(p);
             }
         }
     };

@@ -215,16 +215,6 @@ __device__ __forceinline__ void copy_rows_async(const unsigned char* src, const 
 // The prefetch only pays while a whole layer's K and V stay in L2 until the next launch reads
 // them: above this many bytes per tensor (the grid's total) it is skipped.  Measured at one
 // million positions (0.5 GB per tensor): prefetching cost 15 % of the throughput.
-constexpr long long kL2PrefetchMaxBytes = 24ll << 20;
-
-__device__ __forceinline__ void prefetch_range_l2(const unsigned char* base, long long bytes, int lane) {
-    constexpr long long kPiece = 8192;
-    for (long long off = (long long)lane * kPiece; off < bytes; off += 32 * kPiece) {
-        const unsigned n = (unsigned)((bytes - off < kPiece) ? (bytes - off) : kPiece) & ~15u;
-        if (n) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(base + off), "r"(n) : "memory");
-    }
-}
-
 // Grid-wide barrier for a grid whose CTAs are all resident (grid <= SM count, one CTA
 // per SM).  words[0] counts arrivals and is cleared by the last arriver, words[1] is a
 // generation number; one thread per CTA calls this.  The wait is bounded (kWaitLimitCycles).

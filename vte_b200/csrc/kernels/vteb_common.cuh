@@ -241,6 +241,18 @@ __device__ __forceinline__ void tma_load_box_2d(uint32_t dst_smem, const void* t
         : "memory");
 }
 
+constexpr long long kL2PrefetchMaxBytes = 24ll << 20;   // per tensor and launch: more than this is not asked for ahead (see split_kv_fast.cuh)
+
+// Asks L2 for `bytes` (a multiple of 16) from `base` (16-byte aligned) on: requests of 8 KB, dealt to the
+// lanes of the calling warp.  A hint: no data reaches the SM.
+__device__ __forceinline__ void prefetch_range_l2(const unsigned char* base, long long bytes, int lane) {
+    constexpr long long kPiece = 8192;
+    for (long long off = (long long)lane * kPiece; off < bytes; off += 32 * kPiece) {
+        const unsigned n = (unsigned)((bytes - off < kPiece) ? (bytes - off) : kPiece) & ~15u;
+        if (n) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(base + off), "r"(n) : "memory");
+    }
+}
+
 // Makes the calling thread's earlier async_copy_16 operations count as one
 // arrival on the barrier once they have all landed.
 __device__ __forceinline__ void async_copy_arrive(uint32_t bar) {

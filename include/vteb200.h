@@ -155,6 +155,9 @@ int vteb_split_kv_plan(int num_q_heads, int num_kv_heads, int head_dim, vteb_fas
  * the combine launch, which shortens a layer whose whole split launch lasts only some
  * microseconds.  `ok` is 0 when a head group needs more than six consumer warps. */
 int vteb_split_kv_plan_compact(int num_q_heads, int num_kv_heads, int head_dim, vteb_fast_plan* plan);
+/* The plan of the split kernels for more than eight query heads per KV head (`vteb_split_kv_partial_wide_*`):
+ * ok = 1 when the group can be cut into at most eight equal runs of at most eight heads. */
+int vteb_split_kv_plan_wide(int num_q_heads, int num_kv_heads, int head_dim, vteb_fast_plan* plan);
 /* Encodes the 128-byte tensor map the fast split kernels take for a K or V cache: the cache
  * seen as `n_rows` position rows (all sequences, one after another) of `row_halves` =
  * Hkv * D fp16 values, in boxes of 64 values x `box_rows` rows (the plan's `tile`) with the

@@ -1,0 +1,83 @@
+"""More than eight query heads per KV head: the split kernel's `wide` build, where a group is cut into equal runs
+of at most eight heads that read the same staged rows."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from oracle import attention_oracle as orc
+from vte_b200.bridge.cuda_runtime import FastPlan, load_library
+from vte_b200.core.split_kv_attention import WIDE_SCRATCH_BYTES, choose_split_count
+
+# (heads, consumer heads per KV head): groups of 9 to 64, every head width, one and several KV heads per item
+WIDE = [((32, 2, 128), 2), ((48, 1, 128), 6), ((36, 4, 64), 3), ((20, 2, 64), 2), ((64, 1, 64), 8), ((64, 1, 256), 8),
+        ((24, 2, 256), 2)]
+LENGTHS = [1, 2, 15, 16, 17, 31, 33, 64, 65, 127, 129, 500, 900]
+
+
+def test_plan_covers_groups_with_an_equal_cut(built_library):
+    lib = load_library(str(built_library))
+    plan = FastPlan()
+    for (hq, hkv, d), nv in WIDE:
+        assert lib.vteb_split_kv_plan_wide(hq, hkv, d, ctypes.byref(plan)) == 0
+        assert plan.ok == 1 and plan.hg * nv <= 8 and plan.hg * plan.n_hgroups == hkv
+        assert plan.threads == 320 and plan.nstages >= 2 and plan.smem_bytes <= 227 * 1024 and plan.tile % 16 == 0
+        # the same rows staged as for a group of eight, so the copies' boxes and alignment are the tested ones
+        assert (plan.hg * d) % 64 == 0
+    for hq, hkv, d in [(16, 2, 128), (22, 2, 128), (13, 1, 64), (72, 1, 128), (32, 2, 96), (33, 2, 128)]:
+        assert lib.vteb_split_kv_plan_wide(hq, hkv, d, ctypes.byref(plan)) == 0 and plan.ok == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("batch", [len(LENGTHS), 1], ids=["ragged", "one"])
+@pytest.mark.parametrize("heads", [h for h, _ in WIDE], ids=str)
+def test_wide_groups_match_the_oracle(cuda_runtime, codegen, heads, batch):
+    """Equal shares over a ragged batch, the append among the launches; one sequence through the work queue, and
+    unsplit where the context is short.  Bound: fp32 sums of at most 900 probabilities that carry 22 bits (and 2^-25
+    of the reference at least), values N(0, 1): 900^0.5 * 2^-25 * 4.5 < 5e-6, twice that for the order of the sums."""
+    from vte_b200.core.decode_executor import DecodeAttentionExecutor
+    Hq, Hkv, D = heads
+    rng = np.random.default_rng([Hq, D, batch])
+    meta = {"attention.head_count": Hq, "attention.head_count_kv": Hkv, "attention.key_length": D}
+    lengths = [LENGTHS] if batch > 1 else [[n] for n in (900, 17, 1)]
+    S = 928
+    f16 = lambda *s: rng.standard_normal(s, dtype=np.float32).astype(np.float16)
+    k, v = f16(batch, S, Hkv, D), f16(batch, S, Hkv, D)
+    for capacity in ((S,) if batch > 1 else (S, 64)):
+        ex = DecodeAttentionExecutor(cuda_runtime, codegen, meta, batch, capacity, 1, with_append=True)
+        try:
+            assert ex.dispatcher.wide and ex.dispatcher.split_kernel_name == f"vteb_split_kv_partial_wide_d{D}_kernel"
+            for lens in lengths:
+                if max(lens) > capacity:
+                    continue
+                q, kn, vn = f16(batch, Hq, D), f16(batch, Hkv, D), f16(batch, Hkv, D)
+                off = np.array(lens, dtype=np.int32) - 1
+                kr, vr = k[:, :capacity].copy(), v[:, :capacity].copy()
+                ex.upload_layer(0, q, kr, vr)
+                ex.upload_new_kv(0, kn, vn)
+                out = ex.execute_decode_batch(off)[0]
+                orc.kv_cache_append(kn, vn, kr, vr, off)
+                assert np.max(np.abs(out - orc.decode_attention(q, kr, vr, off))) <= 1e-5
+        finally:
+            ex.cleanup()
+
+
+@pytest.mark.gpu
+def test_wide_only_where_the_split_layout_is_open(cuda_runtime, codegen):
+    from vte_b200.bridge import CudaSafetyError
+    from vte_b200.core.split_kv_attention import SplitKVAttentionDispatcher
+    meta = {"attention.head_count": 32, "attention.head_count_kv": 2, "attention.key_length": 128}
+    make = lambda m=meta, **kw: SplitKVAttentionDispatcher(cuda_runtime, codegen, m, context_length=4096, **kw)
+    assert make(batch_size=8).wide and make(batch_size=8).balanced and make().wide and not make().balanced
+    for kw in ({"num_splits": 16}, {"fixed_chunk_size": 32}, {"compat": True}):
+        d = make(batch_size=8, **kw)
+        assert d.compat and not d.wide and not d.balanced
+    assert not make(dict(meta, **{"attention.head_count": 22})).wide              # 11 heads have no equal cut
+    for batch in (2, 13, 64, 1024):                                               # scratch stays within its limit
+        d = make(dict(meta, **{"attention.head_count": 64, "attention.head_count_kv": 1, "attention.key_length": 256}), batch_size=batch)
+        other = choose_split_count(cuda_runtime.get_num_cus(), batch, 1, 4096)
+        assert d.max_chunks <= max(other, WIDE_SCRATCH_BYTES // (batch * 64 * 258 * 4))
+        assert d.wide == d.balanced and (d.wide or d.max_chunks == other)
+    for kw in ({"fuse_rope": True}, {"fuse_append": True}, {"emit_state": True}):
+        with pytest.raises(CudaSafetyError):
+            make(**kw)

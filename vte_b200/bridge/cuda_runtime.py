@@ -129,6 +129,7 @@ def _declare(lib):
         "vteb_ipc_close_handle": (i, [vp]),
         "vteb_split_kv_plan": (i, [i, i, i, ctypes.POINTER(FastPlan)]),
         "vteb_split_kv_plan_compact": (i, [i, i, i, ctypes.POINTER(FastPlan)]),
+        "vteb_split_kv_plan_wide": (i, [i, i, i, ctypes.POINTER(FastPlan)]),
         "vteb_kv_tensor_map": (i, [vp, vp, ctypes.c_longlong, i, i]),
         "vteb_combine_rows_epl": (i, [i, i]),
         "vteb_split_kv_decode": (i, [vp, vp, vp, vp, vp, i, vp, vp, vp, vp, i, i, i, i, f, ll, i, i, u, i, vp]),
@@ -653,6 +654,13 @@ class CudaRuntime:
         plan = FastPlan()
         fn = self._lib.vteb_split_kv_plan_compact if compact else self._lib.vteb_split_kv_plan
         self._check_error(fn(num_q_heads, num_kv_heads, head_dim, ctypes.byref(plan)), "vteb_split_kv_plan")
+        return plan
+
+    def split_kv_plan_wide(self, num_q_heads: int, num_kv_heads: int, head_dim: int) -> FastPlan:
+        """The plan for more than eight query heads per KV head."""
+        plan = FastPlan()
+        self._check_error(self._lib.vteb_split_kv_plan_wide(num_q_heads, num_kv_heads, head_dim, ctypes.byref(plan)),
+                          "vteb_split_kv_plan_wide")
         return plan
 
     def kv_tensor_map(self, cache_ptr: int, n_rows: int, row_halves: int, box_rows: int) -> KvTensorMap:

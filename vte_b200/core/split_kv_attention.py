@@ -35,6 +35,7 @@ FLAG_DIRECT_OUTPUT = 2
 FLAG_TENSOR_MAPS = 4
 FLAG_PREFETCH_Q = 8
 FLAG_BALANCED = 16
+WIDE_SCRATCH_BYTES = 32 << 20    # partial buffers a group of more than eight heads may take where it took less before; executors reserve 64 MB
 COMPACT_MAX_CONTEXT = 262144      # one sequence up to this long: the compact CTA shape (launches of tens of microseconds)
 SHORT_CONTEXT_MAX = 2048          # one sequence up to this many positions: at most 32 splits (see choose_split_count)
 UNSPLIT_MAX_CONTEXT = 128         # below this, one CTA per (sequence, head group) finishes before a combine could launch
@@ -175,6 +176,7 @@ class SplitKVAttentionDispatcher:
             raise CudaSafetyError(f"variant must be full, compact or auto, not {variant!r}")
         self._plan = None
         self.compact = False
+        self.wide = False           # `compat` stays True with it: what the reference-geometry kernels cannot do is refused as before
         if hip is not None and hasattr(hip, 'split_kv_plan'):
             self._plan = hip.split_kv_plan(self.num_q_heads, self.num_kv_heads, self.head_dim)
             want_compact = variant == "compact" or (variant == "auto" and self.batch_size == 1
@@ -187,8 +189,17 @@ class SplitKVAttentionDispatcher:
         if self.emit_state and (self.compat or self._plan is None or not self._plan.ok):
             raise CudaSafetyError("emit_state needs the fast kernels (group <= 8, head_dim 64/128/256)")
         if not self.compat and (self._plan is None or not self._plan.ok):
-            # geometry outside the fast kernel (group > 8, unusual head_dim): reference-geometry kernels
+            # geometry outside the fast kernel (group > 8, unusual head_dim): reference-geometry kernels.
+            # wide: a group of more than eight query heads that can be cut into equal runs of at most eight
+            # goes to the split kernel's `wide` build, one run per consumer head over the same staged rows
+            # (eight sequences of 500 to 4,096 positions, 32 heads on 2: 20 us a layer against 41).
+            # Only where the caller left the split layout open: a fixed chunk or split count keeps the
+            # reference-geometry kernels and the partial buffers that go with them.
             self.compat = True
+            if not num_splits and fixed_chunk_size is None and hasattr(hip, 'split_kv_plan_wide'):
+                wide_plan = hip.split_kv_plan_wide(self.num_q_heads, self.num_kv_heads, self.head_dim)
+                if wide_plan.ok:
+                    self._plan, self.wide = wide_plan, True
 
         # fused_combine: the split launch also merges the splits (after a grid-wide barrier), so a
         # layer is append + ONE launch.  Needs all eight consumer warps (hg divides 8).
@@ -213,7 +224,7 @@ class SplitKVAttentionDispatcher:
             # balanced: every CTA takes an equal share of all cached positions instead of drawing
             # fixed-size splits from a work queue (split_kv_fast.cuh, BalancedShare).  Chosen when several
             # sequences share the GPU and the caller fixed neither the split count nor a minimum split.
-            fast = (not self.compat) and self._plan is not None and self._plan.ok
+            fast = (not self.compat or self.wide) and self._plan is not None and self._plan.ok
             auto_count = not num_splits
             self.balanced = fast and not self.fused_combine and not self.compact and (
                 (balanced is None and auto_count and min_chunk is None and self.batch_size > 1
@@ -226,6 +237,17 @@ class SplitKVAttentionDispatcher:
                 self.max_chunks = balanced_split_count(num_cus, self.batch_size, n_hg)
             else:
                 self.max_chunks = choose_split_count(num_cus, self.batch_size, n_hg, self.context_length)
+            if self.wide:
+                # scratch no larger than the reference-geometry kernels' own, or WIDE_SCRATCH_BYTES: fewer splits
+                # where those still allow a sequence of 2.5 times the mean length (balanced_split_count)
+                per_split = self.batch_size * self.num_q_heads * (self.head_dim + 2) * 4
+                other = choose_split_count(num_cus, self.batch_size, self.num_kv_heads, self.context_length)
+                fit = max(other, WIDE_SCRATCH_BYTES // per_split)
+                if self.balanced and self.max_chunks > fit >= math.ceil(2.5 * num_cus / (self.batch_size * n_hg)) + 1:
+                    self.max_chunks = fit
+                if self.max_chunks > fit:
+                    self.wide = self.balanced = False
+                    self._plan, self.max_chunks = hip.split_kv_plan(self.num_q_heads, self.num_kv_heads, self.head_dim), other
             if self.balanced and self.max_chunks < 2:
                 raise CudaSafetyError("the balanced partition needs at least two splits")
             if not (1 <= self.max_chunks <= 65535):
@@ -289,8 +311,8 @@ class SplitKVAttentionDispatcher:
         longest_split = -(-self.context_length // max(1, self.max_chunks))
         column_split = (self.compact and not rotating and self.head_dim == 128 and self._plan.hg == 2
                         and self.max_chunks > 1 and longest_split <= 16)
-        return (f"vteb_split_kv_partial_{'compact_' if self.compact else ''}{'cs_' if column_split else ''}"
-                f"{'rope_' if rotating else ''}d{self.head_dim}_kernel")
+        return (f"vteb_split_kv_partial_{'wide_' if self.wide else ''}{'compact_' if self.compact else ''}"
+                f"{'cs_' if column_split else ''}{'rope_' if rotating else ''}d{self.head_dim}_kernel")
 
     # -- tensor-name resolution -------------------------------------------------
     @staticmethod
@@ -328,7 +350,7 @@ class SplitKVAttentionDispatcher:
             load = lambda template, symbol: self.codegen.load_kernel_safe(self.hip, template, arch, symbol, **params)[1]
             self._kernel_cache['append'] = load(
                 'kv_cache_append', 'kv_cache_append_rope_kernel' if self.fuse_rope else 'kv_cache_append_kernel')
-            if self.compat:
+            if self.compat and not self.wide:
                 self._kernel_cache['partial'] = load('flash_attention_split_kv_partial',
                                                      'flash_attention_split_kv_partial_kernel')
                 self._kernel_cache['reduce'] = load(
@@ -490,7 +512,7 @@ class SplitKVAttentionDispatcher:
         reduce_args = [vp(self._partial_m.ptr), vp(self._partial_l.ptr), vp(self._partial_o.ptr),
                        vp(output_ptr), ci(Hq), ci(D), ci(C)]
 
-        if self.compat:
+        if self.compat and not self.wide:
             partial = (partial_fn, reference_partial_args, (batch, Hq, C), (D, 1, 1), 2 * D * 4)
             reduce = (reduce_fn, reduce_args, (batch, Hq, 1), (D, 1, 1), C * 4)
             return [append, partial, reduce]

@@ -114,7 +114,8 @@ __device__ __forceinline__ void mma_hi_lo_acc(float& d0, float& d1, float& e0, f
 
 // Online softmax (log2 domain) of a block's raw scores and O += P V.  `left` = positions of the
 // block that belong to the item (may exceed 16); the rest are masked.  `scale2` = scale * log2(e).
-template <int NT, bool LOACC>
+// kFresh: the products of both parts of P start from zero and are added in fp32 registers.
+template <int NT, bool LOACC, bool kFresh = false>
 __device__ __forceinline__ void softmax_pv(ConsumerState<NT, LOACC>& st, const float (&sraw)[2][2], uint32_t vaddr,
                                            int blk_bytes, int left, float scale2, int t) {
     // V fragments do not depend on the softmax: fetch the first 64 columns now
@@ -204,6 +205,11 @@ __device__ __forceinline__ void softmax_pv(ConsumerState<NT, LOACC>& st, const f
                               vf[ch & 1][i][0], vf[ch & 1][i][1]);
                 mma_hi_lo_acc(st.o[n + 1][0], st.o[n + 1][1], st.o_lo[n + 1][0], st.o_lo[n + 1][1], ph[0], pl[0], ph[1], pl[1],
                               vf[ch & 1][i][2], vf[ch & 1][i][3]);
+            } else if constexpr (kFresh) {
+                float d0 = 0.f, d1 = 0.f, g0 = 0.f, g1 = 0.f, e0, e1, f0, f1;
+                mma_hi_lo(d0, d1, e0, e1, ph[0], pl[0], ph[1], pl[1], vf[ch & 1][i][0], vf[ch & 1][i][1]);
+                mma_hi_lo(g0, g1, f0, f1, ph[0], pl[0], ph[1], pl[1], vf[ch & 1][i][2], vf[ch & 1][i][3]);
+                st.o[n][0] += d0 + e0; st.o[n][1] += d1 + e1; st.o[n + 1][0] += g0 + f0; st.o[n + 1][1] += g1 + f1;
             } else {
                 float e0, e1, f0, f1;
                 mma_hi_lo(st.o[n][0], st.o[n][1], e0, e1, ph[0], pl[0], ph[1], pl[1], vf[ch & 1][i][0], vf[ch & 1][i][1]);
@@ -265,12 +271,15 @@ __device__ __forceinline__ float sum_over_g(float v) {
 }
 
 // Raw scores of one block: s[0] (position g, head 2t), s[1] (g, 2t+1), s[2] (g+8, 2t), s[3] (g+8, 2t+1).
-template <int D>
+// CHAINS accumulation chains; 8 = every product of eight k-steps starts from zero and the sums are taken in fp32
+// registers, which round where the matrix unit's accumulation truncates.
+template <int D, int CHAINS = 2>
 __device__ __forceinline__ void qk_block_t(const uint32_t* __restrict__ q_frag, uint32_t kaddr, int blk_bytes, float (&s)[4]) {
     constexpr int KS = D / 16;
-    float acc[2][4];
+    float acc[CHAINS][4];
 #pragma unroll
-    for (int c = 0; c < 2; ++c) { acc[c][0] = acc[c][1] = acc[c][2] = acc[c][3] = 0.f; }
+    for (int c = 0; c < CHAINS; ++c) { acc[c][0] = acc[c][1] = acc[c][2] = acc[c][3] = 0.f; }
+    if constexpr (CHAINS > 2) { s[0] = s[1] = s[2] = s[3] = 0.f; }
     constexpr int KC = KS < 8 ? KS : 8;
 #pragma unroll
     for (int kc = 0; kc < KS; kc += KC) {
@@ -282,14 +291,26 @@ __device__ __forceinline__ void qk_block_t(const uint32_t* __restrict__ q_frag, 
         for (int i = 0; i < KC; ++i) {
             const int ks = kc + i;
             // kf: (positions 0-7, k 0-7), (0-7, 8-15), (8-15, 0-7), (8-15, 8-15); the A operand wants rows before columns
-            mma_full(acc[ks & 1], kf[i][0], kf[i][2], kf[i][1], kf[i][3], q_frag[(2 * ks) * 32], q_frag[(2 * ks + 1) * 32]);
+            mma_full(acc[ks % CHAINS], kf[i][0], kf[i][2], kf[i][1], kf[i][3], q_frag[(2 * ks) * 32], q_frag[(2 * ks + 1) * 32]);
+        }
+        if constexpr (CHAINS > 2) {
+            static_assert(CHAINS == 8 && KC == 8, "one product per chain");
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                s[i] += ((acc[0][i] + acc[1][i]) + (acc[2][i] + acc[3][i])) + ((acc[4][i] + acc[5][i]) + (acc[6][i] + acc[7][i]));
+#pragma unroll
+                for (int c = 0; c < CHAINS; ++c) acc[c][i] = 0.f;
+            }
         }
     }
+    if constexpr (CHAINS == 2) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) s[i] = acc[0][i] + acc[1][i];
+        for (int i = 0; i < 4; ++i) s[i] = acc[0][i] + acc[1][i];
+    }
 }
 
-template <int MT>
+// kFresh: a block's P V starts from zero and is added to the state in fp32 registers (see qk_block_t).
+template <int MT, bool kFresh = false>
 __device__ __forceinline__ void softmax_pv_t(ConsumerStateT<MT>& st, const float (&sraw)[4], uint32_t vaddr, int blk_bytes,
                                              int left, float scale2, int g) {
     constexpr int VC = (MT >= 4) ? 4 : MT;       // ldmatrix.x4.trans per chunk (4 = 64 output columns)
@@ -344,12 +365,28 @@ __device__ __forceinline__ void softmax_pv_t(ConsumerStateT<MT>& st, const float
                                   vf[(ch + 1) & 1][i][2], vf[(ch + 1) & 1][i][3]);
         }
         // vf: (positions 0-7, columns 0-7)^T, (8-15, 0-7)^T, (0-7, 8-15)^T, (8-15, 8-15)^T
+        if constexpr (kFresh) {
+            float d[VC][4];
 #pragma unroll
-        for (int i = 0; i < VC; ++i)
-            mma_full(st.o[ch * VC + i], vf[ch & 1][i][0], vf[ch & 1][i][2], vf[ch & 1][i][1], vf[ch & 1][i][3], bh[0], bh[1]);
+            for (int i = 0; i < VC; ++i) {
+                d[i][0] = d[i][1] = d[i][2] = d[i][3] = 0.f;
+                mma_full(d[i], vf[ch & 1][i][0], vf[ch & 1][i][2], vf[ch & 1][i][1], vf[ch & 1][i][3], bl[0], bl[1]);
+            }
 #pragma unroll
-        for (int i = 0; i < VC; ++i)
-            mma_full(st.o[ch * VC + i], vf[ch & 1][i][0], vf[ch & 1][i][2], vf[ch & 1][i][1], vf[ch & 1][i][3], bl[0], bl[1]);
+            for (int i = 0; i < VC; ++i)
+                mma_full(d[i], vf[ch & 1][i][0], vf[ch & 1][i][2], vf[ch & 1][i][1], vf[ch & 1][i][3], bh[0], bh[1]);
+#pragma unroll
+            for (int i = 0; i < VC; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) st.o[ch * VC + i][j] += d[i][j];
+        } else {
+#pragma unroll
+            for (int i = 0; i < VC; ++i)
+                mma_full(st.o[ch * VC + i], vf[ch & 1][i][0], vf[ch & 1][i][2], vf[ch & 1][i][1], vf[ch & 1][i][3], bh[0], bh[1]);
+#pragma unroll
+            for (int i = 0; i < VC; ++i)
+                mma_full(st.o[ch * VC + i], vf[ch & 1][i][0], vf[ch & 1][i][2], vf[ch & 1][i][1], vf[ch & 1][i][3], bl[0], bl[1]);
+        }
     }
 }
 

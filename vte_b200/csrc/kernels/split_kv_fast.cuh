@@ -33,6 +33,17 @@
 // warps of a KV head exchange (m, l, o) and the row's true maximum through shared memory and
 // the merged state is stored to partial_m / partial_l / partial_o.
 //
+// The `..._wide_...` build serves more than eight query heads per KV head: the group is cut into nv equal
+// runs of at most eight heads (FastPlan::nv), each run is a consumer head with warps of its own, and all runs
+// of a KV head read the same staged rows, so K and V still cross HBM and L2 once.  Eight sequences of 500 to
+// 4,096 positions, 32 heads on 2 KV heads of 128, append included: 20 us a layer against 41 us with the
+// reference-geometry kernels, which read K and V once per query head; the bytes alone need 3 us, the rest is
+// launches, the Q fetch, the merge and the combine.
+// These groups had fp32 products before, so the wide build rounds every sum in fp32 registers (products of one
+// k-step and of one block start from zero): relative error against 64 bits 1.7e-7 to 2.0e-7 (4.3e-7 with scores
+// four times as wide) where the reference-geometry kernels have 1.9e-7 to 2.4e-7 (4.2e-7), and the same time
+// as with chained accumulation (2.3e-7 to 3.5e-7).
+//
 // Under programmatic dependent launch everything that does not depend on the previous launch runs
 // before griddepcontrol.wait: barrier set-up, the first item's geometry (kv offsets, sequence order),
 // the K/V tiles of positions older than the newest one, and an L2 prefetch of the first item's Q rows.
@@ -357,7 +368,7 @@ __device__ __forceinline__ void append_row_to_tile_and_cache(const __half* __res
     }
 }
 
-template <int D, int CW, bool kRope = false, bool kColSplitKernel = false>
+template <int D, int CW, bool kRope = false, bool kColSplitKernel = false, bool kWide = false>
 __device__ __forceinline__ void fast_partial_body(const FastArgs& a)
 {
     constexpr bool kCompact = (CW == kCompactConsumerWarps);
@@ -370,7 +381,7 @@ __device__ __forceinline__ void fast_partial_body(const FastArgs& a)
     constexpr int kLoaderWarpK = CW;          // loads K rows, owns the work queue
     constexpr int kLoaderWarpV = CW + 1;      // loads V rows, follows the K loader's headers
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    const FastPlan plan = make_fast_plan(a.num_q_heads, a.num_kv_heads, D, kCompact ? 1 : 0);
+    const FastPlan plan = make_fast_plan(a.num_q_heads, a.num_kv_heads, D, kCompact ? 1 : 0, kWide ? 1 : 0);
     const int group = a.num_q_heads / a.num_kv_heads;
 
     volatile int* abort_word = reinterpret_cast<volatile int*>(smem_raw + kAbortOffset);
@@ -709,13 +720,17 @@ __device__ __forceinline__ void fast_partial_body(const FastArgs& a)
     if (warp >= plan.active_warps) return;
 
     // ===================================================================== consumers
-    // warp = (sub * DS + dhalf) * hg + hh
+    // A consumer head is a run of `vgroup` <= 8 query heads: a KV head's whole group, or, in the kernels for
+    // larger groups, one of its nv runs, which read the same staged rows.
+    const int nv = kWide ? plan.nv : 1;
+    const int vhg = plan.hg * nv, vgroup = group / nv;
+    // warp = (sub * DS + dhalf) * vhg + hh
     // 128-wide heads, and 256-wide heads in the full shape, take the transposed form of the block (consumer_block.cuh); its state is `tt`.
     constexpr bool kT = (VTEB_TRANSPOSED != 0) && (D == 128 || (D == 256 && !kCompact));
     constexpr int DS = (D == 256 && !kT) ? 2 : 1;       // warps sharing one (head, block), split by output columns
-    const int hh = warp % plan.hg;                      // KV head within the group
-    const int dhalf = (warp / plan.hg) % DS;            // which part of the output columns this warp owns
-    const int sub = warp / (plan.hg * DS);              // which of the wph interleaved block streams
+    const int hh = warp % vhg;                      // consumer head within the item
+    const int dhalf = (warp / vhg) % DS;            // which part of the output columns this warp owns
+    const int sub = warp / (vhg * DS);              // which of the wph interleaved block streams
     int next_blk = sub;                   // index, within the item, of this warp's next block: sub, sub + wph, ...
     const int g = lane >> 2, t = lane & 3;
     const float scale2 = a.scale * kLog2e;
@@ -729,19 +744,19 @@ __device__ __forceinline__ void fast_partial_body(const FastArgs& a)
     // the item's merge barrier, when no warp of the CTA still reads the old ones.
     uint32_t* q_frag = q_store + hh * (KS * 2 * 32) + lane;
     auto load_q = [&](int b, int hgroup) {
-        const int kv_head = hgroup * plan.hg + hh;
+        const int kv_head = hgroup * vhg + hh;
         const uint32_t* qrow = reinterpret_cast<const uint32_t*>(
-            a.q + ((long long)b * a.num_q_heads + (long long)kv_head * group + g) * D);
+            a.q + ((long long)b * a.num_q_heads + (long long)kv_head * vgroup + g) * D);
         uint32_t tmp[KS * 2];
 #pragma unroll
         for (int ks = 0; ks < KS; ++ks) {
-            tmp[2 * ks] = (g < group) ? qrow[ks * 8 + t] : 0u;
-            tmp[2 * ks + 1] = (g < group) ? qrow[ks * 8 + 4 + t] : 0u;
+            tmp[2 * ks] = (g < vgroup) ? qrow[ks * 8 + t] : 0u;
+            tmp[2 * ks + 1] = (g < vgroup) ? qrow[ks * 8 + 4 + t] : 0u;
         }
         if constexpr (kRope) {
             // q holds the un-rotated projection: rotate it at the sequence's current position, in
             // fp32, and round to fp16 exactly as the standalone rotation kernel would have stored it
-            if (g < group)
+            if (g < vgroup)
                 rope_rotate_q_words<KS>(tmp, a.rope_cos, a.rope_sin, a.kv_offsets[b], a.rope_type, a.rotary_dim, t);
         }
 #pragma unroll
@@ -749,7 +764,7 @@ __device__ __forceinline__ void fast_partial_body(const FastArgs& a)
         __syncwarp();
     };
 
-    ConsumerState<NT, kLoAcc> st;
+    ConsumerState<NT, kLoAcc && !kWide> st;
     ConsumerStateT<D / 16> tt;
     st.reset();
     tt.reset();
@@ -776,10 +791,11 @@ __device__ __forceinline__ void fast_partial_body(const FastArgs& a)
     // (rows 0-7, chunk 1), (rows 8-15, chunk 1).  A lane's row has r & 7 == lane & 7, so the
     // swizzle term of its address is a lane constant XORed with the k-step's chunk pair.
     const int blk_bytes = plan.blk_bytes;
-    const uint32_t k_lane_off = ((lane & 7) + ((lane >> 4) << 3)) * 128 + hh * (D / 64) * blk_bytes;
+    const int kv_hh = hh / nv;                          // KV head whose rows this warp reads
+    const uint32_t k_lane_off = ((lane & 7) + ((lane >> 4) << 3)) * 128 + kv_hh * (D / 64) * blk_bytes;
     const uint32_t k_lane_x = ((((lane >> 3) & 1) ^ (lane & 7)) << 4);
     const uint32_t v_lane_off = ((lane & 7) + (((lane >> 3) & 1) << 3)) * 128 +
-                                (hh * (D / 64) + dhalf * (DW / 64)) * blk_bytes + plan.tile * plan.row_bytes;
+                                (kv_hh * (D / 64) + dhalf * (DW / 64)) * blk_bytes + plan.tile * plan.row_bytes;
     const uint32_t v_lane_x = (((lane >> 4) ^ (lane & 7)) << 4);
 
     // The first item is known without the loader: fetch its Q while the first tile is in flight.
@@ -849,12 +865,12 @@ __device__ __forceinline__ void fast_partial_body(const FastArgs& a)
             if (r0 >= nvalid) break;
             if constexpr (kT) {
                 float sr[4];
-                qk_block_t<D>(q_frag, (tile_base + r0 * 128 + k_lane_off) | k_lane_x, blk_bytes, sr);
-                softmax_pv_t<D / 16>(tt, sr, (tile_base + r0 * 128 + v_lane_off) | v_lane_x, blk_bytes, nvalid - r0, scale2, g);
+                qk_block_t<D, kWide ? 8 : 2>(q_frag, (tile_base + r0 * 128 + k_lane_off) | k_lane_x, blk_bytes, sr);
+                softmax_pv_t<D / 16, kWide>(tt, sr, (tile_base + r0 * 128 + v_lane_off) | v_lane_x, blk_bytes, nvalid - r0, scale2, g);
             } else {
                 float sn[2][2];
-                qk_block<D, kQkChains>(q_frag, (tile_base + r0 * 128 + k_lane_off) | k_lane_x, blk_bytes, sn);
-                softmax_pv<NT, kLoAcc>(st, sn, (tile_base + r0 * 128 + v_lane_off) | v_lane_x, blk_bytes, nvalid - r0, scale2, t);
+                qk_block<D, kWide ? D / 16 : kQkChains>(q_frag, (tile_base + r0 * 128 + k_lane_off) | k_lane_x, blk_bytes, sn);
+                softmax_pv<NT, kLoAcc && !kWide, kWide>(st, sn, (tile_base + r0 * 128 + v_lane_off) | v_lane_x, blk_bytes, nvalid - r0, scale2, t);
             }
         }
         if (flags & kTileLast) {
@@ -878,8 +894,8 @@ __device__ __forceinline__ void fast_partial_body(const FastArgs& a)
                     // maximum and store it; the warps with sub 0 store m and l
                     const bool empty = (flags & kTileEmpty) != 0;
                     const bool write_o = !empty || (a.flags & kFlagWriteEmptyO);
-                    const long long stat_base = ((long long)item_b * a.num_q_heads + (long long)item_hgroup * plan.hg * group +
-                                                 (long long)hh * group) * a.max_chunks + item_c;
+                    const long long stat_base = ((long long)item_b * a.num_q_heads + (long long)item_hgroup * vhg * vgroup +
+                                                 (long long)hh * vgroup) * a.max_chunks + item_c;
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
                         const int r = 2 * t + h;
@@ -891,7 +907,7 @@ __device__ __forceinline__ void fast_partial_body(const FastArgs& a)
 #endif
                         const float f = fast_exp2(tt.m[h] - m_head);
                         l_head *= f;
-                        if (r < group) {
+                        if (r < vgroup) {
                             const long long stat = stat_base + (long long)r * a.max_chunks;
                             if (write_o) {
                                 float* orow = a.partial_o + stat * D + g;
@@ -936,18 +952,18 @@ __device__ __forceinline__ void fast_partial_body(const FastArgs& a)
                     st.m = m_true;
                 }
 #endif
-                if (g < group && (a.flags & kFlagDirectOutput)) {
+                if (g < vgroup && (a.flags & kFlagDirectOutput)) {
                     // unsplit: this warp holds the whole sequence's state for its rows
-                    const long long row = (long long)item_b * a.num_q_heads + (long long)item_hgroup * plan.hg * group +
-                                          (long long)hh * group + g;
+                    const long long row = (long long)item_b * a.num_q_heads + (long long)item_hgroup * vhg * vgroup +
+                                          (long long)hh * vgroup + g;
                     const float inv = 1.f / fmaxf(l_own, 1e-20f);
 #pragma unroll
                     for (int n = 0; n < NT; ++n)
                         store_out2(a.output, a.out_kind, row * D + dhalf * DW + n * 8 + 2 * t,
                                    make_float2(st.o[n][0] * inv, st.o[n][1] * inv));
-                } else if (g < group) {
-                    const long long stat = ((long long)item_b * a.num_q_heads + (long long)item_hgroup * plan.hg * group +
-                                            (long long)hh * group + g) * a.max_chunks + item_c;
+                } else if (g < vgroup) {
+                    const long long stat = ((long long)item_b * a.num_q_heads + (long long)item_hgroup * vhg * vgroup +
+                                            (long long)hh * vgroup + g) * a.max_chunks + item_c;
                     if (!empty1 || (a.flags & kFlagWriteEmptyO)) {
                         float* out = a.partial_o + stat * D + dhalf * DW + 2 * t;
 #pragma unroll
@@ -980,8 +996,8 @@ __device__ __forceinline__ void fast_partial_body(const FastArgs& a)
 #else
                     const float m_head = tt.m[h];
 #endif
-                    if (r < group) {
-                        float* dst = merge + ((size_t)warp * group + r) * pitch;
+                    if (r < vgroup) {
+                        float* dst = merge + ((size_t)warp * vgroup + r) * pitch;
 #pragma unroll
                         for (int mt = 0; mt < D / 16; ++mt) {
                             dst[mt * 16 + g] = tt.o[mt][h];
@@ -995,8 +1011,8 @@ __device__ __forceinline__ void fast_partial_body(const FastArgs& a)
                 l_quad += __shfl_xor_sync(0xffffffffu, l_quad, 1);
                 l_quad += __shfl_xor_sync(0xffffffffu, l_quad, 2);
                 const float m_true = st.true_max();
-                if (g < group) {
-                    float* dst = merge + ((size_t)warp * group + g) * pitch;
+                if (g < vgroup) {
+                    float* dst = merge + ((size_t)warp * vgroup + g) * pitch;
 #pragma unroll
                     for (int n = 0; n < NT; ++n)
                         *reinterpret_cast<float2*>(dst + dhalf * DW + n * 8 + 2 * t) = make_float2(st.o[n][0], st.o[n][1]);
@@ -1017,16 +1033,16 @@ __device__ __forceinline__ void fast_partial_body(const FastArgs& a)
             // weights from broadcast reads and merges D / 16 consecutive columns.  With 12 query heads and six
             // warps the CTA's merge is one pass instead of two.
             const bool empty = (flags & kTileEmpty) != 0;
-            const int heads_item = plan.hg * group;                    // query heads of this item
+            const int heads_item = vhg * vgroup;                    // query heads of this item
             const long long stat0 = ((long long)item_b * a.num_q_heads + (long long)item_hgroup * heads_item) * a.max_chunks + item_c;
             const bool write_o = !empty || (a.flags & kFlagWriteEmptyO);
             for (int hq0 = 2 * warp; hq0 < heads_item; hq0 += 2 * plan.active_warps) {
                 const int hq = hq0 + (lane >> 4), l16 = lane & 15;
                 const bool pair_ok = hq < heads_item;
                 const int hqc = pair_ok ? hq : hq0;                     // an idle half-warp reads the first pair's rows
-                const int kvh = hqc / group, row = hqc - kvh * group;
-                const float* src0 = merge + ((size_t)kvh * group + row) * pitch;        // warp (sub 0, half 0, kvh)
-                const size_t hstride = (size_t)plan.hg * group * pitch;                  // same sub, next column half
+                const int kvh = hqc / vgroup, row = hqc - kvh * vgroup;
+                const float* src0 = merge + ((size_t)kvh * vgroup + row) * pitch;        // warp (sub 0, half 0, kvh)
+                const size_t hstride = (size_t)vhg * vgroup * pitch;                  // same sub, next column half
                 const size_t wstride = hstride * DS;                                     // next sub of the same head
                 constexpr int FPL = D / 16, NV = FPL / 4;                                // floats / float4s per lane
                 const int col0 = l16 * FPL;
@@ -1086,13 +1102,13 @@ __device__ __forceinline__ void fast_partial_body(const FastArgs& a)
             // One (KV head, query row) pair per warp pass: all lanes derive the pair's
             // weights from broadcast reads, then each lane merges its float4 columns.
             const bool empty = (flags & kTileEmpty) != 0;
-            const int heads_item = plan.hg * group;                    // query heads of this item
+            const int heads_item = vhg * vgroup;                    // query heads of this item
             const long long stat0 = ((long long)item_b * a.num_q_heads + (long long)item_hgroup * heads_item) * a.max_chunks + item_c;
             const bool write_o = !empty || (a.flags & kFlagWriteEmptyO);
             for (int hq = warp; hq < heads_item; hq += plan.active_warps) {
-                const int kvh = hq / group, row = hq - kvh * group;
-                const float* src0 = merge + ((size_t)kvh * group + row) * pitch;        // warp (sub 0, half 0, kvh)
-                const size_t hstride = (size_t)plan.hg * group * pitch;                  // same sub, next column half
+                const int kvh = hq / vgroup, row = hq - kvh * vgroup;
+                const float* src0 = merge + ((size_t)kvh * vgroup + row) * pitch;        // warp (sub 0, half 0, kvh)
+                const size_t hstride = (size_t)vhg * vgroup * pitch;                  // same sub, next column half
                 const size_t wstride = hstride * DS;                                     // next sub of the same head
                 constexpr int NV = (D + 127) / 128;                                      // float4 columns per lane
                 const bool col_ok = (D >= 128) || lane < D / 4;
@@ -1199,7 +1215,7 @@ __device__ __forceinline__ void fast_partial_body(const FastArgs& a)
 #endif
 #define VTEB_COMPACT_BOUNDS __maxnreg__(VTEB_COMPACT_MAXNREG)
 
-#define VTEB_FAST_PARTIAL_CS(NAME, DIM, CWARPS, BOUNDS, COLSPLIT)                                     \
+#define VTEB_FAST_PARTIAL_CS(NAME, DIM, CWARPS, BOUNDS, COLSPLIT, WIDE)                               \
     extern "C" __global__ void BOUNDS NAME(                                                           \
         const __half* __restrict__ q, const __half* __restrict__ k_cache,                             \
         const __half* __restrict__ v_cache, float* __restrict__ partial_m,                            \
@@ -1224,7 +1240,7 @@ __device__ __forceinline__ void fast_partial_body(const FastArgs& a)
         a.k_new = nullptr; a.v_new = nullptr;                                                         \
         a.tmap_k = &tmap_k; a.tmap_v = &tmap_v;                                                       \
         (void)head_dim;                                                                               \
-        fast_partial_body<DIM, CWARPS, false, COLSPLIT>(a);                                           \
+        fast_partial_body<DIM, CWARPS, false, COLSPLIT, WIDE>(a);                                     \
     }
 
 // The same kernel with the Q rotation folded into the Q load: `q` is the un-rotated projection,
@@ -1261,17 +1277,21 @@ __device__ __forceinline__ void fast_partial_body(const FastArgs& a)
         fast_partial_body<DIM, CWARPS, true>(a);                                                      \
     }
 
-#define VTEB_FAST_PARTIAL(NAME, DIM, CWARPS, BOUNDS) VTEB_FAST_PARTIAL_CS(NAME, DIM, CWARPS, BOUNDS, false)
+#define VTEB_FAST_PARTIAL(NAME, DIM, CWARPS, BOUNDS) VTEB_FAST_PARTIAL_CS(NAME, DIM, CWARPS, BOUNDS, false, false)
 VTEB_FAST_PARTIAL(vteb_split_kv_partial_d64_kernel, 64, kFullConsumerWarps, __launch_bounds__(kFullThreads, 1))
 VTEB_FAST_PARTIAL(vteb_split_kv_partial_d128_kernel, 128, kFullConsumerWarps, __launch_bounds__(kFullThreads, 1))
 VTEB_FAST_PARTIAL(vteb_split_kv_partial_d256_kernel, 256, kFullConsumerWarps, __launch_bounds__(kFullThreads, 1))
 VTEB_FAST_PARTIAL(vteb_split_kv_partial_compact_d64_kernel, 64, kCompactConsumerWarps, VTEB_COMPACT_BOUNDS)
 VTEB_FAST_PARTIAL(vteb_split_kv_partial_compact_d128_kernel, 128, kCompactConsumerWarps, VTEB_COMPACT_BOUNDS)
 VTEB_FAST_PARTIAL(vteb_split_kv_partial_compact_d256_kernel, 256, kCompactConsumerWarps, VTEB_COMPACT_BOUNDS)
-VTEB_FAST_PARTIAL_CS(vteb_split_kv_partial_compact_cs_d128_kernel, 128, kCompactConsumerWarps, VTEB_COMPACT_BOUNDS, true)
+VTEB_FAST_PARTIAL_CS(vteb_split_kv_partial_compact_cs_d128_kernel, 128, kCompactConsumerWarps, VTEB_COMPACT_BOUNDS, true, false)
 VTEB_FAST_PARTIAL_ROPE(vteb_split_kv_partial_rope_d64_kernel, 64, kFullConsumerWarps, __launch_bounds__(kFullThreads, 1))
 VTEB_FAST_PARTIAL_ROPE(vteb_split_kv_partial_rope_d128_kernel, 128, kFullConsumerWarps, __launch_bounds__(kFullThreads, 1))
 VTEB_FAST_PARTIAL_ROPE(vteb_split_kv_partial_rope_d256_kernel, 256, kFullConsumerWarps, __launch_bounds__(kFullThreads, 1))
 VTEB_FAST_PARTIAL_ROPE(vteb_split_kv_partial_compact_rope_d64_kernel, 64, kCompactConsumerWarps, VTEB_COMPACT_BOUNDS)
 VTEB_FAST_PARTIAL_ROPE(vteb_split_kv_partial_compact_rope_d128_kernel, 128, kCompactConsumerWarps, VTEB_COMPACT_BOUNDS)
 VTEB_FAST_PARTIAL_ROPE(vteb_split_kv_partial_compact_rope_d256_kernel, 256, kCompactConsumerWarps, VTEB_COMPACT_BOUNDS)
+// more than eight query heads per KV head (FastPlan::nv)
+VTEB_FAST_PARTIAL_CS(vteb_split_kv_partial_wide_d64_kernel, 64, kFullConsumerWarps, __launch_bounds__(kFullThreads, 1), false, true)
+VTEB_FAST_PARTIAL_CS(vteb_split_kv_partial_wide_d128_kernel, 128, kFullConsumerWarps, __launch_bounds__(kFullThreads, 1), false, true)
+VTEB_FAST_PARTIAL_CS(vteb_split_kv_partial_wide_d256_kernel, 256, kFullConsumerWarps, __launch_bounds__(kFullThreads, 1), false, true)

@@ -72,8 +72,9 @@ struct TileHeader {
 struct FastPlan {
     int hg;            // KV heads staged together per work item
     int n_hgroups;     // ceil(num_kv_heads / hg)
-    int wph;           // consumer warps per KV head
-    int active_warps;  // wph * hg
+    int nv;            // consumer heads per KV head: runs of group / nv <= 8 query heads (1 up to eight query heads per KV head)
+    int wph;           // consumer warps per consumer head
+    int active_warps;  // wph * hg * nv
     int tile;          // positions per stage
     int row_bytes;     // bytes of one position's K (or V) row for the head group
     int blk_bytes;     // one 128-byte-wide column block of a tile: tile * 128
@@ -102,9 +103,14 @@ __host__ __device__ inline int vteb_round_up(int x, int m) { return (x + m - 1) 
 #define VTEB_TRANSPOSED 1
 #endif
 
-__host__ __device__ inline FastPlan make_fast_plan(int num_q_heads, int num_kv_heads, int head_dim, int compact = 0) {
+// `wide`: the plan of the kernels for more than eight query heads per KV head (full shape only).  The eight
+// columns of an mma hold one run of up to eight query heads, so such a group is cut into `nv` equal runs,
+// each served by warps of its own from the same staged rows; a group without an equal cut into at most one
+// run per consumer warp (11, 13, ... heads) has no such plan.
+__host__ __device__ inline FastPlan make_fast_plan(int num_q_heads, int num_kv_heads, int head_dim, int compact = 0, int wide = 0) {
     FastPlan p;
     p.ok = 0;
+    p.nv = 1;
     p.hg = p.n_hgroups = p.wph = p.active_warps = p.tile = p.row_bytes = p.blk_bytes = 0;
     p.stage_bytes = p.merge_bytes = p.q_bytes = p.nstages = p.smem_bytes = 0;
     const int cw = compact ? kCompactConsumerWarps : kFullConsumerWarps;
@@ -113,14 +119,21 @@ __host__ __device__ inline FastPlan make_fast_plan(int num_q_heads, int num_kv_h
     p.threads = (cw + p.loader_warps) * 32;
     if (num_kv_heads <= 0 || num_q_heads <= 0 || num_q_heads % num_kv_heads != 0) return p;
     int group = num_q_heads / num_kv_heads;
-    if (group > 8) return p;
+    if ((group > 8) != (wide != 0) || (wide && compact)) return p;
+    if (wide) {
+        int nv = 2;
+        while (nv <= cw && (group % nv != 0 || group / nv > 8)) ++nv;
+        if (nv > cw) return p;
+        p.nv = nv;
+        group /= nv;
+    }
     if (head_dim != 64 && head_dim != 128 && head_dim != 256) return p;
     // largest divisor of num_kv_heads with hg * head_dim <= 512 halves and a consumer warp left
     // for every head; 256-wide heads go one per item: a 16-position block of such a head keeps
     // a warp for ~1,500 cycles, and four blocks in flight per head instead of two took the
     // 16-sequence ragged batch from 5.6 to 5.9 TB/s
     int cap = (head_dim == 256) ? 1 : 512 / head_dim;
-    if (cap > cw) cap = cw;
+    if (cap > cw / p.nv) cap = cw / p.nv;
     int hg = 1;
     for (int d = 1; d <= cap; ++d) if (num_kv_heads % d == 0) hg = d;
     // 256-wide heads in the untransposed form: two warps share a (head, block), each owning half of the
@@ -128,9 +141,9 @@ __host__ __device__ inline FastPlan make_fast_plan(int num_q_heads, int num_kv_h
     const int dsplit = (head_dim == 256 && (compact || !VTEB_TRANSPOSED)) ? 2 : 1;
     p.hg = hg;
     p.n_hgroups = num_kv_heads / hg;
-    p.wph = cw / (hg * dsplit);
+    p.wph = cw / (hg * p.nv * dsplit);
     if (p.wph < 1) return p;
-    p.active_warps = p.wph * hg * dsplit;
+    p.active_warps = p.wph * hg * p.nv * dsplit;
     p.row_bytes = hg * head_dim * 2;
     // 16 KB of K (and of V) per stage; 32 KB for 1024-byte rows, whose tensor-map boxes would
     // otherwise be 2 KB each (measured on 64 ragged sequences of 8 x 64-wide heads: 6.5 against 5.7 TB/s)
@@ -141,7 +154,7 @@ __host__ __device__ inline FastPlan make_fast_plan(int num_q_heads, int num_kv_h
     p.blk_bytes = tile * 128;
     p.stage_bytes = 2 * tile * p.row_bytes;
     p.merge_bytes = vteb_round_up(p.active_warps * group * (head_dim + kMergePad) * 4, 128);
-    p.q_bytes = hg * (head_dim / 8) * 32 * 4;   // one fragment image per KV head, shared by its warps
+    p.q_bytes = hg * p.nv * (head_dim / 8) * 32 * 4;   // one fragment image per consumer head, shared by its warps
     int left = kSmemBudget - kCtrlBytes - p.merge_bytes - p.q_bytes - kStageAlign;
     int n = left / p.stage_bytes;
     if (n > kMaxStages) n = kMaxStages;

@@ -552,9 +552,9 @@ int vteb_ipc_close_handle(void* dev_ptr) {
 }
 
 // ---- split-KV decode attention ---------------------------------------------
-static int fill_plan(int num_q_heads, int num_kv_heads, int head_dim, int compact, vteb_fast_plan* plan) {
+static int fill_plan(int num_q_heads, int num_kv_heads, int head_dim, int compact, vteb_fast_plan* plan, int wide = 0) {
     if (!plan) return fail(VTEB_ERR_INVALID_ARGUMENT, "null plan");
-    const vteb::FastPlan p = vteb::make_fast_plan(num_q_heads, num_kv_heads, head_dim, compact);
+    const vteb::FastPlan p = vteb::make_fast_plan(num_q_heads, num_kv_heads, head_dim, compact, wide);
     memset(plan, 0, sizeof(*plan));
     plan->ok = p.ok;
     plan->hg = p.hg;
@@ -574,6 +574,10 @@ int vteb_split_kv_plan(int num_q_heads, int num_kv_heads, int head_dim, vteb_fas
 
 int vteb_split_kv_plan_compact(int num_q_heads, int num_kv_heads, int head_dim, vteb_fast_plan* plan) {
     return fill_plan(num_q_heads, num_kv_heads, head_dim, 1, plan);
+}
+
+int vteb_split_kv_plan_wide(int num_q_heads, int num_kv_heads, int head_dim, vteb_fast_plan* plan) {
+    return fill_plan(num_q_heads, num_kv_heads, head_dim, 0, plan, 1);
 }
 
 int vteb_kv_tensor_map(void* out_128_bytes, const void* cache, long long n_rows, int row_halves, int box_rows) {

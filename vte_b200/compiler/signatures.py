@@ -58,6 +58,7 @@ KERNEL_SIGNATURES = {
     "vteb_split_kv_combine_push_kernel": [P, P, P, P, ctypes.Structure, I, I, I, I, P, I, I, I, I, I, P, P, P, P],
     "vteb_merge_shard_states_ll_kernel": [P, P, I, I, I, I, I, P, P],
     "vteb_advance_step_kernel": [P],
+    "vteb_stage_copy_kernel": [P, P, I],
 }
 
 # template name (what the reference passes to load_kernel_safe) -> source file

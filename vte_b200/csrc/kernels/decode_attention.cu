@@ -146,14 +146,17 @@ extern "C" __global__ void rope_kernel(
 //
 // What bounds it is issue slots and the latency of a warp's chain (K and V come through L2 once per query
 // head).  So a warp takes P = U * 256 / D positions per turn: U = 8 or 16 16-byte loads of K and as many of V
-// per lane are in flight while the previous turn is computed, a row's D / 8 lanes reduce their scores together
-// (one shuffle a score where one score took five), fp32 FMAs go two at a time, one exponential per position, and
+// per lane are in flight while the previous turn is computed, the scores come from mma.sync (exact fp16 products,
+// fp32 sums in four chains added in registers; a turn of 8 positions reduces them over a row's D / 8 lanes
+// instead), the fp32 FMAs of P V go two at a time, one exponential per position, and
 // the maximum moves only when a score passes it by kCompatLazyMax.  Eight sequences of 700 to 3,960 positions,
 // 32 query heads on 2 KV heads of 128, 8 splits, append and reduce included: 88 us a layer with one position
 // per warp and turn, 42 us so (U = 8, 128 registers, four blocks of 128 threads per SM; U = 16 needs 255
 // registers: 56 us).  Unsplit, four sequences of 103 to 1,383 positions, 12 heads of 128: 178 us against 21 us
 // (U = 16; 27 us with 8: there a block has an SM to itself).
-// The unsplit blocks of a sequence ask L2 for its older rows at once: the same launches 18.4 us instead of 21.5.
+// The unsplit blocks of a sequence ask L2 for its older rows at once: the same launches 18.4 us instead of 21.5,
+// and with the scores by mma 16.8 (relative error of fp32 outputs against 64 bits 1.4e-7 to 5.8e-7 over 1 and 8
+// splits of up to 8,192 positions, 1.4e-7 to 5.9e-7 with FMAs, 1.5e-7 to 1.2e-6 with one position a turn).
 // kUnsplit: ONE split covering every position, together with the cache append and the normalisation:
 // flash_attention_kernel below.
 // ---------------------------------------------------------------------------
@@ -207,6 +210,9 @@ __device__ __forceinline__ void compat_partial_body(
     // for four blocks of 128 threads per SM where it has not
     constexpr int U = (kUnsplit && D > 64) ? 16 : 8;
     constexpr int P = U * RPI;         // positions per turn of a warp
+    // scores by mma (positions as the M dimension, the head's Q in every column) where a turn fills its 16 rows
+    constexpr bool kMma = P >= 16;
+    constexpr int MT = kMma ? P / 16 : 1, KK = D / 32;      // row tiles of a turn, 16-byte pieces of K per lane and row
     float* sh_m = sh; float* sh_l = sh + 8; float* sh_t = sh + 16; float* sh_o = sh + 24;
 
     const int b = blockIdx.x, h = blockIdx.y, c = kUnsplit ? 0 : blockIdx.z;
@@ -267,15 +273,47 @@ __device__ __forceinline__ void compat_partial_body(
         }
     };
 
+    // For the mma, lane (g = lane / 4, t = lane % 4) holds channels 32 kk + 8 t .. + 7 of rows g and g + 8: two
+    // k-steps' A fragments.  A dot product does not care which channel is called which k, so Q is dealt alike.
+    const int g = lane >> 2, t = lane & 3;
+    auto load_k = [&](uint4 (&r)[U], int j0) {
+        if constexpr (kMma) {
+            const __half* base = k_cache + head_base + 8 * t + (long long)(j0 + g) * row_stride;
+            if (j0 + P < end) {
+#pragma unroll
+                for (int n = 0; n < 2 * MT; ++n)
+#pragma unroll
+                    for (int kk = 0; kk < KK; ++kk) r[n * KK + kk] = load_8_halves<kVec>(base + (long long)(n * 8) * row_stride + kk * 32);
+            } else {
+#pragma unroll
+                for (int n = 0; n < 2 * MT; ++n) {
+                    const int j = j0 + n * 8 + g;
+                    const __half* p = base + (long long)(n * 8) * row_stride;
+                    if (kUnsplit && j == total - 1) p = k_new + new_base + 8 * t;
+#pragma unroll
+                    for (int kk = 0; kk < KK; ++kk) {
+                        r[n * KK + kk] = make_uint4(0u, 0u, 0u, 0u);
+                        if (j < end) r[n * KK + kk] = load_8_halves<kVec>(p + kk * 32);
+                    }
+                }
+            }
+        } else {
+            load_turn(r, kbase, k_new, j0);
+        }
+    };
     uint4 kr[U], vr[U];
     int j0 = start + warp * P;
-    if (j0 < end) { load_turn(kr, kbase, k_new, j0); load_turn(vr, vbase, v_new, j0); }
-    F32x2 qf[4];
-    {
-        const __half* qp = q + ((long long)b * num_q_heads + h) * D + col;
-        const float f = scale * kLog2e;
+    if (j0 < end) { load_k(kr, j0); load_turn(vr, vbase, v_new, j0); }
+    const float f = scale * kLog2e;
+    const __half* qrow = q + ((long long)b * num_q_heads + h) * D;
+    F32x2 qf[kMma ? 1 : 4];
+    uint4 qb[kMma ? KK : 1];
+    if constexpr (kMma) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) qf[i] = pack_f32x2(__half2float(qp[2 * i]) * f, __half2float(qp[2 * i + 1]) * f);
+        for (int kk = 0; kk < KK; ++kk) qb[kk] = load_8_halves<kVec>(qrow + kk * 32 + 8 * t);
+    } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) qf[i] = pack_f32x2(__half2float(qrow[col + 2 * i]) * f, __half2float(qrow[col + 2 * i + 1]) * f);
     }
     float m = kNeutralM, mt = kNeutralM, l = 0.f;    // reference maximum (warp), largest score seen and sum of weights (lane)
     F32x2 o[4];
@@ -284,6 +322,32 @@ __device__ __forceinline__ void compat_partial_body(
 
     for (; j0 < end; j0 += nwarps * P) {
         const int next = j0 + nwarps * P;
+        float score;
+        bool valid;
+        if constexpr (kMma) {
+            float sc[2 * MT];
+#pragma unroll
+            for (int mt = 0; mt < MT; ++mt) {
+                float acc[4][4];
+#pragma unroll
+                for (int c4 = 0; c4 < 4; ++c4) acc[c4][0] = acc[c4][1] = acc[c4][2] = acc[c4][3] = 0.f;
+#pragma unroll
+                for (int kk = 0; kk < KK; ++kk) {
+                    const uint4 lo = kr[(2 * mt) * KK + kk], hi = kr[(2 * mt + 1) * KK + kk];
+                    mma_full(acc[(2 * kk) & 3], lo.x, hi.x, lo.y, hi.y, qb[kk].x, qb[kk].y);
+                    mma_full(acc[(2 * kk + 1) & 3], lo.z, hi.z, lo.w, hi.w, qb[kk].z, qb[kk].w);
+                }
+                sc[2 * mt] = (acc[0][0] + acc[1][0]) + (acc[2][0] + acc[3][0]);
+                sc[2 * mt + 1] = (acc[0][2] + acc[1][2]) + (acc[2][2] + acc[3][2]);
+            }
+            if (next < end) load_k(kr, next);
+            // every lane has the scores of rows g, g + 8, ...: lane (g, t) keeps that of position 8 t + g
+            // (one row tile: 8 (t & 1) + g, so that two lanes carry every weight)
+            float raw = (t & 1) ? sc[1] : sc[0];
+            if constexpr (MT == 2) { if (t & 2) raw = (t & 1) ? sc[3] : sc[2]; }
+            valid = j0 + 8 * (t & (2 * MT - 1)) + g < end;
+            score = valid ? raw * f : kNeutralM;
+        } else {
         float s[U];
 #pragma unroll
         for (int i = 0; i < U; ++i) {
@@ -295,7 +359,7 @@ __device__ __forceinline__ void compat_partial_body(
             const float2 t = unpack_f32x2(a);
             s[i] = t.x + t.y;
         }
-        if (next < end) load_turn(kr, kbase, k_new, next);
+        if (next < end) load_k(kr, next);
         // U sums over the LPR lanes of a row at once: each exchange halves the number of scores a lane
         // carries; lane (i * LPR / U) of a row's lanes ends with score i (its neighbours with copies of it).
 #pragma unroll
@@ -310,8 +374,9 @@ __device__ __forceinline__ void compat_partial_body(
         }
 #pragma unroll
         for (int mask = LPR / U / 2; mask >= 1; mask >>= 1) s[0] += __shfl_xor_sync(0xffffffffu, s[0], mask);
-        const bool valid = j0 + ((lane % LPR) / (LPR / U)) * RPI + sub < end;
-        const float score = valid ? s[0] : kNeutralM;
+        valid = j0 + ((lane % LPR) / (LPR / U)) * RPI + sub < end;
+        score = valid ? s[0] : kNeutralM;
+        }
         mt = fmaxf(mt, score);
         if (__any_sync(0xffffffffu, score > m + kCompatLazyMax)) {
             float up = score;
@@ -329,7 +394,8 @@ __device__ __forceinline__ void compat_partial_body(
         l += p;
 #pragma unroll
         for (int i = 0; i < U; ++i) {
-            const float pi = __shfl_sync(0xffffffffu, p, sub * LPR + i * (LPR / U));
+            const int r = i * RPI + sub;                       // row of the turn
+            const float pi = __shfl_sync(0xffffffffu, p, kMma ? ((r & 7) << 2) + (r >> 3) : sub * LPR + i * (LPR / U));
             const F32x2 pp = pack_f32x2(pi, pi);
             o[0] = fma_f32x2(pp, widen_half2(vr[i].x), o[0]);
             o[1] = fma_f32x2(pp, widen_half2(vr[i].y), o[1]);
@@ -351,7 +417,7 @@ __device__ __forceinline__ void compat_partial_body(
         l += __shfl_xor_sync(0xffffffffu, l, off);
         mt = fmaxf(mt, __shfl_xor_sync(0xffffffffu, mt, off));
     }
-    if (lane == 0) { sh_m[warp] = m; sh_l[warp] = l * ((float)U / LPR); sh_t[warp] = mt; }   // LPR / U lanes carried every weight
+    if (lane == 0) { sh_m[warp] = m; sh_l[warp] = l * (P / 32.f); sh_t[warp] = mt; }   // 32 / P lanes carried every weight
     if (sub == 0) {
 #pragma unroll
         for (int i = 0; i < 8; ++i) sh_o[warp * D + col + i] = of[i];

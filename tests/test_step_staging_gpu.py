@@ -1,4 +1,4 @@
-"""An end-to-end step's staging copies as launches, and shares long enough for the split kernel to hold its tiles back."""
+"""An end-to-end step's staging copies as launches."""
 import numpy as np
 import pytest
 
@@ -31,34 +31,3 @@ def test_staging_by_launch_and_by_copy_node_give_the_same_step(cuda_runtime, cod
         assert np.array_equal(by_launch, by_node)
         for l in range(L):
             assert np.max(np.abs(by_launch[l] - orc.decode_attention(q[l], k, v, off))) <= 1e-5
-
-
-@pytest.mark.parametrize("heads", [(28, 4, 128), (32, 8, 64)], ids=str)
-def test_long_shares_behind_an_append(cuda_runtime, codegen, heads):
-    """Shares of more than twice the stages' tiles, replayed behind an append: what was not asked for before the
-    dependency wait must still arrive, and the newest rows must be this step's.  Bound as in the wide-group test:
-    fp32 sums of at most 3,000 probabilities, values N(0, 1)."""
-    from vte_b200.core.decode_executor import DecodeAttentionExecutor
-    Hq, Hkv, D = heads
-    B, S = 12, 3000
-    rng = np.random.default_rng([Hq, D])
-    f16 = lambda *s: rng.standard_normal(s, dtype=np.float32).astype(np.float16)
-    k, v = f16(B, S, Hkv, D), f16(B, S, Hkv, D)
-    ex = DecodeAttentionExecutor(cuda_runtime, codegen, {"attention.head_count": Hq, "attention.head_count_kv": Hkv,
-                                                         "attention.key_length": D}, B, S, 2, n_kv_buffers=1, with_append=True)
-    try:
-        plan = ex.dispatcher._plan
-        off = rng.integers(2400, S, size=B).astype(np.int32)
-        assert ex.dispatcher.balanced and (off + 1).sum() // cuda_runtime.get_num_cus() > 2 * plan.nstages * plan.tile
-        q, kn, vn = f16(2, B, Hq, D), f16(2, B, Hkv, D), f16(2, B, Hkv, D)
-        ex.upload_cache(0, k, v)
-        for l in range(2):
-            ex.upload_layer(l, q[l])
-            ex.upload_new_kv(l, kn[l], vn[l])
-        for _ in range(2):
-            out = ex.execute_decode_batch(off)
-        for l in range(2):
-            orc.kv_cache_append(kn[l], vn[l], k, v, off)
-            assert np.max(np.abs(out[l] - orc.decode_attention(q[l], k, v, off))) <= 1e-5
-    finally:
-        ex.cleanup()

@@ -468,15 +468,6 @@ __device__ __forceinline__ void fast_partial_body(const FastArgs& a)
         int stage = 0, filled = 0;
         uint32_t empty_parity = 0;
         bool dep_done = false;
-        // Shares of two to sixteen times what the stages hold: ask for one tile only before the launch in front is
-        // over.  All stages' worth (28 MB over the grid) at once makes the combine in front, which reads its
-        // partials through the same L2, 2 to 3 us longer, and the stream is long enough to make up for the later
-        // start.  Eight sequences of 1,024 to 16,384 positions, 8 x 64: 31.5 -> 30.9 us a layer with one tile,
-        // 30.9 with two, 32.2 with none.  Shorter shares are their first tiles (a group of sixteen, four tiles a CTA:
-        // 20.2 -> 20.4 us with the limit); for longer ones the combine is a few percent (64 sequences: 178.6 us
-        // without, 178.9 with it).
-        const int stages_hold = nstages * plan.tile;
-        const bool few_early = !kWide && balanced && share.per > 2 * stages_hold && share.per <= 16 * stages_hold;
         int item = blockIdx.x;
         long long cursor = share_lo;               // balanced partition: where the next piece starts
         bool alive = true;
@@ -504,7 +495,6 @@ __device__ __forceinline__ void fast_partial_body(const FastArgs& a)
                     empty_parity ^= (1u << stage);
                 }
                 const uint32_t bar = full0 + 8 * stage;
-                if (few_early && !dep_done && filled >= 1) { grid_dependency_wait(); dep_done = true; }
                 const bool empty_item = !stop && g.end <= g.start;
                 const int pos0 = stop ? 0 : g.start + t * plan.tile;
                 const int nvalid = (stop || empty_item) ? 0 : min(plan.tile, g.end - pos0);

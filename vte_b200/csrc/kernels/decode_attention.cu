@@ -147,8 +147,8 @@ extern "C" __global__ void rope_kernel(
 // What bounds it is issue slots and the latency of a warp's chain (K and V come through L2 once per query
 // head).  So a warp takes P = U * 256 / D positions per turn: U = 8 or 16 16-byte loads of K and as many of V
 // per lane are in flight while the previous turn is computed, the scores come from mma.sync (exact fp16 products,
-// fp32 sums in four chains added in registers; a turn of 8 positions reduces them over a row's D / 8 lanes
-// instead), the fp32 FMAs of P V go two at a time, one exponential per position, and
+// fp32 sums in four chains added in registers; the split kernel uses FMAs and reduces them over a row's D / 8
+// lanes), the fp32 FMAs of P V go two at a time, one exponential per position, and
 // the maximum moves only when a score passes it by kCompatLazyMax.  Eight sequences of 700 to 3,960 positions,
 // 32 query heads on 2 KV heads of 128, 8 splits, append and reduce included: 88 us a layer with one position
 // per warp and turn, 42 us so (U = 8, 128 registers, four blocks of 128 threads per SM; U = 16 needs 255
@@ -210,8 +210,10 @@ __device__ __forceinline__ void compat_partial_body(
     // for four blocks of 128 threads per SM where it has not
     constexpr int U = (kUnsplit && D > 64) ? 16 : 8;
     constexpr int P = U * RPI;         // positions per turn of a warp
-    // scores by mma (positions as the M dimension, the head's Q in every column) where a turn fills its 16 rows
-    constexpr bool kMma = P >= 16;
+    // Scores by mma (positions as the M dimension, the head's Q in every column) in the unsplit kernel, whose blocks
+    // have an SM each: there issue slots bound a turn.  The split kernel keeps the FMAs: with four blocks per SM the
+    // other warps fill the slots, and K read in 64-byte pieces of rows costs it more (33.8 -> 36.5 us a layer).
+    constexpr bool kMma = kUnsplit && P >= 16;
     constexpr int MT = kMma ? P / 16 : 1, KK = D / 32;      // row tiles of a turn, 16-byte pieces of K per lane and row
     float* sh_m = sh; float* sh_l = sh + 8; float* sh_t = sh + 16; float* sh_o = sh + 24;
 

@@ -173,7 +173,8 @@ int vteb_combine_rows_epl(int rows, int head_dim);
 /* One layer's decode attention for a batch: split kernel then combine.
  *   q [batch, Hq, D] fp16; k_cache, v_cache [batch, max_seq, Hkv, D] fp16 with
  *   sequence b at element offset b * kv_batch_stride; kv_offsets int32[batch]
- *   (device), sequence b attends to positions 0..kv_offsets[b];
+ *   (device), sequence b attends to positions 0..kv_offsets[b], all of them within its
+ *   kv_batch_stride elements (0 for one sequence: length not known, no tensor-map copies);
  *   partial_m, partial_l fp32[batch*Hq*max_chunks], partial_o
  *   fp32[batch*Hq*max_chunks*D] scratch; work int32[4] scratch that must be
  *   zero before the first call (word 0: work-queue ticket, word 1: status);

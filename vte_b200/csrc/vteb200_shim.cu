@@ -698,9 +698,11 @@ int vteb_split_kv_decode(const void* q, const void* k_cache, const void* v_cache
     memset(&tmk, 0, sizeof(tmk));
     memset(&tmv, 0, sizeof(tmv));
     const int row_halves = num_kv_heads * head_dim;
-    if (!(flags & VTEB_ATTN_NO_TENSOR_MAPS) && kv_batch_stride % row_halves == 0 && row_halves % 64 == 0) {
-        const unsigned long long rows_per_seq = (unsigned long long)(kv_batch_stride / row_halves);
-        const unsigned long long n_rows = batch > 1 ? rows_per_seq * batch : 0xffffffffULL;   // one sequence: its length is not known here
+    // For one sequence a stride of 0 says nothing about the cache's rows: 16-byte copies then.  (A map of 2^32 - 1 rows
+    // in its place raised an illegal-instruction fault at the first whole tile.)
+    if (!(flags & VTEB_ATTN_NO_TENSOR_MAPS) && (kv_batch_stride > 0 || batch > 1) && kv_batch_stride % row_halves == 0 &&
+        row_halves % 64 == 0) {
+        const unsigned long long n_rows = (unsigned long long)(kv_batch_stride / row_halves) * batch;
         if ((rc = encode_kv_tensor_map(&tmk, k_cache, n_rows, row_halves, p.tile))) return rc;
         if ((rc = encode_kv_tensor_map(&tmv, v_cache, n_rows, row_halves, p.tile))) return rc;
         kflags |= kFlagTensorMaps;

@@ -240,7 +240,10 @@ int vteb_split_kv_decode_noalloc(const void* q, const void* k_cache, const void*
 int vteb_noalloc_check_status(void* stream);
 
 /* Writes the current token's K/V rows at position kv_offsets[b]
- * (kv_cache_append.hip.template:13-39; launch built at split_kv_attention.py:186-194). */
+ * (kv_cache_append.hip.template:13-39; launch built at split_kv_attention.py:186-194).
+ * Ordered behind everything before it on the stream, and so is whatever follows it: a
+ * vteb_split_kv_decode behind it, with or without VTEB_ATTN_PROGRAMMATIC, sees offsets and
+ * cache rows that any launch or copy in front of the append wrote. */
 int vteb_kv_cache_append(const void* k, const void* v, void* k_cache, void* v_cache,
                          const int* kv_offsets, int batch, int num_kv_heads, int head_dim,
                          long long kv_batch_stride, void* stream);

@@ -25,6 +25,7 @@ _FAST_COMBINE = _REDUCE + [I, P]                          # dsplit, ticket
 
 KERNEL_SIGNATURES = {
     "kv_cache_append_kernel": [P, P, P, P, I, I, P, I],
+    "vteb_kv_cache_append_ordered_kernel": [P, P, P, P, I, I, P, I],   # the direct entry point's
     "kv_cache_append_rope_kernel": [P, P, P, P, I, I, P, I] + _ROPE_TAIL,
     "rope_kernel": [P, P, P, P, I, I, I, I, P, I, I],
     "flash_attention_kernel": [P, P, P, P, P, P, I, I, I, I, F, P, I],     # flash_attention.hip.template:29-43

@@ -34,18 +34,22 @@ using namespace vteb;
 // kv_cache_append_kernel: grid (B, Hkv, 1), block (D, 1, 1).
 // Replaces vte/compiler/templates/rdna/kv_cache_append.hip.template:13-39.
 // Bound by latency alone: wait, read, store.  The rows are read together with the offset instead of after it
-// (28 layers of one sequence of 1,531 positions: 218.2 -> 213.3 us), and the direct entry point launches it
-// with programmatic dependence, whose wait is the kernel's first action, so any launch may stand before it
-// (32 sequences of 100 to 4,000 positions, append and attention: 41.1 -> 36.9 us).
+// (28 layers of one sequence of 1,531 positions: 218.2 -> 213.3 us).
+//
+// Two builds that differ in when the launch behind may start.  kv_cache_append_kernel releases it at once: the split
+// kernel then reads the offsets and older rows while whatever stands in front of the append may still run, so both
+// must be final before that launch, as an executor's are.  vteb_kv_cache_append_ordered_kernel, which the direct
+// entry point launches, waits first and releases after: everything in front of the append is complete and visible
+// by the time the split kernel starts, whoever launched it, and only the append itself overlaps with it (32 sequences
+// of 100 to 4,000 positions, append and attention, one layer a pass: 39.0 us, 41.1 with an ordinary launch of the
+// append, 36.8 with the early release).
 // ---------------------------------------------------------------------------
-extern "C" __global__ void kv_cache_append_kernel(
+__device__ __forceinline__ void append_body(
     const __half* __restrict__ k, const __half* __restrict__ v,
     __half* __restrict__ k_cache, __half* __restrict__ v_cache,
     int num_kv_heads, int head_dim,
     const int* __restrict__ kv_cache_offset_ptr, int kv_batch_stride)
 {
-    grid_launch_dependents();
-    grid_dependency_wait();
     const int b = blockIdx.x, head = blockIdx.y;
     const long long src = ((long long)b * num_kv_heads + head) * head_dim;
     // the row and its offset are asked for together: only the stores need the offset
@@ -58,6 +62,28 @@ extern "C" __global__ void kv_cache_append_kernel(
         k_cache[dst + d] = k[src + d];
         v_cache[dst + d] = v[src + d];
     }
+}
+
+extern "C" __global__ void kv_cache_append_kernel(
+    const __half* __restrict__ k, const __half* __restrict__ v,
+    __half* __restrict__ k_cache, __half* __restrict__ v_cache,
+    int num_kv_heads, int head_dim,
+    const int* __restrict__ kv_cache_offset_ptr, int kv_batch_stride)
+{
+    grid_launch_dependents();
+    grid_dependency_wait();
+    append_body(k, v, k_cache, v_cache, num_kv_heads, head_dim, kv_cache_offset_ptr, kv_batch_stride);
+}
+
+extern "C" __global__ void vteb_kv_cache_append_ordered_kernel(
+    const __half* __restrict__ k, const __half* __restrict__ v,
+    __half* __restrict__ k_cache, __half* __restrict__ v_cache,
+    int num_kv_heads, int head_dim,
+    const int* __restrict__ kv_cache_offset_ptr, int kv_batch_stride)
+{
+    grid_dependency_wait();
+    grid_launch_dependents();
+    append_body(k, v, k_cache, v_cache, num_kv_heads, head_dim, kv_cache_offset_ptr, kv_batch_stride);
 }
 
 // ---------------------------------------------------------------------------

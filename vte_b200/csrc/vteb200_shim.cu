@@ -796,7 +796,8 @@ int vteb_kv_cache_append(const void* k, const void* v, void* k_cache, void* v_ca
         return fail(VTEB_ERR_INVALID_ARGUMENT, "bad dimension");
     if (kv_batch_stride < 0 || kv_batch_stride > 0x7fffffffLL)
         return fail(VTEB_ERR_INVALID_ARGUMENT, "kv_batch_stride does not fit the kernel ABI's int");
-    return launch_rt(kv_cache_append_kernel, dim3(batch, num_kv_heads, 1), dim3(head_dim), 0,
+    // programmatic, but the kernel releases its dependents only after its own wait (see the kernel)
+    return launch_rt(vteb_kv_cache_append_ordered_kernel, dim3(batch, num_kv_heads, 1), dim3(head_dim), 0,
                      (cudaStream_t)stream, true, (const __half*)k, (const __half*)v, (__half*)k_cache,
                      (__half*)v_cache, num_kv_heads, head_dim, kv_offsets, (int)kv_batch_stride);
 }

@@ -63,6 +63,35 @@ def test_wide_groups_match_the_oracle(cuda_runtime, codegen, heads, batch):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("heads", [(32, 2, 128), (36, 4, 64), (24, 2, 256)], ids=str)
+def test_wide_keeps_weights_far_below_the_maximum(cuda_runtime, codegen, heads):
+    """Every sixteenth position carries all of the weight and values of zero, the others lie 30 octaves under it and
+    make up the whole output.  Bound, relative: a probability of 2^-30 is held to 2^-43, so within 2^-14, and scores of
+    30 octaves in fp32 cost 2e-6; four times that."""
+    from vte_b200.core.decode_executor import DecodeAttentionExecutor
+    Hq, Hkv, D = heads
+    rng = np.random.default_rng([Hq, D, 30])
+    meta = {"attention.head_count": Hq, "attention.head_count_kv": Hkv, "attention.key_length": D}
+    for capacity, lens in ((64, [61]), (928, [900, 100, 17])):
+        B = len(lens)
+        q = np.ones((B, Hq, D), np.float16)
+        k = np.zeros((B, capacity, Hkv, D), np.float16)
+        k[:, ::16] = np.float16(30 * np.log(2) / np.sqrt(D))
+        v = (rng.random((B, capacity, Hkv, D), dtype=np.float32) + 0.5).astype(np.float16)
+        v[:, ::16] = 0
+        off = np.array(lens, dtype=np.int32) - 1
+        ex = DecodeAttentionExecutor(cuda_runtime, codegen, meta, B, capacity, 1)
+        try:
+            assert ex.dispatcher.wide
+            ex.upload_layer(0, q, k, v)
+            out = ex.execute_decode_batch(off)[0]
+        finally:
+            ex.cleanup()
+        ref = orc.decode_attention(q, k, v, off, dtype=np.float64)
+        assert np.max(np.abs(out / ref - 1)) <= 2.5e-4
+
+
+@pytest.mark.gpu
 def test_wide_only_where_the_split_layout_is_open(cuda_runtime, codegen):
     from vte_b200.bridge import CudaSafetyError
     from vte_b200.core.split_kv_attention import SplitKVAttentionDispatcher

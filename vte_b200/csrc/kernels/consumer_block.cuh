@@ -28,6 +28,14 @@ namespace vteb {
 // maximum, the reference maximum's slot (D + 4) otherwise.
 constexpr int kMergeTrueMax = (VTEB_LAZY_MAX > 0) ? 6 : 4;
 
+// P as two fp16 parts in the builds that sum a block on its own (kFresh): the high part of 2^7 P, so that it fills
+// fp16's range, and the low part another 2^11 up; both are scaled back in fp32.  A probability then has 22 bits down to
+// 2^-21 of the reference and is lost only from 2^-43 on, which not even a million such positions lift over fp32's
+// rounding of the sum; with both parts around 1 it was lost from 2^-25 on, though its weight counted in l.
+// (Moving the reference by 7 instead of scaling rounds the exponents: 2.4e-7 where this has 1.9e-7.)
+constexpr float kFreshUp = 128.f, kFreshDown = 1.f / 128.f, kFreshLoUp = 2048.f, kFreshLoDown = 1.f / 2048.f;
+static_assert(VTEB_LAZY_MAX <= 8, "2^7 P has to stay within fp16's range");
+
 // Scores of one block: sn[0] positions 0..7, sn[1] positions 8..15 (raw dot products, unscaled),
 // thread (g = lane / 4, t = lane % 4) holds query row g, positions 2t, 2t+1 of each half.
 // QKC independent accumulation chains per position half: on this part a dependent mma.sync waits
@@ -183,10 +191,12 @@ __device__ __forceinline__ void softmax_pv(ConsumerState<NT, LOACC>& st, const f
     uint32_t ph[2], pl[2];
 #pragma unroll
     for (int n = 0; n < 2; ++n) {
+        if constexpr (kFresh) { p[n][0] *= kFreshUp; p[n][1] *= kFreshUp; }
         const __half2 hi = __floats2half2_rn(p[n][0], p[n][1]);
         const float2 hif = __half22float2(hi);
         ph[n] = *reinterpret_cast<const uint32_t*>(&hi);
-        pl[n] = pack_half2(p[n][0] - hif.x, p[n][1] - hif.y);
+        constexpr float up = kFresh ? kFreshLoUp : 1.f;
+        pl[n] = pack_half2((p[n][0] - hif.x) * up, (p[n][1] - hif.y) * up);
     }
     // O += P V, 64 columns per chunk; the next chunk's fragments load meanwhile
 #pragma unroll
@@ -209,7 +219,10 @@ __device__ __forceinline__ void softmax_pv(ConsumerState<NT, LOACC>& st, const f
                 float d0 = 0.f, d1 = 0.f, g0 = 0.f, g1 = 0.f, e0, e1, f0, f1;
                 mma_hi_lo(d0, d1, e0, e1, ph[0], pl[0], ph[1], pl[1], vf[ch & 1][i][0], vf[ch & 1][i][1]);
                 mma_hi_lo(g0, g1, f0, f1, ph[0], pl[0], ph[1], pl[1], vf[ch & 1][i][2], vf[ch & 1][i][3]);
-                st.o[n][0] += d0 + e0; st.o[n][1] += d1 + e1; st.o[n + 1][0] += g0 + f0; st.o[n + 1][1] += g1 + f1;
+                st.o[n][0] = fmaf(fmaf(e0, kFreshLoDown, d0), kFreshDown, st.o[n][0]);
+                st.o[n][1] = fmaf(fmaf(e1, kFreshLoDown, d1), kFreshDown, st.o[n][1]);
+                st.o[n + 1][0] = fmaf(fmaf(f0, kFreshLoDown, g0), kFreshDown, st.o[n + 1][0]);
+                st.o[n + 1][1] = fmaf(fmaf(f1, kFreshLoDown, g1), kFreshDown, st.o[n + 1][1]);
             } else {
                 float e0, e1, f0, f1;
                 mma_hi_lo(st.o[n][0], st.o[n][1], e0, e1, ph[0], pl[0], ph[1], pl[1], vf[ch & 1][i][0], vf[ch & 1][i][1]);
@@ -351,10 +364,12 @@ __device__ __forceinline__ void softmax_pv_t(ConsumerStateT<MT>& st, const float
     uint32_t bh[2], bl[2];
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
+        if constexpr (kFresh) { p[2 * r] *= kFreshUp; p[2 * r + 1] *= kFreshUp; }
         const __half2 hi = __floats2half2_rn(p[2 * r], p[2 * r + 1]);
         const float2 hif = __half22float2(hi);
         bh[r] = movmatrix_trans(*reinterpret_cast<const uint32_t*>(&hi));
-        bl[r] = movmatrix_trans(pack_half2(p[2 * r] - hif.x, p[2 * r + 1] - hif.y));
+        constexpr float up = kFresh ? kFreshLoUp : 1.f;
+        bl[r] = movmatrix_trans(pack_half2((p[2 * r] - hif.x) * up, (p[2 * r + 1] - hif.y) * up));
     }
 #pragma unroll
     for (int ch = 0; ch < NVC; ++ch) {
@@ -366,19 +381,14 @@ __device__ __forceinline__ void softmax_pv_t(ConsumerStateT<MT>& st, const float
         }
         // vf: (positions 0-7, columns 0-7)^T, (8-15, 0-7)^T, (0-7, 8-15)^T, (8-15, 8-15)^T
         if constexpr (kFresh) {
-            float d[VC][4];
 #pragma unroll
             for (int i = 0; i < VC; ++i) {
-                d[i][0] = d[i][1] = d[i][2] = d[i][3] = 0.f;
-                mma_full(d[i], vf[ch & 1][i][0], vf[ch & 1][i][2], vf[ch & 1][i][1], vf[ch & 1][i][3], bl[0], bl[1]);
+                float hi[4] = {0.f, 0.f, 0.f, 0.f}, lo[4] = {0.f, 0.f, 0.f, 0.f};
+                mma_full(hi, vf[ch & 1][i][0], vf[ch & 1][i][2], vf[ch & 1][i][1], vf[ch & 1][i][3], bh[0], bh[1]);
+                mma_full(lo, vf[ch & 1][i][0], vf[ch & 1][i][2], vf[ch & 1][i][1], vf[ch & 1][i][3], bl[0], bl[1]);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) st.o[ch * VC + i][j] = fmaf(fmaf(lo[j], kFreshLoDown, hi[j]), kFreshDown, st.o[ch * VC + i][j]);
             }
-#pragma unroll
-            for (int i = 0; i < VC; ++i)
-                mma_full(d[i], vf[ch & 1][i][0], vf[ch & 1][i][2], vf[ch & 1][i][1], vf[ch & 1][i][3], bh[0], bh[1]);
-#pragma unroll
-            for (int i = 0; i < VC; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) st.o[ch * VC + i][j] += d[i][j];
         } else {
 #pragma unroll
             for (int i = 0; i < VC; ++i)

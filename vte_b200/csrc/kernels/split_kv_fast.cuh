@@ -39,10 +39,11 @@
 // 4,096 positions, 32 heads on 2 KV heads of 128, append included: 20 us a layer against 41 us with the
 // reference-geometry kernels, which read K and V once per query head; the bytes alone need 3 us, the rest is
 // launches, the Q fetch, the merge and the combine.
-// These groups had fp32 products before, so the wide build rounds every sum in fp32 registers (products of one
-// k-step and of one block start from zero): relative error against 64 bits 1.7e-7 to 2.0e-7 (4.3e-7 with scores
-// four times as wide) where the reference-geometry kernels have 1.9e-7 to 2.4e-7 (4.2e-7), and the same time
-// as with chained accumulation (2.3e-7 to 3.5e-7).
+// The reference-geometry kernels have fp32 products, so the wide build rounds every sum in fp32 registers (products of
+// one k-step and of one block start from zero) and scales the two parts of P (kFreshUp, consumer_block.cuh): relative
+// error against 64 bits over six geometries of up to 4,096 positions 1.8e-7 to 2.1e-7 where those have 1.9e-7 to
+// 2.3e-7 (3.3e-7 to 5.5e-7 and 3.3e-7 to 4.8e-7 with scores four times as wide); eight sequences, 8 layers: 163 us,
+// 161 with unscaled parts, whose error was 1.9e-7 to 2.2e-7.
 //
 // Under programmatic dependent launch everything that does not depend on the previous launch runs
 // before griddepcontrol.wait: barrier set-up, the first item's geometry (kv offsets, sequence order),

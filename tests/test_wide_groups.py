@@ -92,6 +92,42 @@ def test_wide_keeps_weights_far_below_the_maximum(cuda_runtime, codegen, heads):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("heads", [(32, 2, 128), (36, 4, 64), (64, 1, 64), (24, 2, 256)], ids=str)
+def test_wide_keeps_infinite_values(cuda_runtime, codegen, heads):
+    """Every weight is positive, so an infinite value gives an infinite output in its channel, whatever sign the low
+    part of the weight has, and leaves the others finite; both signs give NaN.  The newest row also fills the masked
+    rows of the last tile."""
+    from vte_b200.core.decode_executor import DecodeAttentionExecutor
+    Hq, Hkv, D = heads
+    rng = np.random.default_rng([Hq, D, 7])
+    meta = {"attention.head_count": Hq, "attention.head_count_kv": Hkv, "attention.key_length": D}
+    f16 = lambda *s: rng.standard_normal(s, dtype=np.float32).astype(np.float16)
+    for capacity, lens in ((64, [1]), (64, [61]), (928, [900, 1, 17, 112])):
+        B = len(lens)
+        q, k, v = f16(B, Hq, D), f16(B, capacity, Hkv, D), f16(B, capacity, Hkv, D)
+        for b, n in enumerate(lens):
+            v[b, n - 1, :, 3] = np.inf                      # the newest row
+            v[b, n // 2, :, D - 2] = -np.inf                # a row of its own
+            v[b, : n : 5, :, 9] = np.inf                    # many rows of a channel
+            v[b, 0, :, 40], v[b, n - 1, :, 40] = np.inf, (-np.inf if n > 1 else np.inf)
+        off = np.array(lens, dtype=np.int32) - 1
+        ex = DecodeAttentionExecutor(cuda_runtime, codegen, meta, B, capacity, 1)
+        try:
+            assert ex.dispatcher.wide
+            ex.upload_layer(0, q, k, v)
+            out = ex.execute_decode_batch(off)[0]
+        finally:
+            ex.cleanup()
+        several = np.array(lens) > 1
+        assert np.all(out[:, :, 3] == np.inf) and np.all(out[:, :, 9] == np.inf) and np.all(out[:, :, D - 2] == -np.inf)
+        assert np.all(np.isnan(out[several][:, :, 40])) and np.all(out[~several][:, :, 40] == np.inf)
+        rest = np.delete(np.arange(D), [3, 9, 40, D - 2])
+        v[~np.isfinite(v)] = 0
+        ref = orc.decode_attention(q, k, v, off)
+        assert np.max(np.abs(out[:, :, rest] - ref[:, :, rest])) <= 1e-5
+
+
+@pytest.mark.gpu
 def test_wide_only_where_the_split_layout_is_open(cuda_runtime, codegen):
     from vte_b200.bridge import CudaSafetyError
     from vte_b200.core.split_kv_attention import SplitKVAttentionDispatcher

@@ -400,6 +400,43 @@ __device__ __forceinline__ void softmax_pv_t(ConsumerStateT<MT>& st, const float
     }
 }
 
+// ---------------------------------------------------------------------------------------------
+// P V of a warp's part of an item once more, with fp32 probabilities and products, for builds that promise what fp32
+// kernels give (kFresh).  An infinite V times a zero part of P is NaN where its product with the whole of P is infinite:
+// in a masked row, as the low part of a probability that fp16 holds exactly, or where the two parts differ in sign.  A
+// warp whose sums hold a NaN at the end of an item walks its blocks again, straight from the caches, and rewrites o in
+// its exchange rows (`n_rows` rows of `pitch` floats: o[D], 4 unused, m, ...); m and l stand.  `q`: the rows' queries;
+// `k`, `v`: the KV head's row 0, rows `stride` halves apart; blocks from position `first` on, `step` apart, below `end`.
+// Checked once an item, eight sequences of sixteen heads per KV head, 8 layers: 163.4 -> 164.8 us; a check of every
+// block's products took 170.4.
+template <int D>
+__device__ __noinline__ void redo_rows_fp32(float* rows, int n_rows, int pitch, const __half* q, const __half* k, const __half* v,
+                                            long long stride, int first, int end, int step, float scale2) {
+    const int lane = threadIdx.x & 31;
+    __syncwarp();
+    for (int r = 0; r < n_rows; ++r) {
+        const float m = rows[r * pitch + D + 4];
+        float o[D / 32];
+#pragma unroll
+        for (int c = 0; c < D / 32; ++c) o[c] = 0.f;
+        for (int blk = first; blk < end; blk += step)
+            for (int j = blk; j < min(blk + 16, end); ++j) {
+                float x = 0.f;
+#pragma unroll
+                for (int c = 0; c < D / 32; ++c)
+                    x = fmaf(__half2float(q[r * D + c * 32 + lane]), __half2float(k[j * stride + c * 32 + lane]), x);
+#pragma unroll
+                for (int off = 16; off > 0; off >>= 1) x += __shfl_xor_sync(0xffffffffu, x, off);
+                const float p = fast_exp2(x * scale2 - m);
+#pragma unroll
+                for (int c = 0; c < D / 32; ++c) o[c] = fmaf(p, __half2float(v[j * stride + c * 32 + lane]), o[c]);
+            }
+#pragma unroll
+        for (int c = 0; c < D / 32; ++c) rows[r * pitch + c * 32 + lane] = o[c];
+    }
+    __syncwarp();
+}
+
 // Column-split variant of the transposed form: the warps of a KV head all compute the scores of every
 // block of the item (the same S^T, the same maximum and sum) and each accumulates only its own run of
 // 16-column output tiles [mt0, mt0 + nmt), nmt <= NMT.  No warp holds a partial sum over positions, so

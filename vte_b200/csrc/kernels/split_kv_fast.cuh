@@ -43,7 +43,8 @@
 // one k-step and of one block start from zero) and scales the two parts of P (kFreshUp, consumer_block.cuh): relative
 // error against 64 bits over six geometries of up to 4,096 positions 1.8e-7 to 2.1e-7 where those have 1.9e-7 to
 // 2.3e-7 (3.3e-7 to 5.5e-7 and 3.3e-7 to 4.8e-7 with scores four times as wide); eight sequences, 8 layers: 163 us,
-// 161 with unscaled parts, whose error was 1.9e-7 to 2.2e-7.
+// 161 with unscaled parts, whose error was 1.9e-7 to 2.2e-7.  An infinite V gives what fp32 products give
+// (redo_rows_fp32).
 //
 // Under programmatic dependent launch everything that does not depend on the previous launch runs
 // before griddepcontrol.wait: barrier set-up, the first item's geometry (kv offsets, sequence order),
@@ -878,6 +879,10 @@ __device__ __forceinline__ void fast_partial_body(const FastArgs& a)
             st.fold_lo();
             VTEB_TR(tr, 5);
         }
+        int item_first = 0, item_end = 0;      // wide build, last tile: this warp's first position of the item, the item's end
+        if constexpr (kWide) {
+            if (flags & kTileLast) { item_first = hd->pos0 + (sub - blk0) * kBlockPos; item_end = hd->last_pos + 1; }
+        }
 
 #ifdef VTEB_TRACE
         if (trace_tile < 8) VTEB_TR(tr, 20 + trace_tile);
@@ -935,6 +940,16 @@ __device__ __forceinline__ void fast_partial_body(const FastArgs& a)
             }
             // ---- exchange (m, l, o) between the warps of each KV head and store the item
             const int pitch = D + kMergePad;           // floats per (warp, row): o[D], 4 unused, m, l, true maximum, 1 unused
+            auto redo_if_nan = [&](bool nan) {         // wide build, state in the warp's exchange rows
+                if (!__any_sync(0xffffffffu, nan)) return false;
+                const long long kv0 = (long long)item_b * a.kv_batch_stride + (long long)(item_hgroup * plan.hg + kv_hh) * D;
+                redo_rows_fp32<D>(merge + (size_t)warp * vgroup * pitch, vgroup, pitch,
+                                  a.q + ((long long)item_b * a.num_q_heads + (long long)(item_hgroup * vhg + hh) * vgroup) * D,
+                                  a.k_cache + kv0, a.v_cache + kv0, (long long)a.num_kv_heads * D, item_first, item_end,
+                                  plan.wph * kBlockPos, scale2);
+                return true;
+            };
+            bool nan = false;
             if (plan.wph == 1 && !kT) {
                 // One warp per KV head: nothing to merge, the warp stores its own state.
                 // (The transposed form goes through the exchange area here too: its registers hold
@@ -943,6 +958,20 @@ __device__ __forceinline__ void fast_partial_body(const FastArgs& a)
                 l_own += __shfl_xor_sync(0xffffffffu, l_own, 1);
                 l_own += __shfl_xor_sync(0xffffffffu, l_own, 2);
                 const bool empty1 = (flags & kTileEmpty) != 0;
+                if constexpr (kWide) {
+#pragma unroll
+                    for (int n = 0; n < NT; ++n) nan |= (st.o[n][0] != st.o[n][0]) | (st.o[n][1] != st.o[n][1]);
+                    float* const my_rows = merge + (size_t)warp * vgroup * pitch;
+                    if (t == 0 && g < vgroup) my_rows[g * pitch + D + 4] = st.m;
+                    if (redo_if_nan(nan) && g < vgroup) {
+#pragma unroll
+                        for (int n = 0; n < NT; ++n) {
+                            st.o[n][0] = my_rows[g * pitch + n * 8 + 2 * t];
+                            st.o[n][1] = my_rows[g * pitch + n * 8 + 2 * t + 1];
+                        }
+                    }
+                    __syncwarp();
+                }
 #if VTEB_LAZY_MAX > 0
                 {   // restate (m, l, o) against the row's true maximum, as the partial buffers promise
                     const float m_true = st.true_max();
@@ -1003,6 +1032,7 @@ __device__ __forceinline__ void fast_partial_body(const FastArgs& a)
                         for (int mt = 0; mt < D / 16; ++mt) {
                             dst[mt * 16 + g] = tt.o[mt][h];
                             dst[mt * 16 + g + 8] = tt.o[mt][2 + h];
+                            if constexpr (kWide) nan |= (tt.o[mt][h] != tt.o[mt][h]) | (tt.o[mt][2 + h] != tt.o[mt][2 + h]);
                         }
                         if (g == 0) { dst[D + 4] = tt.m[h]; dst[D + 5] = l_head; dst[D + kMergeTrueMax] = m_head; }
                     }
@@ -1015,11 +1045,14 @@ __device__ __forceinline__ void fast_partial_body(const FastArgs& a)
                 if (g < vgroup) {
                     float* dst = merge + ((size_t)warp * vgroup + g) * pitch;
 #pragma unroll
-                    for (int n = 0; n < NT; ++n)
+                    for (int n = 0; n < NT; ++n) {
                         *reinterpret_cast<float2*>(dst + dhalf * DW + n * 8 + 2 * t) = make_float2(st.o[n][0], st.o[n][1]);
+                        if constexpr (kWide) nan |= (st.o[n][0] != st.o[n][0]) | (st.o[n][1] != st.o[n][1]);
+                    }
                     if (t == 0) { dst[D + 4] = st.m; dst[D + 5] = l_quad; dst[D + kMergeTrueMax] = m_true; }
                 }
             }
+            if constexpr (kWide) redo_if_nan(nan);
             __syncwarp();
             if (lane == 0) mbar_arrive(merge_bar0);
             if (!mbar_wait_bounded(merge_bar0, merge_parity & 1u, abort_word)) {

@@ -128,6 +128,37 @@ def test_wide_keeps_infinite_values(cuda_runtime, codegen, heads):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("f32", [True, False], ids=["fp32", "fp16"])
+@pytest.mark.parametrize("heads", [(32, 2, 128), (36, 4, 64), (64, 1, 64), (24, 2, 256)], ids=str)
+def test_wide_stores_to_an_output_of_any_alignment(cuda_runtime, codegen, heads, f32):
+    """An output that starts one element behind an aligned address, unsplit and combined: the same bits as aligned."""
+    from vte_b200.core.decode_executor import DecodeAttentionExecutor
+    Hq, Hkv, D = heads
+    rng = np.random.default_rng([Hq, D, 4])
+    meta = {"attention.head_count": Hq, "attention.head_count_kv": Hkv, "attention.key_length": D}
+    f16 = lambda *s: rng.standard_normal(s, dtype=np.float32).astype(np.float16)
+    for capacity, lens in ((64, [61, 3]), (928, [900, 17])):
+        q, k, v = f16(2, Hq, D), f16(2, capacity, Hkv, D), f16(2, capacity, Hkv, D)
+        off = np.array(lens, dtype=np.int32) - 1
+        outs = []
+        for skip in (0, 4 if f32 else 2):
+            ex = DecodeAttentionExecutor(cuda_runtime, codegen, meta, 2, capacity, 1, output_f32=f32)
+            try:
+                assert ex.dispatcher.wide
+                ex.tensor_mapping["blk.0.attention.output"] += skip
+                ex.upload_layer(0, q, k, v)
+                ex.execute_decode_batch(off, read_output=False)
+                cuda_runtime.synchronize()
+                raw = np.zeros(ex.out_bytes, dtype=np.uint8)
+                cuda_runtime.safe_memcpy_device_to_host(raw, ctypes.c_void_p(ex.out_all.ptr + skip), "attention output")
+                outs.append(raw.view(np.float32 if f32 else np.float16).reshape(2, Hq, D))
+            finally:
+                ex.cleanup()
+        assert np.array_equal(outs[0], outs[1])
+        assert np.max(np.abs(outs[0] - orc.decode_attention(q, k, v, off))) <= (1e-5 if f32 else 2e-3)
+
+
+@pytest.mark.gpu
 def test_wide_only_where_the_split_layout_is_open(cuda_runtime, codegen):
     from vte_b200.bridge import CudaSafetyError
     from vte_b200.core.split_kv_attention import SplitKVAttentionDispatcher

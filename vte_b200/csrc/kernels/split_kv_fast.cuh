@@ -122,9 +122,18 @@ __device__ __forceinline__ unsigned long long trace_globaltimer() {
 #define VTEB_TR_GT(ctx, slot) do { } while (0)
 #endif
 
-// Stores four (or two) normalised output values; out_kind 1 = fp16, 2 = fp32.
+// Stores four (or two) normalised output values; out_kind 1 = fp16, 2 = fp32.  kAnyAlign: the output need only be aligned
+// to its own element, as for the reference-geometry kernels; otherwise to 16 (8, 4) bytes.
+template <bool kAnyAlign = false>
 __device__ __forceinline__ void store_out4(void* output, int out_kind, long long idx, float4 v) {
-    if (out_kind == 2) {
+    if (kAnyAlign && (reinterpret_cast<uintptr_t>(output) & 15)) {
+        const float x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if (out_kind == 2) reinterpret_cast<float*>(output)[idx + i] = x[i];
+            else reinterpret_cast<__half*>(output)[idx + i] = __float2half(x[i]);
+        }
+    } else if (out_kind == 2) {
         *reinterpret_cast<float4*>(reinterpret_cast<float*>(output) + idx) = v;
     } else {
         __half2* o = reinterpret_cast<__half2*>(reinterpret_cast<__half*>(output) + idx);
@@ -132,8 +141,16 @@ __device__ __forceinline__ void store_out4(void* output, int out_kind, long long
         o[1] = __floats2half2_rn(v.z, v.w);
     }
 }
+template <bool kAnyAlign = false>
 __device__ __forceinline__ void store_out2(void* output, int out_kind, long long idx, float2 v) {
-    if (out_kind == 2) *reinterpret_cast<float2*>(reinterpret_cast<float*>(output) + idx) = v;
+    if (kAnyAlign && (reinterpret_cast<uintptr_t>(output) & 7)) {
+        const float x[2] = {v.x, v.y};
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            if (out_kind == 2) reinterpret_cast<float*>(output)[idx + i] = x[i];
+            else reinterpret_cast<__half*>(output)[idx + i] = __float2half(x[i]);
+        }
+    } else if (out_kind == 2) *reinterpret_cast<float2*>(reinterpret_cast<float*>(output) + idx) = v;
     else *reinterpret_cast<__half2*>(reinterpret_cast<__half*>(output) + idx) = __floats2half2_rn(v.x, v.y);
 }
 
@@ -989,8 +1006,8 @@ __device__ __forceinline__ void fast_partial_body(const FastArgs& a)
                     const float inv = 1.f / fmaxf(l_own, 1e-20f);
 #pragma unroll
                     for (int n = 0; n < NT; ++n)
-                        store_out2(a.output, a.out_kind, row * D + dhalf * DW + n * 8 + 2 * t,
-                                   make_float2(st.o[n][0] * inv, st.o[n][1] * inv));
+                        store_out2<kWide>(a.output, a.out_kind, row * D + dhalf * DW + n * 8 + 2 * t,
+                                          make_float2(st.o[n][0] * inv, st.o[n][1] * inv));
                 } else if (g < vgroup) {
                     const long long stat = ((long long)item_b * a.num_q_heads + (long long)item_hgroup * vhg * vgroup +
                                             (long long)hh * vgroup + g) * a.max_chunks + item_c;
@@ -1117,8 +1134,8 @@ __device__ __forceinline__ void fast_partial_body(const FastArgs& a)
                     const float inv = 1.f / fmaxf(ll, 1e-20f);
 #pragma unroll
                     for (int i = 0; i < NV; ++i)
-                        store_out4(a.output, a.out_kind, orow * D + col0 + 4 * i,
-                                   make_float4(acc[i].x * inv, acc[i].y * inv, acc[i].z * inv, acc[i].w * inv));
+                        store_out4<kWide>(a.output, a.out_kind, orow * D + col0 + 4 * i,
+                                          make_float4(acc[i].x * inv, acc[i].y * inv, acc[i].z * inv, acc[i].w * inv));
                     continue;
                 }
                 const long long stat = stat0 + (long long)hq * a.max_chunks;
@@ -1182,8 +1199,8 @@ __device__ __forceinline__ void fast_partial_body(const FastArgs& a)
                     if (col_ok) {
 #pragma unroll
                         for (int i = 0; i < NV; ++i)
-                            store_out4(a.output, a.out_kind, row * D + i * 128 + lane * 4,
-                                       make_float4(acc[i].x * inv, acc[i].y * inv, acc[i].z * inv, acc[i].w * inv));
+                            store_out4<kWide>(a.output, a.out_kind, row * D + i * 128 + lane * 4,
+                                              make_float4(acc[i].x * inv, acc[i].y * inv, acc[i].z * inv, acc[i].w * inv));
                     }
                     continue;
                 }

@@ -94,6 +94,10 @@ class FakeRuntime:
         plan = FastPlan()
         (self._lib.vteb_split_kv_plan_compact if compact else self._lib.vteb_split_kv_plan)(hq, hkv, d, ctypes.byref(plan))
         return plan
+    def split_kv_plan_wide(self, hq, hkv, d):
+        plan = FastPlan()
+        self._lib.vteb_split_kv_plan_wide(hq, hkv, d, ctypes.byref(plan))
+        return plan
     def safe_malloc(self, n, tag="x"):
         p = self._next
         self._next += (n + 255) // 256 * 256
@@ -331,6 +335,26 @@ def test_compat_launch_list_is_the_reference_geometry():
     assert all(kw == {'split_kv_chunk_size': 8} for _, _, _, kw in cg.calls)
     assert [s for _, s in rt.loaded] == ["kv_cache_append_kernel", "flash_attention_split_kv_partial_kernel",
                                          "flash_attention_split_kv_reduce_kernel"]
+
+
+def test_wide_launch_list_waits_first_unless_the_caller_vouches_for_the_offsets():
+    """More than eight query heads per KV head: the split kernel's wide build, with scratch within its limit; bit 5 of
+    the flags keeps it from reading anything ahead of its dependency wait."""
+    from vte_b200.core.split_kv_attention import FLAG_BALANCED, FLAG_WAIT_FIRST, WIDE_SCRATCH_BYTES
+    meta = {'attention.head_count': 32, 'attention.head_count_kv': 2, 'attention.key_length': 128}
+    d, rt, cg, _ = make_dispatcher(meta, context_length=4096, batch_size=8)
+    assert d.wide and d.compat and d.balanced and d.max_chunks * 8 * 32 * 130 * 4 <= WIDE_SCRATCH_BYTES
+    m = mapping(stride=4096 * 2 * 128)
+    append, split, combine = d.build_launches(0, m, 0x7200_0000_0000, batch=8)
+    assert len(split[1]) == len(KERNEL_SIGNATURES["vteb_split_kv_partial_wide_d128_kernel"])
+    assert split[1][15].value & FLAG_WAIT_FIRST and split[1][15].value & FLAG_BALANCED and split[2] == (148, 1, 1)
+    assert [s for _, s in rt.loaded] == ["kv_cache_append_kernel", "vteb_split_kv_partial_wide_d128_kernel",
+                                         "vteb_split_kv_combine_rows_kernel"]
+    d.offsets_final = True
+    assert not d.build_launches(0, m, 0x7200_0000_0000, batch=8)[1][1][15].value & FLAG_WAIT_FIRST
+    # groups of at most eight heads ask their caller for final offsets in any case
+    d, *_ = make_dispatcher(context_length=4096, batch_size=8)
+    assert not d.wide and not d.build_launches(0, mapping(stride=4096 * 2 * 128), 0x7200_0000_0000, batch=8)[1][1][15].value & FLAG_WAIT_FIRST
 
 
 def test_dispatcher_switches_and_fallbacks(monkeypatch):

@@ -159,6 +159,66 @@ def test_wide_stores_to_an_output_of_any_alignment(cuda_runtime, codegen, heads,
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("batch", [1, 5])
+def test_wide_reads_offsets_behind_the_launch_in_front(cuda_runtime, codegen, batch):
+    """A dispatcher's launches under programmatic launch, three appends and an attention per step, with a launch in
+    front of each append that writes the offsets: right for the reference-geometry kernels, so right for `wide`."""
+    from vte_b200.core.split_kv_attention import SplitKVAttentionDispatcher
+    from vte_b200.bridge.memory import SlabAllocator
+    rt, (Hq, Hkv, D), S, steps = cuda_runtime, (32, 2, 128), 288, 16
+    rng = np.random.default_rng(batch)
+    f16 = lambda *s: rng.standard_normal(s, dtype=np.float32).astype(np.float16)
+    k, v = f16(batch, S, Hkv, D), f16(batch, S, Hkv, D)
+    q, kn, vn = f16(steps, batch, Hq, D), f16(3 * steps, batch, Hkv, D), f16(3 * steps, batch, Hkv, D)
+    offs = np.zeros((3 * steps, 8), dtype=np.int32)
+    offs[:, :batch] = np.arange(3 * steps)[:, None] + np.array([40, 1, 200, 61, 15][:batch])
+    alloc = SlabAllocator(rt, rt.get_real_mem_info()[1], requested_pool_size=64 << 20)
+    alloc.initialize()
+    bufs = []
+
+    def dev(arr):
+        bufs.append(rt.safe_malloc(arr.nbytes, "wide order output"))
+        rt.safe_memcpy_host_to_device(bufs[-1], arr, "wide order output")
+        return bufs[-1].value
+    try:
+        d = SplitKVAttentionDispatcher(rt, codegen, {"attention.head_count": Hq, "attention.head_count_kv": Hkv,
+                                                     "attention.key_length": D}, allocator=alloc, context_length=S,
+                                       batch_size=batch, output_f32=True)
+        assert d.wide
+        dk, dv, dq, dkn, dvn, doffs = (dev(x) for x in (k, v, q, kn, vn, offs))
+        cur, dout = dev(np.zeros(8, np.int32)), dev(np.zeros((steps, batch, Hq, D), np.float32))
+        copy = codegen.load_kernel_safe(rt, "decode_attention", rt.get_gpu_architecture(), "vteb_stage_copy_kernel")[1]
+        vp, ci, row = ctypes.c_void_p, ctypes.c_int, batch * Hkv * D * 2
+        d._get_kernels()
+        rt.synchronize()
+        for step in range(steps):
+            for a in range(3 * step, 3 * step + 3):
+                rt.launch_kernel(copy, (1, 1, 1), (32, 1, 1), [vp(doffs + a * 32), vp(cur), ci(2)])
+                rt.programmatic_launch = True
+                launches = d.build_launches(0, {
+                    "blk.0.q_proj.output": dq + step * batch * Hq * D * 2, "blk.0.k_proj.output": dkn + a * row,
+                    "blk.0.v_proj.output": dvn + a * row, "blk.0.kv_cache.k": dk, "blk.0.kv_cache.v": dv,
+                    "blk.0.attention.output": dout + step * batch * Hq * D * 4,
+                    "kv_batch_stride_elements": S * Hkv * D}, cur, batch=batch)
+                for fn, args, grid, block, smem in launches[:1] if a % 3 < 2 else launches:
+                    rt.launch_kernel_recorded(fn, args, grid, block, smem)
+                rt.programmatic_launch = False
+        rt.check_status(d.work_ptr)
+        out = np.zeros((steps, batch, Hq, D), np.float32)
+        rt.safe_memcpy_device_to_host(out, ctypes.c_void_p(dout), "wide order output")
+    finally:
+        rt.programmatic_launch = False
+        for p in bufs:
+            rt.safe_free(p, "wide order cleanup")
+        alloc.cleanup()
+    for step in range(steps):
+        for a in range(3 * step, 3 * step + 3):
+            orc.kv_cache_append(kn[a], vn[a], k, v, offs[a, :batch])
+        ref = orc.decode_attention(q[step], k, v, offs[3 * step + 2, :batch])
+        assert np.max(np.abs(out[step] - ref)) <= 1e-5, step
+
+
+@pytest.mark.gpu
 def test_wide_only_where_the_split_layout_is_open(cuda_runtime, codegen):
     from vte_b200.bridge import CudaSafetyError
     from vte_b200.core.split_kv_attention import SplitKVAttentionDispatcher

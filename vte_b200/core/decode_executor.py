@@ -208,6 +208,8 @@ class DecodeAttentionExecutor:
     def _record_all(self, after_copy: bool = False):
         n = 0
         programmatic = self.hip.programmatic_launch
+        # within a captured step of nothing but the layers' own launches, offsets and older rows do not change
+        self.dispatcher.offsets_final = self.use_graph and self.per_layer_hook is None and self.launch_rewriter is None
         for l in range(self.L):
             launches = self.dispatcher.build_launches(l, self.tensor_mapping, self.offsets.ptr, batch=self.B)
             if not self.with_append and not self.dispatcher.fuse_append:

@@ -35,6 +35,7 @@ FLAG_DIRECT_OUTPUT = 2
 FLAG_TENSOR_MAPS = 4
 FLAG_PREFETCH_Q = 8
 FLAG_BALANCED = 16
+FLAG_WAIT_FIRST = 32
 WIDE_SCRATCH_BYTES = 32 << 20    # partial buffers a group of more than eight heads may take where it took less before; executors reserve 64 MB
 COMPACT_MAX_CONTEXT = 262144      # one sequence up to this long: the compact CTA shape (launches of tens of microseconds)
 SHORT_CONTEXT_MAX = 2048          # one sequence up to this many positions: at most 32 splits (see choose_split_count)
@@ -292,6 +293,11 @@ class SplitKVAttentionDispatcher:
         # results; by default they come from the allocator with the other scratch
         self._external_work_ptr = int(work_ptr) if work_ptr else None
 
+        # offsets_final: whoever launches sees to it that kv offsets and older cache rows are final before the launch
+        # in front of the split kernel starts.  Groups of at most eight heads ask for that in any case; the wide build
+        # waits for the launch in front first unless this is set, as the reference-geometry kernels do.
+        self.offsets_final = False
+
         self._kernel_cache = {}
         self._rows_combine = False
         self._small_combine = False
@@ -523,6 +529,8 @@ class SplitKVAttentionDispatcher:
         flags = FLAG_WRITE_EMPTY_O if self.strict_empty_splits else 0
         if self.balanced:
             flags |= FLAG_BALANCED
+        if self.wide and not self.offsets_final:
+            flags |= FLAG_WAIT_FIRST
         # Under programmatic dependent launch the split CTAs start while the launch before them still runs:
         # the loader asks L2 for the Q rows (a hint only, no data reaches the SM) so that the consumers'
         # fetch after the dependency wait does not go to DRAM.  With plain stream order the wait returns at

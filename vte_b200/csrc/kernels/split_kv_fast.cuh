@@ -101,6 +101,7 @@ constexpr int kFlagWriteEmptyO = 1;   // also zero partial_o of empty splits (re
 constexpr int kFlagDirectOutput = 2;  // max_chunks == 1: normalise and store the attention output here, no partials
 constexpr int kFlagTensorMaps = 4;    // tmap_k / tmap_v are valid: whole tiles are fetched with tensor-map copies
 constexpr int kFlagBalanced = 16;     // several sequences: every CTA takes an equal share of all cached positions (see BalancedShare), no work queue
+constexpr int kFlagWaitFirst = 32;    // wide build: touch nothing ahead of the dependency wait, so that the launch in front may write offsets and older rows
 constexpr int kFlagPrefetchQ = 8;     // ask L2 for an item's Q rows ahead of their use (the first item's before the dependency wait); a hint, no data is read
 
 // ---- optional timeline trace (compiled in with -DVTEB_TRACE=1, used by vte_b200/trace_timeline.py) ----
@@ -416,6 +417,11 @@ __device__ __forceinline__ void fast_partial_body(const FastArgs& a)
     const uint32_t merge_bar0 = bar0 + kBarMerge;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nstages = plan.nstages;
+
+    if constexpr (kWide) {
+        // The reference-geometry kernels, which serve these groups elsewhere, read nothing ahead of their wait.
+        if (a.flags & kFlagWaitFirst) grid_dependency_wait();
+    }
 
     // The first item's geometry needs one global load (the sequence's kv offset): start it
     // before the barrier set-up so its latency is hidden.

@@ -502,6 +502,39 @@ def test_every_kernel_of_the_signature_table_is_in_the_cubin():
     assert in_cubin == set(KERNEL_SIGNATURES), in_cubin ^ set(KERNEL_SIGNATURES)
 
 
+def test_a_cubin_is_loaded_once_and_again_when_it_changes(tmp_path, built_library):
+    class FakeLib:
+        def __init__(self): self.loads, self.unloads, self.failing = [], [], False
+        def vteb_module_load(self, out, path):
+            self.loads.append(path)
+            out._obj.value = 0x100 + len(self.loads)
+            return 0
+        def vteb_module_get_function(self, out, module, name):
+            out._obj.value = module.value * 0x1000 + len(name)
+            return 500 if self.failing else 0
+        def vteb_func_set_shared_carveout(self, fn, percent): return 0
+        def vteb_module_unload(self, module): self.unloads.append(module.value)
+        def vteb_last_error_string(self): return b"fake"
+        def vteb_device_synchronize(self): return 0
+    rt = CudaRuntime(str(built_library))
+    rt._lib, rt._initialized = FakeLib(), True
+    a, b = tmp_path / "a.cubin", tmp_path / "b.cubin"
+    a.write_bytes(b"one"), b.write_bytes(b"one")
+    m1, f1 = rt.load_kernel(str(a), "kv_cache_append_kernel")
+    m2, f2 = rt.load_kernel(str(a), "rope_kernel")
+    assert m1.value == m2.value and f1.value != f2.value and len(rt._lib.loads) == 1
+    assert rt.load_kernel(str(b), "rope_kernel")[0].value != m1.value
+    rt._lib.failing = True
+    with pytest.raises(CudaRuntimeError):
+        rt.load_kernel(str(a), "rope_kernel")
+    rt._lib.failing = False
+    a.write_bytes(b"recompiled")                                  # what load_kernel_safe does after a failure
+    assert rt.load_kernel(str(a), "rope_kernel")[0].value not in (m1.value, m2.value)
+    assert len(rt._lib.loads) == 3
+    rt.cleanup()
+    assert sorted(rt._lib.unloads) == [0x101, 0x102, 0x103] and not rt._modules
+
+
 def test_oom_error_is_a_safety_error():
     assert issubclass(MemoryGuardianOOMError, CudaSafetyError)
 

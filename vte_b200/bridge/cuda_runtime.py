@@ -191,7 +191,8 @@ class CudaRuntime:
         self._counted_as_live = False
         self._active_allocations: dict[int, tuple[int, str]] = {}
         self._host_allocations: dict[int, int] = {}
-        self._modules: list[int] = []
+        self._module_lock = threading.Lock()
+        self._modules: dict[tuple, int] = {}      # loaded cubin (path and what stat says of the file) -> module
         self._stream = ctypes.c_void_p()
         self._device_index = device_index
         self._vram_total = 0
@@ -456,11 +457,21 @@ class CudaRuntime:
 
     # ------------------------------------------------------------------ kernels
     def load_kernel(self, cubin_path: str, kernel_name: str):
-        """Load a cubin and return (module, function) as c_void_p."""
+        """Load a cubin and return (module, function) as c_void_p.  A file is loaded once: its other kernels are looked
+        up in the same module.  A file that has changed since is loaded anew."""
         self._require_init()
         module, function = ctypes.c_void_p(), ctypes.c_void_p()
-        self._check_error(self._lib.vteb_module_load(ctypes.byref(module), str(cubin_path).encode("utf-8")), "cuModuleLoad")
-        self._modules.append(module.value)
+        path = os.path.realpath(cubin_path)
+        try:
+            st = os.stat(path)
+            key = (path, st.st_ino, st.st_size, st.st_mtime_ns)
+        except OSError:
+            key = None                            # the load below says what is wrong with it
+        with self._module_lock:
+            module.value = self._modules.get(key) if key else None
+            if not module.value:
+                self._check_error(self._lib.vteb_module_load(ctypes.byref(module), str(cubin_path).encode("utf-8")), "cuModuleLoad")
+                self._modules[key or (path, module.value)] = module.value
         self._check_error(self._lib.vteb_module_get_function(ctypes.byref(function), module, kernel_name.encode("utf-8")),
                           "cuModuleGetFunction")
         from ..compiler.signatures import KERNEL_SIGNATURES
@@ -768,7 +779,7 @@ class CudaRuntime:
                 self.host_free(ctypes.c_void_p(val))
             except Exception as e:
                 logger.error("error freeing pinned 0x%016X: %s", val, e)
-        for m in self._modules:
+        for m in self._modules.values():
             self._lib.vteb_module_unload(ctypes.c_void_p(m))
         self._modules.clear()
         self._signatures.clear()

@@ -535,6 +535,30 @@ def test_a_cubin_is_loaded_once_and_again_when_it_changes(tmp_path, built_librar
     assert sorted(rt._lib.unloads) == [0x101, 0x102, 0x103] and not rt._modules
 
 
+def test_the_unsplit_kernel_has_a_build_for_every_number_of_blocks(built_library):
+    """The first build whose resident blocks cover the grid, else the last; a kernel without builds is itself."""
+    rt = CudaRuntime(str(built_library))
+    rt._props = {"multiprocessor_count": 148}
+    rt.get_num_cus = lambda: 148
+    few, mid, many, other = (ctypes.c_void_p(x) for x in (1, 2, 3, 4))
+    rt._by_blocks = {2: [(few, 208), (mid, 128), (many, 64)]}
+    for threads, n_few, n_mid in ((64, 592, 1184), (128, 296, 592), (256, 148, 296)):
+        for blocks, want in ((1, few), (n_few, few), (n_few + 1, mid), (n_mid, mid), (n_mid + 1, many), (10 * n_mid, many)):
+            assert rt._build_for(mid, (blocks, 1, 1), (threads, 1, 1)) is want
+    assert rt._build_for(other, (10 ** 6, 1, 1), (128, 1, 1)) is other
+
+
+def test_short_splits_take_the_short_build_of_the_reference_geometry():
+    from vte_b200.core.split_kv_attention import compat_short_splits
+    names = lambda **kw: (lambda d, rt, cg, a: (d.build_launches(0, mapping(), 0x7200_0000_0000), rt.loaded[1][1])[1])(
+        *make_dispatcher(compat=True, **kw))
+    assert names(context_length=500, num_splits=32) == "vteb_split_kv_partial_compat_short_kernel"
+    assert names(context_length=500, num_splits=8) == "flash_attention_split_kv_partial_kernel"       # 96 blocks
+    assert names(context_length=500, fixed_chunk_size=8) == "flash_attention_split_kv_partial_kernel"   # cut at compile time
+    assert not compat_short_splits(148, 1, 12, 128, 128 * 49, 49) and compat_short_splits(148, 1, 12, 128, 128 * 50, 50)
+    assert not compat_short_splits(148, 64, 64, 256, 129 * 64, 64)                                    # long splits
+
+
 def test_oom_error_is_a_safety_error():
     assert issubclass(MemoryGuardianOOMError, CudaSafetyError)
 

@@ -16,9 +16,16 @@ pytestmark = pytest.mark.gpu
 LENGTHS = [1, 2, 7, 8, 9, 15, 16, 17, 31, 32, 33, 63, 64, 65, 127, 128, 129, 255, 256, 257, 513, 700]
 
 
+NAMED = ("flash_attention_kernel", "flash_attention_split_kv_partial_kernel")
+SHORT = ("vteb_flash_attention_many_kernel", "vteb_split_kv_partial_compat_short_kernel")
+
+
 @pytest.mark.parametrize("skew", [0, 4], ids=["aligned", "8-byte"])
-@pytest.mark.parametrize("heads", [(12, 2, 128), (6, 2, 64), (16, 1, 128), (4, 2, 256)], ids=str)
-def test_unsplit_and_split_walks_at_turn_boundaries(cuda_runtime, codegen, heads, skew):
+@pytest.mark.parametrize("builds, heads", [(NAMED, h) for h in ((12, 2, 128), (6, 2, 64), (16, 1, 128), (4, 2, 256))] +
+                         [(NAMED, h) for h in ((30, 2, 64), (8, 2, 256))] +          # grids of the build between few and many
+                         [(SHORT, h) for h in ((12, 2, 128), (6, 2, 64), (4, 2, 256))],
+                         ids=lambda x: str(x) if isinstance(x[0], int) else "named" if x is NAMED else "short")
+def test_unsplit_and_split_walks_at_turn_boundaries(cuda_runtime, codegen, builds, heads, skew):
     rt = cuda_runtime
     Hq, Hkv, D = heads
     B, S, C = len(LENGTHS), 700, 3
@@ -47,7 +54,7 @@ def test_unsplit_and_split_walks_at_turn_boundaries(cuda_runtime, codegen, heads
         dout = dev(np.zeros((B, Hq, D), np.float16))
         vp, ci, cf = ctypes.c_void_p, ctypes.c_int, ctypes.c_float
         stride, scale = S * Hkv * D, 1.0 / np.sqrt(D)
-        _, unsplit = codegen.load_kernel_safe(rt, 'flash_attention', arch, 'flash_attention_kernel')
+        _, unsplit = codegen.load_kernel_safe(rt, 'flash_attention', arch, builds[0])
         rt.launch_kernel(unsplit, (B, Hq, 1), (D, 1, 1),
                          [dq, dkn, dvn, dk, dv, dout, ci(1), ci(Hq), ci(Hkv), ci(D), cf(scale), doff, ci(stride)], 2 * D * 4)
         rt.synchronize()
@@ -57,8 +64,7 @@ def test_unsplit_and_split_walks_at_turn_boundaries(cuda_runtime, codegen, heads
         # the same caches, now with the new rows in them, cut into three splits
         dm, dl = dev(np.zeros((B, Hq, C), np.float32)), dev(np.zeros((B, Hq, C), np.float32))
         do = dev(np.zeros((B, Hq, C, D), np.float32))
-        _, partial = codegen.load_kernel_safe(rt, 'flash_attention_split_kv_partial', arch,
-                                              'flash_attention_split_kv_partial_kernel')
+        _, partial = codegen.load_kernel_safe(rt, 'flash_attention_split_kv_partial', arch, builds[1])
         rt.launch_kernel(partial, (B, Hq, C), (D, 1, 1),
                          [dq, dk, dv, dm, dl, do, ci(Hq), ci(Hkv), ci(D), cf(scale), doff, ci(stride), ci(C)], 2 * D * 4)
         rt.synchronize()

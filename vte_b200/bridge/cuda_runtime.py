@@ -199,6 +199,7 @@ class CudaRuntime:
         self._props: dict = {}
         self._smem_optin_set: dict[int, int] = {}
         self._signatures: dict[int, tuple[str, int]] = {}
+        self._by_blocks: dict[int, list] = {}     # function -> [(build, registers a thread)], see KERNEL_BY_BLOCKS
         self._panic = False
         self._sync_timeout_s = sync_timeout_s
         self.programmatic_launch = False   # when True, recorded launches carry the PDL attribute
@@ -460,7 +461,7 @@ class CudaRuntime:
         """Load a cubin and return (module, function) as c_void_p.  A file is loaded once: its other kernels are looked
         up in the same module.  A file that has changed since is loaded anew."""
         self._require_init()
-        module, function = ctypes.c_void_p(), ctypes.c_void_p()
+        module = ctypes.c_void_p()
         path = os.path.realpath(cubin_path)
         try:
             st = os.stat(path)
@@ -472,16 +473,40 @@ class CudaRuntime:
             if not module.value:
                 self._check_error(self._lib.vteb_module_load(ctypes.byref(module), str(cubin_path).encode("utf-8")), "cuModuleLoad")
                 self._modules[key or (path, module.value)] = module.value
+        from ..compiler.signatures import KERNEL_BY_BLOCKS, KERNEL_SIGNATURES
+        function = self._module_function(module, kernel_name)
+        if kernel_name in KERNEL_BY_BLOCKS:
+            try:
+                self._by_blocks[function.value] = [(self._module_function(module, symbol), registers)
+                                                   for symbol, registers in KERNEL_BY_BLOCKS[kernel_name]]
+            except CudaRuntimeError:
+                pass                              # a cubin of someone else's with a kernel of that name: one build
+        if kernel_name in KERNEL_SIGNATURES:
+            self._signatures[function.value] = (kernel_name, len(KERNEL_SIGNATURES[kernel_name]))
+        return module, function
+
+    def _module_function(self, module, kernel_name: str):
+        function = ctypes.c_void_p()
         self._check_error(self._lib.vteb_module_get_function(ctypes.byref(function), module, kernel_name.encode("utf-8")),
                           "cuModuleGetFunction")
         from ..compiler.signatures import KERNEL_SIGNATURES
         if kernel_name in KERNEL_SIGNATURES:
-            self._signatures[function.value] = (kernel_name, len(KERNEL_SIGNATURES[kernel_name]))
             # Every kernel of the attention path asks for the same (maximum) shared-memory
             # carve-out: the SMs then never have to drain to re-split L1 / shared memory
             # between the split launch and the small launches around it.
             self._check_error(self._lib.vteb_func_set_shared_carveout(function, 100), "cuFuncSetAttribute")
-        return module, function
+        return function
+
+    def _build_for(self, function, grid, block):
+        """The build of a kernel that suits a grid's number of blocks (KERNEL_BY_BLOCKS); most kernels have one."""
+        builds = self._by_blocks.get(_ptr_value(function)) if self._by_blocks else None
+        if not builds:
+            return function
+        blocks, threads = int(grid[0]) * int(grid[1]) * int(grid[2]), int(block[0]) * int(block[1]) * int(block[2])
+        for build, registers in builds:
+            if blocks <= self.get_num_cus() * (65536 // (registers * threads)):
+                break
+        return build
 
     def register_kernel_signature(self, function, name: str, n_args: int) -> None:
         self._signatures[_ptr_value(function)] = (name, n_args)
@@ -510,10 +535,6 @@ class CudaRuntime:
         sig = self._signatures.get(fval)
         if sig is not None and sig[1] != n_args:
             raise CudaSafetyError(f"ABI mismatch: kernel {sig[0]} takes {sig[1]} arguments, got {n_args}")
-        if shared_mem > self._props["shared_mem_per_block"] and self._smem_optin_set.get(fval, 0) < shared_mem:
-            self._check_error(self._lib.vteb_func_set_max_dynamic_smem(ctypes.c_void_p(fval), int(shared_mem)),
-                              "cuFuncSetAttribute")
-            self._smem_optin_set[fval] = int(shared_mem)
 
     @staticmethod
     def _marshal(args: list):
@@ -533,6 +554,12 @@ class CudaRuntime:
 
     def _launch(self, function, grid, block, args, shared_mem: int, flags: int):
         arr, keep = self._marshal(args)
+        function = self._build_for(function, grid, block)
+        fval = _ptr_value(function)
+        if shared_mem > self._props["shared_mem_per_block"] and self._smem_optin_set.get(fval, 0) < shared_mem:
+            self._check_error(self._lib.vteb_func_set_max_dynamic_smem(ctypes.c_void_p(fval), int(shared_mem)),
+                              "cuFuncSetAttribute")
+            self._smem_optin_set[fval] = int(shared_mem)
         err = self._lib.vteb_launch(ctypes.c_void_p(_ptr_value(function)), int(grid[0]), int(grid[1]), int(grid[2]),
                                     int(block[0]), int(block[1]), int(block[2]), int(shared_mem), self._stream,
                                     arr, flags)
@@ -783,6 +810,7 @@ class CudaRuntime:
             self._lib.vteb_module_unload(ctypes.c_void_p(m))
         self._modules.clear()
         self._signatures.clear()
+        self._by_blocks.clear()
         self._smem_optin_set.clear()
         if self._initialized and self._stream:
             self._lib.vteb_stream_destroy(self._stream)

@@ -29,7 +29,10 @@ KERNEL_SIGNATURES = {
     "kv_cache_append_rope_kernel": [P, P, P, P, I, I, P, I] + _ROPE_TAIL,
     "rope_kernel": [P, P, P, P, I, I, I, I, P, I, I],
     "flash_attention_kernel": [P, P, P, P, P, P, I, I, I, I, F, P, I],     # flash_attention.hip.template:29-43
+    "vteb_flash_attention_few_kernel": [P, P, P, P, P, P, I, I, I, I, F, P, I],       # flash_attention_kernel for few / many blocks
+    "vteb_flash_attention_many_kernel": [P, P, P, P, P, P, I, I, I, I, F, P, I],
     "flash_attention_split_kv_partial_kernel": _REFERENCE_PARTIAL,
+    "vteb_split_kv_partial_compat_short_kernel": _REFERENCE_PARTIAL,                  # the same for short splits
     "flash_attention_split_kv_reduce_kernel": _REDUCE,
     "flash_attention_split_kv_reduce_f32_kernel": _REDUCE,
     "vteb_split_kv_partial_d64_kernel": _FAST_PARTIAL,
@@ -60,6 +63,13 @@ KERNEL_SIGNATURES = {
     "vteb_merge_shard_states_ll_kernel": [P, P, I, I, I, I, I, P, P],
     "vteb_advance_step_kernel": [P],
     "vteb_stage_copy_kernel": [P, P, I],
+}
+
+# Builds of a kernel that differ in registers a thread: a launch takes the first whose resident blocks
+# (65,536 registers per SM) cover its grid, so that the grid is one wave, else the last.
+KERNEL_BY_BLOCKS = {
+    "flash_attention_kernel": (("vteb_flash_attention_few_kernel", 208), ("flash_attention_kernel", 128),
+                               ("vteb_flash_attention_many_kernel", 64)),
 }
 
 # template name (what the reference passes to load_kernel_safe) -> source file

@@ -136,6 +136,16 @@ def choose_split_count(num_sms: int, batch: int, n_hgroups: int, context_length:
     return max(1, min(MAX_SPLITS, math.ceil(context_length / chunk)))
 
 
+def compat_short_splits(num_sms: int, batch: int, num_q_heads: int, head_dim: int, context_length: int, max_chunks: int) -> bool:
+    """Whether the reference-geometry split kernel's build for short splits is taken: two loads in flight a lane and 64
+    registers instead of eight and 128 (decode_attention.cu).  Up to 32 positions a split always, up to 128 where the
+    other build's blocks would not fit the SMs at once.  12 heads on 2 KV heads of 128, short / other: one sequence,
+    32 splits of 16 positions 6.3 / 6.7 us, 64 of 250 20.8 / 16.9; eight sequences, 64 of 63 33.9 / 39.0, of 250 97 / 94."""
+    per_split = -(-context_length // max_chunks)
+    resident = num_sms * (65536 // (128 * head_dim))              # blocks of the ordinary build, 128 registers a thread
+    return per_split <= 32 or (per_split <= 128 and batch * num_q_heads * max_chunks > resident)
+
+
 class SplitKVAttentionDispatcher:
     def __init__(self, hip, codegen, metadata: dict, allocator=None, context_length: int = 4096,
                  batch_size: int = 1, *, num_splits: int | None = None, fixed_chunk_size=None,
@@ -357,8 +367,11 @@ class SplitKVAttentionDispatcher:
             self._kernel_cache['append'] = load(
                 'kv_cache_append', 'kv_cache_append_rope_kernel' if self.fuse_rope else 'kv_cache_append_kernel')
             if self.compat and not self.wide:
+                short = not self.fixed_chunk and compat_short_splits(self.num_sms, self.batch_size, self.num_q_heads, self.head_dim,
+                                                                     self.context_length, self.max_chunks)
                 self._kernel_cache['partial'] = load('flash_attention_split_kv_partial',
-                                                     'flash_attention_split_kv_partial_kernel')
+                                                     'vteb_split_kv_partial_compat_short_kernel' if short
+                                                     else 'flash_attention_split_kv_partial_kernel')
                 self._kernel_cache['reduce'] = load(
                     'flash_attention_split_kv_reduce',
                     'flash_attention_split_kv_reduce_f32_kernel' if self.output_f32

@@ -170,19 +170,26 @@ extern "C" __global__ void rope_kernel(
 // and the warps are merged at the end.  This is the compatibility kernel; the
 // fast path is further down.
 //
-// What bounds it is issue slots and the latency of a warp's chain (K and V come through L2 once per query
-// head).  So a warp takes P = U * 256 / D positions per turn: U = 8 or 16 16-byte loads of K and as many of V
-// per lane are in flight while the previous turn is computed, the scores come from mma.sync (exact fp16 products,
-// fp32 sums in four chains added in registers; the split kernel uses FMAs and reduces them over a row's D / 8
-// lanes), the fp32 FMAs of P V go two at a time, one exponential per position, and
-// the maximum moves only when a score passes it by kCompatLazyMax.  Eight sequences of 700 to 3,960 positions,
-// 32 query heads on 2 KV heads of 128, 8 splits, append and reduce included: 88 us a layer with one position
-// per warp and turn, 42 us so (U = 8, 128 registers, four blocks of 128 threads per SM; U = 16 needs 255
-// registers: 56 us).  Unsplit, four sequences of 103 to 1,383 positions, 12 heads of 128: 178 us against 21 us
-// (U = 16; 27 us with 8: there a block has an SM to itself).
-// The unsplit blocks of a sequence ask L2 for its older rows at once: the same launches 18.4 us instead of 21.5,
-// and with the scores by mma 16.8 (relative error of fp32 outputs against 64 bits 1.4e-7 to 5.8e-7 over 1 and 8
-// splits of up to 8,192 positions, 1.4e-7 to 5.9e-7 with FMAs, 1.5e-7 to 1.2e-6 with one position a turn).
+// What bounds it is issue slots and the latency of a warp's chain (K and V come through L2 once per query head).  So a
+// warp takes P = U * 256 / D positions per turn: U 16-byte loads of K and as many of V per lane are in flight while the
+// previous turn is computed, the scores of a turn are reduced together over a row's D / 8 lanes (by mma.sync in the
+// unsplit kernel from 16 positions on: exact fp16 products, fp32 sums in four chains added in registers), the fp32 FMAs
+// of P V go two at a time, one exponential per position, and the maximum moves only when a score passes it by
+// kCompatLazyMax.  Relative error of fp32 outputs against 64 bits 1.4e-7 to 5.9e-7 over 1 and 8 splits of up to 8,192
+// positions; 1.5e-7 to 1.2e-6 with one position a turn.
+//
+// U trades loads in flight within a warp against warps on an SM, so there are builds of it:
+//   splits: U = 8 in 128 registers for long ones, U = 2 in 64 for short ones, whose blocks are many and do little
+//     (compat_short_splits in core/split_kv_attention.py is the rule; a fixed chunk length sets U at compile time, one
+//     turn of the block's warps a chunk).  Eight sequences, 12 heads on 2 KV heads of 128, 64 splits: 500 positions
+//     21.9 us with U = 8, 16.3 with U = 2 (15.9 with one position a turn); 16,000 positions in 8 splits 95 and 117
+//     (265).  4,000 positions in chunks of 8: 45 us with U = 8, 36 with U = 1 (35).
+//   unsplit: U = 16, 8 or 2 in 208, 128 or 64 registers, whichever the grid's blocks still fit with in one wave
+//     (KERNEL_BY_BLOCKS in compiler/signatures.py).  12 heads of 128, 1,000 positions: 1 sequence 11.3 / 13.3 / 28.9 us,
+//     32 sequences 24.5 / 20.7 / 34.5, 64 sequences of 64 positions 11.7 / 8.2 / 6.8 (one position a turn: 74, 75, 8.2).
+//     Sequences that one turn of every warp covers take that turn with U = 4: 16 positions 4.5 -> 3.5 us.
+// The unsplit blocks of a sequence ask L2 for its older rows at once: four sequences of 103 to 1,383 positions, 12
+// heads of 128, 18.4 us a layer instead of 21.5, and 16.8 with the scores by mma.
 // kUnsplit: ONE split covering every position, together with the cache append and the normalisation:
 // flash_attention_kernel below.
 // ---------------------------------------------------------------------------
@@ -221,7 +228,7 @@ __device__ __forceinline__ F32x2 widen_half2(uint32_t w) {
     return pack_f32x2(f.x, f.y);
 }
 
-template <int D, bool kUnsplit, bool kVec>
+template <int D, bool kUnsplit, bool kVec, int U>
 __device__ __forceinline__ void compat_partial_body(
     float* sh, const __half* __restrict__ q, const __half* k_cache, const __half* v_cache,
     float* __restrict__ partial_m, float* __restrict__ partial_l, float* __restrict__ partial_o,
@@ -232,13 +239,12 @@ __device__ __forceinline__ void compat_partial_body(
 {
     constexpr int LPR = D / 8;         // lanes per cache row, 16 bytes each
     constexpr int RPI = 32 / LPR;      // rows per load instruction of a warp
-    // load instructions per turn and tensor (at most LPR): more where a block has an SM to itself, few enough
-    // for four blocks of 128 threads per SM where it has not
-    constexpr int U = (kUnsplit && D > 64) ? 16 : 8;
-    constexpr int P = U * RPI;         // positions per turn of a warp
-    // Scores by mma (positions as the M dimension, the head's Q in every column) in the unsplit kernel, whose blocks
-    // have an SM each: there issue slots bound a turn.  The split kernel keeps the FMAs: with four blocks per SM the
-    // other warps fill the slots, and K read in 64-byte pieces of rows costs it more (33.8 -> 36.5 us a layer).
+    static_assert(U <= LPR, "at most one score per lane");
+    constexpr int P = U * RPI;         // positions per turn of a warp: U load instructions per tensor (see kSplitTurn)
+    // Scores by mma (positions as the M dimension, the head's Q in every column) in the unsplit kernel, few of whose
+    // blocks share an SM: there issue slots bound a turn.  The split kernel keeps the FMAs: with four blocks per SM the
+    // other warps fill the slots, and K read in 64-byte pieces of rows costs it more (eight sequences of 500 to 4,096
+    // positions, 32 heads on 2 KV heads of 128, 8 splits: 33.8 -> 36.5 us a layer without the append).
     constexpr bool kMma = kUnsplit && P >= 16;
     constexpr int MT = kMma ? P / 16 : 1, KK = D / 32;      // row tiles of a turn, 16-byte pieces of K per lane and row
     float* sh_m = sh; float* sh_l = sh + 8; float* sh_t = sh + 16; float* sh_o = sh + 24;
@@ -451,13 +457,14 @@ __device__ __forceinline__ void compat_partial_body(
         for (int i = 0; i < 8; ++i) sh_o[warp * D + col + i] = of[i];
     }
     __syncthreads();
+    const int used = min(nwarps, (end - start + P - 1) / P);       // warps that had a turn
     float mm = kNeutralM;
-    for (int w = 0; w < nwarps; ++w) mm = fmaxf(mm, sh_t[w]);
+    for (int w = 0; w < used; ++w) mm = fmaxf(mm, sh_t[w]);
     float ll = 0.f;
-    for (int w = 0; w < nwarps; ++w) ll += sh_l[w] * fast_exp2(sh_m[w] - mm);
+    for (int w = 0; w < used; ++w) ll += sh_l[w] * fast_exp2(sh_m[w] - mm);
     for (int d = threadIdx.x; d < D; d += blockDim.x) {
         float acc = 0.f;
-        for (int w = 0; w < nwarps; ++w) acc += sh_o[w * D + d] * fast_exp2(sh_m[w] - mm);
+        for (int w = 0; w < used; ++w) acc += sh_o[w * D + d] * fast_exp2(sh_m[w] - mm);
         if constexpr (kUnsplit) output[((long long)b * num_q_heads + h) * D + d] = __float2half(acc / fmaxf(ll, 1e-20f));
         else partial_o[stat * D + d] = acc;
     }
@@ -467,20 +474,34 @@ __device__ __forceinline__ void compat_partial_body(
     }
 }
 
-template <int D>
-__device__ __forceinline__ void compat_partial_dispatch(
+template <int U>
+__device__ __forceinline__ void split_walk(
     float* sh, const __half* q, const __half* k_cache, const __half* v_cache, float* partial_m, float* partial_l, float* partial_o,
-    int num_q_heads, int num_kv_heads, float scale, const int* kv_cache_offset_ptr, int kv_batch_stride, int max_chunks)
+    int num_q_heads, int num_kv_heads, int head_dim, float scale, const int* kv_cache_offset_ptr, int kv_batch_stride, int max_chunks)
 {
-    if ((((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)v_cache) & 15) == 0 && (kv_batch_stride & 7) == 0)
-        compat_partial_body<D, false, true>(sh, q, k_cache, v_cache, partial_m, partial_l, partial_o, num_q_heads, num_kv_heads,
-                                            scale, kv_cache_offset_ptr, kv_batch_stride, max_chunks);
-    else
-        compat_partial_body<D, false, false>(sh, q, k_cache, v_cache, partial_m, partial_l, partial_o, num_q_heads, num_kv_heads,
-                                             scale, kv_cache_offset_ptr, kv_batch_stride, max_chunks);
+    const bool vec = (((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)v_cache) & 15) == 0 && (kv_batch_stride & 7) == 0;
+#define VTEB_ARGS sh, q, k_cache, v_cache, partial_m, partial_l, partial_o, num_q_heads, num_kv_heads, scale, \
+                  kv_cache_offset_ptr, kv_batch_stride, max_chunks
+    if (vec) {
+        if (head_dim == 64) compat_partial_body<64, false, true, U>(VTEB_ARGS);
+        else if (head_dim == 128) compat_partial_body<128, false, true, U>(VTEB_ARGS);
+        else if (head_dim == 256) compat_partial_body<256, false, true, U>(VTEB_ARGS);
+    } else {
+        constexpr int UU = U < 4 ? U : 4;
+        if (head_dim == 64) compat_partial_body<64, false, false, UU>(VTEB_ARGS);
+        else if (head_dim == 128) compat_partial_body<128, false, false, UU>(VTEB_ARGS);
+        else if (head_dim == 256) compat_partial_body<256, false, false, UU>(VTEB_ARGS);
+    }
+    // the host refuses other head sizes before launching
+#undef VTEB_ARGS
 }
 
-extern "C" __global__ void __launch_bounds__(256) flash_attention_split_kv_partial_kernel(
+// Turn of the split kernel under its reference name: a chunk of fixed length is one turn of the block's warps (8 U
+// positions for every head width).
+constexpr int kSplitTurn = (SPLIT_KV_CHUNK_SIZE <= 0 || SPLIT_KV_CHUNK_SIZE > 32) ? 8
+                         : SPLIT_KV_CHUNK_SIZE > 16 ? 4 : SPLIT_KV_CHUNK_SIZE > 8 ? 2 : 1;
+
+extern "C" __global__ void __launch_bounds__(256, kSplitTurn == 8 ? 2 : kSplitTurn == 4 ? 3 : kSplitTurn == 2 ? 4 : 5) flash_attention_split_kv_partial_kernel(
     const __half* __restrict__ q, const __half* __restrict__ k_cache, const __half* __restrict__ v_cache,
     float* __restrict__ partial_m, float* __restrict__ partial_l, float* __restrict__ partial_o,
     int num_q_heads, int num_kv_heads, int head_dim, float scale,
@@ -489,13 +510,22 @@ extern "C" __global__ void __launch_bounds__(256) flash_attention_split_kv_parti
     __shared__ float sh[kCompatSharedFloats];
     grid_launch_dependents();
     grid_dependency_wait();
-#define VTEB_ARGS sh, q, k_cache, v_cache, partial_m, partial_l, partial_o, num_q_heads, num_kv_heads, scale, \
-                  kv_cache_offset_ptr, kv_batch_stride, max_chunks
-    if (head_dim == 64) compat_partial_dispatch<64>(VTEB_ARGS);
-    else if (head_dim == 128) compat_partial_dispatch<128>(VTEB_ARGS);
-    else if (head_dim == 256) compat_partial_dispatch<256>(VTEB_ARGS);
-    // the host refuses other head sizes before launching
-#undef VTEB_ARGS
+    split_walk<kSplitTurn>(sh, q, k_cache, v_cache, partial_m, partial_l, partial_o, num_q_heads, num_kv_heads, head_dim, scale,
+                           kv_cache_offset_ptr, kv_batch_stride, max_chunks);
+}
+
+// The same for short splits; chosen by compat_short_splits (core/split_kv_attention.py) and by vteb_split_kv_decode.
+extern "C" __global__ void __launch_bounds__(256, 4) vteb_split_kv_partial_compat_short_kernel(
+    const __half* __restrict__ q, const __half* __restrict__ k_cache, const __half* __restrict__ v_cache,
+    float* __restrict__ partial_m, float* __restrict__ partial_l, float* __restrict__ partial_o,
+    int num_q_heads, int num_kv_heads, int head_dim, float scale,
+    const int* __restrict__ kv_cache_offset_ptr, int kv_batch_stride, int max_chunks)
+{
+    __shared__ float sh[kCompatSharedFloats];
+    grid_launch_dependents();
+    grid_dependency_wait();
+    split_walk<2>(sh, q, k_cache, v_cache, partial_m, partial_l, partial_o, num_q_heads, num_kv_heads, head_dim, scale,
+                  kv_cache_offset_ptr, kv_batch_stride, max_chunks);
 }
 
 // ---------------------------------------------------------------------------
@@ -509,30 +539,64 @@ extern "C" __global__ void __launch_bounds__(256) flash_attention_split_kv_parti
 // are read once per query head (through L2); the dispatcher's own one-launch path for short
 // contexts is the split kernel with one split, which reads them once per KV head.
 // ---------------------------------------------------------------------------
-extern "C" __global__ void __launch_bounds__(256) flash_attention_kernel(
+template <int U>
+__device__ __forceinline__ void unsplit_walk(
+    float* sh, const __half* q, const __half* k, const __half* v, __half* k_cache, __half* v_cache, __half* output,
+    int num_q_heads, int num_kv_heads, int head_dim, float scale, const int* kv_cache_offset_ptr, int kv_batch_stride)
+{
+    grid_launch_dependents();
+    grid_dependency_wait();
+    const bool vec = (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)k_cache | (uintptr_t)v_cache) & 15) == 0 && (kv_batch_stride & 7) == 0;
+    constexpr int kShort = U < 4 ? U : 4;          // one turn of every warp: 8 * kShort positions
+    const bool one_turn = U > 4 && kv_cache_offset_ptr[blockIdx.x] < 8 * kShort;
+#define VTEB_ARGS sh, q, k_cache, v_cache, nullptr, nullptr, nullptr, num_q_heads, num_kv_heads, scale, \
+                  kv_cache_offset_ptr, kv_batch_stride, 1, k, v, output
+#define VTEB_WALK(DIM, UU)                                                                                        \
+    do {                                                                                                          \
+        if (!vec) compat_partial_body<DIM, true, false, kShort>(VTEB_ARGS);                                       \
+        else if (one_turn) compat_partial_body<DIM, true, true, kShort>(VTEB_ARGS);                               \
+        else compat_partial_body<DIM, true, true, UU>(VTEB_ARGS);                                                 \
+    } while (0)
+    if (head_dim == 64) VTEB_WALK(64, (U < 8 ? U : 8));
+    else if (head_dim == 128) VTEB_WALK(128, U);
+    else if (head_dim == 256) VTEB_WALK(256, U);
+    // the host refuses other head sizes before launching
+#undef VTEB_WALK
+#undef VTEB_ARGS
+}
+
+extern "C" __global__ void __launch_bounds__(256, 2) flash_attention_kernel(
     const __half* __restrict__ q, const __half* __restrict__ k, const __half* __restrict__ v,
     __half* __restrict__ k_cache, __half* __restrict__ v_cache, __half* __restrict__ output,
     int seq_len, int num_q_heads, int num_kv_heads, int head_dim, float scale,
     const int* __restrict__ kv_cache_offset_ptr, int kv_batch_stride)
 {
     __shared__ float sh[kCompatSharedFloats];
-    grid_launch_dependents();
-    grid_dependency_wait();
-    (void)seq_len;
-    const bool vec = (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)k_cache | (uintptr_t)v_cache) & 15) == 0 && (kv_batch_stride & 7) == 0;
-#define VTEB_ARGS sh, q, k_cache, v_cache, nullptr, nullptr, nullptr, num_q_heads, num_kv_heads, scale, \
-                  kv_cache_offset_ptr, kv_batch_stride, 1, k, v, output
-    if (vec) {
-        if (head_dim == 64) compat_partial_body<64, true, true>(VTEB_ARGS);
-        else if (head_dim == 128) compat_partial_body<128, true, true>(VTEB_ARGS);
-        else if (head_dim == 256) compat_partial_body<256, true, true>(VTEB_ARGS);
-    } else {
-        if (head_dim == 64) compat_partial_body<64, true, false>(VTEB_ARGS);
-        else if (head_dim == 128) compat_partial_body<128, true, false>(VTEB_ARGS);
-        else if (head_dim == 256) compat_partial_body<256, true, false>(VTEB_ARGS);
-    }
-    // the host refuses other head sizes before launching
-#undef VTEB_ARGS
+    unsplit_walk<8>(sh, q, k, v, k_cache, v_cache, output, num_q_heads, num_kv_heads, head_dim, scale, kv_cache_offset_ptr,
+                     kv_batch_stride);
+}
+
+// The builds for grids of few and of many blocks (KERNEL_BY_BLOCKS in compiler/signatures.py).
+extern "C" __global__ void __launch_bounds__(256) vteb_flash_attention_few_kernel(
+    const __half* __restrict__ q, const __half* __restrict__ k, const __half* __restrict__ v,
+    __half* __restrict__ k_cache, __half* __restrict__ v_cache, __half* __restrict__ output,
+    int seq_len, int num_q_heads, int num_kv_heads, int head_dim, float scale,
+    const int* __restrict__ kv_cache_offset_ptr, int kv_batch_stride)
+{
+    __shared__ float sh[kCompatSharedFloats];
+    unsplit_walk<16>(sh, q, k, v, k_cache, v_cache, output, num_q_heads, num_kv_heads, head_dim, scale, kv_cache_offset_ptr,
+                     kv_batch_stride);
+}
+
+extern "C" __global__ void __launch_bounds__(256, 4) vteb_flash_attention_many_kernel(
+    const __half* __restrict__ q, const __half* __restrict__ k, const __half* __restrict__ v,
+    __half* __restrict__ k_cache, __half* __restrict__ v_cache, __half* __restrict__ output,
+    int seq_len, int num_q_heads, int num_kv_heads, int head_dim, float scale,
+    const int* __restrict__ kv_cache_offset_ptr, int kv_batch_stride)
+{
+    __shared__ float sh[kCompatSharedFloats];
+    unsplit_walk<2>(sh, q, k, v, k_cache, v_cache, output, num_q_heads, num_kv_heads, head_dim, scale, kv_cache_offset_ptr,
+                     kv_batch_stride);
 }
 
 // ---------------------------------------------------------------------------

@@ -638,8 +638,16 @@ int vteb_split_kv_decode(const void* q, const void* k_cache, const void* v_cache
     const __half* vh = (const __half*)v_cache;
 
     if (flags & VTEB_ATTN_COMPAT) {
-        rc = launch_rt(flash_attention_split_kv_partial_kernel, dim3(batch, num_q_heads, max_chunks),
-                       dim3(head_dim), 0, s, pdl, qh, kh, vh, partial_m, partial_l, partial_o, num_q_heads,
+        // short splits: their own build, as compat_short_splits (core/split_kv_attention.py) chooses it; the stride
+        // stands for the context, and 0 (not known) for a long one
+        const long long context = kv_batch_stride / ((long long)num_kv_heads * head_dim);
+        const long long per_split = context > 0 ? (context + max_chunks - 1) / max_chunks : 0x7fffffffLL;
+        int sms = 0;
+        if ((rc = check_rt(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, g_device), "sm count"))) return rc;
+        const bool short_splits = per_split <= 32 || (per_split <= 128 && (long long)batch * num_q_heads * max_chunks >
+                                                                              (long long)sms * (65536 / (128 * head_dim)));
+        rc = launch_rt(short_splits ? vteb_split_kv_partial_compat_short_kernel : flash_attention_split_kv_partial_kernel,
+                       dim3(batch, num_q_heads, max_chunks), dim3(head_dim), 0, s, pdl, qh, kh, vh, partial_m, partial_l, partial_o, num_q_heads,
                        num_kv_heads, head_dim, scale, kv_offsets, (int)kv_batch_stride, max_chunks);
         if (rc) return rc;
         if (out_is_f32)

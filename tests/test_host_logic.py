@@ -357,6 +357,25 @@ def test_wide_launch_list_waits_first_unless_the_caller_vouches_for_the_offsets(
     assert not d.wide and not d.build_launches(0, mapping(stride=4096 * 2 * 128), 0x7200_0000_0000, batch=8)[1][1][15].value & FLAG_WAIT_FIRST
 
 
+def test_wide_is_taken_where_it_pays_or_is_asked_for():
+    meta = lambda hq, hkv, d: {'attention.head_count': hq, 'attention.head_count_kv': hkv, 'attention.key_length': d}
+    make = lambda m, **kw: make_dispatcher(m, **kw)[0]
+    for heads, batch, context, want in (((32, 2, 128), 1, 3000, True), ((32, 2, 128), 1, 2999, False), ((64, 1, 256), 1, 128, False),
+                                        ((64, 1, 256), 8, 375, True), ((64, 1, 256), 8, 374, False), ((36, 4, 64), 1, 128, True),
+                                        ((36, 4, 64), 1, 129, False), ((32, 2, 128), 12, 128, True), ((32, 2, 128), 11, 128, False)):
+        d = make(meta(*heads), context_length=context, batch_size=batch)
+        assert d.compat and d.wide == want, (heads, batch, context)
+        assert make(meta(*heads), context_length=context, batch_size=batch, wide=True).wide
+        assert not make(meta(*heads), context_length=context, batch_size=batch, wide=False).wide
+    for kw in ({"num_splits": 8}, {"fixed_chunk_size": 32}):
+        assert not make(meta(32, 2, 128), context_length=4096, **kw).wide
+        with pytest.raises(CudaSafetyError):
+            make(meta(32, 2, 128), context_length=4096, wide=True, **kw)
+    for heads in ((22, 2, 128), (12, 2, 128)):                     # no equal cut; a group the split kernel serves anyway
+        with pytest.raises(CudaSafetyError):
+            make(meta(*heads), context_length=4096, wide=True)
+
+
 def test_dispatcher_switches_and_fallbacks(monkeypatch):
     d, *_ = make_dispatcher({'attention.head_count': 32, 'attention.head_count_kv': 2, 'attention.key_length': 128})
     assert d.compat                                               # group 16 is outside the fast kernel

@@ -44,7 +44,7 @@ def test_wide_groups_match_the_oracle(cuda_runtime, codegen, heads, batch):
     f16 = lambda *s: rng.standard_normal(s, dtype=np.float32).astype(np.float16)
     k, v = f16(batch, S, Hkv, D), f16(batch, S, Hkv, D)
     for capacity in ((S,) if batch > 1 else (S, 64)):
-        ex = DecodeAttentionExecutor(cuda_runtime, codegen, meta, batch, capacity, 1, with_append=True)
+        ex = DecodeAttentionExecutor(cuda_runtime, codegen, meta, batch, capacity, 1, with_append=True, wide=True)
         try:
             assert ex.dispatcher.wide and ex.dispatcher.split_kernel_name == f"vteb_split_kv_partial_wide_d{D}_kernel"
             for lens in lengths:
@@ -80,7 +80,7 @@ def test_wide_keeps_weights_far_below_the_maximum(cuda_runtime, codegen, heads):
         v = (rng.random((B, capacity, Hkv, D), dtype=np.float32) + 0.5).astype(np.float16)
         v[:, ::16] = 0
         off = np.array(lens, dtype=np.int32) - 1
-        ex = DecodeAttentionExecutor(cuda_runtime, codegen, meta, B, capacity, 1)
+        ex = DecodeAttentionExecutor(cuda_runtime, codegen, meta, B, capacity, 1, wide=True)
         try:
             assert ex.dispatcher.wide
             ex.upload_layer(0, q, k, v)
@@ -111,7 +111,7 @@ def test_wide_keeps_infinite_values(cuda_runtime, codegen, heads):
             v[b, : n : 5, :, 9] = np.inf                    # many rows of a channel
             v[b, 0, :, 40], v[b, n - 1, :, 40] = np.inf, (-np.inf if n > 1 else np.inf)
         off = np.array(lens, dtype=np.int32) - 1
-        ex = DecodeAttentionExecutor(cuda_runtime, codegen, meta, B, capacity, 1)
+        ex = DecodeAttentionExecutor(cuda_runtime, codegen, meta, B, capacity, 1, wide=True)
         try:
             assert ex.dispatcher.wide
             ex.upload_layer(0, q, k, v)
@@ -142,7 +142,7 @@ def test_wide_stores_to_an_output_of_any_alignment(cuda_runtime, codegen, heads,
         off = np.array(lens, dtype=np.int32) - 1
         outs = []
         for skip in (0, 4 if f32 else 2):
-            ex = DecodeAttentionExecutor(cuda_runtime, codegen, meta, 2, capacity, 1, output_f32=f32)
+            ex = DecodeAttentionExecutor(cuda_runtime, codegen, meta, 2, capacity, 1, output_f32=f32, wide=True)
             try:
                 assert ex.dispatcher.wide
                 ex.tensor_mapping["blk.0.attention.output"] += skip
@@ -183,7 +183,7 @@ def test_wide_reads_offsets_behind_the_launch_in_front(cuda_runtime, codegen, ba
     try:
         d = SplitKVAttentionDispatcher(rt, codegen, {"attention.head_count": Hq, "attention.head_count_kv": Hkv,
                                                      "attention.key_length": D}, allocator=alloc, context_length=S,
-                                       batch_size=batch, output_f32=True)
+                                       batch_size=batch, output_f32=True, wide=True)
         assert d.wide
         dk, dv, dq, dkn, dvn, doffs = (dev(x) for x in (k, v, q, kn, vn, offs))
         cur, dout = dev(np.zeros(8, np.int32)), dev(np.zeros((steps, batch, Hq, D), np.float32))

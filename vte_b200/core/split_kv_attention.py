@@ -146,6 +146,20 @@ def compat_short_splits(num_sms: int, batch: int, num_q_heads: int, head_dim: in
     return per_split <= 32 or (per_split <= 128 and batch * num_q_heads * max_chunks > resident)
 
 
+def wide_pays(batch: int, head_dim: int, context_length: int) -> bool:
+    """Whether a group of more than eight heads goes to the `wide` build of the split kernel: from 3,000 positions of a
+    batch on; in one split (up to UNSPLIT_MAX_CONTEXT positions) from 1,536 on, 64-wide heads always.  Below that the
+    build's fixed costs (Q, merge, combine of a full-shape launch) outweigh that it reads K and V once.  Over 966 calls
+    of 11 head geometries, 1 to 32 sequences of 64 to 16,000 positions, append included: the rule is within 1.3 % of
+    the better one on the whole and at most 1.4 times it; wide everywhere 8 % and 2.4 times.  32 heads on 2 KV heads of
+    128, wide / reference geometry, us a layer: one sequence of 2,000 positions 12.3 / 11.3, of 4,000 10.7 / 17.4;
+    eight of 300 15.0 / 11.3, of 1,000 16.9 / 18.9, of 16,000 39.6 / 186.6."""
+    positions = batch * context_length
+    if context_length <= UNSPLIT_MAX_CONTEXT:
+        return head_dim == 64 or positions >= 1536
+    return positions >= 3000
+
+
 class SplitKVAttentionDispatcher:
     def __init__(self, hip, codegen, metadata: dict, allocator=None, context_length: int = 4096,
                  batch_size: int = 1, *, num_splits: int | None = None, fixed_chunk_size=None,
@@ -153,7 +167,7 @@ class SplitKVAttentionDispatcher:
                  strict_empty_splits: bool = False, emit_state: bool = False, prefetch_next_layer: bool = True,
                  fused_combine: bool | None = None, variant: str = "auto", fuse_rope: bool = False,
                  tensor_maps: bool = True, work_ptr: int | None = None, fuse_append: bool = False,
-                 balanced: bool | None = None):
+                 balanced: bool | None = None, wide: bool | None = None):
         self.hip = hip
         self.codegen = codegen
         self.metadata = metadata or {}
@@ -202,12 +216,13 @@ class SplitKVAttentionDispatcher:
         if not self.compat and (self._plan is None or not self._plan.ok):
             # geometry outside the fast kernel (group > 8, unusual head_dim): reference-geometry kernels.
             # wide: a group of more than eight query heads that can be cut into equal runs of at most eight
-            # goes to the split kernel's `wide` build, one run per consumer head over the same staged rows
-            # (eight sequences of 500 to 4,096 positions, 32 heads on 2: 20 us a layer against 41).
+            # goes to the split kernel's `wide` build, one run per consumer head over the same staged rows,
+            # where that pays (wide_pays; `wide=` decides otherwise).
             # Only where the caller left the split layout open: a fixed chunk or split count keeps the
             # reference-geometry kernels and the partial buffers that go with them.
             self.compat = True
-            if not num_splits and fixed_chunk_size is None and hasattr(hip, 'split_kv_plan_wide'):
+            if (self._plan is not None and not num_splits and fixed_chunk_size is None and
+                    (wide_pays(self.batch_size, self.head_dim, self.context_length) if wide is None else wide)):
                 wide_plan = hip.split_kv_plan_wide(self.num_q_heads, self.num_kv_heads, self.head_dim)
                 if wide_plan.ok:
                     self._plan, self.wide = wide_plan, True
@@ -220,6 +235,8 @@ class SplitKVAttentionDispatcher:
         # combine launch (the grid barrier costs more than the launch it saves), so it is opt-in.
         self.fused_combine = bool(fused_combine) and can_fuse
 
+        if wide and fixed_chunk_size is not None:
+            raise CudaSafetyError("wide and a fixed chunk size exclude each other")
         if fixed_chunk_size is not None:
             self.chunk_size = _chunk_size_for_cus(num_cus) if fixed_chunk_size == "auto" else int(fixed_chunk_size)
             if self.chunk_size <= 0:
@@ -259,6 +276,9 @@ class SplitKVAttentionDispatcher:
                 if self.max_chunks > fit:
                     self.wide = self.balanced = False
                     self._plan, self.max_chunks = hip.split_kv_plan(self.num_q_heads, self.num_kv_heads, self.head_dim), other
+            if wide and not self.wide:
+                raise CudaSafetyError("wide needs more than eight query heads per KV head that an equal cut brings to "
+                                      "eight or fewer, an open split layout and partial buffers within their limit")
             if self.balanced and self.max_chunks < 2:
                 raise CudaSafetyError("the balanced partition needs at least two splits")
             if not (1 <= self.max_chunks <= 65535):

@@ -63,6 +63,34 @@ def test_wide_groups_match_the_oracle(cuda_runtime, codegen, heads, batch):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("heads, batch, capacity, longest", [((64, 1, 256), 13, 4096, 700), ((48, 1, 128), 200, 64, 64)],
+                         ids=["fewer splits for the scratch limit", "more unsplit items than SMs"])
+def test_wide_batches_at_the_limits_match_the_oracle(cuda_runtime, codegen, heads, batch, capacity, longest):
+    """The balanced partition with its splits cut to the scratch limit; the work queue with more items than CTAs.
+    Bound as above."""
+    from vte_b200.core.decode_executor import DecodeAttentionExecutor
+    Hq, Hkv, D = heads
+    rng = np.random.default_rng([Hq, batch])
+    f16 = lambda *s: rng.standard_normal(s, dtype=np.float32).astype(np.float16)
+    q, k, v = f16(batch, Hq, D), f16(batch, capacity, Hkv, D), f16(batch, capacity, Hkv, D)
+    off = rng.integers(0, longest, size=batch).astype(np.int32)
+    off[0], off[-1] = longest - 1, 0
+    ex = DecodeAttentionExecutor(cuda_runtime, codegen, {"attention.head_count": Hq, "attention.head_count_kv": Hkv,
+                                                         "attention.key_length": D}, batch, capacity, 1, wide=True)
+    try:
+        d = ex.dispatcher
+        if d.balanced:
+            assert d.max_chunks * batch * Hq * (D + 2) * 4 <= WIDE_SCRATCH_BYTES < (d.max_chunks + 1) * batch * Hq * (D + 2) * 4
+        else:
+            assert d.max_chunks == 1 and batch > cuda_runtime.get_num_cus()
+        ex.upload_layer(0, q, k, v)
+        out = ex.execute_decode_batch(off)[0]
+    finally:
+        ex.cleanup()
+    assert np.max(np.abs(out - orc.decode_attention(q, k, v, off))) <= 1e-5
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("heads", [(32, 2, 128), (36, 4, 64), (24, 2, 256)], ids=str)
 def test_wide_keeps_weights_far_below_the_maximum(cuda_runtime, codegen, heads):
     """Every sixteenth position carries all of the weight and values of zero, the others lie 30 octaves under it and

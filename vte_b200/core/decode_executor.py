@@ -194,14 +194,11 @@ class DecodeAttentionExecutor:
     # ---- graph ----------------------------------------------------------------------
     def _stage_copy(self, dst: int, src: int, nbytes: int, first: bool = False):
         """Record a staging copy as a launch.  Both ends are 256-byte aligned and padded to 256 bytes."""
-        if self._copy_fn is None:
-            self._copy_fn = self.codegen.load_kernel_safe(self.hip, 'decode_attention', self.hip.get_gpu_architecture(),
-                                                          'vteb_stage_copy_kernel')[1]
         words = -(-nbytes // 16)
         programmatic, self.hip.programmatic_launch = self.hip.programmatic_launch, self.programmatic and not first
         try:
             self.hip.launch_kernel_recorded(self._copy_fn, [ctypes.c_void_p(src), ctypes.c_void_p(dst), ctypes.c_int(words)],
-                                            (max(1, min(148, -(-words // 256))), 1, 1), (256, 1, 1), 0)
+                                            (max(1, min(self.hip.get_num_cus(), -(-words // 256))), 1, 1), (256, 1, 1), 0)
         finally:
             self.hip.programmatic_launch = programmatic
 
@@ -255,11 +252,15 @@ class DecodeAttentionExecutor:
     def build_io_graph(self):
         """One graph for a whole end-to-end step: kv offsets and every layer's Q from pinned
         staging to the device, every layer's launches, every layer's output back to pinned
-        staging.  Copies up to STAGE_COPY_MAX_BYTES are launches on the compute queue, larger ones copy nodes.  A step is then one graph launch instead of three copies and a launch (the
+        staging.  Copies up to STAGE_COPY_MAX_BYTES are launches on the compute queue, larger ones
+        copy nodes.  A step is then one graph launch instead of three copies and a launch (the
         reference stages its offsets with a separate copy before each launch,
         vte/core/hip_graph_executor.py:772-789)."""
         if self._io_graph_exec is not None or not self.use_graph:
             return
+        if self._copy_fn is None:                         # before the capture begins
+            self._copy_fn = self.codegen.load_kernel_safe(self.hip, 'decode_attention', self.hip.get_gpu_architecture(),
+                                                          'vteb_stage_copy_kernel')[1]
         self.hip.programmatic_launch = self.programmatic
         try:
             self.hip.stream_begin_capture()

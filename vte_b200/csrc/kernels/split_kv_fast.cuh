@@ -35,8 +35,8 @@
 //
 // The `..._wide_...` build serves more than eight query heads per KV head: the group is cut into nv equal
 // runs of at most eight heads (FastPlan::nv), each run is a consumer head with warps of its own, and all runs
-// of a KV head read the same staged rows, so K and V still cross HBM and L2 once.  Eight sequences of 500 to
-// 4,096 positions, 32 heads on 2 KV heads of 128, append included: 20 us a layer against 41 us with the
+// of a KV head read the same staged rows, so K and V still cross HBM and L2 once.  Eight sequences of 400 to
+// 4,000 positions, 32 heads on 2 KV heads of 128, append included: 19.4 us a layer against 34.0 us with the
 // reference-geometry kernels, which read K and V once per query head; the bytes alone need 3 us, the rest is
 // launches, the Q fetch, the merge and the combine.
 // The reference-geometry kernels have fp32 products, so the wide build rounds every sum in fp32 registers (products of
@@ -233,19 +233,6 @@ __device__ __forceinline__ void copy_rows_async(const unsigned char* src, const 
     }
 }
 
-// When a CTA owns exactly one item (one sequence, splits <= CTAs) and the
-// dispatcher passed the next layer's cache, a loader warp that has issued its last
-// copy asks L2 to fetch the byte range the same CTA will stream in the next
-// layer's launch.  HBM then stays busy while this launch drains its tail and the
-// combine runs, and the next launch starts from L2.  Every byte is still read
-// from HBM once per step.  Requests are 8 KB each, spread over the lanes.
-// Its place matters: issued right after the loader's last tile and its (fruitless) ticket
-// draw it is worth 0.35 us per 32k-context layer (1.2 us per launch when split launches run back to
-// back); issued one atomic round trip earlier it is worth 0.07 us less, and held back until the
-// consumers have released the last tile it costs 1.2 us.
-// The prefetch only pays while a whole layer's K and V stay in L2 until the next launch reads
-// them: above this many bytes per tensor (the grid's total) it is skipped.  Measured at one
-// million positions (0.5 GB per tensor): prefetching cost 15 % of the throughput.
 // Grid-wide barrier for a grid whose CTAs are all resident (grid <= SM count, one CTA
 // per SM).  words[0] counts arrivals and is cleared by the last arriver, words[1] is a
 // generation number; one thread per CTA calls this.  The wait is bounded (kWaitLimitCycles).
@@ -614,6 +601,19 @@ __device__ __forceinline__ void fast_partial_body(const FastArgs& a)
             if (lane == 0) next = gridDim.x + atomicAdd(a.ticket, 1);
             item = __shfl_sync(0xffffffffu, next, 0);
         }
+        // When a CTA owns exactly one item (one sequence, splits <= CTAs) and the
+        // dispatcher passed the next layer's cache, a loader warp that has issued its last
+        // copy asks L2 to fetch the byte range the same CTA will stream in the next
+        // layer's launch.  HBM then stays busy while this launch drains its tail and the
+        // combine runs, and the next launch starts from L2.  Every byte is still read
+        // from HBM once per step.  Requests are 8 KB each, spread over the lanes.
+        // Its place matters: issued right after the loader's last tile and its (fruitless) ticket
+        // draw it is worth 0.35 us per 32k-context layer (1.2 us per launch when split launches run back to
+        // back); issued one atomic round trip earlier it is worth 0.07 us less, and held back until the
+        // consumers have released the last tile it costs 1.2 us.
+        // The prefetch only pays while a whole layer's K and V stay in L2 until the next launch reads
+        // them: above this many bytes per tensor (the grid's total) it is skipped.  Measured at one
+        // million positions (0.5 GB per tensor): prefetching cost 15 % of the throughput.
         if (a.next_k_cache != nullptr && plan.n_hgroups == 1 && total_items <= (int)gridDim.x && (int)blockIdx.x < total_items) {
             const ItemGeometry g = first_geom;
             if (g.end > g.start && (long long)(g.end - g.start) * pos_stride * total_items <= kL2PrefetchMaxBytes)

@@ -31,7 +31,7 @@ def _round_up(x: int, m: int) -> int:
 
 
 # Staging copies of an end-to-end step up to this size are launches (build_io_graph).  Measured, copy nodes against
-# launches, a step of 12 query heads: 3 KB of Q 38.6 / 27.4 us, 84 KB (28 layers) 182 / 173, 336 KB 289 / 284;
+# launches, a step of 12 query heads: 3 KB of Q 34.2 / 27.1 us, 84 KB (28 layers) 182 / 173, 336 KB 289 / 284;
 # of 32 heads of 64: 1.8 MB 730 / 730, 7 MB 2,099 / 2,104.
 STAGE_COPY_MAX_BYTES = 1 << 20
 

@@ -44,6 +44,8 @@ extern "C" {
 #define VTEB_LAUNCH_PROGRAMMATIC 1  /* programmatic dependent launch: the kernel may start
                                        before its predecessor in the stream has finished and
                                        orders itself with griddepcontrol.wait */
+#define VTEB_LAUNCH_CLUSTER_SHIFT 8 /* bits 8 and up: blocks per thread-block cluster along x, 0 or 1
+                                       for none, at most 16; has to divide the grid */
 
 const char* vteb_last_error_string(void);
 int vteb_version(void);
@@ -158,6 +160,20 @@ int vteb_split_kv_plan_compact(int num_q_heads, int num_kv_heads, int head_dim, 
 /* The plan of the split kernels for more than eight query heads per KV head (`vteb_split_kv_partial_wide_*`):
  * ok = 1 when the group can be cut into at most eight equal runs of at most eight heads. */
 int vteb_split_kv_plan_wide(int num_q_heads, int num_kv_heads, int head_dim, vteb_fast_plan* plan);
+/* What a launch of the kernels with one work item per CTA needs (`vteb_decode_cluster_*`, `vteb_split_kv_lean_*`):
+ * a (sequence, KV head) is cut into `n_parts` (at most 16 with `cluster` != 0: the parts are one thread-block
+ * cluster), the longest sequence has `context` positions.  ok = 0: not covered (groups of more than 16 query heads,
+ * more than 8 with 256-wide heads or without clusters). */
+typedef struct vteb_lean_plan_t {
+    int ok;
+    int threads;
+    int smem_bytes;
+    int depth;         /* blocks of 16 positions a warp has in flight: the kernels' `depth` argument */
+} vteb_lean_plan_t;
+int vteb_lean_plan(int num_q_heads, int num_kv_heads, int head_dim, int n_parts, long long context, int cluster,
+                   vteb_lean_plan_t* plan);
+/* How many clusters of `cluster` blocks of a loaded kernel the device runs at once (cuOccupancyMaxActiveClusters). */
+int vteb_max_active_clusters(void* function, int cluster, int threads, int smem_bytes, int* count);
 /* Encodes the 128-byte tensor map the fast split kernels take for a K or V cache: the cache
  * seen as `n_rows` position rows (all sequences, one after another) of `row_halves` =
  * Hkv * D fp16 values, in boxes of 64 values x `box_rows` rows (the plan's `tile`) with the

@@ -1,0 +1,183 @@
+"""Routes with one work item per CTA (core/lean_route.py): what is chosen, on the CPU, and the kernels against the oracle
+where lengths, parts and blocks meet."""
+import ctypes
+import math
+
+import numpy as np
+import pytest
+
+from oracle import attention_oracle as orc
+from vte_b200.bridge.cuda_runtime import LeanPlan, load_library
+from vte_b200.core.decode_executor import DecodeAttentionExecutor
+from vte_b200.core.lean_route import CLUSTER_PARTS, LEAN_SPLIT_MAX_CONTEXT, choose_lean_route
+
+
+def lean_plan(*a):
+    plan = LeanPlan()
+    assert load_library().vteb_lean_plan(*a, ctypes.byref(plan)) == 0
+    return plan
+
+
+@pytest.mark.parametrize("D", [64, 128, 256])
+@pytest.mark.parametrize("group", [1, 6, 8, 9, 16, 17])
+def test_plan_holds_exchange_rows_and_received_states(built_library, group, D):
+    for parts in (1, 2, 7, 16, 17, 148):
+        for cluster in (0, 1):
+            for context in (1, 128, 129, 4096, 1 << 20):
+                p = lean_plan(2 * group, 2, D, parts, context, cluster)
+                covered = group <= (8 if D == 256 or not cluster else 16) and (not cluster or 2 <= parts <= 16)
+                assert bool(p.ok) == covered
+                if not covered:
+                    continue
+                warps = p.threads // 32
+                assert p.threads % (D // 8) == 0 and 1 <= p.depth <= (2 if D == 256 else 3)
+                assert p.depth * 64 * D >= group * (D + 8) * 4                   # a warp's exchange rows in its own blocks
+                blocks = -(-(-(-context // parts)) // 16)
+                assert p.depth * warps >= min(blocks, 3 * warps if D < 256 else 2 * warps)
+                need = 128 + (2 if group > 8 else 1) * D * 16 + warps * p.depth * 64 * D
+                need += -(-(group * D // 32) // parts) * parts * 144 if cluster else 0
+                assert p.smem_bytes == need <= 225 * 1024
+
+
+class FakeHip:
+    lean_plan = staticmethod(lambda hq, hkv, d, parts, context, cluster: lean_plan(hq, hkv, d, parts, context, int(cluster)))
+    get_gpu_architecture = staticmethod(lambda: "sm_100a")
+
+    @staticmethod
+    def max_active_clusters(fn, cluster, threads, smem):
+        return {2: 74, 3: 45, 4: 33, 5: 26, 6: 22, 8: 15, 9: 15, 12: 7, 16: 7}[cluster]
+
+
+class FakeDispatcher:
+    def __init__(self, heads, batch, context):
+        self.num_q_heads, self.num_kv_heads, self.head_dim = heads
+        self.batch_size, self.context_length, self.num_sms, self.max_chunks = batch, context, 148, 148
+        self.hip, self.codegen = FakeHip, self
+
+    def load_kernel_safe(self, *a):
+        return None, ctypes.c_void_p(1)
+
+
+def test_the_route_follows_the_size(built_library):
+    route = lambda *a: choose_lean_route(FakeDispatcher(*a), True)
+    assert route((12, 2, 128), 1, 4096) == (16, True)             # one short sequence
+    assert route((12, 2, 128), 1, 16384) == (74, False)           # one long one: split and combine over the whole GPU
+    assert route((12, 2, 128), 1, LEAN_SPLIT_MAX_CONTEXT + 1) == (0, False)
+    assert route((32, 8, 64), 64, 16384) == (0, False)            # a batch that streams: equal shares
+    assert route((32, 2, 128), 8, 4096)[1] and route((12, 2, 128), 4, 2048)[1]
+    assert route((34, 2, 128), 4, 2048) == (0, False)             # seventeen query heads on a KV head
+    assert route((32, 2, 256), 4, 2048) == (0, False)             # sixteen with 256-wide heads
+    assert route((12, 2, 96), 4, 2048) == (0, False)
+    for batch in (1, 3, 17, 64):
+        for context in (1, 130, 1000, 9000, 70000):
+            parts, cluster = route((28, 4, 128), batch, context)
+            assert parts == 0 or (parts in CLUSTER_PARTS if cluster else batch == 1 and parts == 37)
+
+
+LENGTHS = [1, 15, 16, 17, 127, 128, 129, 255, 257, 385, 600]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("heads", [(12, 2, 128), (8, 8, 64), (8, 1, 256), (16, 1, 64), (22, 2, 128), (32, 2, 128)])
+@pytest.mark.parametrize("route", [(2, True), (5, True), (16, True), (37, False)])
+@pytest.mark.parametrize("append", [True, False], ids=["append", "attend"])
+def test_lean_kernels_match_the_oracle(cuda_runtime, codegen, heads, route, append):
+    """Every length at which a block, a warp's turn or a part starts or ends, two layers on one cache.  fp32 sums of fp16
+    products: 2e-5 of the result's norm; the newest rows are the projections' bits."""
+    Hq, Hkv, D = heads
+    if not route[1] and Hq // Hkv > 8:
+        pytest.skip("split and combine serve groups of up to eight heads")
+    B = len(LENGTHS) if route[1] else 1
+    rng = np.random.default_rng(7)
+    f16 = lambda *s: rng.standard_normal(s, dtype=np.float32).astype(np.float16)
+    S = 640
+    ex = DecodeAttentionExecutor(cuda_runtime, codegen, {"attention.head_count": Hq, "attention.head_count_kv": Hkv,
+                                                         "attention.key_length": D}, B, S, 2, n_kv_buffers=1,
+                                 with_append=append, lean=route, **({} if route[1] else {"num_splits": 148}))
+    try:
+        q, k0, v0 = f16(2, B, Hq, D), f16(B, S, Hkv, D), f16(B, S, Hkv, D)
+        kn, vn = f16(2, B, Hkv, D), f16(2, B, Hkv, D)
+        for lengths in ([LENGTHS] if B > 1 else [[n] for n in LENGTHS]):
+            off, k, v = np.array(lengths, dtype=np.int32) - 1, k0.copy(), v0.copy()
+            for b, n in enumerate(lengths):
+                k[b, n:], v[b, n:] = np.inf, np.nan                   # nothing behind the end counts
+            ex.upload_cache(0, k, v)
+            for l in range(2):
+                ex.upload_layer(l, q[l])
+                ex.upload_new_kv(l, kn[l], vn[l])
+            out = ex.execute_decode_batch(off)
+            assert ex.kernel_launches_per_step == (2 if route[1] else 4)
+            for l in range(2):
+                for b, n in enumerate(lengths):
+                    if append:
+                        k[b, n - 1], v[b, n - 1] = kn[l, b], vn[l, b]
+                ref = orc.decode_attention(q[l], np.where(np.isfinite(k), k, 0), np.where(np.isfinite(v), v, 0), off)
+                assert np.linalg.norm(out[l] - ref) <= 2e-5 * np.linalg.norm(ref)
+            got_k, got_v = ex.download_cache_rows(0, 0, S)
+            assert np.array_equal(got_k.view(np.uint16), k[0].view(np.uint16)) and np.array_equal(got_v.view(np.uint16), v[0].view(np.uint16))
+    finally:
+        ex.cleanup()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rope_type,rotary", [(0, 0), (1, 0), (2, 32), (2, 64)])
+@pytest.mark.parametrize("D", [64, 128, 256])
+def test_rotation_in_the_lean_kernels_gives_the_separate_launch_s_bits(cuda_runtime, codegen, D, rope_type, rotary):
+    """The rotated row in the cache is the standalone rotation's, bit for bit, and so are the outputs of the same route."""
+    meta = {"attention.head_count": 12, "attention.head_count_kv": 2, "attention.key_length": D, "rope_type": rope_type}
+    if rotary:
+        meta["rotary_dim"] = rotary
+    rng = np.random.default_rng(3)
+    f16 = lambda *s: rng.standard_normal(s, dtype=np.float32).astype(np.float16)
+    B, S = 2, 300
+    q, k, v, kn, vn = f16(B, 12, D), f16(B, S, 2, D), f16(B, S, 2, D), f16(B, 2, D), f16(B, 2, D)
+    off, got = np.array([250, 16], dtype=np.int32), []
+    for rope in ("separate", "fused", "fused-append"):
+        ex = DecodeAttentionExecutor(cuda_runtime, codegen, meta, B, S, 1, rope=rope, lean=(6, True))
+        try:
+            ex.upload_layer(0, q, k, v)
+            ex.upload_new_kv(0, kn, vn)
+            out = ex.execute_decode_batch(off)
+            got.append((out, *ex.download_cache_rows(0, 0, 251)))
+            m, l, o = ex.read_partials()                             # the split launch's, on demand
+            assert np.isfinite(m).all() and l.max() > 0
+        finally:
+            ex.cleanup()
+    for other in got[1:]:
+        for a, b in zip(got[0], other):
+            assert np.array_equal(a, b)
+
+
+@pytest.mark.gpu
+def test_an_infinite_value_stays_infinite_in_a_cluster(cuda_runtime, codegen):
+    """As fp32 products give it: infinite where its weight is not zero, the other columns finite."""
+    rng = np.random.default_rng(5)
+    f16 = lambda *s: rng.standard_normal(s, dtype=np.float32).astype(np.float16)
+    q, k, v = f16(1, 12, 128), f16(1, 200, 2, 128), f16(1, 200, 2, 128)
+    v[0, 3, 0, 5], v[0, 199, 1, 7] = np.inf, -np.inf
+    ex = DecodeAttentionExecutor(cuda_runtime, codegen, {"attention.head_count": 12, "attention.head_count_kv": 2,
+                                                         "attention.key_length": 128}, 1, 200, 1, lean=(8, True))
+    try:
+        ex.upload_layer(0, q, k, v)
+        out = ex.execute_decode_batch(np.array([199], dtype=np.int32))[0, 0]
+    finally:
+        ex.cleanup()
+    assert np.all(out[:6, 5] == np.inf) and np.all(out[6:, 7] == -np.inf)
+    out[:6, 5], out[6:, 7] = 0, 0
+    assert np.isfinite(out).all()
+
+
+@pytest.mark.gpu
+def test_a_cluster_kernel_refuses_a_launch_without_its_clusters(cuda_runtime, codegen):
+    """The grid's clusters have to be the parts: otherwise the status word says so and nothing is written."""
+    meta = {"attention.head_count": 12, "attention.head_count_kv": 2, "attention.key_length": 128}
+    ex = DecodeAttentionExecutor(cuda_runtime, codegen, meta, 1, 256, 1, lean=(4, True))
+    try:
+        ex._choose_route()
+        fn, args, grid, block, smem = ex._route.launches(0, ex.tensor_mapping, ex.offsets.ptr, 1)[0]
+        ex._update_staging_buffers(np.array([200], dtype=np.int32))
+        cuda_runtime.launch_kernel_recorded(fn, args, tuple(grid), block, smem)
+        with pytest.raises(Exception, match="bounded wait"):
+            ex.dispatcher_check()
+    finally:
+        ex.cleanup()

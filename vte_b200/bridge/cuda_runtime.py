@@ -42,6 +42,7 @@ ATTR_L2_BYTES = 6
 ATTR_CLOCK_KHZ = 7
 
 LAUNCH_PROGRAMMATIC = 1
+LAUNCH_CLUSTER_SHIFT = 8
 
 ATTN_COMPAT = 1
 ATTN_WRITE_EMPTY_O = 2
@@ -62,9 +63,22 @@ class FastPlan(ctypes.Structure):
                 ("combine_smem_bytes", ctypes.c_int)]
 
 
+class LeanPlan(ctypes.Structure):
+    """Mirror of `vteb_lean_plan_t` (include/vteb200.h)."""
+    _fields_ = [("ok", ctypes.c_int), ("threads", ctypes.c_int), ("smem_bytes", ctypes.c_int), ("depth", ctypes.c_int)]
+
+
 class KvTensorMap(ctypes.Structure):
     """The 128-byte tensor map of a K or V cache, passed to the fast split kernels by value."""
     _fields_ = [("opaque", ctypes.c_uint64 * 16)]
+
+
+class ClusterGrid(tuple):
+    """Grid dimensions of a launch whose blocks form thread-block clusters of `cluster` along x."""
+    def __new__(cls, dims, cluster: int):
+        self = super().__new__(cls, dims)
+        self.cluster = int(cluster)
+        return self
 
 
 def default_library_path() -> Path:
@@ -130,6 +144,8 @@ def _declare(lib):
         "vteb_split_kv_plan": (i, [i, i, i, ctypes.POINTER(FastPlan)]),
         "vteb_split_kv_plan_compact": (i, [i, i, i, ctypes.POINTER(FastPlan)]),
         "vteb_split_kv_plan_wide": (i, [i, i, i, ctypes.POINTER(FastPlan)]),
+        "vteb_lean_plan": (i, [i, i, i, i, ll, i, ctypes.POINTER(LeanPlan)]),
+        "vteb_max_active_clusters": (i, [vp, i, i, i, ip]),
         "vteb_kv_tensor_map": (i, [vp, vp, ctypes.c_longlong, i, i]),
         "vteb_combine_rows_epl": (i, [i, i]),
         "vteb_split_kv_decode": (i, [vp, vp, vp, vp, vp, i, vp, vp, vp, vp, i, i, i, i, f, ll, i, i, u, i, vp]),
@@ -199,6 +215,7 @@ class CudaRuntime:
         self._props: dict = {}
         self._smem_optin_set: dict[int, int] = {}
         self._signatures: dict[int, tuple[str, int]] = {}
+        self._active_clusters: dict[tuple, int] = {}   # what the device said of a kernel's clusters
         self._by_blocks: dict[int, list] = {}     # function -> [(build, registers a thread)], see KERNEL_BY_BLOCKS
         self._panic = False
         self._sync_timeout_s = sync_timeout_s
@@ -560,6 +577,9 @@ class CudaRuntime:
             self._check_error(self._lib.vteb_func_set_max_dynamic_smem(ctypes.c_void_p(fval), int(shared_mem)),
                               "cuFuncSetAttribute")
             self._smem_optin_set[fval] = int(shared_mem)
+        cluster = getattr(grid, "cluster", 1)
+        if cluster > 1:
+            flags |= cluster << LAUNCH_CLUSTER_SHIFT
         err = self._lib.vteb_launch(ctypes.c_void_p(_ptr_value(function)), int(grid[0]), int(grid[1]), int(grid[2]),
                                     int(block[0]), int(block[1]), int(block[2]), int(shared_mem), self._stream,
                                     arr, flags)
@@ -701,6 +721,23 @@ class CudaRuntime:
                           "vteb_split_kv_plan_wide")
         return plan
 
+    def lean_plan(self, num_q_heads: int, num_kv_heads: int, head_dim: int, n_parts: int, context: int, cluster: bool) -> LeanPlan:
+        """What a launch of the kernels with one work item per CTA needs."""
+        plan = LeanPlan()
+        self._check_error(self._lib.vteb_lean_plan(num_q_heads, num_kv_heads, head_dim, n_parts, context, int(cluster),
+                                                   ctypes.byref(plan)), "vteb_lean_plan")
+        return plan
+
+    def max_active_clusters(self, function, cluster: int, threads: int, smem_bytes: int) -> int:
+        """Clusters of `cluster` blocks of a loaded kernel that the device runs at once."""
+        key = (_ptr_value(function), cluster, threads, smem_bytes)
+        if key not in self._active_clusters:
+            n = ctypes.c_int(0)
+            self._check_error(self._lib.vteb_max_active_clusters(ctypes.c_void_p(key[0]), cluster, threads, smem_bytes,
+                                                                 ctypes.byref(n)), "cuOccupancyMaxActiveClusters")
+            self._active_clusters[key] = n.value
+        return self._active_clusters[key]
+
     def kv_tensor_map(self, cache_ptr: int, n_rows: int, row_halves: int, box_rows: int) -> KvTensorMap:
         """Tensor map over a cache of `n_rows` position rows of `row_halves` fp16 values (boxes of
         64 values x `box_rows` rows, 128-byte swizzle) for the fast split kernels."""
@@ -811,6 +848,7 @@ class CudaRuntime:
         self._modules.clear()
         self._signatures.clear()
         self._by_blocks.clear()
+        self._active_clusters.clear()
         self._smem_optin_set.clear()
         if self._initialized and self._stream:
             self._lib.vteb_stream_destroy(self._stream)

@@ -20,6 +20,7 @@ _FAST_PARTIAL = _REFERENCE_PARTIAL + [I, I, I, P, P, P, P, P, P, I, ctypes.Struc
 # ... batch, min_chunk, flags, seq_order, ticket, status, next K, next V, output, out_kind,
 #     tensor map of the K cache, tensor map of the V cache (128 bytes each, by value)
 _ROPE_TAIL = [P, P, I, I]                                 # cos table, sin table, rope_type, rotary_dim
+_LEAN = _REFERENCE_PARTIAL + [P, P, P, I, I, I, P, P, P] + _ROPE_TAIL   # ... new K, new V, output, out_kind, flags, depth, status, next K, next V
 _REDUCE = [P, P, P, P, I, I, I]
 _FAST_COMBINE = _REDUCE + [I, P]                          # dsplit, ticket
 
@@ -51,6 +52,14 @@ KERNEL_SIGNATURES = {
     "vteb_split_kv_partial_wide_d64_kernel": _FAST_PARTIAL,           # more than eight query heads per KV head
     "vteb_split_kv_partial_wide_d128_kernel": _FAST_PARTIAL,
     "vteb_split_kv_partial_wide_d256_kernel": _FAST_PARTIAL,
+    "vteb_decode_cluster_d64_kernel": _LEAN,                          # a thread-block cluster per (sequence, KV head)
+    "vteb_decode_cluster_d128_kernel": _LEAN,
+    "vteb_decode_cluster_d256_kernel": _LEAN,
+    "vteb_decode_cluster_2_d64_kernel": _LEAN,                        # nine to sixteen query heads per KV head
+    "vteb_decode_cluster_2_d128_kernel": _LEAN,
+    "vteb_split_kv_lean_d64_kernel": _LEAN,                           # one sequence: a part of one KV head per CTA
+    "vteb_split_kv_lean_d128_kernel": _LEAN,
+    "vteb_split_kv_lean_d256_kernel": _LEAN,
     "vteb_split_kv_combine_f16_kernel": _FAST_COMBINE,
     "vteb_split_kv_combine_f32_kernel": _FAST_COMBINE,
     "vteb_split_kv_combine_state_kernel": _FAST_COMBINE,

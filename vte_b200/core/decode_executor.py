@@ -23,6 +23,7 @@ import numpy as np
 from ..bridge.errors import CudaSafetyError
 from ..bridge.memory import MemoryRegion, SlabAllocator
 from ..config import ENV_NO_PDL, env_flag
+from .lean_route import LeanRoute, choose_lean_route
 from .split_kv_attention import SplitKVAttentionDispatcher
 
 
@@ -45,7 +46,7 @@ class DecodeAttentionExecutor:
                  emit_state: bool = False, per_layer_hook=None, prefetch_next_layer: bool = True,
                  fused_combine: Optional[bool] = None, variant: str = "auto", rope: str = "off",
                  rope_theta: float = 1e6, tensor_maps: bool = True, fuse_append: bool = False,
-                 balanced: Optional[bool] = None, wide: Optional[bool] = None):
+                 balanced: Optional[bool] = None, wide: Optional[bool] = None, lean: Optional[tuple] = None):
         self.hip = hip
         # rope: "off" = Q and K arrive rotated; "separate" = the reference's standalone rotation
         # launch runs before the append (rotating the projections in place); "fused" = the append
@@ -110,6 +111,13 @@ class DecodeAttentionExecutor:
             fuse_rope=rope in ("fused", "fused-append"), fuse_append=(rope == "fused-append" or fuse_append), tensor_maps=tensor_maps,
             work_ptr=self.out_all.ptr + self._out_tail, balanced=balanced, wide=wide)
 
+        # lean: (CTAs per (sequence, KV head), whether they are a cluster), the launches of lean_route.py; (0, False) never,
+        # None where they pay and the caller has asked for nothing that the dispatcher's own launches have and these have not.
+        open_layout = not (num_splits or compat or strict_empty_splits or emit_state or fused_combine or balanced is not None or
+                           wide is not None) and (fixed_chunk_size is None and min_chunk is None and variant == "auto" and
+                                                  tensor_maps and prefetch_next_layer)
+        self._lean = lean if lean is not None else None if open_layout else (0, False)
+        self._route = None
         self.k_cache = [A(self.kv_bytes, f"kv_cache.k.{i}", MemoryRegion.KV_CACHE) for i in range(self.n_kv)]
         self.v_cache = [A(self.kv_bytes, f"kv_cache.v.{i}", MemoryRegion.KV_CACHE) for i in range(self.n_kv)]
         # all layers' Q (and outputs) are contiguous so one copy moves a whole step's worth
@@ -207,10 +215,14 @@ class DecodeAttentionExecutor:
         programmatic = self.hip.programmatic_launch
         # within a captured step of nothing but the layers' own launches, offsets and older rows do not change
         self.dispatcher.offsets_final = self.use_graph and self.per_layer_hook is None and self.launch_rewriter is None
+        route = self._route if self.dispatcher.offsets_final else None
         for l in range(self.L):
-            launches = self.dispatcher.build_launches(l, self.tensor_mapping, self.offsets.ptr, batch=self.B)
-            if not self.with_append and not self.dispatcher.fuse_append:
-                launches = launches[1:]
+            if route is not None:
+                launches = route.launches(l, self.tensor_mapping, self.offsets.ptr, self.B)
+            else:
+                launches = self.dispatcher.build_launches(l, self.tensor_mapping, self.offsets.ptr, batch=self.B)
+                if not self.with_append and not self.dispatcher.fuse_append:
+                    launches = launches[1:]
             if self.launch_rewriter is not None:
                 launches = self.launch_rewriter(l, launches)
             if self.rope == "separate":
@@ -228,6 +240,19 @@ class DecodeAttentionExecutor:
                 n += int(self.per_layer_hook(l) or 0)
         return n
 
+    def _choose_route(self):
+        """Before a step is captured: whether its layers' launches are the dispatcher's own or a route of lean_route.py."""
+        d = self.dispatcher
+        if (self._route is not None or self._lean == (0, False) or not self.use_graph or self.per_layer_hook is not None or
+                self.launch_rewriter is not None or not d.enabled or not hasattr(self.hip, 'lean_plan')):
+            return
+        d._allocate_scratch()                         # and the work words
+        append = self.with_append or d.fuse_append
+        if self._lean is None:
+            self._lean = choose_lean_route(d, append)
+        if self._lean[0]:
+            self._route = LeanRoute(d, self._lean[0], append, self._lean[1])
+
     def build_decode_graph(self):
         """Capture all layers' launches once (hip_graph_executor.py:504-725)."""
         if self._graph_exec is not None:
@@ -239,6 +264,7 @@ class DecodeAttentionExecutor:
                 n += 1 if self.rope == "separate" else 0
                 self.kernel_launches_per_step = (n if (self.with_append or self.dispatcher.fuse_append) else n - 1) * self.L
                 return
+            self._choose_route()
             self.hip.stream_begin_capture()
             try:
                 self.kernel_launches_per_step = self._record_all()
@@ -261,6 +287,7 @@ class DecodeAttentionExecutor:
         if self._copy_fn is None:                         # before the capture begins
             self._copy_fn = self.codegen.load_kernel_safe(self.hip, 'decode_attention', self.hip.get_gpu_architecture(),
                                                           'vteb_stage_copy_kernel')[1]
+        self._choose_route()
         self.hip.programmatic_launch = self.programmatic
         try:
             self.hip.stream_begin_capture()
@@ -375,6 +402,12 @@ class DecodeAttentionExecutor:
 
     def read_partials(self):
         """(partial_m, partial_l [B,Hq,C], partial_o [B,Hq,C,D]) of the last layer run."""
+        if self._route is not None:
+            # the step had no partials: the last layer's split launch now, on the caches and offsets as they are
+            launches = self.dispatcher.build_launches(self.L - 1, self.tensor_mapping, self.offsets.ptr, batch=self.B)
+            for fn, args, grid, block, smem in launches[0 if self.dispatcher.fuse_append else 1:][:1]:
+                self.hip.launch_kernel_recorded(fn, args, grid, block, smem)
+            self.hip.stream_synchronize()
         pm, pl, po = self.dispatcher.partial_buffers
         C = self.dispatcher.max_chunks
         m = np.empty((self.B, self.Hq, C), dtype=np.float32)

@@ -414,6 +414,11 @@ class SplitKVAttentionDispatcher:
                     'vteb_split_kv_combine_state_kernel' if self.emit_state else
                     'vteb_split_kv_combine_f32_kernel' if self.output_f32 else 'vteb_split_kv_combine_f16_kernel')
 
+        self._allocate_scratch()
+        return self._kernel_cache['append'], self._kernel_cache['partial'], self._kernel_cache['reduce']
+
+    def _allocate_scratch(self):
+        if self._partial_m is None:
             # One scratch set shared by every layer: layers run strictly one after
             # another inside a decode step, so rewriting the same buffers is safe.
             stats_size = self.batch_size * self.num_q_heads * self.max_chunks * 4
@@ -429,7 +434,6 @@ class SplitKVAttentionDispatcher:
                 self._work = self.allocator.allocate(16, "attn_splitkv_work", MemoryRegion.SCRATCH)
             if hasattr(self.hip, 'safe_memset'):
                 self.hip.safe_memset(ctypes.c_void_p(self._work.ptr), 16, "attn_splitkv_work")
-        return self._kernel_cache['append'], self._kernel_cache['partial'], self._kernel_cache['reduce']
 
     def build_rope_launch(self, tensor_mapping: dict, kv_offset_ptr: int, batch: int = 1,
                           q_name: str = None, k_name: str = None, layer_idx: int = 0, block_size: int = 256):

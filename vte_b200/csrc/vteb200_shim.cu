@@ -43,6 +43,7 @@ struct DriverApi {
     CUresult (*LaunchKernel)(CUfunction, unsigned, unsigned, unsigned, unsigned, unsigned, unsigned,
                              unsigned, CUstream, void**, void**) = nullptr;
     CUresult (*LaunchKernelEx)(const CUlaunchConfig*, CUfunction, void**, void**) = nullptr;
+    CUresult (*OccupancyMaxActiveClusters)(int*, CUfunction, const CUlaunchConfig*) = nullptr;
     CUresult (*GetErrorString)(CUresult, const char**) = nullptr;
     CUresult (*TensorMapEncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                      const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
@@ -72,6 +73,7 @@ int driver_api() {
     if ((rc = resolve("cuFuncSetAttribute", &g_drv.FuncSetAttribute))) return rc;
     if ((rc = resolve("cuLaunchKernel", &g_drv.LaunchKernel))) return rc;
     if ((rc = resolve("cuLaunchKernelEx", &g_drv.LaunchKernelEx))) return rc;
+    if ((rc = resolve("cuOccupancyMaxActiveClusters", &g_drv.OccupancyMaxActiveClusters))) return rc;
     if ((rc = resolve("cuGetErrorString", &g_drv.GetErrorString))) return rc;
     if ((rc = resolve("cuTensorMapEncodeTiled", &g_drv.TensorMapEncodeTiled))) return rc;
     g_drv.ready = true;
@@ -364,19 +366,34 @@ int vteb_launch(void* function, unsigned gx, unsigned gy, unsigned gz, unsigned 
     REQUIRE_INIT();
     if (!function) return fail(VTEB_ERR_INVALID_ARGUMENT, "null function");
     if (!gx || !gy || !gz || !bx || !by || !bz) return fail(VTEB_ERR_INVALID_ARGUMENT, "zero launch dimension");
-    if (flags & VTEB_LAUNCH_PROGRAMMATIC) {
+    const unsigned cluster = flags >> VTEB_LAUNCH_CLUSTER_SHIFT;
+    if (cluster > 16 || (cluster > 1 && gx % cluster))
+        return fail(VTEB_ERR_INVALID_ARGUMENT, "clusters of %u blocks do not divide a grid of %u", cluster, gx);
+    if ((flags & VTEB_LAUNCH_PROGRAMMATIC) || cluster > 1) {
         CUlaunchConfig cfg;
         memset(&cfg, 0, sizeof(cfg));
         cfg.gridDimX = gx; cfg.gridDimY = gy; cfg.gridDimZ = gz;
         cfg.blockDimX = bx; cfg.blockDimY = by; cfg.blockDimZ = bz;
         cfg.sharedMemBytes = shared_mem_bytes;
         cfg.hStream = (CUstream)stream;
-        CUlaunchAttribute attr;
-        memset(&attr, 0, sizeof(attr));
-        attr.id = CU_LAUNCH_ATTRIBUTE_PROGRAMMATIC_STREAM_SERIALIZATION;
-        attr.value.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = &attr;
-        cfg.numAttrs = 1;
+        CUlaunchAttribute attr[2];
+        memset(attr, 0, sizeof(attr));
+        cfg.attrs = attr;
+        if (flags & VTEB_LAUNCH_PROGRAMMATIC) {
+            attr[cfg.numAttrs].id = CU_LAUNCH_ATTRIBUTE_PROGRAMMATIC_STREAM_SERIALIZATION;
+            attr[cfg.numAttrs++].value.programmaticStreamSerializationAllowed = 1;
+        }
+        if (cluster > 1) {
+            attr[cfg.numAttrs].id = CU_LAUNCH_ATTRIBUTE_CLUSTER_DIMENSION;
+            attr[cfg.numAttrs].value.clusterDim.x = cluster;
+            attr[cfg.numAttrs].value.clusterDim.y = 1;
+            attr[cfg.numAttrs++].value.clusterDim.z = 1;
+            if (cluster > 8) {             // more than every device has to offer
+                const int rc = check_drv(g_drv.FuncSetAttribute((CUfunction)function, CU_FUNC_ATTRIBUTE_NON_PORTABLE_CLUSTER_SIZE_ALLOWED, 1),
+                                         "cuFuncSetAttribute(cluster size)");
+                if (rc) return rc;
+            }
+        }
         return check_drv(g_drv.LaunchKernelEx(&cfg, (CUfunction)function, params, nullptr), "cuLaunchKernelEx");
     }
     return check_drv(g_drv.LaunchKernel((CUfunction)function, gx, gy, gz, bx, by, bz, shared_mem_bytes,
@@ -578,6 +595,35 @@ int vteb_split_kv_plan_compact(int num_q_heads, int num_kv_heads, int head_dim, 
 
 int vteb_split_kv_plan_wide(int num_q_heads, int num_kv_heads, int head_dim, vteb_fast_plan* plan) {
     return fill_plan(num_q_heads, num_kv_heads, head_dim, 0, plan, 1);
+}
+
+int vteb_lean_plan(int num_q_heads, int num_kv_heads, int head_dim, int n_parts, long long context, int cluster, vteb_lean_plan_t* plan) {
+    if (!plan) return fail(VTEB_ERR_INVALID_ARGUMENT, "null plan");
+    const LeanPlan p = make_lean_plan(num_q_heads, num_kv_heads, head_dim, n_parts, context, cluster);
+    plan->ok = p.ok; plan->threads = p.threads; plan->smem_bytes = p.smem_bytes; plan->depth = p.depth;
+    return 0;
+}
+
+int vteb_max_active_clusters(void* function, int cluster, int threads, int smem_bytes, int* count) {
+    REQUIRE_INIT();
+    if (!function || !count || cluster < 1 || cluster > 16 || threads < 1 || smem_bytes < 0)
+        return fail(VTEB_ERR_INVALID_ARGUMENT, "clusters of %d blocks of %d threads and %d bytes", cluster, threads, smem_bytes);
+    CUlaunchConfig cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDimX = cluster; cfg.gridDimY = 1; cfg.gridDimZ = 1;
+    cfg.blockDimX = threads; cfg.blockDimY = 1; cfg.blockDimZ = 1;
+    cfg.sharedMemBytes = smem_bytes;
+    CUlaunchAttribute attr;
+    memset(&attr, 0, sizeof(attr));
+    attr.id = CU_LAUNCH_ATTRIBUTE_CLUSTER_DIMENSION;
+    attr.value.clusterDim.x = cluster; attr.value.clusterDim.y = 1; attr.value.clusterDim.z = 1;
+    cfg.attrs = &attr; cfg.numAttrs = 1;
+    int rc = 0;
+    if (cluster > 8 && (rc = check_drv(g_drv.FuncSetAttribute((CUfunction)function, CU_FUNC_ATTRIBUTE_NON_PORTABLE_CLUSTER_SIZE_ALLOWED, 1),
+                                       "cuFuncSetAttribute(cluster size)"))) return rc;
+    if ((rc = check_drv(g_drv.FuncSetAttribute((CUfunction)function, CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, vteb::kSmemBudget),
+                        "cuFuncSetAttribute(max dynamic shared memory)"))) return rc;
+    return check_drv(g_drv.OccupancyMaxActiveClusters(count, (CUfunction)function, &cfg), "cuOccupancyMaxActiveClusters");
 }
 
 int vteb_kv_tensor_map(void* out_128_bytes, const void* cache, long long n_rows, int row_halves, int box_rows) {

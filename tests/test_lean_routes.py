@@ -74,6 +74,34 @@ def test_the_route_follows_the_size(built_library):
             assert parts == 0 or (parts in CLUSTER_PARTS if cluster else batch == 1 and parts == 37)
 
 
+def test_the_unsplit_kernel_goes_to_clusters_where_they_pay(built_library):
+    """Which launches of flash_attention_kernel do, and with which arguments; all others keep their own builds."""
+    from vte_b200.compiler.signatures import CLUSTER_KERNELS, KERNEL_SIGNATURES
+    from vte_b200.core.lean_route import unsplit_as_clusters
+    hip = FakeHip()
+    hip.get_num_cus = lambda: 148
+    kernels = {name: name for name in CLUSTER_KERNELS}
+    vp, ci = ctypes.c_void_p, ctypes.c_int
+
+    def served(B=4, heads=(12, 2, 128), capacity=2048, grid=None, block=None, at=0, stride=None):
+        Hq, Hkv, D = heads
+        args = [vp(0x1000 * (i + 1)) for i in range(6)] + [ci(1), ci(Hq), ci(Hkv), ci(D), ctypes.c_float(0.5), vp(0x9000),
+                                                          ci(capacity * Hkv * D if stride is None else stride)]
+        args[0] = vp(0x1000 + at)
+        return unsplit_as_clusters(hip, kernels, args, grid or (B, Hq, 1), block or (D, 1, 1))
+    fn, args, grid, block, smem = served()
+    parts = args[12].value
+    assert fn == "vteb_decode_cluster_d128_kernel" and parts in CLUSTER_PARTS and grid == (8 * parts, 1, 1) and grid.cluster == parts
+    assert [isinstance(a, t) for a, t in zip(args, KERNEL_SIGNATURES[fn])] == [True] * len(KERNEL_SIGNATURES[fn]) and block == (256, 1, 1)
+    assert [a.value for a in (args[0], args[1], args[2], args[13], args[14], args[15])] == [0x1000, 0x4000, 0x5000, 0x2000, 0x3000, 0x6000]
+    assert args[16].value == 1 and args[17].value == 32 and args[9].value == 0.5 and args[11].value == 2048 * 256
+    assert served(heads=(32, 2, 128))[0] == "vteb_decode_cluster_2_d128_kernel" and served(B=37)[1][12].value == 2
+    for refused in (dict(capacity=256), dict(capacity=512, heads=(32, 2, 128)), dict(B=38), dict(heads=(34, 2, 128)), dict(stride=0),
+                    dict(stride=2048 * 256 + 4), dict(at=8), dict(grid=(4, 6, 1)), dict(block=(64, 1, 1)), dict(heads=(32, 2, 256)),
+                    dict(heads=(12, 2, 96)), dict(grid=(4, 12, 2))):
+        assert served(**refused) is None, refused
+
+
 LENGTHS = [1, 15, 16, 17, 127, 128, 129, 255, 257, 385, 600]
 
 

@@ -153,6 +153,7 @@ def _declare(lib):
         "vteb_kv_cache_append": (i, [vp, vp, vp, vp, vp, i, i, i, ll, vp]),
         "vteb_check_status": (i, [vp, vp]),
         "vteb_noalloc_check_status": (i, [vp]),
+        "vteb_module_check_status": (i, [vp]),
         "vteb_fill_normal_f16": (i, [vp, sz, ull, f, f, f, vp]),
         "vteb_read_bandwidth_probe": (i, [vp, sz, vp, i, vp]),
     }
@@ -215,6 +216,8 @@ class CudaRuntime:
         self._props: dict = {}
         self._smem_optin_set: dict[int, int] = {}
         self._signatures: dict[int, tuple[str, int]] = {}
+        self._clustered: dict[int, dict] = {}     # unsplit kernel -> the cluster kernels that serve it where that pays, and its module
+        self._status_modules: set[int] = set()    # modules whose launches report to a status word of the module's
         self._active_clusters: dict[tuple, int] = {}   # what the device said of a kernel's clusters
         self._by_blocks: dict[int, list] = {}     # function -> [(build, registers a thread)], see KERNEL_BY_BLOCKS
         self._panic = False
@@ -490,12 +493,15 @@ class CudaRuntime:
             if not module.value:
                 self._check_error(self._lib.vteb_module_load(ctypes.byref(module), str(cubin_path).encode("utf-8")), "cuModuleLoad")
                 self._modules[key or (path, module.value)] = module.value
-        from ..compiler.signatures import KERNEL_BY_BLOCKS, KERNEL_SIGNATURES
+        from ..compiler.signatures import CLUSTER_KERNELS, KERNEL_BY_BLOCKS, KERNEL_SIGNATURES
         function = self._module_function(module, kernel_name)
         if kernel_name in KERNEL_BY_BLOCKS:
             try:
                 self._by_blocks[function.value] = [(self._module_function(module, symbol), registers)
                                                    for symbol, registers in KERNEL_BY_BLOCKS[kernel_name]]
+                if kernel_name == "flash_attention_kernel":
+                    self._clustered[function.value] = {name: self._module_function(module, name) for name in CLUSTER_KERNELS}
+                    self._clustered[function.value]["module"] = module.value
             except CudaRuntimeError:
                 pass                              # a cubin of someone else's with a kernel of that name: one build
         if kernel_name in KERNEL_SIGNATURES:
@@ -570,8 +576,17 @@ class CudaRuntime:
         return arr, keep
 
     def _launch(self, function, grid, block, args, shared_mem: int, flags: int):
+        kernels = self._clustered.get(_ptr_value(function)) if self._clustered else None
+        served = None
+        if kernels:
+            from ..core.lean_route import unsplit_as_clusters
+            served = unsplit_as_clusters(self, kernels, args, grid, block)
+        if served:
+            function, args, grid, block, shared_mem = served
+            self._status_modules.add(kernels["module"])
         arr, keep = self._marshal(args)
-        function = self._build_for(function, grid, block)
+        if not served:
+            function = self._build_for(function, grid, block)
         fval = _ptr_value(function)
         if shared_mem > self._props["shared_mem_per_block"] and self._smem_optin_set.get(fval, 0) < shared_mem:
             self._check_error(self._lib.vteb_func_set_max_dynamic_smem(ctypes.c_void_p(fval), int(shared_mem)),
@@ -621,6 +636,11 @@ class CudaRuntime:
         finally:
             done.set()
         self._check_error(err, "cudaDeviceSynchronize")
+        for module in self._status_modules:
+            err = self._lib.vteb_module_check_status(ctypes.c_void_p(module))
+            if err == ERR_DEVICE_STATUS:
+                raise CudaRuntimeError(self._last_error(), code=err)
+            self._check_error(err, "vteb_module_check_status")
         if timed_out.is_set():
             raise CudaRuntimeError(f"cudaDeviceSynchronize took longer than {self._sync_timeout_s} s")
         return True
@@ -849,6 +869,8 @@ class CudaRuntime:
         self._signatures.clear()
         self._by_blocks.clear()
         self._active_clusters.clear()
+        self._clustered.clear()
+        self._status_modules.clear()
         self._smem_optin_set.clear()
         if self._initialized and self._stream:
             self._lib.vteb_stream_destroy(self._stream)

@@ -81,6 +81,9 @@ KERNEL_BY_BLOCKS = {
                                ("vteb_flash_attention_many_kernel", 64)),
 }
 
+# Kernels of a thread-block cluster per (sequence, KV head): flash_attention_kernel goes to them where they pay (lean_route.py).
+CLUSTER_KERNELS = tuple(k for k in KERNEL_SIGNATURES if k.startswith("vteb_decode_cluster_"))
+
 # template name (what the reference passes to load_kernel_safe) -> source file
 TEMPLATE_SOURCES = {
     "kv_cache_append": "decode_attention.cu",

@@ -14,6 +14,7 @@ from ..bridge.cuda_runtime import ClusterGrid
 from ..bridge.errors import CudaSafetyError
 
 FLAG_PREFETCH_Q = 8
+FLAG_WAIT_FIRST = 32
 FLAG_ROWS_FINAL = 64
 
 
@@ -134,3 +135,56 @@ def choose_lean_route(d, append: bool) -> tuple:
             d.hip.lean_plan(Hq, Hkv, D, parts, context, False).ok and _split_us(parts, positions, D, cache_bytes) < best):
         route = parts, False
     return route
+
+
+UNSPLIT_MIN_CAPACITY = 256          # cache positions a sequence, by the stride; above them flash_attention_kernel goes to clusters
+
+
+def _unsplit_parts(hip, kernels: dict, name: str, Hq: int, Hkv: int, D: int, pairs: int, capacity: int):
+    """(parts, plan), or (0, None).  Sizes alone decide, so `kernels` remembers a thousand of them."""
+    known = kernels.setdefault("parts", {})
+    key = (Hq, Hkv, D, pairs, capacity)
+    if key not in known:
+        if len(known) >= 1024:
+            known.clear()
+        best = (math.inf, 0, None)
+        for parts in CLUSTER_PARTS:
+            plan = hip.lean_plan(Hq, Hkv, D, parts, capacity, True)
+            if not plan.ok or hip.max_active_clusters(kernels[name], parts, plan.threads, plan.smem_bytes) < pairs:
+                continue
+            us = _cluster_us(parts, pairs, pairs, _LONGEST * capacity, _PER_POSITION[D], hip.get_num_cus(), 0.0)
+            if us < best[0]:
+                best = (us, parts, plan)
+        known[key] = best[1:]
+    return known[key]
+
+
+def unsplit_as_clusters(hip, kernels: dict, args: list, grid, block):
+    """flash_attention_kernel's launch (13 arguments, grid (batch, query heads, 1), block (head_dim)) as a launch of the
+    cluster kernels, (function, args, grid, block, shared_mem), or None where its own builds serve it.
+
+    Its geometry has one block walk a whole sequence; a cluster per (sequence, KV head) has as many SMs on it as the grid
+    leaves and reads K and V once for the group.  us a layer, plain stream order, builds / clusters: four sequences of 12
+    heads on 2 of 128, 64 positions 4.8 / 5.3, 200: 5.9 / 5.3, 600: 8.6 / 5.4, 1,500: 15.3 / 6.3, 4,000: 43 / 9.6.  So:
+    caches with room for more than 256 positions (512 with two runs of query heads: 6.5 us at the least), and no more
+    pairs than clusters run at once (a second wave costs more than short sequences take: 64 sequences of 200 positions
+    19 / 21, of 64 8 / 17)."""
+    if len(args) != 13:
+        return None
+    value = lambda a: a if isinstance(a, int) else getattr(a, "value", None) or 0
+    q, k, v, k_cache, v_cache, out, _, Hq, Hkv, D, scale, offsets, stride = (value(a) for a in args)
+    batch = int(grid[0])
+    if (D not in _PER_POSITION or Hkv <= 0 or Hq <= 0 or Hq % Hkv or stride <= 0 or stride % 8 or (q | k | v | k_cache | v_cache) % 16 or
+            tuple(int(x) for x in grid) != (batch, Hq, 1) or tuple(int(x) for x in block) != (D, 1, 1)):
+        return None
+    group, pairs, capacity = Hq // Hkv, batch * Hkv, stride // (Hkv * D)
+    name = cluster_kernel_name(group, D)
+    if name not in kernels or capacity <= UNSPLIT_MIN_CAPACITY * (2 if group > 8 else 1):
+        return None
+    parts, plan = _unsplit_parts(hip, kernels, name, Hq, Hkv, D, pairs, capacity)
+    if not parts:
+        return None
+    vp, ci, cf = ctypes.c_void_p, ctypes.c_int, ctypes.c_float
+    lean = [vp(q), vp(k_cache), vp(v_cache), vp(0), vp(0), vp(0), ci(Hq), ci(Hkv), ci(D), cf(scale), vp(offsets), ci(stride), ci(parts),
+            vp(k), vp(v), vp(out), ci(1), ci(FLAG_WAIT_FIRST), ci(plan.depth), vp(0), vp(0), vp(0), vp(0), vp(0), ci(-1), ci(0)]
+    return kernels[name], lean, ClusterGrid((pairs * parts, 1, 1), parts), (plan.threads, 1, 1), plan.smem_bytes

@@ -48,6 +48,10 @@ __host__ __device__ inline LeanPlan make_lean_plan(int num_q_heads, int num_kv_h
     return p;
 }
 
+// Where a launch without a status word of its own (flash_attention_kernel's arguments have none) reports a wait that ran
+// out; read by vteb_module_check_status.
+extern "C" { __device__ int vteb_lean_status = 0; }
+
 constexpr int kLeanRowsFinal = 64;      // flag: the newest row is in the cache before the launch in front starts
 constexpr int kLeanCtrlBytes = 128;     // barriers and the abort word
 constexpr int kLeanUnit = 36;           // floats a CTA sends per 32 output columns: o[32], m, l, 2 unused
@@ -562,7 +566,7 @@ __device__ __forceinline__ void lean_body(const LeanArgs& a)
         a.partial_m = partial_m; a.partial_l = partial_l; a.partial_o = partial_o;                                      \
         a.num_q_heads = num_q_heads; a.num_kv_heads = num_kv_heads; a.scale = scale;                                    \
         a.kv_offsets = kv_cache_offset_ptr; a.kv_batch_stride = kv_batch_stride; a.n_parts = n_parts;                   \
-        a.k_new = k_new; a.v_new = v_new; a.output = output; a.out_kind = out_kind; a.flags = flags; a.status = status; \
+        a.k_new = k_new; a.v_new = v_new; a.output = output; a.out_kind = out_kind; a.flags = flags; a.status = status ? status : &vteb_lean_status; \
         a.depth = depth;                                                                                                \
         a.next_k_cache = next_k_cache; a.next_v_cache = next_v_cache;                                                   \
         a.rope_cos = cos_cache; a.rope_sin = sin_cache; a.rope_type = rope_type; a.rotary_dim = rotary_dim;             \

@@ -39,6 +39,7 @@ struct DriverApi {
     CUresult (*ModuleLoad)(CUmodule*, const char*) = nullptr;
     CUresult (*ModuleGetFunction)(CUfunction*, CUmodule, const char*) = nullptr;
     CUresult (*ModuleUnload)(CUmodule) = nullptr;
+    CUresult (*ModuleGetGlobal)(CUdeviceptr*, size_t*, CUmodule, const char*) = nullptr;
     CUresult (*FuncSetAttribute)(CUfunction, CUfunction_attribute, int) = nullptr;
     CUresult (*LaunchKernel)(CUfunction, unsigned, unsigned, unsigned, unsigned, unsigned, unsigned,
                              unsigned, CUstream, void**, void**) = nullptr;
@@ -70,6 +71,7 @@ int driver_api() {
     if ((rc = resolve("cuModuleLoad", &g_drv.ModuleLoad))) return rc;
     if ((rc = resolve("cuModuleGetFunction", &g_drv.ModuleGetFunction))) return rc;
     if ((rc = resolve("cuModuleUnload", &g_drv.ModuleUnload))) return rc;
+    if ((rc = resolve("cuModuleGetGlobal", &g_drv.ModuleGetGlobal))) return rc;
     if ((rc = resolve("cuFuncSetAttribute", &g_drv.FuncSetAttribute))) return rc;
     if ((rc = resolve("cuLaunchKernel", &g_drv.LaunchKernel))) return rc;
     if ((rc = resolve("cuLaunchKernelEx", &g_drv.LaunchKernelEx))) return rc;
@@ -872,6 +874,20 @@ int vteb_check_status(int* work, void* stream) {
                                   : "another CTA or another rank never arrived");
     }
     return 0;
+}
+
+int vteb_module_check_status(void* module) {
+    REQUIRE_INIT();
+    if (!module) return fail(VTEB_ERR_INVALID_ARGUMENT, "null module");
+    CUdeviceptr p = 0;
+    size_t bytes = 0;
+    int rc = check_drv(g_drv.ModuleGetGlobal(&p, &bytes, (CUmodule)module, "vteb_lean_status"), "cuModuleGetGlobal");
+    if (rc) return rc;
+    int status = 0;
+    if ((rc = check_rt(cudaMemcpy(&status, (const void*)p, sizeof(int), cudaMemcpyDeviceToHost), "status read"))) return rc;
+    if (status == 0) return 0;
+    cudaMemset((void*)p, 0, sizeof(int));
+    return fail(VTEB_ERR_DEVICE_STATUS, "a kernel gave up on a bounded wait (code %d)", status);
 }
 
 int vteb_noalloc_check_status(void* stream) {

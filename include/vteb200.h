@@ -161,17 +161,22 @@ int vteb_split_kv_plan_compact(int num_q_heads, int num_kv_heads, int head_dim, 
  * ok = 1 when the group can be cut into at most eight equal runs of at most eight heads. */
 int vteb_split_kv_plan_wide(int num_q_heads, int num_kv_heads, int head_dim, vteb_fast_plan* plan);
 /* What a launch of the kernels with one work item per CTA needs (`vteb_decode_cluster_*`, `vteb_split_kv_lean_*`):
- * a (sequence, KV head) is cut into `n_parts` (at most 16 with `cluster` != 0: the parts are one thread-block
- * cluster), the longest sequence has `context` positions.  ok = 0: not covered (groups of more than 16 query heads,
- * more than 8 with 256-wide heads or without clusters). */
+ * a (sequence, KV head) is cut into `n_parts`, the longest sequence has `context` positions.  `kind` 0: split and
+ * combine; 1: the parts, 2 to 16, are one thread-block cluster; 2: the same with half the warps a block
+ * (`vteb_decode_cluster_half_*`).  ok = 0: not covered (groups of more than 16 query heads, more than 8 with 256-wide
+ * heads or without clusters, half blocks of 64-wide heads). */
 typedef struct vteb_lean_plan_t {
     int ok;
     int threads;
     int smem_bytes;
     int depth;         /* blocks of 16 positions a warp has in flight: the kernels' `depth` argument */
 } vteb_lean_plan_t;
-int vteb_lean_plan(int num_q_heads, int num_kv_heads, int head_dim, int n_parts, long long context, int cluster,
+int vteb_lean_plan(int num_q_heads, int num_kv_heads, int head_dim, int n_parts, long long context, int kind,
                    vteb_lean_plan_t* plan);
+/* Estimated microseconds of one layer on a route of `kind` and `n_parts` with `resident` clusters at once (kind -1: the
+ * launches of vteb_split_kv_decode), by which routes are chosen. */
+double vteb_lean_estimate(int kind, int n_parts, int num_q_heads, int num_kv_heads, int head_dim, int batch, long long context,
+                          int resident, int num_sms);
 /* How many clusters of `cluster` blocks of a loaded kernel the device runs at once (cuOccupancyMaxActiveClusters). */
 int vteb_max_active_clusters(void* function, int cluster, int threads, int smem_bytes, int* count);
 /* Encodes the 128-byte tensor map the fast split kernels take for a K or V cache: the cache
@@ -212,7 +217,10 @@ int vteb_combine_rows_epl(int rows, int head_dim);
                                       split the output columns instead of the blocks.  Correct at any length */
 #define VTEB_ATTN_BALANCED 64   /* several sequences: every CTA takes an equal share of all cached positions; a
                                    (sequence, KV head group) is cut where shares end, into at most max_chunks
-                                   splits (max_chunks >= 2; min_chunk is ignored); no work queue */
+                                   splits (max_chunks >= 2; min_chunk is ignored); no work queue.  With no other
+                                   flag but VTEB_ATTN_PROGRAMMATIC and n_ctas <= 0, a call that thread-block
+                                   clusters serve faster (vteb_lean_estimate; kv_batch_stride stands for the
+                                   context) is ONE launch of those, which leaves the scratch as it is */
 int vteb_split_kv_decode(const void* q, const void* k_cache, const void* v_cache,
                          const int* kv_offsets, void* output, int out_is_f32,
                          float* partial_m, float* partial_l, float* partial_o, int* work,

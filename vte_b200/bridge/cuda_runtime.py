@@ -145,6 +145,7 @@ def _declare(lib):
         "vteb_split_kv_plan_compact": (i, [i, i, i, ctypes.POINTER(FastPlan)]),
         "vteb_split_kv_plan_wide": (i, [i, i, i, ctypes.POINTER(FastPlan)]),
         "vteb_lean_plan": (i, [i, i, i, i, ll, i, ctypes.POINTER(LeanPlan)]),
+        "vteb_lean_estimate": (ctypes.c_double, [i, i, i, i, i, i, ll, i, i]),
         "vteb_max_active_clusters": (i, [vp, i, i, i, ip]),
         "vteb_kv_tensor_map": (i, [vp, vp, ctypes.c_longlong, i, i]),
         "vteb_combine_rows_epl": (i, [i, i]),
@@ -584,6 +585,7 @@ class CudaRuntime:
         if served:
             function, args, grid, block, shared_mem = served
             self._status_modules.add(kernels["module"])
+            flags |= LAUNCH_PROGRAMMATIC          # it waits for everything in front before it touches anything, and releases after
         arr, keep = self._marshal(args)
         if not served:
             function = self._build_for(function, grid, block)
@@ -741,12 +743,17 @@ class CudaRuntime:
                           "vteb_split_kv_plan_wide")
         return plan
 
-    def lean_plan(self, num_q_heads: int, num_kv_heads: int, head_dim: int, n_parts: int, context: int, cluster: bool) -> LeanPlan:
+    def lean_plan(self, num_q_heads: int, num_kv_heads: int, head_dim: int, n_parts: int, context: int, kind: int) -> LeanPlan:
         """What a launch of the kernels with one work item per CTA needs."""
         plan = LeanPlan()
-        self._check_error(self._lib.vteb_lean_plan(num_q_heads, num_kv_heads, head_dim, n_parts, context, int(cluster),
+        self._check_error(self._lib.vteb_lean_plan(num_q_heads, num_kv_heads, head_dim, n_parts, context, int(kind),
                                                    ctypes.byref(plan)), "vteb_lean_plan")
         return plan
+
+    def lean_estimate(self, kind: int, n_parts: int, num_q_heads: int, num_kv_heads: int, head_dim: int, batch: int, context: int,
+                      resident: int) -> float:
+        """Estimated microseconds of one layer, by which routes are chosen (kind -1: the dispatcher's launches)."""
+        return self._lib.vteb_lean_estimate(kind, n_parts, num_q_heads, num_kv_heads, head_dim, batch, context, resident, self.get_num_cus())
 
     def max_active_clusters(self, function, cluster: int, threads: int, smem_bytes: int) -> int:
         """Clusters of `cluster` blocks of a loaded kernel that the device runs at once."""

@@ -111,12 +111,12 @@ class DecodeAttentionExecutor:
             fuse_rope=rope in ("fused", "fused-append"), fuse_append=(rope == "fused-append" or fuse_append), tensor_maps=tensor_maps,
             work_ptr=self.out_all.ptr + self._out_tail, balanced=balanced, wide=wide)
 
-        # lean: (CTAs per (sequence, KV head), whether they are a cluster), the launches of lean_route.py; (0, False) never,
-        # None where they pay and the caller has asked for nothing that the dispatcher's own launches have and these have not.
+        # lean: (CTAs per (sequence, KV head), kind) of a route of lean_route.py; (0, 0) never, None where one pays and
+        # the caller has asked for nothing that the dispatcher's own launches have and these have not.
         open_layout = not (num_splits or compat or strict_empty_splits or emit_state or fused_combine or balanced is not None or
                            wide is not None) and (fixed_chunk_size is None and min_chunk is None and variant == "auto" and
                                                   tensor_maps and prefetch_next_layer)
-        self._lean = lean if lean is not None else None if open_layout else (0, False)
+        self._lean = lean if lean is not None else None if open_layout else (0, 0)
         self._route = None
         self.k_cache = [A(self.kv_bytes, f"kv_cache.k.{i}", MemoryRegion.KV_CACHE) for i in range(self.n_kv)]
         self.v_cache = [A(self.kv_bytes, f"kv_cache.v.{i}", MemoryRegion.KV_CACHE) for i in range(self.n_kv)]
@@ -243,7 +243,7 @@ class DecodeAttentionExecutor:
     def _choose_route(self):
         """Before a step is captured: whether its layers' launches are the dispatcher's own or a route of lean_route.py."""
         d = self.dispatcher
-        if (self._route is not None or self._lean == (0, False) or not self.use_graph or self.per_layer_hook is not None or
+        if (self._route is not None or self._lean == (0, 0) or not self.use_graph or self.per_layer_hook is not None or
                 self.launch_rewriter is not None or not d.enabled or not hasattr(self.hip, 'lean_plan')):
             return
         d._allocate_scratch()                         # and the work words
@@ -251,7 +251,7 @@ class DecodeAttentionExecutor:
         if self._lean is None:
             self._lean = choose_lean_route(d, append)
         if self._lean[0]:
-            self._route = LeanRoute(d, self._lean[0], append, self._lean[1])
+            self._route = LeanRoute(d, *self._lean, append)
 
     def build_decode_graph(self):
         """Capture all layers' launches once (hip_graph_executor.py:504-725)."""

@@ -18,22 +18,25 @@ FLAG_WAIT_FIRST = 32
 FLAG_ROWS_FINAL = 64
 
 
-def cluster_kernel_name(group: int, head_dim: int) -> str:
-    return f"vteb_decode_cluster_{'2_' if group > 8 else ''}d{head_dim}_kernel"
+SPLIT, CLUSTER, HALF = 0, 1, 2      # kinds of route: split and combine; clusters; clusters of blocks of half the warps
+
+
+def cluster_kernel_name(kind: int, group: int, head_dim: int) -> str:
+    return f"vteb_decode_cluster_{'half_' if kind == HALF else ''}{'2_' if group > 8 else ''}d{head_dim}_kernel"
 
 
 class LeanRoute:
-    """`parts` CTAs per (sequence, KV head): one launch a layer (`cluster`), or split and combine."""
+    """`parts` CTAs per (sequence, KV head): one launch a layer (CLUSTER, HALF), or split and combine."""
 
-    def __init__(self, dispatcher, parts: int, append: bool, cluster: bool):
+    def __init__(self, dispatcher, parts: int, kind: int, append: bool):
         d = self.d = dispatcher
-        self.parts, self.append, self.cluster = int(parts), bool(append), bool(cluster)
-        self.plan = d.hip.lean_plan(d.num_q_heads, d.num_kv_heads, d.head_dim, self.parts, d.context_length, self.cluster)
+        self.parts, self.append, self.cluster = int(parts), bool(append), kind != SPLIT
+        self.plan = d.hip.lean_plan(d.num_q_heads, d.num_kv_heads, d.head_dim, self.parts, d.context_length, kind)
         if not self.plan.ok:
             raise CudaSafetyError(f"{self.parts} CTAs per (sequence, KV head) are not covered for this geometry")
         load = lambda symbol: d.codegen.load_kernel_safe(d.hip, 'decode_attention', d.hip.get_gpu_architecture(), symbol)[1]
         if self.cluster:
-            self.function = load(cluster_kernel_name(d.num_q_heads // d.num_kv_heads, d.head_dim))
+            self.function = load(cluster_kernel_name(kind, d.num_q_heads // d.num_kv_heads, d.head_dim))
         else:
             self.function = load(f"vteb_split_kv_lean_d{d.head_dim}_kernel")
             self.combine = load('vteb_split_kv_combine_small_kernel' if self.parts <= 32 else
@@ -76,86 +79,66 @@ class LeanRoute:
         return [split, (self.combine, args + [ci(slices), vp(d.work_ptr)], (rows * slices, 1, 1), (256, 1, 1), min(N, 256) * 4)]
 
 
-# Estimated microseconds a layer, by which a route is chosen.  Fitted to 1,536 steps of 12 head geometries, 1 to 64
-# sequences of 130 to 80,000 positions (the shortest down to a twentieth of the longest) in caches with room for 1 to 2.5
-# times the longest, every route timed on each: the choice is within 1.6 % of the best route on the whole, takes 0.63 times
-# as long as the dispatcher's launches, and at most 1.17 times (more than 1.05 in 8 of them).
-_PER_POSITION = {64: 0.0038, 128: 0.0065, 256: 0.0145}      # K and V of one KV head through one CTA, alone on its SM
-_TWO_RUNS = 1.34                                            # nine to sixteen query heads per KV head
-_LONGEST, _MEAN = 0.75, 0.5                                 # of a batch, as shares of the cache's capacity
-_ONE = 0.92                                                 # the same for one sequence
 CLUSTER_PARTS = (2, 3, 4, 5, 6, 8, 9, 12, 16)              # more than 8 only where the device has room for such clusters
 LEAN_SPLIT_MAX_CONTEXT = 131072
+APPEND_US = 2.0                                            # the append launch that the other routes have
+MARGIN = 0.95                                              # a route has to be estimated this much below the dispatcher's launches
 
 
-def _dispatcher_us(batch: int, cache_bytes: float, append: bool) -> float:
-    return (7.2 if batch == 1 else 12.7) + cache_bytes / 5.8e6 + (2.0 if append else 0.0)
-
-
-def _cluster_us(parts: int, pairs: int, resident: int, positions: float, per_position: float, num_sms: int, cache_bytes: float) -> float:
-    """`resident` clusters run at once, one wave after the other; CTAs that share an SM share its load rate.  The stream
-    of all of them and the stream of one CTA overlap (a smooth maximum)."""
-    waves = -(-pairs // resident)
-    one = per_position * max(1.0, min(pairs, resident) * parts / num_sms) * positions / parts * waves * (0.9 if waves > 1 else 1.0)
-    return 3.4 + 0.21 * math.log2(parts) + 3.5 * (waves - 1) + ((cache_bytes / 6.1e6) ** 3.4 + one ** 3.4) ** (1 / 3.4)
-
-
-def _split_us(parts: int, positions: float, head_dim: int, cache_bytes: float) -> float:
-    return 5.2 + 0.0125 * head_dim + max(cache_bytes / 12e6, 0.57 * _PER_POSITION[head_dim] * positions / parts)
+def cluster_options(hip, load, Hq: int, Hkv: int, D: int, batch: int, context: int, below: float):
+    """(estimated us, kind, parts, function, plan, clusters at once) of every cluster route estimated `below` that many
+    us.  `load(name)` loads a kernel; None where it is not to be had."""
+    for kind in (CLUSTER, HALF):
+        function = None
+        for parts in CLUSTER_PARTS:
+            plan = hip.lean_plan(Hq, Hkv, D, parts, context, kind)
+            if not plan.ok or hip.lean_estimate(kind, parts, Hq, Hkv, D, batch, context, batch * Hkv) >= below:
+                continue                                   # not even with room for all clusters at once
+            function = function or load(cluster_kernel_name(kind, Hq // Hkv, D))
+            if function is None:
+                break
+            resident = hip.max_active_clusters(function, parts, plan.threads, plan.smem_bytes)
+            us = hip.lean_estimate(kind, parts, Hq, Hkv, D, batch, context, resident)
+            if resident > 0 and us < below:
+                yield us, kind, parts, function, plan, resident
 
 
 def choose_lean_route(d, append: bool) -> tuple:
-    """(CTAs per (sequence, KV head), whether they are a cluster) for a dispatcher's geometry; (0, False): its own launches.
+    """(CTAs per (sequence, KV head), kind) for a dispatcher's geometry; (0, 0): its own launches.  The estimates and what
+    they are fitted to: csrc/kernels/lean_decode.cuh.
 
     Clusters win wherever latency counts: a layer is one dependent launch of 3.3 us instead of two or three (7.1).  They
-    lose to the dispatcher's equal shares where a batch streams for tens of microseconds, because a cluster's CTAs stay
+    lose to the dispatcher's equal shares where a batch streams for a hundred microseconds, because a cluster's CTAs stay
     with their sequence, and to split and combine for one long sequence, whose parts fill the GPU."""
     Hq, Hkv, D, batch, context = d.num_q_heads, d.num_kv_heads, d.head_dim, d.batch_size, d.context_length
-    if D not in _PER_POSITION or Hq % Hkv:
-        return 0, False
-    group, pairs, positions = Hq // Hkv, batch * Hkv, (_ONE if batch == 1 else _LONGEST) * context
-    cache_bytes = 4.0 * D * pairs * (_ONE if batch == 1 else _MEAN) * context
-    per_position = _PER_POSITION[D] * (_TWO_RUNS if group > 8 else 1.0)
-    best, route = 0.95 * _dispatcher_us(batch, cache_bytes, append), (0, False)
-    function = None
-    for parts in CLUSTER_PARTS:
-        plan = d.hip.lean_plan(Hq, Hkv, D, parts, context, True)
-        if not plan.ok or _cluster_us(parts, pairs, pairs, positions, per_position, 1 << 30, cache_bytes) >= best:
-            continue                                        # not even with an SM for every CTA
-        if function is None:
-            function = d.codegen.load_kernel_safe(d.hip, 'decode_attention', d.hip.get_gpu_architecture(), cluster_kernel_name(group, D))[1]
-        resident = d.hip.max_active_clusters(function, parts, plan.threads, plan.smem_bytes)
-        if resident < 1:
-            continue
-        us = _cluster_us(parts, pairs, resident, positions, per_position, d.num_sms, cache_bytes)
+    if Hkv <= 0 or Hq % Hkv or D not in (64, 128, 256):
+        return 0, 0
+    best, route = MARGIN * (d.hip.lean_estimate(-1, 0, Hq, Hkv, D, batch, context, 0) + (APPEND_US if append else 0.0)), (0, 0)
+    load = lambda name: d.codegen.load_kernel_safe(d.hip, 'decode_attention', d.hip.get_gpu_architecture(), name)[1]
+    for us, kind, parts, *_ in cluster_options(d.hip, load, Hq, Hkv, D, batch, context, best):
         if us < best:
-            best, route = us, (parts, True)
+            best, route = us, (parts, kind)
     parts = d.num_sms // Hkv
-    if (batch == 1 and context <= LEAN_SPLIT_MAX_CONTEXT and 1 < parts <= d.max_chunks and
-            d.hip.lean_plan(Hq, Hkv, D, parts, context, False).ok and _split_us(parts, positions, D, cache_bytes) < best):
-        route = parts, False
+    if (batch == 1 and context <= LEAN_SPLIT_MAX_CONTEXT and 1 < parts <= d.max_chunks and d.hip.lean_plan(Hq, Hkv, D, parts, context, SPLIT).ok
+            and d.hip.lean_estimate(SPLIT, parts, Hq, Hkv, D, 1, context, 0) < best):
+        route = parts, SPLIT
     return route
 
 
 UNSPLIT_MIN_CAPACITY = 256          # cache positions a sequence, by the stride; above them flash_attention_kernel goes to clusters
 
 
-def _unsplit_parts(hip, kernels: dict, name: str, Hq: int, Hkv: int, D: int, pairs: int, capacity: int):
-    """(parts, plan), or (0, None).  Sizes alone decide, so `kernels` remembers a thousand of them."""
+def _unsplit_option(hip, kernels: dict, Hq: int, Hkv: int, D: int, pairs: int, capacity: int):
+    """(us, parts, function, plan), parts 0 where no clusters hold all pairs at once.  Sizes alone decide, so `kernels`
+    remembers a thousand of them."""
     known = kernels.setdefault("parts", {})
     key = (Hq, Hkv, D, pairs, capacity)
     if key not in known:
         if len(known) >= 1024:
             known.clear()
-        best = (math.inf, 0, None)
-        for parts in CLUSTER_PARTS:
-            plan = hip.lean_plan(Hq, Hkv, D, parts, capacity, True)
-            if not plan.ok or hip.max_active_clusters(kernels[name], parts, plan.threads, plan.smem_bytes) < pairs:
-                continue
-            us = _cluster_us(parts, pairs, pairs, _LONGEST * capacity, _PER_POSITION[D], hip.get_num_cus(), 0.0)
-            if us < best[0]:
-                best = (us, parts, plan)
-        known[key] = best[1:]
+        options = cluster_options(hip, kernels.get, Hq, Hkv, D, pairs // Hkv, capacity, math.inf)
+        known[key] = min(((us, parts, function, plan) for us, _, parts, function, plan, resident in options if resident >= pairs),
+                         key=lambda o: o[0], default=(0.0, 0, None, None))
     return known[key]
 
 
@@ -174,17 +157,16 @@ def unsplit_as_clusters(hip, kernels: dict, args: list, grid, block):
     value = lambda a: a if isinstance(a, int) else getattr(a, "value", None) or 0
     q, k, v, k_cache, v_cache, out, _, Hq, Hkv, D, scale, offsets, stride = (value(a) for a in args)
     batch = int(grid[0])
-    if (D not in _PER_POSITION or Hkv <= 0 or Hq <= 0 or Hq % Hkv or stride <= 0 or stride % 8 or (q | k | v | k_cache | v_cache) % 16 or
+    if (D not in (64, 128, 256) or Hkv <= 0 or Hq <= 0 or Hq % Hkv or stride <= 0 or stride % 8 or (q | k | v | k_cache | v_cache) % 16 or
             tuple(int(x) for x in grid) != (batch, Hq, 1) or tuple(int(x) for x in block) != (D, 1, 1)):
         return None
     group, pairs, capacity = Hq // Hkv, batch * Hkv, stride // (Hkv * D)
-    name = cluster_kernel_name(group, D)
-    if name not in kernels or capacity <= UNSPLIT_MIN_CAPACITY * (2 if group > 8 else 1):
+    if capacity <= UNSPLIT_MIN_CAPACITY * (2 if group > 8 else 1):
         return None
-    parts, plan = _unsplit_parts(hip, kernels, name, Hq, Hkv, D, pairs, capacity)
+    _, parts, function, plan = _unsplit_option(hip, kernels, Hq, Hkv, D, pairs, capacity)
     if not parts:
         return None
     vp, ci, cf = ctypes.c_void_p, ctypes.c_int, ctypes.c_float
     lean = [vp(q), vp(k_cache), vp(v_cache), vp(0), vp(0), vp(0), ci(Hq), ci(Hkv), ci(D), cf(scale), vp(offsets), ci(stride), ci(parts),
             vp(k), vp(v), vp(out), ci(1), ci(FLAG_WAIT_FIRST), ci(plan.depth), vp(0), vp(0), vp(0), vp(0), vp(0), ci(-1), ci(0)]
-    return kernels[name], lean, ClusterGrid((pairs * parts, 1, 1), parts), (plan.threads, 1, 1), plan.smem_bytes
+    return function, lean, ClusterGrid((pairs * parts, 1, 1), parts), (plan.threads, 1, 1), plan.smem_bytes

@@ -14,6 +14,8 @@
 // position puts them, rotated if asked to, into the cache and into its block; no append launch.
 #pragma once
 
+#include <cmath>
+
 struct LeanArgs {
     const __half* q; __half* k_cache; __half* v_cache;
     float* partial_m; float* partial_l; float* partial_o;
@@ -27,16 +29,21 @@ struct LeanArgs {
 };
 
 __host__ __device__ constexpr int lean_warps(int D) { return D == 256 ? 6 : 8; }
+__host__ __device__ constexpr int lean_half_warps(int D) { return D == 256 ? 3 : 4; }  // two CTAs an SM with rings of full depth
 __host__ __device__ constexpr int lean_depth(int D) { return D == 256 ? 2 : 3; }      // most blocks a warp has in flight
+
+constexpr int kLeanSplit = 0, kLeanCluster = 1, kLeanHalf = 2;      // split and combine; clusters; clusters of CTAs of half the warps
 
 // What a launch of these kernels needs; `context` is the longest sequence.  A ring no deeper than its blocks need leaves
 // room on the SM for the CTAs of the launch behind.  ok = 0: a geometry the kernels do not cover.
 struct LeanPlan { int ok, threads, smem_bytes, depth; };
-__host__ __device__ inline LeanPlan make_lean_plan(int num_q_heads, int num_kv_heads, int head_dim, int n_parts, long long context, int cluster) {
+__host__ __device__ inline LeanPlan make_lean_plan(int num_q_heads, int num_kv_heads, int head_dim, int n_parts, long long context, int kind) {
+    const bool cluster = kind != kLeanSplit;
     LeanPlan p = {0, 0, 0, 0};
     if ((head_dim != 64 && head_dim != 128 && head_dim != 256) || num_kv_heads <= 0 || num_q_heads <= 0 ||
-        num_q_heads % num_kv_heads || n_parts < 1 || (cluster && (n_parts < 2 || n_parts > 16)) || context < 1) return p;
-    const int group = num_q_heads / num_kv_heads, runs = group > 8 ? 2 : 1, warps = lean_warps(head_dim), block = 64 * head_dim;
+        num_q_heads % num_kv_heads || n_parts < 1 || kind < kLeanSplit || kind > kLeanHalf || (kind == kLeanHalf && head_dim == 64) || (cluster && (n_parts < 2 || n_parts > 16)) || context < 1) return p;
+    const int group = num_q_heads / num_kv_heads, runs = group > 8 ? 2 : 1, block = 64 * head_dim;
+    const int warps = kind == kLeanHalf ? lean_half_warps(head_dim) : lean_warps(head_dim);
     if (group > 16 || (runs > 1 && (head_dim == 256 || !cluster))) return p;
     const long long blocks = (vteb::vteb_round_up((int)((context + n_parts - 1) / n_parts), vteb::kBlockPos) / vteb::kBlockPos + warps - 1) / warps;
     p.depth = blocks < lean_depth(head_dim) ? (int)blocks : lean_depth(head_dim);
@@ -47,6 +54,35 @@ __host__ __device__ inline LeanPlan make_lean_plan(int num_q_heads, int num_kv_h
     p.ok = 1;
     return p;
 }
+
+// Estimated microseconds of one layer, by which a route is chosen; `kind` -1: the append / split / combine launches
+// these kernels compete with (without the append, 2 us).  `resident`: clusters the device runs at once.  `context`: room in
+// the cache, of which a sequence is expected to use three quarters (a batch's mean: half).
+// The figures are fitted to 971 steps of 12 head geometries, 1 to 64 sequences of 130 to 80,000 positions (the shortest down to
+// a twentieth of the longest) in caches with room for 1 to 2.5 times the longest, 14 routes timed on each.  The choice
+// is within 3.5 % of the best route on the whole and takes 0.61 times as long as the launches of kind -1, at most 1.08
+// times (above 1.03 in 3 of them).
+//   per_position: K and V rows of one KV head through one CTA alone, us; CTAs of an SM share its rate, so a launch lasts as
+//   long as its longest part or as all positions spread over the SMs, whichever is longer, but no less than the
+//   bytes; a second wave starts when the first one's clusters end.
+inline double lean_estimate_us(int kind, int n_parts, int num_q_heads, int num_kv_heads, int head_dim, int batch, long long context,
+                               int resident, int num_sms) {
+    (void)num_q_heads;
+    const double pairs = (double)batch * num_kv_heads;
+    const double longest = (batch == 1 ? 0.765 : 0.72) * (double)context, mean = batch == 1 ? longest : 0.504 * (double)context;
+    const double bytes = pairs * mean * 4.0 * head_dim;
+    const double per_position = head_dim == 64 ? 0.0045 : head_dim == 128 ? 0.00706 : 0.0168;
+    if (kind < 0) return batch == 1 ? 9.0 + bytes / 8.2e6 : 12.0 + bytes / 5.5e6;
+    if (kind == kLeanSplit) {
+        const double stream = bytes / 8.0e6, walk = 0.62 * per_position * longest / n_parts;
+        return 4.8 + 0.0117 * head_dim + (stream > walk ? stream : walk);
+    }
+    const double waves = resident > 0 ? std::ceil(pairs / resident) : 1e9;
+    const double part = per_position * (kind == kLeanHalf ? 1.7 : 1.0) * longest / n_parts, spread = 0.96 * per_position * mean * pairs / num_sms;
+    const double walk = waves > 1.0 ? 0.84 * part + spread : part > spread ? part : spread;
+    return 3.5 + 0.2 * std::log2((double)n_parts) + 2.6 * (waves - 1.0) + std::pow(std::pow(bytes / 6.1e6, 4.0) + std::pow(walk, 4.0), 0.25);
+}
+constexpr double kLeanMargin = 0.95;       // a route has to be estimated this much below kind -1
 
 // Where a launch without a status word of its own (flash_attention_kernel's arguments have none) reports a wait that ran
 // out; read by vteb_module_check_status.
@@ -259,18 +295,18 @@ __device__ __forceinline__ void lean_softmax_pv(ConsumerStateT<D / 16> (&st)[NV]
     }
 }
 
-// D: head width; NV: runs of eight query heads a warp serves.
-template <int D, int NV, bool kFresh, bool kCluster>
+// D: head width; NV: runs of eight query heads a warp serves; CW: warps.
+template <int D, int NV, int CW, bool kFresh, bool kCluster>
 __device__ __forceinline__ void lean_body(const LeanArgs& a)
 {
-    constexpr int CW = lean_warps(D), P = lean_depth(D);
+    constexpr int P = lean_depth(D);
     constexpr int ROW = 2 * D, CPR = D / 8, BLK = 2 * 16 * ROW;      // bytes of a row, its 16-byte chunks, bytes of a block (K, then V)
     constexpr int PITCH = D + kMergePad;                             // floats of an exchange row: o[D], 4 unused, m, l, true maximum, 1 unused
     constexpr int THREADS = CW * 32;
     const int depth = a.depth;                                       // blocks a warp has in flight, at most P; the host sizes the ring for it
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    const uint32_t bar_q = smem_u32(smem_raw), bar_merge = bar_q + 8, bar_recv = bar_q + 16;
-    volatile int* abort_word = reinterpret_cast<volatile int*>(smem_raw + 24);
+    const uint32_t bar_recv = smem_u32(smem_raw);
+    volatile int* abort_word = reinterpret_cast<volatile int*>(smem_raw + 8);
     uint32_t* q_store = reinterpret_cast<uint32_t*>(smem_raw + kLeanCtrlBytes);              // Q as mma fragments: [run][chunk / 4][head, word][chunk % 4]
     unsigned char* ring = smem_raw + kLeanCtrlBytes + NV * CPR * 128;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -308,8 +344,6 @@ __device__ __forceinline__ void lean_body(const LeanArgs& a)
 
     const int units = group * (D / 32), my_units = kCluster && part < units ? (units - part + N - 1) / N : 0;
     if (threadIdx.x == 0) {
-        mbar_init(bar_q, CW);
-        mbar_init(bar_merge, CW);
         mbar_init(bar_recv, 1);
         *abort_word = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -409,8 +443,6 @@ __device__ __forceinline__ void lean_body(const LeanArgs& a)
         uint32_t* dst = q_store + ((h >> 3) * CPR + (q_chunk & ~3)) * 32 + (h & 7) * 16 + (q_chunk & 3);
         dst[0] = x.x; dst[4] = x.y; dst[8] = x.z; dst[12] = x.w;
     }
-    __syncwarp();
-    if (lane == 0) mbar_arrive(bar_q);
     if (my_late && a.k_new != nullptr) {
         if (rotate && lane < CPR && rope_touches(a.rope_type, a.rotary_dim, lane * 8))
             fresh[0] = rope_chunk(fresh[0], a.k_new + new_row, lane * 8, k_words, a.rope_type, a.rotary_dim, D);
@@ -420,11 +452,7 @@ __device__ __forceinline__ void lean_body(const LeanArgs& a)
             if (p < 2 * CPR) *reinterpret_cast<uint4*>((p < CPR ? a.k_cache : a.v_cache) + cache_row + c * 8) = fresh[i];
         }
     }
-    auto give_up = [&](int code) {                                   // a wait ran out: nobody leaves while another CTA may still send to it
-        raise_abort(abort_word, a.status, code);
-        if constexpr (kCluster) cluster_rejoin();
-    };
-    if (!mbar_wait_bounded(bar_q, 0, abort_word)) { give_up(kStatusMergeTimeout); return; }
+    __syncthreads();                                                 // Q is in place
 
     const int g = lane >> 2, t = lane & 3;
     const float scale2 = a.scale * kLog2e;
@@ -466,7 +494,7 @@ __device__ __forceinline__ void lean_body(const LeanArgs& a)
 
     // ---- the warps' states meet in shared memory: row h of warp w lies in warp w's own blocks' memory
     float* const mine = reinterpret_cast<float*>(ring + (size_t)warp * depth * BLK);
-    bool nan = false;
+    float probe[4] = {0.f, 0.f, 0.f, 0.f};                           // NaN if any sum is (and sometimes if some are infinite)
 #pragma unroll
     for (int v = 0; v < NV; ++v)
 #pragma unroll
@@ -479,19 +507,18 @@ __device__ __forceinline__ void lean_body(const LeanArgs& a)
                 for (int mt = 0; mt < D / 16; ++mt) {
                     dst[mt * 16 + g] = st[v].o[mt][h];
                     dst[mt * 16 + g + 8] = st[v].o[mt][2 + h];
-                    if constexpr (kFresh) nan |= (st[v].o[mt][h] != st[v].o[mt][h]) | (st[v].o[mt][2 + h] != st[v].o[mt][2 + h]);
+                    if constexpr (kFresh) { probe[2 * h] += st[v].o[mt][h]; probe[2 * h + 1] += st[v].o[mt][2 + h]; }
                 }
                 if (g == 0) { dst[D + 4] = st[v].m[h]; dst[D + 5] = l_head; dst[D + kMergeTrueMax] = m_head; }
             }
         }
     if constexpr (kFresh) {
-        if (__any_sync(0xffffffffu, nan) && !rotate)
+        const float all = (probe[0] + probe[1]) + (probe[2] + probe[3]);
+        if (__any_sync(0xffffffffu, all != all) && !rotate)
             redo_rows_fp32<D>(mine, group, PITCH, a.q + ((long long)b * a.num_q_heads + (long long)kv_head * group) * D, a.k_cache + base,
                               a.v_cache + base, pos_stride, start + warp * kBlockPos, end, CW * kBlockPos, scale2);
     }
-    __syncwarp();
-    if (lane == 0) mbar_arrive(bar_merge);
-    if (!mbar_wait_bounded(bar_merge, 0, abort_word)) { give_up(kStatusMergeTimeout); return; }
+    __syncthreads();
 
     const long long head0 = (long long)b * a.num_q_heads + (long long)kv_head * group;
     for (int idx = threadIdx.x; idx < group * (D / 4); idx += THREADS) {
@@ -526,21 +553,27 @@ __device__ __forceinline__ void lean_body(const LeanArgs& a)
     }
     if constexpr (kCluster) {
         if (my_units == 0) return;
-        if (!mbar_wait_bounded(bar_recv, 0, abort_word)) { give_up(kStatusGridTimeout); return; }
+        if (!mbar_wait_bounded(bar_recv, 0, abort_word)) {           // nobody leaves while another CTA may still send to it
+            raise_abort(abort_word, a.status, kStatusGridTimeout);
+            cluster_rejoin();
+            return;
+        }
         for (int slot = warp; slot < my_units; slot += CW) {
             const float* src = recv + slot * N * kLeanUnit;
-            const float m = lane < N ? src[lane * kLeanUnit + 32] : kNeutralM, l = lane < N ? src[lane * kLeanUnit + 33] : 0.f;
-            float top = m;
+            // every lane takes all the weights itself: broadcast reads instead of shuffles
+            float m[16], top = kNeutralM, sum = 0.f, acc = 0.f;
 #pragma unroll
-            for (int off = 8; off > 0; off >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, off));
-            const float wt = fast_exp2(m - top);                     // lanes 16 .. 31 hold nothing and are not read
-            float sum = l * wt;
+            for (int k = 0; k < 16; ++k) {
+                m[k] = k < N ? src[k * kLeanUnit + 32] : kNeutralM;
+                top = fmaxf(top, m[k]);
+            }
 #pragma unroll
-            for (int off = 8; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
-            sum = __shfl_sync(0xffffffffu, sum, 0);
-            float acc = 0.f;
-#pragma unroll 8
-            for (int k = 0; k < N; ++k) acc = fmaf(src[k * kLeanUnit + lane], __shfl_sync(0xffffffffu, wt, k), acc);
+            for (int k = 0; k < 16; ++k)
+                if (k < N) {
+                    const float wt = fast_exp2(m[k] - top);
+                    sum = fmaf(src[k * kLeanUnit + 33], wt, sum);
+                    acc = fmaf(src[k * kLeanUnit + lane], wt, acc);
+                }
             const int unit = slot * N + part, h = unit / (D / 32);
             const long long at = (head0 + h) * D + (unit - h * (D / 32)) * 32 + lane;
             const float v = acc / fmaxf(sum, 1e-20f);
@@ -550,7 +583,7 @@ __device__ __forceinline__ void lean_body(const LeanArgs& a)
     }
 }
 
-#define VTEB_LEAN_KERNEL(NAME, DIM, NV, FRESH, CLUSTER, BOUNDS)                                                         \
+#define VTEB_LEAN_KERNEL(NAME, DIM, NV, WARPS, FRESH, CLUSTER, BOUNDS)                                                  \
     extern "C" __global__ void BOUNDS NAME(                                                                             \
         const __half* __restrict__ q, __half* k_cache, __half* v_cache, float* __restrict__ partial_m,                  \
         float* __restrict__ partial_l, float* __restrict__ partial_o, int num_q_heads, int num_kv_heads, int head_dim,  \
@@ -567,17 +600,20 @@ __device__ __forceinline__ void lean_body(const LeanArgs& a)
         a.num_q_heads = num_q_heads; a.num_kv_heads = num_kv_heads; a.scale = scale;                                    \
         a.kv_offsets = kv_cache_offset_ptr; a.kv_batch_stride = kv_batch_stride; a.n_parts = n_parts;                   \
         a.k_new = k_new; a.v_new = v_new; a.output = output; a.out_kind = out_kind; a.flags = flags; a.status = status ? status : &vteb_lean_status; \
-        a.depth = depth;                                                                                                \
+        a.depth = depth;                                                                                                    \
         a.next_k_cache = next_k_cache; a.next_v_cache = next_v_cache;                                                   \
         a.rope_cos = cos_cache; a.rope_sin = sin_cache; a.rope_type = rope_type; a.rotary_dim = rotary_dim;             \
-        lean_body<DIM, NV, FRESH, CLUSTER>(a);                                                                          \
+        lean_body<DIM, NV, WARPS, FRESH, CLUSTER>(a);                                                                   \
     }
 
-VTEB_LEAN_KERNEL(vteb_decode_cluster_d64_kernel, 64, 1, true, true, __launch_bounds__(256, 2))
-VTEB_LEAN_KERNEL(vteb_decode_cluster_d128_kernel, 128, 1, true, true, __launch_bounds__(256, 2))
-VTEB_LEAN_KERNEL(vteb_decode_cluster_d256_kernel, 256, 1, true, true, __launch_bounds__(192, 1))
-VTEB_LEAN_KERNEL(vteb_decode_cluster_2_d64_kernel, 64, 2, true, true, __launch_bounds__(256, 2))
-VTEB_LEAN_KERNEL(vteb_decode_cluster_2_d128_kernel, 128, 2, true, true, __launch_bounds__(256, 1))
-VTEB_LEAN_KERNEL(vteb_split_kv_lean_d64_kernel, 64, 1, false, false, __maxnreg__(160))
-VTEB_LEAN_KERNEL(vteb_split_kv_lean_d128_kernel, 128, 1, false, false, __maxnreg__(160))
-VTEB_LEAN_KERNEL(vteb_split_kv_lean_d256_kernel, 256, 1, true, false, __maxnreg__(168))
+VTEB_LEAN_KERNEL(vteb_decode_cluster_d64_kernel, 64, 1, lean_warps(64), true, true, __launch_bounds__(256, 2))
+VTEB_LEAN_KERNEL(vteb_decode_cluster_d128_kernel, 128, 1, lean_warps(128), true, true, __launch_bounds__(256, 2))
+VTEB_LEAN_KERNEL(vteb_decode_cluster_d256_kernel, 256, 1, lean_warps(256), true, true, __launch_bounds__(192, 1))
+VTEB_LEAN_KERNEL(vteb_decode_cluster_2_d64_kernel, 64, 2, lean_warps(64), true, true, __launch_bounds__(256, 2))
+VTEB_LEAN_KERNEL(vteb_decode_cluster_2_d128_kernel, 128, 2, lean_warps(128), true, true, __launch_bounds__(256, 1))
+VTEB_LEAN_KERNEL(vteb_decode_cluster_half_d128_kernel, 128, 1, lean_half_warps(128), true, true, __launch_bounds__(128, 2))
+VTEB_LEAN_KERNEL(vteb_decode_cluster_half_d256_kernel, 256, 1, lean_half_warps(256), true, true, __launch_bounds__(96, 2))
+VTEB_LEAN_KERNEL(vteb_decode_cluster_half_2_d128_kernel, 128, 2, lean_half_warps(128), true, true, __launch_bounds__(128, 2))
+VTEB_LEAN_KERNEL(vteb_split_kv_lean_d64_kernel, 64, 1, lean_warps(64), false, false, __maxnreg__(160))
+VTEB_LEAN_KERNEL(vteb_split_kv_lean_d128_kernel, 128, 1, lean_warps(128), false, false, __maxnreg__(160))
+VTEB_LEAN_KERNEL(vteb_split_kv_lean_d256_kernel, 256, 1, lean_warps(256), true, false, __maxnreg__(168))

@@ -640,6 +640,7 @@ def run_ours(args, rank, world, local_rank):
                                    "programmatic_dependent_launch": not args.no_pdl,
                                    "kv_tile_copies": "tensor-map (TMA) boxes for whole tiles, 16-byte cp.async for ragged ends" if ex.dispatcher.tensor_maps else "16-byte cp.async",
                                    "next_layer_l2_prefetch": not args.no_prefetch and cfg.batch == 1,
+                                   "route": "%s, %d CTAs per (sequence, KV head)" % ex.route_name if ex.route_name else "the dispatcher's launches",
                                    "combine": "inside the split launch (grid barrier)" if ex.dispatcher.fused_combine else "separate launch", "kernels": "compat" if args.compat else ("fast, compact CTAs" if ex.dispatcher.compact else "fast, full CTAs"),
                                    "step_contents": {"off": "split + combine per layer",
                                                      "separate": "rotation launch + cache append + split + combine per layer",
@@ -709,19 +710,24 @@ def kernel_durations(rt, ex, n_layers, reps=20):
     on the launching stream: duration = elapsed / (replays * layers), which
     includes the in-graph launch gap between consecutive kernels."""
     disp = ex.dispatcher
-    name = "flash_attention_split_kv_partial_kernel" if disp.compat else disp.split_kernel_name
+    name = (ex.route_name[0] if ex.route_name else "flash_attention_split_kv_partial_kernel" if disp.compat
+            else disp.split_kernel_name)
     out = {}
-    kinds = ((0, "split_us"),) if disp.fused_combine else ((0, "split_us"), (1, "combine_us"))
+    one_launch = len(ex.layer_launches(0)) == 1 if ex.route_name else disp.fused_combine
+    kinds = ((0, "split_us"),) if one_launch else ((0, "split_us"), (1, "combine_us"))
     out["combine_us"] = 0.0
     for which, key in kinds:
         rt.stream_begin_capture()
         try:
             for l in range(n_layers):
-                launches = disp.build_launches(l, ex.tensor_mapping, ex.offsets.ptr, batch=ex.B)
-                if not disp.fuse_append:
-                    launches = launches[1:]                     # drop the append launch
+                if ex.route_name:
+                    launches = ex.layer_launches(l)
+                else:
+                    launches = disp.build_launches(l, ex.tensor_mapping, ex.offsets.ptr, batch=ex.B)
+                    if not disp.fuse_append:
+                        launches = launches[1:]                 # drop the append launch
                 fn, args, grid, block, smem = launches[which]
-                if (which == 0 and not disp.compat and not disp.fused_combine
+                if (which == 0 and not ex.route_name and not disp.compat and not disp.fused_combine
                         and ex.B * disp._plan.n_hgroups * disp.max_chunks > grid[0]):
                     # more items than CTAs: the work-queue ticket, normally cleared by the
                     # combine launch, has to start from zero

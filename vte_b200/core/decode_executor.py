@@ -210,19 +210,25 @@ class DecodeAttentionExecutor:
         finally:
             self.hip.programmatic_launch = programmatic
 
+    def layer_launches(self, layer: int):
+        """What a step launches for a layer (without a rotation launch of its own)."""
+        if self._route is not None and self.dispatcher.offsets_final:
+            return self._route.launches(layer, self.tensor_mapping, self.offsets.ptr, self.B)
+        launches = self.dispatcher.build_launches(layer, self.tensor_mapping, self.offsets.ptr, batch=self.B)
+        return launches if self.with_append or self.dispatcher.fuse_append else launches[1:]
+
+    @property
+    def route_name(self):
+        """(kernel, CTAs per (sequence, KV head)) where a captured step does not take the dispatcher's launches, else None."""
+        return (self._route.name, self._route.parts) if self._route is not None else None
+
     def _record_all(self, after_copy: bool = False):
         n = 0
         programmatic = self.hip.programmatic_launch
         # within a captured step of nothing but the layers' own launches, offsets and older rows do not change
         self.dispatcher.offsets_final = self.use_graph and self.per_layer_hook is None and self.launch_rewriter is None
-        route = self._route if self.dispatcher.offsets_final else None
         for l in range(self.L):
-            if route is not None:
-                launches = route.launches(l, self.tensor_mapping, self.offsets.ptr, self.B)
-            else:
-                launches = self.dispatcher.build_launches(l, self.tensor_mapping, self.offsets.ptr, batch=self.B)
-                if not self.with_append and not self.dispatcher.fuse_append:
-                    launches = launches[1:]
+            launches = self.layer_launches(l)
             if self.launch_rewriter is not None:
                 launches = self.launch_rewriter(l, launches)
             if self.rope == "separate":

@@ -35,10 +35,10 @@ class LeanRoute:
         if not self.plan.ok:
             raise CudaSafetyError(f"{self.parts} CTAs per (sequence, KV head) are not covered for this geometry")
         load = lambda symbol: d.codegen.load_kernel_safe(d.hip, 'decode_attention', d.hip.get_gpu_architecture(), symbol)[1]
-        if self.cluster:
-            self.function = load(cluster_kernel_name(kind, d.num_q_heads // d.num_kv_heads, d.head_dim))
-        else:
-            self.function = load(f"vteb_split_kv_lean_d{d.head_dim}_kernel")
+        self.name = (cluster_kernel_name(kind, d.num_q_heads // d.num_kv_heads, d.head_dim) if self.cluster
+                     else f"vteb_split_kv_lean_d{d.head_dim}_kernel")
+        self.function = load(self.name)
+        if not self.cluster:
             self.combine = load('vteb_split_kv_combine_small_kernel' if self.parts <= 32 else
                                 'vteb_split_kv_combine_f32_kernel' if d.output_f32 else 'vteb_split_kv_combine_f16_kernel')
 

@@ -535,7 +535,8 @@ extern "C" __global__ void __launch_bounds__(256, 4) vteb_split_kv_partial_compa
 // (head_dim, 1, 1) (dynamic shared memory is accepted and not used).  It is what the reference's
 // batched executor records (vte/core/batched_hip_graph_executor.py:231-247): append this step's
 // K/V rows at position kv_offset, attend to positions 0..kv_offset, store the normalised fp16
-// output.  `seq_len` must be 1, as in the reference.  One block serves one query head, so K and V
+// output.  `seq_len` must be 1, as in the reference.  CudaRuntime serves launches with room for more than 256
+// positions by clusters instead (core/lean_route.py).  One block serves one query head, so K and V
 // are read once per query head (through L2); the dispatcher's own one-launch path for short
 // contexts is the split kernel with one split, which reads them once per KV head.
 // ---------------------------------------------------------------------------

@@ -10,6 +10,16 @@
 //   split (`vteb_split_kv_lean_...`): each CTA stores its state to partial_m / partial_l / partial_o for a combine
 //     launch, as the persistent split kernel does.
 //
+// What bounds them, us: a cluster layer of one sequence of 1,531 positions (12 heads on 2 KV heads of 128) takes 3.3 (7.1
+// with append, split and combine): 1.5 between the end of one launch and the end of the next one's wait, 0.4 block
+// arithmetic, 0.5 the warps' exchange, 0.6 merge and send, 0.4 last merge and store.  A CTA alone streams about 72 B/ns, two
+// warps a scheduler (568 instructions a block before the copies' addresses and Q's words were simplified: 24.8 -> 23.0 for 6,000
+// positions on two CTAs); with every SM busy HBM bounds them: 64 (sequence, KV head) pairs of 6,000 positions 33, 6.5 TB/s
+// while streaming.  A lean split layer takes 4.6 plus its bytes at 6.6 TB/s: 6.3 for 11,003 positions (8.5), 9.6 for 32,768 (9.9).
+// Rings are as deep as the longest part needs, three blocks a warp (two of 256-wide heads) at most: 192 KB in flight an SM.
+// Half blocks (four or three warps, two CTAs an SM) serve more pairs than whole-SM clusters fit at once: 40 sequences of 8
+// heads 42.4 -> 35.8, 37 of 300 positions 24.3 -> 15.4, 32 sequences of 28 heads on 4 27.3 -> 26.6.
+//
 // Either way this step's K and V rows may be handed over (`k_new`, `v_new`): the warp whose block ends with the newest
 // position puts them, rotated if asked to, into the cache and into its block; no append launch.
 #pragma once

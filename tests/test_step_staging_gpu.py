@@ -31,3 +31,29 @@ def test_staging_by_launch_and_by_copy_node_give_the_same_step(cuda_runtime, cod
         assert np.array_equal(by_launch, by_node)
         for l in range(L):
             assert np.max(np.abs(by_launch[l] - orc.decode_attention(q[l], k, v, off))) <= 1e-5
+
+
+def test_queued_steps_keep_their_own_offsets(cuda_runtime, codegen):
+    """More steps in flight than there are staging slots, each appending at its own position: every row is written."""
+    from vte_b200.core import decode_executor as de
+    n, S = 2 * de.OFFSET_SLOTS + 5, 256
+    ex = de.DecodeAttentionExecutor(cuda_runtime, codegen, {"attention.head_count": 12, "attention.head_count_kv": 2,
+                                                            "attention.key_length": 128}, 2, S, 3, n_kv_buffers=1, with_append=True)
+    try:
+        rng = np.random.default_rng(0)
+        new = [rng.standard_normal((2, 2, 128), dtype=np.float32).astype(np.float16) for _ in range(2)]
+        zero = np.zeros((2, S, 2, 128), np.float16)
+        ex.upload_cache(0, zero, zero)
+        for l in range(3):
+            ex.upload_layer(l, np.zeros((2, 12, 128), np.float16))
+            ex.upload_new_kv(l, *new)
+        for i in range(n):
+            ex.execute_decode_batch(np.array([i, S - 1 - i], dtype=np.int32), read_output=False)
+        cuda_runtime.stream_synchronize()
+        k, v = ex.download_cache_rows(0, 0, S)
+        assert np.array_equal(k[:n], np.broadcast_to(new[0][0], (n, 2, 128))) and not k[n:].any()
+        k, v = ex.download_cache_rows(0, 1, S)
+        assert np.array_equal(v[S - n:], np.broadcast_to(new[1][1], (n, 2, 128))) and not v[:S - n].any()
+        ex.dispatcher_check()
+    finally:
+        ex.cleanup()

@@ -9,7 +9,8 @@ import pytest
 from oracle import attention_oracle as orc
 from vte_b200.bridge.cuda_runtime import LeanPlan, load_library
 from vte_b200.core.decode_executor import DecodeAttentionExecutor
-from vte_b200.core.lean_route import CLUSTER_PARTS, LEAN_SPLIT_MAX_CONTEXT, choose_lean_route
+from vte_b200.bridge.errors import CudaSafetyError
+from vte_b200.core.lean_route import CLUSTER_PARTS, LEAN_SPLIT_MAX_CONTEXT, LeanRoute, choose_lean_route
 
 
 def lean_plan(*a):
@@ -57,7 +58,7 @@ class FakeDispatcher:
     def __init__(self, heads, batch, context):
         self.num_q_heads, self.num_kv_heads, self.head_dim = heads
         self.batch_size, self.context_length, self.num_sms, self.max_chunks = batch, context, 148, 148
-        self.hip, self.codegen = FakeHip, self
+        self.hip, self.codegen, self.output_f32 = FakeHip, self, True
 
     def load_kernel_safe(self, *a):
         return None, ctypes.c_void_p(1)
@@ -78,6 +79,16 @@ def test_the_route_follows_the_size(built_library):
         for context in (1, 130, 1000, 9000, 70000):
             parts, kind = route((28, 4, 128), batch, context)
             assert parts == 0 or (parts in CLUSTER_PARTS if kind else batch == 1 and parts == 37)
+
+
+def test_a_forced_split_route_stays_within_the_partial_buffers(built_library):
+    """Each (sequence, query head) has room for max_chunks partials: one sequence of up to 2,048 positions for 32."""
+    d = FakeDispatcher((12, 2, 128), 1, 2048)
+    d.max_chunks = 32
+    assert LeanRoute(d, 32, 0, False).parts == 32 and LeanRoute(d, 16, 1, False).parts == 16
+    for parts in (33, 37, 148):
+        with pytest.raises(CudaSafetyError, match="room for 32"):
+            LeanRoute(d, parts, 0, False)
 
 
 def test_the_unsplit_kernel_goes_to_clusters_where_they_pay(built_library):

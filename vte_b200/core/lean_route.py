@@ -34,6 +34,8 @@ class LeanRoute:
         self.plan = d.hip.lean_plan(d.num_q_heads, d.num_kv_heads, d.head_dim, self.parts, d.context_length, kind)
         if not self.plan.ok:
             raise CudaSafetyError(f"{self.parts} CTAs per (sequence, KV head) are not covered for this geometry")
+        if not self.cluster and self.parts > d.max_chunks:      # the partial buffers hold max_chunks a row
+            raise CudaSafetyError(f"{self.parts} splits, the partial buffers have room for {d.max_chunks}")
         load = lambda symbol: d.codegen.load_kernel_safe(d.hip, 'decode_attention', d.hip.get_gpu_architecture(), symbol)[1]
         self.name = (cluster_kernel_name(kind, d.num_q_heads // d.num_kv_heads, d.head_dim) if self.cluster
                      else f"vteb_split_kv_lean_d{d.head_dim}_kernel")

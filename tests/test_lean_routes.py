@@ -91,6 +91,12 @@ def test_a_forced_split_route_stays_within_the_partial_buffers(built_library):
             LeanRoute(d, parts, 0, False)
 
 
+@pytest.mark.parametrize("option", ["compat", "strict_empty_splits", "emit_state", "fused_combine"])
+def test_a_forced_route_refuses_what_it_would_drop(option):
+    with pytest.raises(CudaSafetyError, match="lean_route"):
+        DecodeAttentionExecutor(None, None, {}, 1, 256, 1, lean=(4, 1), **{option: True})
+
+
 def test_the_unsplit_kernel_goes_to_clusters_where_they_pay(built_library):
     """Which launches of flash_attention_kernel do, and with which arguments; all others keep their own builds."""
     from vte_b200.compiler.signatures import CLUSTER_KERNELS, KERNEL_SIGNATURES

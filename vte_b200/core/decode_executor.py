@@ -53,6 +53,8 @@ class DecodeAttentionExecutor:
                  rope_theta: float = 1e6, tensor_maps: bool = True, fuse_append: bool = False,
                  balanced: Optional[bool] = None, wide: Optional[bool] = None, lean: Optional[tuple] = None):
         self.hip = hip
+        if lean is not None and lean[0] and (compat or strict_empty_splits or emit_state or fused_combine):
+            raise CudaSafetyError("a route of lean_route.py has no compat kernels, empty-split partials, shard states or fused combine")
         # rope: "off" = Q and K arrive rotated; "separate" = the reference's standalone rotation
         # launch runs before the append (rotating the projections in place); "fused" = the append
         # rotates K and the split kernel rotates Q.  Either way the step includes the append.

@@ -91,6 +91,33 @@ def test_a_forced_split_route_stays_within_the_partial_buffers(built_library):
             LeanRoute(d, parts, 0, False)
 
 
+def real_dispatcher(**kw):
+    from tests import test_host_logic as host
+    d = host.make_dispatcher(**{"context_length": 4096, "batch_size": 1, **kw})[0]
+    d.hip.lean_plan, d.hip.programmatic_launch = lean_plan, False
+    d._allocate_scratch()
+    return d, {**host.mapping(stride=4096 * 256), "rope_cos": 0x7300_0000_0000, "rope_sin": 0x7300_0010_0000}
+
+
+@pytest.mark.parametrize("kind", [0, 1])
+def test_a_route_checks_the_rows_to_append(built_library, kind):
+    """Null new rows would mean to the kernel that the row is in the cache already; rows that 16-byte loads cannot read
+    go through an append launch where the step has one, and are refused where the caller left it out."""
+    d, m = real_dispatcher()
+    names = [fn_args[1] for fn_args in LeanRoute(d, 16, kind, True).launches(0, m, 0x7200_0000_0000, 1)[:1]]
+    assert [a.value for a in names[0][13:15]] == [m['blk.0.k_proj.output'], m['blk.0.v_proj.output']]
+    for name in ('blk.0.k_proj.output', 'blk.0.v_proj.output'):
+        with pytest.raises(CudaSafetyError, match="null"):
+            LeanRoute(d, 16, kind, True).launches(0, {k: v for k, v in m.items() if k != name}, 0x7200_0000_0000, 1)
+        odd = {**m, name: m[name] + 2}
+        got = LeanRoute(d, 16, kind, True).launches(0, odd, 0x7200_0000_0000, 1)
+        assert [x[2:] for x in got] == [x[2:] for x in d.build_launches(0, odd, 0x7200_0000_0000, 1)] and len(got) == 3
+        assert m[name] + 2 in [a.value for a in got[0][1][:2]]
+        folded, _ = real_dispatcher(fuse_append=True)
+        with pytest.raises(CudaSafetyError, match="16-byte aligned"):
+            LeanRoute(folded, 16, kind, True).launches(0, odd, 0x7200_0000_0000, 1)
+
+
 @pytest.mark.parametrize("option", ["compat", "strict_empty_splits", "emit_state", "fused_combine"])
 def test_a_forced_route_refuses_what_it_would_drop(option):
     with pytest.raises(CudaSafetyError, match="lean_route"):

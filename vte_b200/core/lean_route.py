@@ -54,7 +54,13 @@ class LeanRoute:
         k_cache, v_cache = d._resolve_kv_cache_ptrs(layer, tensor_mapping)
         stride = int(tensor_mapping.get('kv_batch_stride_elements', 0))
         d._validate(batch, q, k_cache, v_cache, out, kv_offset_ptr, stride)
-        k_new, v_new = (ptr(f'blk.{layer}.k_proj.output'), ptr(f'blk.{layer}.v_proj.output')) if self.append else (0, 0)
+        k_new = v_new = 0
+        if self.append:
+            k_new, v_new = ptr(f'blk.{layer}.k_proj.output'), ptr(f'blk.{layer}.v_proj.output')
+            if not k_new or not v_new:                     # null means to the kernels that the row is in the cache already
+                raise CudaSafetyError(f"layer {layer}: the new K / V rows could not be resolved (null)")
+            if (k_new | v_new) % 16:                       # 16-byte loads; an append launch takes rows of any alignment
+                return d.build_launches(layer, tensor_mapping, kv_offset_ptr, batch)
         flags = (0 if self.append else FLAG_ROWS_FINAL) | (FLAG_PREFETCH_Q if d.hip.programmatic_launch else 0)
         rope = [vp(0), vp(0), ci(-1), ci(0)]
         if d.fuse_rope:

@@ -118,6 +118,17 @@ def test_a_route_checks_the_rows_to_append(built_library, kind):
             LeanRoute(folded, 16, kind, True).launches(0, odd, 0x7200_0000_0000, 1)
 
 
+@pytest.mark.parametrize("kind", [0, 1])
+def test_a_route_checks_the_rotation_s_tables(built_library, kind):
+    d, m = real_dispatcher(fuse_rope=True)
+    args = LeanRoute(d, 16, kind, True).launches(0, m, 0x7200_0000_0000, 1)[0][1]
+    assert [a.value for a in args[22:24]] == [m['rope_cos'], m['rope_sin']]
+    for name in ('rope_cos', 'rope_sin'):
+        for bad in ({k: v for k, v in m.items() if k != name}, {**m, name: m[name] + 2}):
+            with pytest.raises(CudaSafetyError, match="rope_cos / rope_sin"):
+                LeanRoute(d, 16, kind, True).launches(0, bad, 0x7200_0000_0000, 1)
+
+
 @pytest.mark.parametrize("option", ["compat", "strict_empty_splits", "emit_state", "fused_combine"])
 def test_a_forced_route_refuses_what_it_would_drop(option):
     with pytest.raises(CudaSafetyError, match="lean_route"):

@@ -62,9 +62,7 @@ class LeanRoute:
             if (k_new | v_new) % 16:                       # 16-byte loads; an append launch takes rows of any alignment
                 return d.build_launches(layer, tensor_mapping, kv_offset_ptr, batch)
         flags = (0 if self.append else FLAG_ROWS_FINAL) | (FLAG_PREFETCH_Q if d.hip.programmatic_launch else 0)
-        rope = [vp(0), vp(0), ci(-1), ci(0)]
-        if d.fuse_rope:
-            rope = [vp(ptr('rope_cos')), vp(ptr('rope_sin')), ci(d.rope_type), ci(d.rotary_dim)]
+        rope = d._rope_arguments(tensor_mapping) if d.fuse_rope else [vp(0), vp(0), ci(-1), ci(0)]
         Hq, Hkv, D, N = d.num_q_heads, d.num_kv_heads, d.head_dim, self.parts
         out_kind = 2 if d.output_f32 else 1
         next_k = next_v = 0

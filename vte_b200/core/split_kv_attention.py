@@ -486,6 +486,13 @@ class SplitKVAttentionDispatcher:
         return self._tensor_map_cache[key]
 
     # -- launches -----------------------------------------------------------------
+    def _rope_arguments(self, tensor_mapping: dict) -> list:
+        """Tables, type and width of the rotation, as the rotating kernels take them."""
+        cos_ptr, sin_ptr = (self._resolve_ptr(tensor_mapping, name) for name in ('rope_cos', 'rope_sin'))
+        if not cos_ptr or not sin_ptr or cos_ptr % 4 or sin_ptr % 4:
+            raise CudaSafetyError("fuse_rope: rope_cos / rope_sin missing from the tensor mapping or misaligned")
+        return [ctypes.c_void_p(cos_ptr), ctypes.c_void_p(sin_ptr), ctypes.c_int(self.rope_type), ctypes.c_int(self.rotary_dim)]
+
     def _validate(self, batch, q_ptr, k_cache_ptr, v_cache_ptr, output_ptr, kv_offset_ptr, kv_batch_stride):
         if batch <= 0 or batch > self.batch_size:
             raise CudaSafetyError(f"batch {batch} outside 1..{self.batch_size} (scratch is sized for batch_size)")
@@ -530,13 +537,7 @@ class SplitKVAttentionDispatcher:
         vp, ci, cf = ctypes.c_void_p, ctypes.c_int, ctypes.c_float
         append_args = [vp(k_proj_ptr), vp(v_proj_ptr), vp(k_cache_ptr), vp(v_cache_ptr),
                        ci(Hkv), ci(D), vp(kv_offset_ptr), ci(kv_batch_stride)]
-        rope_tail = []
-        if self.fuse_rope:
-            cos_ptr = self._resolve_ptr(tensor_mapping, 'rope_cos')
-            sin_ptr = self._resolve_ptr(tensor_mapping, 'rope_sin')
-            if not cos_ptr or not sin_ptr or cos_ptr % 4 or sin_ptr % 4:
-                raise CudaSafetyError("fuse_rope: rope_cos / rope_sin missing from the tensor mapping or misaligned")
-            rope_tail = [vp(cos_ptr), vp(sin_ptr), ci(self.rope_type), ci(self.rotary_dim)]
+        rope_tail = self._rope_arguments(tensor_mapping) if self.fuse_rope else []
         append = (append_fn, append_args + rope_tail, (batch, Hkv, 1), (D, 1, 1), 0)
         split_tail = list(rope_tail)
         if self.fuse_rope or self.fuse_append:

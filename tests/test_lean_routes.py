@@ -129,6 +129,18 @@ def test_a_route_checks_the_rotation_s_tables(built_library, kind):
                 LeanRoute(d, 16, kind, True).launches(0, bad, 0x7200_0000_0000, 1)
 
 
+def test_a_route_looks_no_further_than_a_pool_for_the_next_layer_s_rows(built_library):
+    """The L2 prefetch reads the next layer's caches by name only (a pool's last layer has none behind it), at 16 bytes."""
+    d, m = real_dispatcher()
+    ahead = lambda m: [a.value or 0 for a in LeanRoute(d, 16, 0, True).launches(0, m, 0x7200_0000_0000, 1)[0][1][20:22]]
+    next_k, next_v = 0x7400_0000_0000, 0x7500_0000_0000
+    assert ahead({**m, 'blk.1.kv_cache.k': next_k, 'blk.1.kv_cache.v': next_v}) == [next_k, next_v]
+    pooled = {k: v for k, v in m.items() if 'kv_cache' not in k}
+    for without in ({**pooled, 'KV Cache Pool': 0x7600_0000_0000}, {**m, 'blk.1.kv_cache.k': next_k},
+                    {**m, 'blk.1.kv_cache.k': next_k, 'blk.1.kv_cache.v': next_v + 8}):
+        assert ahead(without) == [0, 0]
+
+
 @pytest.mark.parametrize("option", ["compat", "strict_empty_splits", "emit_state", "fused_combine"])
 def test_a_forced_route_refuses_what_it_would_drop(option):
     with pytest.raises(CudaSafetyError, match="lean_route"):

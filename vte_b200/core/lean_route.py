@@ -69,10 +69,10 @@ class LeanRoute:
         partials = [vp(0), vp(0), vp(0)]
         if not self.cluster:
             partials = [vp(p.ptr) for p in d.partial_buffers]
-            next_k, next_v = d._resolve_kv_cache_ptrs(layer + 1, tensor_mapping)
+            next_k, next_v = d._next_caches(layer, tensor_mapping)
         args = [vp(q), vp(k_cache), vp(v_cache), *partials, ci(Hq), ci(Hkv), ci(D), cf(scale), vp(kv_offset_ptr), ci(stride),
                 ci(N), vp(k_new), vp(v_new), vp(out), ci(out_kind), ci(flags), ci(self.plan.depth), vp(d.work_ptr + 4),
-                vp(next_k if next_v else 0), vp(next_v if next_k else 0)] + rope
+                vp(next_k), vp(next_v)] + rope
         dims = (batch * Hkv * N, 1, 1)
         split = (self.function, args, ClusterGrid(dims, N) if self.cluster else dims, (self.plan.threads, 1, 1), self.plan.smem_bytes)
         if self.cluster:

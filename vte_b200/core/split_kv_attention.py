@@ -493,6 +493,13 @@ class SplitKVAttentionDispatcher:
             raise CudaSafetyError("fuse_rope: rope_cos / rope_sin missing from the tensor mapping or misaligned")
         return [ctypes.c_void_p(cos_ptr), ctypes.c_void_p(sin_ptr), ctypes.c_int(self.rope_type), ctypes.c_int(self.rotary_dim)]
 
+    def _next_caches(self, layer_idx: int, tensor_mapping: dict):
+        """The next layer's caches for the L2 prefetch, (0, 0) where there are none: the last layer of a pool has no next."""
+        if not self.prefetch_next_layer:
+            return 0, 0
+        next_k, next_v = self._resolve_kv_cache_ptrs(layer_idx + 1, {k: v for k, v in tensor_mapping.items() if k != 'KV Cache Pool'})
+        return (next_k, next_v) if next_k and next_v and not (next_k | next_v) % 16 else (0, 0)
+
     def _validate(self, batch, q_ptr, k_cache_ptr, v_cache_ptr, output_ptr, kv_offset_ptr, kv_batch_stride):
         if batch <= 0 or batch > self.batch_size:
             raise CudaSafetyError(f"batch {batch} outside 1..{self.batch_size} (scratch is sized for batch_size)")
@@ -576,12 +583,7 @@ class SplitKVAttentionDispatcher:
         # launch in a graph of split launches only), so the flag is left off.
         if getattr(self.hip, 'programmatic_launch', False):
             flags |= FLAG_PREFETCH_Q
-        next_k = next_v = 0
-        if self.prefetch_next_layer:
-            next_k, next_v = self._resolve_kv_cache_ptrs(layer_idx + 1, {k: v for k, v in tensor_mapping.items()
-                                                                         if k != 'KV Cache Pool'})
-            if not (next_k and next_v) or next_k % 16 or next_v % 16:
-                next_k = next_v = 0
+        next_k, next_v = self._next_caches(layer_idx, tensor_mapping)
         out_kind = 3 if self.emit_state else (2 if self.output_f32 else 1)
         # One split and an ordinary output: the split launch normalises and stores the attention
         # output itself (the reference's unsplit kernel, flash_attention.hip.template:29-113, in one

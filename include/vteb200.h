@@ -263,8 +263,8 @@ int vteb_split_kv_decode_noalloc(const void* q, const void* k_cache, const void*
  * counterpart in the reference. */
 int vteb_noalloc_check_status(void* stream);
 
-/* The same for the launches of a loaded module whose arguments name no status word (flash_attention_kernel, where it is
- * served by thread-block clusters).  Waits for the device. */
+/* The same for the launches of a loaded module's cluster and lean kernels whose `status` argument is null.  Waits for the
+ * device. */
 int vteb_module_check_status(void* module);
 
 /* Writes the current token's K/V rows at position kv_offsets[b]

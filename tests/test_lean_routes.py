@@ -156,12 +156,13 @@ def test_the_unsplit_kernel_goes_to_clusters_where_they_pay(built_library):
     kernels = {name: name for name in CLUSTER_KERNELS}
     vp, ci = ctypes.c_void_p, ctypes.c_int
 
-    def served(B=4, heads=(12, 2, 128), capacity=2048, grid=None, block=None, at=0, stride=None):
+    def served(B=4, heads=(12, 2, 128), capacity=2048, grid=None, block=None, at=0, stride=None, **status):
         Hq, Hkv, D = heads
         args = [vp(0x1000 * (i + 1)) for i in range(6)] + [ci(1), ci(Hq), ci(Hkv), ci(D), ctypes.c_float(0.5), vp(0x9000),
                                                           ci(capacity * Hkv * D if stride is None else stride)]
         args[0] = vp(0x1000 + at)
-        return unsplit_as_clusters(hip, kernels, args, grid or (B, Hq, 1), block or (D, 1, 1))
+        return unsplit_as_clusters(hip, kernels, args, grid or (B, Hq, 1), block or (D, 1, 1), **status)
+    assert served(status=0x4440)[1][19].value == 0x4440
     fn, args, grid, block, smem = served()
     parts = args[12].value
     assert fn.startswith("vteb_decode_cluster_") and fn.endswith("d128_kernel") and parts in CLUSTER_PARTS and grid == (8 * parts, 1, 1) and grid.cluster == parts
@@ -173,6 +174,25 @@ def test_the_unsplit_kernel_goes_to_clusters_where_they_pay(built_library):
                     dict(stride=2048 * 256 + 4), dict(at=8), dict(grid=(4, 6, 1)), dict(block=(64, 1, 1)), dict(heads=(32, 2, 256)),
                     dict(heads=(12, 2, 96)), dict(grid=(4, 12, 2))):
         assert served(**refused) is None, refused
+
+
+def test_a_wait_that_ran_out_is_raised_wherever_the_host_waits(built_library):
+    """Launches whose arguments have no status word report to one of the runtime's: raised once, by whichever wait is next."""
+    from vte_b200.bridge.cuda_runtime import CudaRuntime, ERR_DEVICE_STATUS
+    from vte_b200.bridge.errors import CudaRuntimeError
+
+    class FakeLib:
+        def __getattr__(self, name):
+            return lambda *a: 0
+    rt = CudaRuntime(str(built_library))
+    rt._lib, rt._initialized, rt._launch_status = FakeLib(), True, ctypes.c_int(0)
+    for wait in (rt.synchronize, rt.stream_synchronize, lambda: rt.event_synchronize(ctypes.c_void_p(1))):
+        wait()
+        rt._launch_status.value = 4
+        with pytest.raises(CudaRuntimeError, match="bounded wait") as e:
+            wait()
+        assert e.value.code == ERR_DEVICE_STATUS
+        wait()
 
 
 LENGTHS = [1, 15, 16, 17, 127, 128, 129, 255, 257, 385, 600]
@@ -278,10 +298,20 @@ def test_a_cluster_kernel_refuses_a_launch_without_its_clusters(cuda_runtime, co
     try:
         ex._choose_route()
         fn, args, grid, block, smem = ex._route.launches(0, ex.tensor_mapping, ex.offsets.ptr, 1)[0]
+        module = codegen.load_kernel_safe(cuda_runtime, 'decode_attention', cuda_runtime.get_gpu_architecture(), ex._route.name)[0]
         ex._update_staging_buffers(np.array([200], dtype=np.int32))
         cuda_runtime.launch_kernel_recorded(fn, args, tuple(grid), block, smem)
         with pytest.raises(Exception, match="bounded wait"):
             ex.dispatcher_check()
+        # without a status word of its own: the runtime's, as launches of flash_attention_kernel get it, or the module's
+        for word, wait in ((ctypes.addressof(cuda_runtime._launch_status), cuda_runtime.stream_synchronize),
+                           (0, lambda: cuda_runtime.module_check_status(module))):
+            wait()
+            args[19] = ctypes.c_void_p(word)
+            cuda_runtime.launch_kernel_recorded(fn, args, tuple(grid), block, smem)
+            with pytest.raises(Exception, match="bounded wait"):
+                wait()
+            wait()
     finally:
         ex.cleanup()
 

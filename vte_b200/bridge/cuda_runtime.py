@@ -217,8 +217,8 @@ class CudaRuntime:
         self._props: dict = {}
         self._smem_optin_set: dict[int, int] = {}
         self._signatures: dict[int, tuple[str, int]] = {}
-        self._clustered: dict[int, dict] = {}     # unsplit kernel -> the cluster kernels that serve it where that pays, and its module
-        self._status_modules: set[int] = set()    # modules whose launches report to a status word of the module's
+        self._clustered: dict[int, dict] = {}     # unsplit kernel -> the cluster kernels that serve it where that pays
+        self._launch_status: Optional[ctypes.c_int] = None   # pinned; where launches whose arguments have no status word report
         self._active_clusters: dict[tuple, int] = {}   # what the device said of a kernel's clusters
         self._by_blocks: dict[int, list] = {}     # function -> [(build, registers a thread)], see KERNEL_BY_BLOCKS
         self._panic = False
@@ -268,6 +268,9 @@ class CudaRuntime:
         self._device_index = idx
         self._check_error(self._lib.vteb_stream_create(ctypes.byref(self._stream)), "cudaStreamCreate")
         self._initialized = True
+        word = self.host_alloc(ctypes.sizeof(ctypes.c_int))
+        ctypes.memset(word.value, 0, ctypes.sizeof(ctypes.c_int))
+        self._launch_status = ctypes.c_int.from_address(word.value)
         self._props = self._query_properties(idx)
         free_b, total_b = self.get_real_mem_info()
         self._vram_total = total_b
@@ -502,7 +505,6 @@ class CudaRuntime:
                                                    for symbol, registers in KERNEL_BY_BLOCKS[kernel_name]]
                 if kernel_name == "flash_attention_kernel":
                     self._clustered[function.value] = {name: self._module_function(module, name) for name in CLUSTER_KERNELS}
-                    self._clustered[function.value]["module"] = module.value
             except CudaRuntimeError:
                 pass                              # a cubin of someone else's with a kernel of that name: one build
         if kernel_name in KERNEL_SIGNATURES:
@@ -581,10 +583,10 @@ class CudaRuntime:
         served = None
         if kernels:
             from ..core.lean_route import unsplit_as_clusters
-            served = unsplit_as_clusters(self, kernels, args, grid, block)
+            served = unsplit_as_clusters(self, kernels, args, grid, block,
+                                         ctypes.addressof(self._launch_status) if self._launch_status is not None else 0)
         if served:
             function, args, grid, block, shared_mem = served
-            self._status_modules.add(kernels["module"])
             flags |= LAUNCH_PROGRAMMATIC          # it waits for everything in front before it touches anything, and releases after
         arr, keep = self._marshal(args)
         if not served:
@@ -638,14 +640,24 @@ class CudaRuntime:
         finally:
             done.set()
         self._check_error(err, "cudaDeviceSynchronize")
-        for module in self._status_modules:
-            err = self._lib.vteb_module_check_status(ctypes.c_void_p(module))
-            if err == ERR_DEVICE_STATUS:
-                raise CudaRuntimeError(self._last_error(), code=err)
-            self._check_error(err, "vteb_module_check_status")
+        self._check_launch_status()
         if timed_out.is_set():
             raise CudaRuntimeError(f"cudaDeviceSynchronize took longer than {self._sync_timeout_s} s")
         return True
+
+    def _check_launch_status(self):
+        """Raise, once, if a launch that has completed gave up on a bounded wait and its arguments name no status word."""
+        if self._launch_status is not None and self._launch_status.value:
+            code, self._launch_status.value = self._launch_status.value, 0
+            raise CudaRuntimeError(f"a kernel gave up on a bounded wait (code {code})", code=ERR_DEVICE_STATUS)
+
+    def module_check_status(self, module) -> None:
+        """Raise, once, if a launch of a loaded module's cluster kernels with a null status gave up.  Waits for the device."""
+        self._require_init()
+        err = self._lib.vteb_module_check_status(ctypes.c_void_p(_ptr_value(module)))
+        if err == ERR_DEVICE_STATUS:
+            raise CudaRuntimeError(self._last_error(), code=err)
+        self._check_error(err, "vteb_module_check_status")
 
     def is_panic_state(self) -> bool:
         return self._panic
@@ -691,6 +703,7 @@ class CudaRuntime:
 
     def event_synchronize(self, event):
         self._check_error(self._lib.vteb_event_synchronize(event), "cudaEventSynchronize")
+        self._check_launch_status()
 
     def event_elapsed_ms(self, start, stop) -> float:
         self._check_error(self._lib.vteb_event_synchronize(stop), "cudaEventSynchronize")
@@ -704,6 +717,7 @@ class CudaRuntime:
     def stream_synchronize(self):
         self._require_init()
         self._check_error(self._lib.vteb_stream_synchronize(self._stream), "cudaStreamSynchronize")
+        self._check_launch_status()
 
     # ------------------------------------------------------------------ peer memory
     def ipc_export(self, ptr) -> bytes:
@@ -865,6 +879,7 @@ class CudaRuntime:
                 self.safe_free(ctypes.c_void_p(val), f"{tag}_cleanup")
             except Exception as e:   # keep going: cleanup is fail-safe
                 logger.error("error freeing 0x%016X: %s", val, e)
+        self._launch_status = None
         for val in list(self._host_allocations):
             try:
                 self.host_free(ctypes.c_void_p(val))
@@ -877,7 +892,6 @@ class CudaRuntime:
         self._by_blocks.clear()
         self._active_clusters.clear()
         self._clustered.clear()
-        self._status_modules.clear()
         self._smem_optin_set.clear()
         if self._initialized and self._stream:
             self._lib.vteb_stream_destroy(self._stream)

@@ -148,9 +148,10 @@ def _unsplit_option(hip, kernels: dict, Hq: int, Hkv: int, D: int, pairs: int, c
     return known[key]
 
 
-def unsplit_as_clusters(hip, kernels: dict, args: list, grid, block):
+def unsplit_as_clusters(hip, kernels: dict, args: list, grid, block, status: int = 0):
     """flash_attention_kernel's launch (13 arguments, grid (batch, query heads, 1), block (head_dim)) as a launch of the
-    cluster kernels, (function, args, grid, block, shared_mem), or None where its own builds serve it.
+    cluster kernels, (function, args, grid, block, shared_mem), or None where its own builds serve it.  `status`: where a
+    launch reports a wait that ran out.
 
     Its geometry has one block walk a whole sequence; a cluster per (sequence, KV head) has as many SMs on it as the grid
     leaves and reads K and V once for the group.  us a layer, plain stream order, builds / clusters: four sequences of 12
@@ -174,5 +175,5 @@ def unsplit_as_clusters(hip, kernels: dict, args: list, grid, block):
         return None
     vp, ci, cf = ctypes.c_void_p, ctypes.c_int, ctypes.c_float
     lean = [vp(q), vp(k_cache), vp(v_cache), vp(0), vp(0), vp(0), ci(Hq), ci(Hkv), ci(D), cf(scale), vp(offsets), ci(stride), ci(parts),
-            vp(k), vp(v), vp(out), ci(1), ci(FLAG_WAIT_FIRST), ci(plan.depth), vp(0), vp(0), vp(0), vp(0), vp(0), ci(-1), ci(0)]
+            vp(k), vp(v), vp(out), ci(1), ci(FLAG_WAIT_FIRST), ci(plan.depth), vp(status), vp(0), vp(0), vp(0), vp(0), ci(-1), ci(0)]
     return function, lean, ClusterGrid((pairs * parts, 1, 1), parts), (plan.threads, 1, 1), plan.smem_bytes

@@ -195,6 +195,27 @@ def test_a_wait_that_ran_out_is_raised_wherever_the_host_waits(built_library):
         wait()
 
 
+@pytest.mark.parametrize("off", [False, True])
+def test_cluster_launches_of_the_unsplit_kernel_obey_the_programmatic_switch(built_library, monkeypatch, off):
+    from vte_b200.bridge.cuda_runtime import CudaRuntime, LAUNCH_CLUSTER_SHIFT, LAUNCH_PROGRAMMATIC
+    from vte_b200.compiler.signatures import CLUSTER_KERNELS
+    monkeypatch.setenv("VTE_B200_NO_PDL", "1") if off else monkeypatch.delenv("VTE_B200_NO_PDL", raising=False)
+    rt, flags = CudaRuntime(str(built_library)), []
+
+    class FakeLib:
+        def __getattr__(self, name):
+            return lambda *a: flags.append(a[-1]) or 0 if name == "vteb_launch" else 0
+    rt.get_num_cus, rt.max_active_clusters, rt.lean_plan = lambda: 148, FakeHip.max_active_clusters, lean_plan
+    rt.lean_estimate = FakeHip.lean_estimate
+    rt._lib, rt._initialized, rt._props = FakeLib(), True, {"max_threads_per_block": 1024, "shared_mem_per_block": 49152,
+                                                            "shared_mem_per_block_optin": 232448}
+    rt._clustered = {2: {name: ctypes.c_void_p(3) for name in CLUSTER_KERNELS}}
+    vp, ci = ctypes.c_void_p, ctypes.c_int
+    args = [vp(0x1000 * (i + 1)) for i in range(6)] + [ci(1), ci(12), ci(2), ci(128), ctypes.c_float(0.5), vp(0x9000), ci(2048 * 256)]
+    rt.launch_kernel_recorded(vp(2), args, (4, 12, 1), (128, 1, 1), 1024)
+    assert flags[0] >> LAUNCH_CLUSTER_SHIFT > 1 and flags[0] & LAUNCH_PROGRAMMATIC == (0 if off else LAUNCH_PROGRAMMATIC)
+
+
 LENGTHS = [1, 15, 16, 17, 127, 128, 129, 255, 257, 385, 600]
 
 

@@ -25,7 +25,7 @@ from pathlib import Path
 from typing import Optional
 
 from ..config import (MAX_ALLOCATION_SIZE, MAX_GRID_DIMENSIONS, VRAM_USAGE_LIMIT, DEFAULT_SYNC_TIMEOUT_S,
-                      ENV_DEVICE_INDEX)
+                      ENV_DEVICE_INDEX, ENV_NO_PDL, env_flag)
 from .errors import CudaRuntimeError, CudaSafetyError, MemoryGuardianOOMError
 
 logger = logging.getLogger(__name__)
@@ -223,6 +223,7 @@ class CudaRuntime:
         self._by_blocks: dict[int, list] = {}     # function -> [(build, registers a thread)], see KERNEL_BY_BLOCKS
         self._panic = False
         self._sync_timeout_s = sync_timeout_s
+        self._no_pdl = env_flag(ENV_NO_PDL)
         self.programmatic_launch = False   # when True, recorded launches carry the PDL attribute
 
     # ------------------------------------------------------------------ errors
@@ -587,7 +588,8 @@ class CudaRuntime:
                                          ctypes.addressof(self._launch_status) if self._launch_status is not None else 0)
         if served:
             function, args, grid, block, shared_mem = served
-            flags |= LAUNCH_PROGRAMMATIC          # it waits for everything in front before it touches anything, and releases after
+            if not self._no_pdl:
+                flags |= LAUNCH_PROGRAMMATIC      # it waits for everything in front before it touches anything, and releases after
         arr, keep = self._marshal(args)
         if not served:
             function = self._build_for(function, grid, block)

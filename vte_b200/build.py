@@ -33,7 +33,7 @@ def _newer(target: Path, sources) -> bool:
 
 
 def build_library(force: bool = False, verbose: bool = False) -> Path:
-    sources = [CSRC / "vteb200_shim.cu", *sorted((CSRC / "kernels").glob("*.cu*")),
+    sources = [CSRC / "vteb200_shim.cu", *sorted(CSRC.glob("*.h")), *sorted((CSRC / "kernels").glob("*.cu*")),
                PKG.parent / "include" / "vteb200.h"]
     if not force and _newer(LIB, sources):
         return LIB

@@ -6,12 +6,12 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <dlfcn.h>
-#include <pthread.h>
 #include <stdarg.h>
 #include <stdio.h>
 #include <string.h>
 
 #include "../../include/vteb200.h"
+#include "cluster_choice.h"
 #include "kernels/decode_attention.cu"
 #include "kernels/aux_kernels.cu"
 
@@ -138,9 +138,9 @@ int check_nccl(int r, const char* what) {
     return r;
 }
 
-// Per-process record of which in-library kernels already had their dynamic
-// shared memory limit raised.
-bool g_fast_attr_set[7] = {false, false, false, false, false, false, false};
+// Which in-library kernels had their dynamic shared memory limit raised, on each device.
+constexpr int kMaxDevices = 64;
+bool g_fast_attr_set[kMaxDevices][7];
 
 // Tensor map over a K or V cache seen as a matrix of `n_rows` position rows of `row_halves`
 // fp16 values: boxes of 64 halves x `box_rows` rows, 128-byte swizzle.
@@ -683,52 +683,31 @@ static LeanKernel lean_cluster_kernel(int kind, int head_dim) {          // grou
     return head_dim == 64 ? vteb_decode_cluster_d64_kernel : head_dim == 128 ? vteb_decode_cluster_d128_kernel : vteb_decode_cluster_d256_kernel;
 }
 
-struct LeanChoice { int hq, hkv, d, batch, sms; long long context; int kind, parts; };   // parts 0: no clusters
-static pthread_mutex_t g_lean_lock = PTHREAD_MUTEX_INITIALIZER;
-static LeanChoice g_lean_known[64];
-static unsigned g_lean_count = 0;
+static ClusterChoices g_cluster_choices;
 
-// Whether a call goes to clusters, and to which; sizes alone decide, so the last 64 answers are kept.
-static int choose_clusters(int hq, int hkv, int d, int batch, long long context, int sms, LeanChoice* out) {
-    pthread_mutex_lock(&g_lean_lock);
-    for (unsigned i = 0; i < g_lean_count && i < 64; ++i) {
-        const LeanChoice& k = g_lean_known[i];
-        if (k.hq == hq && k.hkv == hkv && k.d == d && k.batch == batch && k.context == context && k.sms == sms) {
-            *out = k;
-            pthread_mutex_unlock(&g_lean_lock);
-            return 0;
-        }
-    }
-    pthread_mutex_unlock(&g_lean_lock);
-    LeanChoice best = {hq, hkv, d, batch, sms, context, 0, 0};
-    double least = kLeanMargin * lean_estimate_us(-1, 0, hq, hkv, d, batch, context, 0, sms);
-    static const int kParts[] = {2, 3, 4, 5, 6, 8, 9, 12, 16};
-    for (int kind = kLeanCluster; kind <= kLeanHalf; ++kind)
-        for (int parts : kParts) {
-            const LeanPlan p = make_lean_plan(hq, hkv, d, parts, context, kind);
-            if (!p.ok || lean_estimate_us(kind, parts, hq, hkv, d, batch, context, batch * hkv, sms) >= least) continue;
-            const LeanKernel fn = lean_cluster_kernel(kind, d);
-            int rc = check_rt(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, vteb::kSmemBudget), "cudaFuncSetAttribute");
-            if (!rc && parts > 8) rc = check_rt(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1), "cudaFuncSetAttribute");
-            if (rc) return rc;
-            cudaLaunchConfig_t cfg;
-            memset(&cfg, 0, sizeof(cfg));
-            cfg.gridDim = dim3(parts); cfg.blockDim = dim3(p.threads); cfg.dynamicSmemBytes = p.smem_bytes;
-            cudaLaunchAttribute attr;
-            attr.id = cudaLaunchAttributeClusterDimension;
-            attr.val.clusterDim.x = parts; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
-            cfg.attrs = &attr; cfg.numAttrs = 1;
-            int resident = 0;
-            if ((rc = check_rt(cudaOccupancyMaxActiveClusters(&resident, fn, &cfg), "cudaOccupancyMaxActiveClusters"))) return rc;
-            const double us = lean_estimate_us(kind, parts, hq, hkv, d, batch, context, resident, sms);
-            if (resident > 0 && us < least) { least = us; best.kind = kind; best.parts = parts; }
-        }
-    pthread_mutex_lock(&g_lean_lock);
-    g_lean_known[g_lean_count++ % 64] = best;
-    if (g_lean_count >= 128) g_lean_count -= 64;
-    pthread_mutex_unlock(&g_lean_lock);
-    *out = best;
-    return 0;
+// Whether a call goes to clusters, and to which.
+static ClusterChoice choose_clusters(int hq, int hkv, int d, int batch, long long context, int sms) {
+    const ClusterCall call = {g_device, hq, hkv, d, batch, sms, context};
+    const auto estimate = [&](int kind, int parts, int resident) {
+        return make_lean_plan(hq, hkv, d, parts, context, kind).ok ? lean_estimate_us(kind, parts, hq, hkv, d, batch, context, resident, sms) : -1.0;
+    };
+    const auto resident = [&](int kind, int parts, int* n) {
+        const LeanKernel fn = lean_cluster_kernel(kind, d);
+        const LeanPlan p = make_lean_plan(hq, hkv, d, parts, context, kind);
+        cudaLaunchConfig_t cfg;
+        memset(&cfg, 0, sizeof(cfg));
+        cfg.gridDim = dim3(parts); cfg.blockDim = dim3(p.threads); cfg.dynamicSmemBytes = p.smem_bytes;
+        cudaLaunchAttribute attr;
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = parts; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+        cfg.attrs = &attr; cfg.numAttrs = 1;
+        if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, vteb::kSmemBudget) == cudaSuccess &&
+            (parts <= 8 || cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) &&
+            cudaOccupancyMaxActiveClusters(n, fn, &cfg) == cudaSuccess) return true;
+        cudaGetLastError();                              // not to be had here: another route serves the call
+        return false;
+    };
+    return g_cluster_choices.choose(call, kLeanMargin * lean_estimate_us(-1, 0, hq, hkv, d, batch, context, 0, sms), estimate, resident);
 }
 
 int vteb_split_kv_decode(const void* q, const void* k_cache, const void* v_cache, const int* kv_offsets,
@@ -796,8 +775,8 @@ int vteb_split_kv_decode(const void* q, const void* k_cache, const void* v_cache
     // positions, 28 heads on 4 of 128, append included: 38.8 us and 31.1).  The stride stands for the context.
     if (balanced && all_sms && kv_batch_stride > 0 && !(flags & ~(unsigned)(VTEB_ATTN_BALANCED | VTEB_ATTN_PROGRAMMATIC))) {
         const long long context = kv_batch_stride / ((long long)num_kv_heads * head_dim);
-        LeanChoice c = {};
-        if (context > 0 && (rc = choose_clusters(num_q_heads, num_kv_heads, head_dim, batch, context, n_ctas, &c))) return rc;
+        ClusterChoice c = {0, 0};
+        if (context > 0) c = choose_clusters(num_q_heads, num_kv_heads, head_dim, batch, context, n_ctas);
         if (c.parts) {
             const LeanPlan lp = make_lean_plan(num_q_heads, num_kv_heads, head_dim, c.parts, context, c.kind);
             cudaLaunchConfig_t cfg;
@@ -831,10 +810,11 @@ int vteb_split_kv_decode(const void* q, const void* k_cache, const void* v_cache
     else if (head_dim == 64) { fk = vteb_split_kv_partial_d64_kernel; slot = 0; }
     else if (head_dim == 128) { fk = vteb_split_kv_partial_d128_kernel; slot = 1; }
     else { fk = vteb_split_kv_partial_d256_kernel; slot = 2; }
-    if (!g_fast_attr_set[slot]) {
+    const bool recorded = g_device >= 0 && g_device < kMaxDevices;
+    if (!recorded || !g_fast_attr_set[g_device][slot]) {
         if ((rc = check_rt(cudaFuncSetAttribute(fk, cudaFuncAttributeMaxDynamicSharedMemorySize, vteb::kSmemBudget),
                            "cudaFuncSetAttribute(max dynamic shared memory)"))) return rc;
-        g_fast_attr_set[slot] = true;
+        if (recorded) g_fast_attr_set[g_device][slot] = true;
     }
     int kflags = (flags & VTEB_ATTN_WRITE_EMPTY_O) ? kFlagWriteEmptyO : 0;
     if (balanced) kflags |= kFlagBalanced;

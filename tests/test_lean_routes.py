@@ -264,6 +264,82 @@ def test_lean_kernels_match_the_oracle(cuda_runtime, codegen, heads, route, appe
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("heads,B,S,route,kw", [
+    ((12, 2, 128), 3, 700, (8, 1), {}), ((12, 2, 128), 1, 4096, (37, 0), dict(rope="fused-append")),
+    ((12, 2, 128), 1, 4096, (16, 1), dict(rope="fused")), ((32, 8, 64), 5, 300, (3, 1), dict(with_append=True)),
+    ((8, 2, 256), 4, 300, (5, 2), dict(fuse_append=True)), ((32, 2, 128), 4, 2048, (6, 1), dict(with_append=True))])
+def test_partials_after_a_routed_step_are_the_step_s_own(cuda_runtime, codegen, heads, B, S, route, kw):
+    """Bit for bit what the dispatcher's own launches leave, although Q, offsets, new rows and caches change between the
+    step and the call; neither the outputs nor the caches change with the call, twice in a row."""
+    Hq, Hkv, D = heads
+    meta = {"attention.head_count": Hq, "attention.head_count_kv": Hkv, "attention.key_length": D}
+    rng = np.random.default_rng(B)
+    f16 = lambda *s: rng.standard_normal(s, dtype=np.float32).astype(np.float16)
+    k, v, steps = f16(B, S, Hkv, D), f16(B, S, Hkv, D), []
+    for _ in range(2):
+        steps.append((f16(2, B, Hq, D), f16(2, B, Hkv, D), f16(2, B, Hkv, D), rng.integers(S // 2, S, B).astype(np.int32)))
+    got = []
+    for lean in (route, (0, 0)):
+        ex = DecodeAttentionExecutor(cuda_runtime, codegen, meta, B, S, 2, n_kv_buffers=1, lean=lean, **kw)
+        try:
+            ex.upload_cache(0, k, v)
+
+            def rows_and_q(q, kn, vn):
+                for l in range(2):
+                    ex.upload_layer(l, q[l])
+                    ex.upload_new_kv(l, kn[l], vn[l])
+            mine = []
+            for i, (q, kn, vn, off) in enumerate(steps):
+                rows_and_q(q, kn, vn)
+                out = ex.execute_decode_batch(off)
+                caches = ex.download_cache_rows(0, 0, S)
+                rows_and_q(*steps[1 - i][:3])                        # the next step's inputs
+                ex._update_staging_buffers(steps[1 - i][3])
+                if i:
+                    ex.upload_cache(0, v, k)
+                partials = ex.read_partials()
+                again = ex.read_partials()
+                assert all(np.array_equal(a, b) for a, b in zip(partials, again))
+                if not i:
+                    left = np.empty_like(out)
+                    cuda_runtime.safe_memcpy_device_to_host(left, ctypes.c_void_p(ex.out_all.ptr), "output")
+                    assert np.array_equal(left, out)
+                    assert all(np.array_equal(a, b) for a, b in zip(caches, ex.download_cache_rows(0, 0, S)))
+                mine.append(partials)
+            got.append(mine)
+        finally:
+            ex.cleanup()
+    for a, b in zip(*got):
+        m, l, o = zip(a, b)
+        used = l[1] > 0
+        assert used.any() and np.array_equal(used, l[0] > 0)
+        assert np.array_equal(m[0][used], m[1][used]) and np.array_equal(l[0], l[1]) and np.array_equal(o[0][used], o[1][used])
+
+
+@pytest.mark.gpu
+def test_partials_of_more_items_than_sms_each_time(cuda_runtime, codegen):
+    """256 work items, one split: the launch behind read_partials draws them from a queue, whose ticket is zero every time."""
+    B, S, Hkv, D = 32, 128, 8, 256
+    rng = np.random.default_rng(1)
+    f16 = lambda *s: rng.standard_normal(s, dtype=np.float32).astype(np.float16)
+    q, k, v = f16(B, Hkv, D), f16(B, S, Hkv, D), f16(B, S, Hkv, D)
+    ex = DecodeAttentionExecutor(cuda_runtime, codegen, {"attention.head_count": Hkv, "attention.head_count_kv": Hkv,
+                                                         "attention.key_length": D}, B, S, 1, lean=(2, 1))
+    try:
+        ex.upload_layer(0, q, k, v)
+        for _ in range(3):
+            off = rng.integers(0, S, B).astype(np.int32)
+            out = ex.execute_decode_batch(off)[0]
+            m, l, o = ex.read_partials()
+            assert m.shape == (B, Hkv, 1)
+            whole = o[:, :, 0] / l
+            assert np.linalg.norm(whole - out) <= 2e-5 * np.linalg.norm(out)
+            assert np.linalg.norm(out - orc.decode_attention(q, k, v, off)) <= 2e-5 * np.linalg.norm(out)
+    finally:
+        ex.cleanup()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("rope_type,rotary", [(0, 0), (1, 0), (2, 32), (2, 64)])
 @pytest.mark.parametrize("D", [64, 128, 256])
 def test_rotation_in_the_lean_kernels_gives_the_separate_launch_s_bits(cuda_runtime, codegen, D, rope_type, rotary):

@@ -24,7 +24,7 @@ from ..bridge.errors import CudaSafetyError
 from ..bridge.memory import MemoryRegion, SlabAllocator
 from ..config import ENV_NO_PDL, env_flag
 from .lean_route import LeanRoute, choose_lean_route
-from .split_kv_attention import SplitKVAttentionDispatcher
+from .split_kv_attention import FLAG_DIRECT_OUTPUT, SplitKVAttentionDispatcher
 
 
 def _round_up(x: int, m: int) -> int:
@@ -125,6 +125,9 @@ class DecodeAttentionExecutor:
                                                   tensor_maps and prefetch_next_layer)
         self._lean = lean if lean is not None else None if open_layout else (0, 0)
         self._route = None
+        # what partials of a routed step can be had from: the last layer's Q and offsets as the step saw them, the names it
+        # was captured with, and whether the partial buffers are still to be filled
+        self._kept, self._kept_names, self._partials_due = None, None, False
         self.k_cache = [A(self.kv_bytes, f"kv_cache.k.{i}", MemoryRegion.KV_CACHE) for i in range(self.n_kv)]
         self.v_cache = [A(self.kv_bytes, f"kv_cache.v.{i}", MemoryRegion.KV_CACHE) for i in range(self.n_kv)]
         # all layers' Q (and outputs) are contiguous so one copy moves a whole step's worth
@@ -180,6 +183,8 @@ class DecodeAttentionExecutor:
             self.upload_cache(layer % self.n_kv, k_cache, v_cache)
 
     def upload_cache(self, buf: int, k_cache: np.ndarray, v_cache: np.ndarray):
+        if buf == (self.L - 1) % self.n_kv:
+            self._fill_partials()
         for dst, src in ((self.k_cache[buf], k_cache), (self.v_cache[buf], v_cache)):
             src = np.ascontiguousarray(src, dtype=np.float16)
             if src.shape != (self.B, self.S, self.Hkv, self.D):
@@ -195,6 +200,8 @@ class DecodeAttentionExecutor:
     def fill_cache_on_device(self, buf: int, seed: int, sigma: float = 1.0, outlier_prob: float = 0.0,
                              outlier_scale: float = 1.0):
         """Synthetic N(0, sigma) cache contents generated on the device."""
+        if buf == (self.L - 1) % self.n_kv:
+            self._fill_partials()
         n = self.B * self.kv_batch_stride
         self.hip.fill_normal_f16(ctypes.c_void_p(self.k_cache[buf].ptr), n, 2 * seed + 1, sigma, outlier_prob, outlier_scale)
         self.hip.fill_normal_f16(ctypes.c_void_p(self.v_cache[buf].ptr), n, 2 * seed + 2, sigma, outlier_prob, outlier_scale)
@@ -224,7 +231,12 @@ class DecodeAttentionExecutor:
     def layer_launches(self, layer: int):
         """What a step launches for a layer (without a rotation launch of its own)."""
         if self._route is not None and self.dispatcher.offsets_final:
-            return self._route.launches(layer, self.tensor_mapping, self.offsets.ptr, self.B)
+            last = layer == self.L - 1
+            launches = self._route.launches(layer, self.tensor_mapping, self.offsets.ptr, self.B,
+                                            (self._kept.ptr, self._kept.ptr + _round_up(self.q_bytes, 256)) if last else (0, 0))
+            if last:
+                self._kept_names = dict(self.tensor_mapping) if launches[0][0] is self._route.function else None
+            return launches
         launches = self.dispatcher.build_launches(layer, self.tensor_mapping, self.offsets.ptr, batch=self.B)
         return launches if self.with_append or self.dispatcher.fuse_append else launches[1:]
 
@@ -269,6 +281,8 @@ class DecodeAttentionExecutor:
             self._lean = choose_lean_route(d, append)
         if self._lean[0]:
             self._route = LeanRoute(d, *self._lean, append)
+            self._kept = self.allocator.allocate(_round_up(self.q_bytes, 256) + _round_up(4 * self.B, 256), "attn_partials_source",
+                                                 MemoryRegion.SCRATCH)
 
     def build_decode_graph(self):
         """Capture all layers' launches once (hip_graph_executor.py:504-725)."""
@@ -361,6 +375,7 @@ class DecodeAttentionExecutor:
         """Enqueue one decode step (no host synchronisation)."""
         if self._graph_exec is not None:
             self.hip.graph_launch(self._graph_exec)
+            self._partials_due = self._kept_names is not None
         else:
             self.hip.programmatic_launch = self.programmatic
             try:
@@ -388,6 +403,7 @@ class DecodeAttentionExecutor:
             ctypes.memmove(self._stage_offsets.value, off.ctypes.data, off.nbytes)
             ctypes.memmove(self._stage_q.value, qh.ctypes.data, qh.nbytes)
             self.hip.graph_launch(self._io_graph_exec)
+            self._partials_due = self._kept_names is not None
             self.hip.stream_synchronize()
             # the status word travelled with the outputs: only a non-zero one needs the slow path
             if ctypes.c_int.from_address(self._stage_out.value + self._out_tail + 4).value != 0:
@@ -423,14 +439,32 @@ class DecodeAttentionExecutor:
         if self.dispatcher.work_ptr and hasattr(self.hip, "check_status"):
             self.hip.check_status(ctypes.c_void_p(self.dispatcher.work_ptr))
 
+    def _fill_partials(self):
+        """Where the last step took a route without partials: its last layer's split launch, now, on the Q and offsets that
+        the step left a copy of.  The layer's caches have to be the step's still."""
+        if not self._partials_due:
+            return
+        self._partials_due = False
+        d, ci, vp = self.dispatcher, ctypes.c_int, ctypes.c_void_p
+        names = {**self._kept_names, f'blk.{self.L - 1}.q_proj.output': self._kept.ptr}
+        fn, args, grid, block, smem = d.build_launches(self.L - 1, names, self._kept.ptr + _round_up(self.q_bytes, 256),
+                                                       batch=self.B)[0 if d.fuse_append else 1]
+        if len(args) > 13:                            # not the reference-geometry kernels
+            args[15] = ci(args[15].value & ~FLAG_DIRECT_OUTPUT)
+            args[21], args[22] = vp(0), ci(0)         # partials, no output
+            if d.fuse_append:
+                args[-2:] = [vp(0), vp(0)]            # the step has appended its row
+        # the ticket is zero only behind a combine launch
+        self.hip.memset_async(vp(d.work_ptr), 4, 0, "work ticket")
+        self.hip.launch_kernel_recorded(fn, args, grid, block, smem)
+        self.hip.memset_async(vp(d.work_ptr), 4, 0, "work ticket")
+        self.hip.stream_synchronize()
+        self.dispatcher_check()
+
     def read_partials(self):
-        """(partial_m, partial_l [B,Hq,C], partial_o [B,Hq,C,D]) of the last layer run."""
-        if self._route is not None:
-            # the step had no partials: the last layer's split launch now, on the caches and offsets as they are
-            launches = self.dispatcher.build_launches(self.L - 1, self.tensor_mapping, self.offsets.ptr, batch=self.B)
-            for fn, args, grid, block, smem in launches[0 if self.dispatcher.fuse_append else 1:][:1]:
-                self.hip.launch_kernel_recorded(fn, args, grid, block, smem)
-            self.hip.stream_synchronize()
+        """(partial_m, partial_l [B,Hq,C], partial_o [B,Hq,C,D]) of the last layer of the last step.  Cache rows that the step
+        read must not have been overwritten since by anything but this executor's own upload and fill methods."""
+        self._fill_partials()
         pm, pl, po = self.dispatcher.partial_buffers
         C = self.dispatcher.max_chunks
         m = np.empty((self.B, self.Hq, C), dtype=np.float32)

@@ -16,6 +16,7 @@ from ..bridge.errors import CudaSafetyError
 FLAG_PREFETCH_Q = 8
 FLAG_WAIT_FIRST = 32
 FLAG_ROWS_FINAL = 64
+FLAG_KEEP = 128
 
 
 SPLIT, CLUSTER, HALF = 0, 1, 2      # kinds of route: split and combine; clusters; clusters of blocks of half the warps
@@ -44,7 +45,8 @@ class LeanRoute:
             self.combine = load('vteb_split_kv_combine_small_kernel' if self.parts <= 32 else
                                 'vteb_split_kv_combine_f32_kernel' if d.output_f32 else 'vteb_split_kv_combine_f16_kernel')
 
-    def launches(self, layer: int, tensor_mapping: dict, kv_offset_ptr: int, batch: int):
+    def launches(self, layer: int, tensor_mapping: dict, kv_offset_ptr: int, batch: int, keep: tuple = (0, 0)):
+        """`keep`: where the kernel leaves a copy of Q and of the offsets, for a layer whose partials may be asked for."""
         d = self.d
         vp, ci, cf = ctypes.c_void_p, ctypes.c_int, ctypes.c_float
         attention_scale = d.metadata.get('attention_scale')
@@ -70,6 +72,9 @@ class LeanRoute:
         if not self.cluster:
             partials = [vp(p.ptr) for p in d.partial_buffers]
             next_k, next_v = d._next_caches(layer, tensor_mapping)
+        if keep[0]:
+            next_k, next_v = keep
+            flags |= FLAG_KEEP
         args = [vp(q), vp(k_cache), vp(v_cache), *partials, ci(Hq), ci(Hkv), ci(D), cf(scale), vp(kv_offset_ptr), ci(stride),
                 ci(N), vp(k_new), vp(v_new), vp(out), ci(out_kind), ci(flags), ci(self.plan.depth), vp(d.work_ptr + 4),
                 vp(next_k), vp(next_v)] + rope

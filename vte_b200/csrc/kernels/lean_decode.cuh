@@ -34,7 +34,8 @@ struct LeanArgs {
     const __half* k_new; const __half* v_new;             // this step's projections [B, Hkv, D]; null: the newest row is in the cache
     void* output; int out_kind;                           // cluster kernels: 1 fp16, 2 fp32
     int flags; int* status;
-    const __half* next_k_cache; const __half* next_v_cache;   // split kernels, optional: the next layer's caches, for L2
+    const __half* next_k_cache; const __half* next_v_cache;   // split kernels, optional: the next layer's caches, for L2;
+                                                              // with kLeanKeep: where Q and the offsets are kept instead
     const __half* rope_cos; const __half* rope_sin; int rope_type, rotary_dim;   // rope_type < 0: Q and K arrive rotated
 };
 
@@ -99,6 +100,8 @@ constexpr double kLeanMargin = 0.95;       // a route has to be estimated this m
 extern "C" { __device__ int vteb_lean_status = 0; }
 
 constexpr int kLeanRowsFinal = 64;      // flag: the newest row is in the cache before the launch in front starts
+constexpr int kLeanKeep = 128;          // flag: Q as it came goes to next_k_cache [B, Hq, D], the offsets to next_v_cache [B], so that
+                                        // the partials of this launch can be had later
 constexpr int kLeanCtrlBytes = 128;     // barriers and the abort word
 constexpr int kLeanUnit = 36;           // floats a CTA sends per 32 output columns: o[32], m, l, 2 unused
 
@@ -404,7 +407,8 @@ __device__ __forceinline__ void lean_body(const LeanArgs& a)
         if (i < depth) fetch(i, i);
 
     // the next layer's rows of this part
-    bool ahead = !kCluster && a.next_k_cache != nullptr && warp < 2 && end > start &&
+    const bool keep = (a.flags & kLeanKeep) != 0 && part == 0;
+    bool ahead = !kCluster && a.next_k_cache != nullptr && !(a.flags & kLeanKeep) && warp < 2 && end > start &&
                  (long long)total * pos_stride * 2 <= kL2PrefetchMaxBytes;
     auto fetch_ahead = [&]() {
         ahead = false;
@@ -448,11 +452,13 @@ __device__ __forceinline__ void lean_body(const LeanArgs& a)
     for (int h = threadIdx.x / CPR; h < group; h += THREADS / CPR) {
         const __half* row = a.q + ((long long)b * a.num_q_heads + (long long)kv_head * group + h) * D;
         uint4 x = *reinterpret_cast<const uint4*>(row + q_chunk * 8);
+        if (keep) *reinterpret_cast<uint4*>(const_cast<__half*>(a.next_k_cache) + (row - a.q) + q_chunk * 8) = x;
         if (rotate && rope_touches(a.rope_type, a.rotary_dim, q_chunk * 8))
             x = rope_chunk(x, row, q_chunk * 8, q_words, a.rope_type, a.rotary_dim, D);
         uint32_t* dst = q_store + ((h >> 3) * CPR + (q_chunk & ~3)) * 32 + (h & 7) * 16 + (q_chunk & 3);
         dst[0] = x.x; dst[4] = x.y; dst[8] = x.z; dst[12] = x.w;
     }
+    if (keep && kv_head == 0 && threadIdx.x == 0) reinterpret_cast<int*>(const_cast<__half*>(a.next_v_cache))[b] = total - 1;
     if (my_late && a.k_new != nullptr) {
         if (rotate && lane < CPR && rope_touches(a.rope_type, a.rotary_dim, lane * 8))
             fresh[0] = rope_chunk(fresh[0], a.k_new + new_row, lane * 8, k_words, a.rope_type, a.rotary_dim, D);

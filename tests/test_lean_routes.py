@@ -264,6 +264,27 @@ def test_lean_kernels_match_the_oracle(cuda_runtime, codegen, heads, route, appe
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("heads,S", [((32, 8, 64), 16384), ((8, 1, 64), 131072)])
+def test_the_lean_split_is_as_exact_as_the_dispatcher_s(cuda_runtime, codegen, heads, S):
+    """64-wide heads: no further from 64-bit sums than the launches that the route replaces (the products of the low parts
+    of P chained with those of the high parts were, by 10 to 22 %)."""
+    Hq, Hkv, D = heads
+    rng = np.random.default_rng([0, S, Hq])
+    f16 = lambda *s: rng.standard_normal(s, dtype=np.float32).astype(np.float16)
+    q, k, v, off = f16(1, Hq, D), f16(1, S, Hkv, D), f16(1, S, Hkv, D), np.array([S - 1], dtype=np.int32)
+    ref, error = orc.decode_attention(q, k, v, off, dtype=np.float64), []
+    for lean in ((148 // Hkv, 0), (0, 0)):
+        ex = DecodeAttentionExecutor(cuda_runtime, codegen, {"attention.head_count": Hq, "attention.head_count_kv": Hkv,
+                                                             "attention.key_length": D}, 1, S, 1, lean=lean)
+        try:
+            ex.upload_layer(0, q, k, v)
+            error.append(np.linalg.norm(ex.execute_decode_batch(off)[0] - ref))
+        finally:
+            ex.cleanup()
+    assert error[0] <= error[1]
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("heads,B,S,route,kw", [
     ((12, 2, 128), 3, 700, (8, 1), {}), ((12, 2, 128), 1, 4096, (37, 0), dict(rope="fused-append")),
     ((12, 2, 128), 1, 4096, (16, 1), dict(rope="fused")), ((32, 8, 64), 5, 300, (3, 1), dict(with_append=True)),

@@ -292,6 +292,16 @@ __device__ __forceinline__ void lean_softmax_pv(ConsumerStateT<D / 16> (&st)[NV]
                     for (int j = 0; j < 4; ++j)
                         st[v].o[ch * 4 + i][j] = fmaf(fmaf(lo[j], kFreshLoDown, hi[j]), kFreshDown, st[v].o[ch * 4 + i][j]);
                 }
+            } else if constexpr (D == 64) {                              // the low parts' products on their own, added in fp32
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const uint32_t* f = vf[ch & 1][i];
+                    float lo[4] = {0.f, 0.f, 0.f, 0.f};
+                    mma_full(st[v].o[ch * 4 + i], f[0], f[2], f[1], f[3], bh[v][0], bh[v][1]);
+                    mma_full(lo, f[0], f[2], f[1], f[3], bl[v][0], bl[v][1]);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) st[v].o[ch * 4 + i][j] += lo[j];
+                }
             } else {
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {

@@ -177,6 +177,10 @@ int vteb_lean_plan(int num_q_heads, int num_kv_heads, int head_dim, int n_parts,
  * launches of vteb_split_kv_decode), by which routes are chosen. */
 double vteb_lean_estimate(int kind, int n_parts, int num_q_heads, int num_kv_heads, int head_dim, int batch, long long context,
                           int resident, int num_sms);
+/* The same for a step whose lengths are known: `longest` positions at the most, `total` in all sequences together, in caches with
+ * room for `capacity` a sequence (up to 128, kind -1 is the dispatcher's one launch). */
+double vteb_lean_step_estimate(int kind, int n_parts, int num_q_heads, int num_kv_heads, int head_dim, int batch,
+                               long long capacity, long long longest, long long total, int resident);
 /* How many clusters of `cluster` blocks of a loaded kernel the device runs at once (cuOccupancyMaxActiveClusters). */
 int vteb_max_active_clusters(void* function, int cluster, int threads, int smem_bytes, int* count);
 /* Encodes the 128-byte tensor map the fast split kernels take for a K or V cache: the cache

@@ -44,6 +44,7 @@ def test_plan_holds_exchange_rows_and_received_states(built_library, group, D):
 class FakeHip:
     lean_plan = staticmethod(lean_plan)
     lean_estimate = staticmethod(lambda *a: load_library().vteb_lean_estimate(*a, 148))
+    lean_step_estimate = staticmethod(lambda *a: load_library().vteb_lean_step_estimate(*a))
     get_gpu_architecture = staticmethod(lambda: "sm_100a")
 
     @staticmethod
@@ -79,6 +80,19 @@ def test_the_route_follows_the_size(built_library):
         for context in (1, 130, 1000, 9000, 70000):
             parts, kind = route((28, 4, 128), batch, context)
             assert parts == 0 or (parts in CLUSTER_PARTS if kind else batch == 1 and parts == 37)
+
+
+def test_small_caches_keep_the_one_launch_that_is_shorter(built_library):
+    """Up to 128 positions the dispatcher's layer is one launch.  Timed, dispatcher / clusters, us: 64 sequences of 32 heads on
+    8 of 64 3.1 / 14.1 (room for 16) and 6.4 / 16.2 (128), of 28 on 4 of 128 4.9 / 9.5, of 8 on 2 of 256 5.4 / 6.4; one
+    sequence of 8 on 2 of 256 3.1 / 4.1; of 12 on 2 of 128 with room for 128 4.9 / 3.1, eight of 28 on 4 7.2 / 4.0."""
+    route = lambda *a, append=False: choose_lean_route(FakeDispatcher(*a), append)
+    for append in (False, True):
+        for capacity in (16, 64, 128):
+            assert route((32, 8, 64), 64, capacity, append=append) == (0, 0)
+            assert route((28, 4, 128), 64, capacity, append=append) == (0, 0)
+        assert route((8, 2, 256), 64, 16, append=append) == (0, 0) and route((8, 2, 256), 1, 16) == (0, 0)
+        assert route((12, 2, 128), 1, 128, append=append)[1] and route((28, 4, 128), 8, 128, append=append)[1]
 
 
 def test_a_forced_split_route_stays_within_the_partial_buffers(built_library):

@@ -146,6 +146,7 @@ def _declare(lib):
         "vteb_split_kv_plan_wide": (i, [i, i, i, ctypes.POINTER(FastPlan)]),
         "vteb_lean_plan": (i, [i, i, i, i, ll, i, ctypes.POINTER(LeanPlan)]),
         "vteb_lean_estimate": (ctypes.c_double, [i, i, i, i, i, i, ll, i, i]),
+        "vteb_lean_step_estimate": (ctypes.c_double, [i, i, i, i, i, i, ll, ll, ll, i]),
         "vteb_max_active_clusters": (i, [vp, i, i, i, ip]),
         "vteb_kv_tensor_map": (i, [vp, vp, ctypes.c_longlong, i, i]),
         "vteb_combine_rows_epl": (i, [i, i]),
@@ -770,6 +771,11 @@ class CudaRuntime:
                       resident: int) -> float:
         """Estimated microseconds of one layer, by which routes are chosen (kind -1: the dispatcher's launches)."""
         return self._lib.vteb_lean_estimate(kind, n_parts, num_q_heads, num_kv_heads, head_dim, batch, context, resident, self.get_num_cus())
+
+    def lean_step_estimate(self, kind: int, n_parts: int, num_q_heads: int, num_kv_heads: int, head_dim: int, batch: int, capacity: int,
+                           longest: int, total: int, resident: int) -> float:
+        """Estimated microseconds of one layer of a step with these lengths (kind -1: the dispatcher's launches)."""
+        return self._lib.vteb_lean_step_estimate(kind, n_parts, num_q_heads, num_kv_heads, head_dim, batch, capacity, longest, total, resident)
 
     def max_active_clusters(self, function, cluster: int, threads: int, smem_bytes: int) -> int:
         """Clusters of `cluster` blocks of a loaded kernel that the device runs at once."""

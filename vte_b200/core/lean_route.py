@@ -12,6 +12,7 @@ import math
 
 from ..bridge.cuda_runtime import ClusterGrid
 from ..bridge.errors import CudaSafetyError
+from .split_kv_attention import UNSPLIT_MAX_CONTEXT
 
 FLAG_PREFETCH_Q = 8
 FLAG_WAIT_FIRST = 32
@@ -92,7 +93,8 @@ class LeanRoute:
 
 CLUSTER_PARTS = (2, 3, 4, 5, 6, 8, 9, 12, 16)              # more than 8 only where the device has room for such clusters
 LEAN_SPLIT_MAX_CONTEXT = 131072
-APPEND_US = 2.0                                            # the append launch that the other routes have
+APPEND_US = 2.0                                            # the append launch that the other routes have,
+SMALL_APPEND_US = 0.5                                      # in front of the one launch of a small cache
 MARGIN = 0.95                                              # a route has to be estimated this much below the dispatcher's launches
 
 
@@ -120,15 +122,20 @@ def choose_lean_route(d, append: bool) -> tuple:
 
     Clusters win wherever latency counts: a layer is one dependent launch of 3.3 us instead of two or three (7.1).  They
     lose to the dispatcher's equal shares where a batch streams for a hundred microseconds, because a cluster's CTAs stay
-    with their sequence, and to split and combine for one long sequence, whose parts fill the GPU."""
+    with their sequence, and to split and combine for one long sequence, whose parts fill the GPU.  Up to
+    UNSPLIT_MAX_CONTEXT positions the dispatcher's layer is one launch too, and many clusters take longer to start than
+    its CTAs: 64 sequences of 32 heads on 8 of 64, room for 16 positions 4.9 us, in clusters 15.9.."""
     Hq, Hkv, D, batch, context = d.num_q_heads, d.num_kv_heads, d.head_dim, d.batch_size, d.context_length
     if Hkv <= 0 or Hq % Hkv or D not in (64, 128, 256):
         return 0, 0
     best, route = MARGIN * (d.hip.lean_estimate(-1, 0, Hq, Hkv, D, batch, context, 0) + (APPEND_US if append else 0.0)), (0, 0)
     load = lambda name: d.codegen.load_kernel_safe(d.hip, 'decode_attention', d.hip.get_gpu_architecture(), name)[1]
-    for us, kind, parts, *_ in cluster_options(d.hip, load, Hq, Hkv, D, batch, context, best):
+    for us, kind, parts, _, _, resident in cluster_options(d.hip, load, Hq, Hkv, D, batch, context, best):
         if us < best:
-            best, route = us, (parts, kind)
+            best, route, clusters = us, (parts, kind), resident
+    if context <= UNSPLIT_MAX_CONTEXT and route[0]:
+        us = lambda kind, parts, resident: d.hip.lean_step_estimate(kind, parts, Hq, Hkv, D, batch, context, context, batch * context, resident)
+        return route if us(route[1], route[0], clusters) <= MARGIN * (us(-1, 0, 0) + (SMALL_APPEND_US if append else 0.0)) else (0, 0)
     parts = d.num_sms // Hkv
     if (batch == 1 and context <= LEAN_SPLIT_MAX_CONTEXT and 1 < parts <= d.max_chunks and d.hip.lean_plan(Hq, Hkv, D, parts, context, SPLIT).ok
             and d.hip.lean_estimate(SPLIT, parts, Hq, Hkv, D, 1, context, 0) < best):

@@ -95,6 +95,55 @@ inline double lean_estimate_us(int kind, int n_parts, int num_q_heads, int num_k
 }
 constexpr double kLeanMargin = 0.95;       // a route has to be estimated this much below kind -1
 
+// The same where the lengths are known: the longest sequence has `longest` positions, all together `total`, in caches with room
+// for `capacity`.  Fitted to 3,444 steps of 8 head geometries, 1 to 64 sequences, room for 16 to 65,536 positions, lengths
+// all the same, uniform, one or a quarter of them long and the others a fiftieth to a twentieth of it, up to 19 routes timed on
+// each: 90 % within a sixth.  Of 2,340 batches in caches above 128 positions, the clusters chosen by capacity took up to 3.3
+// times as long as kind -1 and longer than 1.03 times in 252; where every step takes the one that this finds shorter (by
+// kLeanMargin), at most 1.28 times and in 20.
+//   a cluster layer: its longest part, the starts of all clusters and the bytes overlap (a p-norm); every further wave costs as
+//   much again; merges and starts grow with the query heads of a KV head
+//   kind -1: bytes over a rate, what grows with the work items and with the longest over the mean length; up to 128 positions it
+//   is one launch that stores the output itself
+struct LeanStepFit { double base, per_position, per_pair, wave, bytes_per_us, norm, base_8, per_pair_8, wave_8; };   // _8: for eight query heads a KV head
+struct PlainStepFit { double base, bytes_per_us, per_pair_log, per_row, skew, longest_log; };
+inline double lean_step_us(int kind, int n_parts, int num_q_heads, int num_kv_heads, int head_dim, int batch, long long capacity, long long longest,
+                           double total, int resident) {
+    const int runs = num_q_heads > 8 * num_kv_heads ? 1 : 0, d = head_dim == 64 ? 0 : head_dim == 128 ? 1 : 2;
+    const double pairs = (double)batch * num_kv_heads, bytes = total * num_kv_heads * 4.0 * head_dim, g = num_q_heads / (8.0 * num_kv_heads);
+    if (kind < 0 && capacity <= 128) {
+        static const double kSmall[2][3][4] = {{{2.55, .0205, .10, 0.}, {3.4, .0135, .09, .26}, {3.9, .0075, .19, 0.}},
+                                               {{3.2, .0045, .06, 0.}, {4.45, .011, .25, .3}, {4.45, .011, .25, .3}}};
+        const double* c = kSmall[runs][d];
+        return c[0] + c[1] * (double)longest + c[2] * std::log2((double)batch) + c[3] * pairs / 148.0;
+    }
+    if (kind < 0) {
+        static const PlainStepFit kOne[2][3] = {{{3.52, 6.87e6, .25, .0027, 0., .25}, {4.42, 7.41e6, .01, .0557, 0., .31}, {5.44, 7.88e6, 0., 0., 0., .36}},
+                                                {{5.88, 7.37e6, .25, .002, 0., .50}, {6.42, 7.36e6, .64, .006, 0., .75}, {6.42, 7.36e6, .64, .006, 0., .75}}};
+        static const PlainStepFit kBatch[2][3] = {{{3.37, 7.20e6, .89, .0005, .65, .42}, {7.28, 7.13e6, .25, .0057, .80, .48}, {9.51, 7.32e6, .04, .0102, 1.20, .32}},
+                                                  {{6.94, 4.02e6, .66, .0023, .66, .26}, {7.89, 5.75e6, 1.15, 0., .83, .68}, {7.89, 5.75e6, 1.15, 0., .83, .68}}};
+        const PlainStepFit& c = batch == 1 ? kOne[runs][d] : kBatch[runs][d];
+        const double skew = (double)longest * batch / total;
+        return c.base + bytes / c.bytes_per_us + c.per_pair_log * std::log2(pairs) + c.per_row * batch * num_q_heads +
+               c.skew * std::log2(skew > 1.0 ? skew : 1.0) + c.longest_log * std::log2(longest > 512 ? longest / 512.0 : 1.0);
+    }
+    if (kind == kLeanSplit) {
+        const double stream = bytes / 8.0e6, walk = 0.62 * (d == 0 ? 0.0045 : d == 1 ? 0.00706 : 0.0168) * (double)longest / n_parts;
+        return 4.8 + 0.0117 * head_dim + (stream > walk ? stream : walk);
+    }
+    static const LeanStepFit kCluster[2][3] = {{{2.84, .0038, .0057, 2.80, 6.56e6, 2.0, .29, .0014, .14}, {2.96, .0055, .0062, 2.95, 6.66e6, 3.2, .61, .0118, .56},
+                                                {2.99, .0121, .0147, 2.93, 5.95e6, 3.4, 1.51, .0329, .95}},
+                                               {{2.90, .0060, .0194, 2.34, 4.39e6, 2.0, .34, .0035, .44}, {3.25, .0080, .0051, 2.99, 5.24e6, 2.8, .73, .0149, .59},
+                                                {3.25, .0080, .0051, 2.99, 5.24e6, 2.8, .73, .0149, .59}}};
+    static const LeanStepFit kHalf[2][2] = {{{2.76, .0078, .0046, 2.41, 7.00e6, 2.0, .66, .0139, .84}, {3.35, .0165, .0048, 2.93, 6.53e6, 2.0, 1.67, .0417, 1.30}},
+                                            {{3.24, .0125, .0092, 2.92, 6.60e6, 3.0, .80, .0143, .76}, {3.24, .0125, .0092, 2.92, 6.60e6, 3.0, .80, .0143, .76}}};
+    const LeanStepFit& c = kind == kLeanHalf ? kHalf[runs][d == 2 ? 1 : 0] : kCluster[runs][d];
+    const double waves = resident > 0 ? std::ceil(pairs / resident) : 1e9;
+    const double part = c.per_position * (double)longest / n_parts, start = (c.per_pair + c.per_pair_8 * g) * pairs, stream = bytes / c.bytes_per_us;
+    return c.base + c.base_8 * g + std::pow(std::pow(part, c.norm) + std::pow(start, c.norm) + std::pow(stream, c.norm), 1.0 / c.norm) +
+           (c.wave + c.wave_8 * g) * (waves - 1.0);
+}
+
 // Where a launch without a status word of its own (flash_attention_kernel's arguments have none) reports a wait that ran
 // out; read by vteb_module_check_status.
 extern "C" { __device__ int vteb_lean_status = 0; }

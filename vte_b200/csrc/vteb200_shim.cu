@@ -612,6 +612,11 @@ double vteb_lean_estimate(int kind, int n_parts, int num_q_heads, int num_kv_hea
     return lean_estimate_us(kind, n_parts, num_q_heads, num_kv_heads, head_dim, batch, context, resident, num_sms);
 }
 
+double vteb_lean_step_estimate(int kind, int n_parts, int num_q_heads, int num_kv_heads, int head_dim, int batch, long long capacity,
+                               long long longest, long long total, int resident) {
+    return lean_step_us(kind, n_parts, num_q_heads, num_kv_heads, head_dim, batch, capacity, longest, (double)total, resident);
+}
+
 int vteb_max_active_clusters(void* function, int cluster, int threads, int smem_bytes, int* count) {
     REQUIRE_INIT();
     if (!function || !count || cluster < 1 || cluster > 16 || threads < 1 || smem_bytes < 0)

@@ -95,6 +95,27 @@ def test_small_caches_keep_the_one_launch_that_is_shorter(built_library):
         assert route((12, 2, 128), 1, 128, append=append)[1] and route((28, 4, 128), 8, 128, append=append)[1]
 
 
+def chosen_route(heads, batch, capacity, append=True):
+    d = FakeDispatcher(heads, batch, capacity)
+    parts, kind = choose_lean_route(d, append)
+    return LeanRoute(d, parts, kind, append)
+
+
+def test_one_long_sequence_among_short_ones_leaves_the_clusters(built_library):
+    """Timed, clusters / dispatcher, us a layer, append included: 71 / 29, 74 / 33, 46 / 37, 40 / 23; with all sequences
+    short 6.8 / 14, 7.6 / 15, 5.5 / 15, 7.7 / 15."""
+    for heads, batch, capacity, others in (((12, 2, 128), 32, 32768, 500), ((12, 2, 128), 16, 65536, 1000),
+                                           ((28, 4, 128), 8, 32768, 500), ((8, 2, 256), 16, 16384, 400)):
+        route = chosen_route(heads, batch, capacity)
+        assert route.cluster
+        assert not route.pays(capacity, capacity + (batch - 1) * others) and route.pays(others, batch * others)
+        known = route.pays_up_to()
+        assert others < known < capacity and route.pays(known, known + batch - 1) and route.pays(known, known * batch)
+    for heads, batch, capacity in (((12, 2, 128), 8, 2048), ((28, 4, 128), 4, 4096), ((32, 2, 128), 8, 4096), ((12, 2, 128), 8, 128)):
+        assert chosen_route(heads, batch, capacity).pays_up_to() == capacity       # no lengths for which they do not
+    assert chosen_route((12, 2, 128), 1, 16384).pays_up_to() == 16384              # one sequence, split and combine
+
+
 def test_a_forced_split_route_stays_within_the_partial_buffers(built_library):
     """Each (sequence, query head) has room for max_chunks partials: one sequence of up to 2,048 positions for 32."""
     d = FakeDispatcher((12, 2, 128), 1, 2048)
@@ -349,6 +370,50 @@ def test_partials_after_a_routed_step_are_the_step_s_own(cuda_runtime, codegen, 
         used = l[1] > 0
         assert used.any() and np.array_equal(used, l[0] > 0)
         assert np.array_equal(m[0][used], m[1][used]) and np.array_equal(l[0], l[1]) and np.array_equal(o[0][used], o[1][used])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rope", ["off", "fused-append"])
+@pytest.mark.parametrize("from_host", [False, True])
+def test_each_step_takes_the_route_that_its_lengths_ask_for(cuda_runtime, codegen, rope, from_host):
+    """Steps of one executor, long among short and all short in turn: the oracle's outputs, the newest rows, the step's own
+    partials, and as many launches as the route has.  fp32 sums of fp16 products: 2e-5 of the result's norm."""
+    heads, B, S, L = (8, 2, 256), 16, 16384, 2
+    Hq, Hkv, D = heads
+    rng = np.random.default_rng(2)
+    f16 = lambda *s: rng.standard_normal(s, dtype=np.float32).astype(np.float16)
+    k, v = np.zeros((B, S, Hkv, D), np.float16), np.zeros((B, S, Hkv, D), np.float16)
+    k[:, :600], v[:, :600], k[3], v[3] = f16(B, 600, Hkv, D), f16(B, 600, Hkv, D), f16(S, Hkv, D), f16(S, Hkv, D)
+    ex = DecodeAttentionExecutor(cuda_runtime, codegen, {"attention.head_count": Hq, "attention.head_count_kv": Hkv,
+                                                         "attention.key_length": D}, B, S, L, n_kv_buffers=1, with_append=True, rope=rope)
+    if rope != "off":
+        cos, sin = orc.rope_tables(S, D, 1e6)
+    try:
+        ex.upload_cache(0, k, v)
+        for step, longest in enumerate((500, S - 3, 500, S - 2)):
+            q, kn, vn = f16(L, B, Hq, D), f16(L, B, Hkv, D), f16(L, B, Hkv, D)
+            off = rng.integers(300, 500, B).astype(np.int32)
+            off[3] = longest - 1
+            for l in range(L):
+                ex.upload_new_kv(l, kn[l], vn[l])
+                ex.upload_layer(l, q[l])
+            out = ex.execute_decode_batch(off, q if from_host else None)
+            skewed = longest > 500
+            assert (ex.route_name is None) == skewed
+            assert ex.kernel_launches_per_step == (L * (2 if rope != "off" else 3) if skewed else L)
+            for l in range(L):
+                ql, kl = (q[l], kn[l]) if rope == "off" else orc.rope_step(q[l], kn[l], cos, sin, off, 0, D)
+                orc.kv_cache_append(kl, vn[l], k, v, off)
+                ref = orc.decode_attention(ql, k, v, off)
+                assert np.linalg.norm(out[l] - ref) <= 2e-5 * np.linalg.norm(ref)
+            m, lsum, o = ex.read_partials()
+            w = np.exp(np.where(lsum > 0, m, -np.inf) - m.max(axis=2, keepdims=True))
+            whole = (np.where(lsum > 0, w, 0)[..., None] * np.where((lsum > 0)[..., None], o, 0)).sum(axis=2) / (w * lsum).sum(axis=2)[..., None]
+            assert np.linalg.norm(whole - out[L - 1]) <= 2e-5 * np.linalg.norm(out[L - 1])
+        rows_k, rows_v = ex.download_cache_rows(0, 3, S - 1)
+        assert np.array_equal(rows_k, k[3, :S - 1]) and np.array_equal(rows_v, v[3, :S - 1])
+    finally:
+        ex.cleanup()
 
 
 @pytest.mark.gpu

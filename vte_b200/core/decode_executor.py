@@ -124,7 +124,11 @@ class DecodeAttentionExecutor:
                            wide is not None) and (fixed_chunk_size is None and min_chunk is None and variant == "auto" and
                                                   tensor_maps and prefetch_next_layer)
         self._lean = lean if lean is not None else None if open_layout else (0, 0)
-        self._route = None
+        self._route, self._forced_route = None, lean is not None
+        # where lengths can make the dispatcher's launches the shorter ones: a step of those is captured beside the route's, and
+        # each step takes one by its longest and total length; up to _route_pays_to positions it is the route's in any case
+        self._route_pays_to, self._on_route, self._launches = self.S, True, (0, 0)
+        self._plain_graph_exec = self._plain_io_graph_exec = None
         # what partials of a routed step can be had from: the last layer's Q and offsets as the step saw them, the names it
         # was captured with, and whether the partial buffers are still to be filled
         self._kept, self._kept_names, self._partials_due = None, None, False
@@ -228,9 +232,9 @@ class DecodeAttentionExecutor:
         finally:
             self.hip.programmatic_launch = programmatic
 
-    def layer_launches(self, layer: int):
-        """What a step launches for a layer (without a rotation launch of its own)."""
-        if self._route is not None and self.dispatcher.offsets_final:
+    def layer_launches(self, layer: int, plain: bool = False):
+        """What a step launches for a layer (without a rotation launch of its own); `plain`: in the dispatcher's launches."""
+        if self._route is not None and not plain and self.dispatcher.offsets_final:
             last = layer == self.L - 1
             launches = self._route.launches(layer, self.tensor_mapping, self.offsets.ptr, self.B,
                                             (self._kept.ptr, self._kept.ptr + _round_up(self.q_bytes, 256)) if last else (0, 0))
@@ -242,16 +246,16 @@ class DecodeAttentionExecutor:
 
     @property
     def route_name(self):
-        """(kernel, CTAs per (sequence, KV head)) where a captured step does not take the dispatcher's launches, else None."""
-        return (self._route.name, self._route.parts) if self._route is not None else None
+        """(kernel, CTAs per (sequence, KV head)) where the last captured step did not take the dispatcher's launches, else None."""
+        return (self._route.name, self._route.parts) if self._route is not None and self._on_route else None
 
-    def _record_all(self, after_copy: bool = False):
+    def _record_all(self, after_copy: bool = False, plain: bool = False):
         n = 0
         programmatic = self.hip.programmatic_launch
         # within a captured step of nothing but the layers' own launches, offsets and older rows do not change
         self.dispatcher.offsets_final = self.use_graph and self.per_layer_hook is None and self.launch_rewriter is None
         for l in range(self.L):
-            launches = self.layer_launches(l)
+            launches = self.layer_launches(l, plain)
             if self.launch_rewriter is not None:
                 launches = self.launch_rewriter(l, launches)
             if self.rope == "separate":
@@ -281,6 +285,8 @@ class DecodeAttentionExecutor:
             self._lean = choose_lean_route(d, append)
         if self._lean[0]:
             self._route = LeanRoute(d, *self._lean, append)
+            if not self._forced_route:
+                self._route_pays_to = self._route.pays_up_to()
             self._kept = self.allocator.allocate(_round_up(self.q_bytes, 256) + _round_up(4 * self.B, 256), "attn_partials_source",
                                                  MemoryRegion.SCRATCH)
 
@@ -296,15 +302,32 @@ class DecodeAttentionExecutor:
                 self.kernel_launches_per_step = (n if (self.with_append or self.dispatcher.fuse_append) else n - 1) * self.L
                 return
             self._choose_route()
-            self.hip.stream_begin_capture()
-            try:
-                self.kernel_launches_per_step = self._record_all()
-            finally:
-                graph = self.hip.stream_end_capture()
-            self._graph_exec = self.hip.graph_instantiate(graph)
-            self.hip.graph_destroy(graph)
+            self._graph_exec, n = self._capture(self._record_all)
+            plain = n
+            if self._route_pays_to < self.S:
+                self._plain_graph_exec, plain = self._capture(lambda: self._record_all(plain=True))
+            self._launches = n, plain
+            self.kernel_launches_per_step = n
         finally:
             self.hip.programmatic_launch = False
+
+    def _capture(self, record):
+        """(executable graph, what `record` returns) of what `record` launches."""
+        self.hip.stream_begin_capture()
+        try:
+            n = record()
+        finally:
+            graph = self.hip.stream_end_capture()
+        graph_exec = self.hip.graph_instantiate(graph)
+        self.hip.graph_destroy(graph)
+        return graph_exec, n
+
+    def _pick(self, offsets: np.ndarray, newest: int):
+        """Which of the captured steps serves these offsets, the largest of which is `newest`."""
+        self._on_route = self._route is not None and (newest < self._route_pays_to or
+                                                      self._route.pays(newest + 1, int(offsets.sum(dtype=np.int64)) + self.B))
+        if self._plain_graph_exec is not None:
+            self.kernel_launches_per_step = self._launches[not self._on_route]
 
     def build_io_graph(self):
         """One graph for a whole end-to-end step: kv offsets and every layer's Q from pinned
@@ -321,24 +344,23 @@ class DecodeAttentionExecutor:
         self._choose_route()
         self.hip.programmatic_launch = self.programmatic
         try:
-            self.hip.stream_begin_capture()
-            try:
-                if max(self._q_tail, self._out_tail) <= STAGE_COPY_MAX_BYTES:
-                    self._stage_copy(self.q_all.ptr, self._stage_q.value, self._q_tail + 4 * self.B, first=True)
-                    self._record_all(after_copy=True)
-                    self._stage_copy(self._stage_out.value, self.out_all.ptr, self._out_tail + 16)
-                else:
-                    self.hip.memcpy_h2d_async(ctypes.c_void_p(self.q_all.ptr), self._stage_q, self._q_tail + 4 * self.B,
-                                              "q and kv offsets staging")
-                    self._record_all()
-                    self.hip.memcpy_d2h_async(self._stage_out, ctypes.c_void_p(self.out_all.ptr), self._out_tail + 16,
-                                              "attention output and status word")
-            finally:
-                graph = self.hip.stream_end_capture()
-            self._io_graph_exec = self.hip.graph_instantiate(graph)
-            self.hip.graph_destroy(graph)
+            self._io_graph_exec, _ = self._capture(self._record_io)
+            if self._route_pays_to < self.S:
+                self._plain_io_graph_exec, _ = self._capture(lambda: self._record_io(plain=True))
         finally:
             self.hip.programmatic_launch = False
+
+    def _record_io(self, plain: bool = False):
+        if max(self._q_tail, self._out_tail) <= STAGE_COPY_MAX_BYTES:
+            self._stage_copy(self.q_all.ptr, self._stage_q.value, self._q_tail + 4 * self.B, first=True)
+            self._record_all(after_copy=True, plain=plain)
+            self._stage_copy(self._stage_out.value, self.out_all.ptr, self._out_tail + 16)
+        else:
+            self.hip.memcpy_h2d_async(ctypes.c_void_p(self.q_all.ptr), self._stage_q, self._q_tail + 4 * self.B,
+                                      "q and kv offsets staging")
+            self._record_all(plain=plain)
+            self.hip.memcpy_d2h_async(self._stage_out, ctypes.c_void_p(self.out_all.ptr), self._out_tail + 16,
+                                      "attention output and status word")
 
     def _wait_for_staging(self):
         """The pinned Q staging may be rewritten only after the previous step's asynchronous copy has read it (a step
@@ -357,8 +379,10 @@ class DecodeAttentionExecutor:
         off = np.ascontiguousarray(kv_offsets, dtype=np.int32)
         if off.shape != (self.B,):
             raise CudaSafetyError(f"kv_offsets shape {off.shape} != ({self.B},)")
-        if off.min() < 0 or off.max() >= self.S:
+        newest = int(off.max())
+        if off.min() < 0 or newest >= self.S:
             raise CudaSafetyError(f"kv offset outside 0..{self.S - 1}")
+        self._pick(off, newest)
         half, slot = divmod(self._offset_slot, OFFSET_SLOTS // 2)
         if slot == 0 and self._offset_events[half] is not None:
             self.hip.event_synchronize(self._offset_events[half])
@@ -374,8 +398,9 @@ class DecodeAttentionExecutor:
     def launch_step(self):
         """Enqueue one decode step (no host synchronisation)."""
         if self._graph_exec is not None:
-            self.hip.graph_launch(self._graph_exec)
-            self._partials_due = self._kept_names is not None
+            plain = self._plain_graph_exec is not None and not self._on_route
+            self.hip.graph_launch(self._plain_graph_exec if plain else self._graph_exec)
+            self._partials_due = self._kept_names is not None and not plain
         else:
             self.hip.programmatic_launch = self.programmatic
             try:
@@ -394,7 +419,8 @@ class DecodeAttentionExecutor:
             # the whole step as one graph launch
             self.build_io_graph()
             off = np.ascontiguousarray(kv_offsets, dtype=np.int32)
-            if off.shape != (self.B,) or off.min() < 0 or off.max() >= self.S:
+            newest = int(off.max()) if off.shape == (self.B,) else self.S
+            if newest >= self.S or off.min() < 0:
                 raise CudaSafetyError(f"kv_offsets must be int32[{self.B}] within 0..{self.S - 1}")
             qh = np.ascontiguousarray(q_host, dtype=np.float16)
             if qh.nbytes != self.L * self.q_bytes:
@@ -402,8 +428,10 @@ class DecodeAttentionExecutor:
             self._wait_for_staging()
             ctypes.memmove(self._stage_offsets.value, off.ctypes.data, off.nbytes)
             ctypes.memmove(self._stage_q.value, qh.ctypes.data, qh.nbytes)
-            self.hip.graph_launch(self._io_graph_exec)
-            self._partials_due = self._kept_names is not None
+            self._pick(off, newest)
+            plain = self._plain_io_graph_exec is not None and not self._on_route
+            self.hip.graph_launch(self._plain_io_graph_exec if plain else self._io_graph_exec)
+            self._partials_due = self._kept_names is not None and not plain
             self.hip.stream_synchronize()
             # the status word travelled with the outputs: only a non-zero one needs the slow path
             if ctypes.c_int.from_address(self._stage_out.value + self._out_tail + 4).value != 0:
@@ -486,6 +514,10 @@ class DecodeAttentionExecutor:
         if self._io_graph_exec is not None:
             self.hip.graph_exec_destroy(self._io_graph_exec)
             self._io_graph_exec = None
+        for graph_exec in (self._plain_graph_exec, self._plain_io_graph_exec):
+            if graph_exec is not None:
+                self.hip.graph_exec_destroy(graph_exec)
+        self._plain_graph_exec = self._plain_io_graph_exec = None
         for i, event in enumerate(self._offset_events):
             if event is not None:
                 self.hip.event_synchronize(event)

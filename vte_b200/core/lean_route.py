@@ -32,7 +32,7 @@ class LeanRoute:
 
     def __init__(self, dispatcher, parts: int, kind: int, append: bool):
         d = self.d = dispatcher
-        self.parts, self.append, self.cluster = int(parts), bool(append), kind != SPLIT
+        self.parts, self.kind, self.append, self.cluster = int(parts), int(kind), bool(append), kind != SPLIT
         self.plan = d.hip.lean_plan(d.num_q_heads, d.num_kv_heads, d.head_dim, self.parts, d.context_length, kind)
         if not self.plan.ok:
             raise CudaSafetyError(f"{self.parts} CTAs per (sequence, KV head) are not covered for this geometry")
@@ -41,10 +41,35 @@ class LeanRoute:
         load = lambda symbol: d.codegen.load_kernel_safe(d.hip, 'decode_attention', d.hip.get_gpu_architecture(), symbol)[1]
         self.name = (cluster_kernel_name(kind, d.num_q_heads // d.num_kv_heads, d.head_dim) if self.cluster
                      else f"vteb_split_kv_lean_d{d.head_dim}_kernel")
-        self.function = load(self.name)
+        self.function, self._resident = load(self.name), None
         if not self.cluster:
             self.combine = load('vteb_split_kv_combine_small_kernel' if self.parts <= 32 else
                                 'vteb_split_kv_combine_f32_kernel' if d.output_f32 else 'vteb_split_kv_combine_f16_kernel')
+
+    def pays(self, longest: int, total: int) -> bool:
+        """Whether a step whose longest sequence has `longest` positions, and all together `total`, is estimated shorter on
+        this route than in the dispatcher's launches.  A route is chosen by capacity, but its CTAs stay with their sequence: one
+        long sequence among short ones takes as long as its parts, where equal shares spread it over the GPU (32 sequences of
+        12 heads on 2 of 128, one of 32,768 positions, 31 of 500: 71 us a layer in clusters, 29)."""
+        d = self.d
+        if not self.cluster or d.context_length <= UNSPLIT_MAX_CONTEXT:
+            return True
+        us = lambda kind, parts, resident: d.hip.lean_step_estimate(kind, parts, d.num_q_heads, d.num_kv_heads, d.head_dim, d.batch_size,
+                                                                    d.context_length, longest, total, resident)
+        if self._resident is None:
+            self._resident = d.hip.max_active_clusters(self.function, self.parts, self.plan.threads, self.plan.smem_bytes)
+        return us(self.kind, self.parts, self._resident) <= MARGIN * (us(-1, 0, 0) + (LEAST_APPEND_US if self.append else 0.0))
+
+    def pays_up_to(self) -> int:
+        """A length up to which the route pays whatever the other sequences have."""
+        batch, lo, hi = self.d.batch_size, 0, self.d.context_length
+        while lo < hi:
+            mid = (lo + hi + 1) // 2
+            if self.pays(mid, mid + batch - 1) and self.pays(mid, mid * batch):
+                lo = mid
+            else:
+                hi = mid - 1
+        return lo
 
     def launches(self, layer: int, tensor_mapping: dict, kv_offset_ptr: int, batch: int, keep: tuple = (0, 0)):
         """`keep`: where the kernel leaves a copy of Q and of the offsets, for a layer whose partials may be asked for."""
@@ -94,6 +119,7 @@ class LeanRoute:
 CLUSTER_PARTS = (2, 3, 4, 5, 6, 8, 9, 12, 16)              # more than 8 only where the device has room for such clusters
 LEAN_SPLIT_MAX_CONTEXT = 131072
 APPEND_US = 2.0                                            # the append launch that the other routes have,
+LEAST_APPEND_US = 1.5                                      # at the least,
 SMALL_APPEND_US = 0.5                                      # in front of the one launch of a small cache
 MARGIN = 0.95                                              # a route has to be estimated this much below the dispatcher's launches
 

@@ -222,9 +222,11 @@ int vteb_combine_rows_epl(int rows, int head_dim);
 #define VTEB_ATTN_BALANCED 64   /* several sequences: every CTA takes an equal share of all cached positions; a
                                    (sequence, KV head group) is cut where shares end, into at most max_chunks
                                    splits (max_chunks >= 2; min_chunk is ignored); no work queue.  With no other
-                                   flag but VTEB_ATTN_PROGRAMMATIC and n_ctas <= 0, a call that thread-block
-                                   clusters serve faster (vteb_lean_estimate; kv_batch_stride stands for the
-                                   context) is ONE launch of those, which leaves the scratch as it is */
+                                   flag but VTEB_ATTN_PROGRAMMATIC and n_ctas <= 0, a call
+                                   that thread-block clusters serve faster whatever the lengths are
+                                   (vteb_lean_estimate, vteb_lean_step_estimate; kv_batch_stride stands for the
+                                   context) is ONE launch of those, which leaves the scratch as it is.  n_ctas = the
+                                   number of SMs asks for the equal shares themselves */
 int vteb_split_kv_decode(const void* q, const void* k_cache, const void* v_cache,
                          const int* kv_offsets, void* output, int out_is_f32,
                          float* partial_m, float* partial_l, float* partial_o, int* work,

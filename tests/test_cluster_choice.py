@@ -11,11 +11,12 @@ HARNESS = r"""
 #include <cstdio>
 #include "cluster_choice.h"
 
-static int queries = 0, failing = 0;
+static int queries = 0, failing = 0, slower_up_to = 0;
 static ClusterChoice ask(ClusterChoices& c, int device, long long context) {
     const ClusterCall call = {device, 12, 2, 128, 4, 148, context};
     return c.choose(call, 10.0,
         [&](int kind, int parts, int resident) { return kind == 2 && parts == 16 ? -1.0 : resident < 8 ? 50.0 : 12.0 / parts + kind; },
+        [&](int kind, int parts, int resident) { return parts > slower_up_to && resident > 0; },
         [&](int kind, int parts, int* n) { ++queries; *n = parts > 9 ? 4 : 16; return !(failing == 1 || (failing == 2 && parts == 9)); });
 }
 #define SAY(x) std::printf("%s %d\n", #x, (int)(x))
@@ -29,6 +30,9 @@ int main() {
     failing = 2; SAY(ask(c, 0, 5000).parts);                // one answer missing: the next best
     failing = 1; SAY(ask(c, 0, 5000).parts);                // none to be had
     failing = 0; SAY(ask(c, 0, 5000).parts);                // neither was recorded
+    slower_up_to = 8; SAY(ask(c, 2, 4096).parts);           // what a skewed batch could make slower is passed over,
+    slower_up_to = 9; SAY(ask(c, 2, 5000).parts);           // down to no clusters at all
+    slower_up_to = 0;
     for (int i = 0; i < 1000; ++i) ask(c, 0, 6000 + i);
     before = queries; ask(c, 0, 6999); SAY(queries - before);        // the last is known,
     ask(c, 0, 4096); SAY(queries - before > 0);                      // the first of a thousand not any more
@@ -46,4 +50,4 @@ def said(tmp_path_factory):
 
 
 def test_choices_are_kept_for_each_device_and_only_when_every_candidate_answered(said):
-    assert said == ["1", "9", "0", "1", "8", "0", "9", "0", "1"]
+    assert said == ["1", "9", "0", "1", "8", "0", "9", "9", "0", "0", "1"]

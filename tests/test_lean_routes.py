@@ -553,3 +553,24 @@ def test_balanced_calls_through_the_direct_entry_point(cuda_runtime, heads, B, S
     orc.kv_cache_append(kn, vn, k, v, off)
     ref = orc.decode_attention(q, k, v, off)
     assert np.linalg.norm(out - ref) <= (2e-5 if f32 else 5e-4) * np.linalg.norm(ref)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("heads,B,S,clusters", [((28, 4, 128), 32, 4096, True), ((12, 2, 128), 8, 2048, True), ((12, 2, 128), 32, 32768, False),
+                                                ((8, 2, 256), 16, 16384, False)])
+def test_balanced_calls_that_a_long_sequence_could_slow_keep_the_equal_shares(cuda_runtime, heads, B, S, clusters):
+    """The entry point sees no lengths.  Launches are captured and counted, not run: one of clusters, or split and combine,
+    which a caller gets in any case who names the number of CTAs."""
+    from vte_b200.bridge.cuda_runtime import ATTN_BALANCED, ATTN_PROGRAMMATIC
+    rt, (Hq, Hkv, D) = cuda_runtime, heads
+    p = rt.safe_malloc(4096, "direct entry output")
+    try:
+        for n_ctas, nodes in ((0, 1 if clusters else 2), (rt.get_num_cus(), 2)):
+            rt.stream_begin_capture()
+            rt.split_kv_decode(p, p, p, p, p, True, p, p, p, p, B, Hq, Hkv, D, 1 / math.sqrt(D), S * Hkv * D, 8, 0,
+                               ATTN_BALANCED | ATTN_PROGRAMMATIC, n_ctas)
+            graph = rt.stream_end_capture()
+            assert rt.graph_node_count(graph) == nodes
+            rt.graph_destroy(graph)
+    finally:
+        rt.safe_free(p, "direct entry cleanup")

@@ -19,10 +19,11 @@ struct ClusterChoice { int kind, parts; };            // parts 0: no clusters
 class ClusterChoices {
 public:
     // `estimate(kind, parts, resident)`: microseconds, negative where the kernels do not cover the geometry.
+    // `never_slower(kind, parts, resident)`: whether that holds whatever the lengths are, which the host does not see here.
     // `resident(kind, parts, &n)`: readies the kernel on the device and says how many clusters run at once; false where
     // that cannot be had, and then another answer serves the call and nothing is recorded.
-    template <class Estimate, class Resident>
-    ClusterChoice choose(const ClusterCall& call, double below, Estimate estimate, Resident resident) {
+    template <class Estimate, class NeverSlower, class Resident>
+    ClusterChoice choose(const ClusterCall& call, double below, Estimate estimate, NeverSlower never_slower, Resident resident) {
         ClusterChoice best = {0, 0};
         bool found = false;
         pthread_mutex_lock(&lock_);
@@ -39,7 +40,7 @@ public:
                 int n = 0;
                 if (!resident(kind, parts, &n)) { all_answered = false; continue; }
                 const double us = n > 0 ? estimate(kind, parts, n) : below;
-                if (us < below) { below = us; best.kind = kind; best.parts = parts; }
+                if (us < below && never_slower(kind, parts, n)) { below = us; best.kind = kind; best.parts = parts; }
             }
         if (all_answered) {
             pthread_mutex_lock(&lock_);

@@ -696,6 +696,15 @@ static ClusterChoice choose_clusters(int hq, int hkv, int d, int batch, long lon
     const auto estimate = [&](int kind, int parts, int resident) {
         return make_lean_plan(hq, hkv, d, parts, context, kind).ok ? lean_estimate_us(kind, parts, hq, hkv, d, batch, context, resident, sms) : -1.0;
     };
+    // One sequence at its capacity among short ones, and all at theirs: between them a batch is.  32 sequences of 12 heads on
+    // 2 of 128 with room for 32,768, one full and 31 of 500: 31 us in equal shares, 74 in clusters of four half blocks.
+    const auto never_slower = [&](int kind, int parts, int n) {
+        const long long split = context > 128 ? context : 129;       // kind -1 is split and combine here at any capacity
+        for (const double total : {(double)context + batch - 1, (double)context * batch})
+            if (lean_step_us(kind, parts, hq, hkv, d, batch, context, context, total, n) >
+                lean_step_us(-1, 0, hq, hkv, d, batch, split, context, total, 0)) return false;
+        return true;
+    };
     const auto resident = [&](int kind, int parts, int* n) {
         const LeanKernel fn = lean_cluster_kernel(kind, d);
         const LeanPlan p = make_lean_plan(hq, hkv, d, parts, context, kind);
@@ -712,7 +721,8 @@ static ClusterChoice choose_clusters(int hq, int hkv, int d, int batch, long lon
         cudaGetLastError();                              // not to be had here: another route serves the call
         return false;
     };
-    return g_cluster_choices.choose(call, kLeanMargin * lean_estimate_us(-1, 0, hq, hkv, d, batch, context, 0, sms), estimate, resident);
+    return g_cluster_choices.choose(call, kLeanMargin * lean_estimate_us(-1, 0, hq, hkv, d, batch, context, 0, sms), estimate,
+                                    never_slower, resident);
 }
 
 int vteb_split_kv_decode(const void* q, const void* k_cache, const void* v_cache, const int* kv_offsets,
@@ -777,7 +787,8 @@ int vteb_split_kv_decode(const void* q, const void* k_cache, const void* v_cache
     if (balanced && compact) return fail(VTEB_ERR_INVALID_ARGUMENT, "VTEB_ATTN_BALANCED and VTEB_ATTN_COMPACT exclude each other");
     // Equal shares over all SMs, partials and a combine, or a cluster per (sequence, KV head) that needs neither: whichever is
     // estimated shorter, where the caller asked for nothing that only the former has (32 sequences of 100 to 4,000
-    // positions, 28 heads on 4 of 128, append included: 38.8 us and 31.1).  The stride stands for the context.
+    // positions, 28 heads on 4 of 128, append included: 38.8 us and 31.1).  The stride stands for the context; clusters that a
+    // skewed batch could make the longer ones are not taken (choose_clusters).
     if (balanced && all_sms && kv_batch_stride > 0 && !(flags & ~(unsigned)(VTEB_ATTN_BALANCED | VTEB_ATTN_PROGRAMMATIC))) {
         const long long context = kv_batch_stride / ((long long)num_kv_heads * head_dim);
         ClusterChoice c = {0, 0};

@@ -70,6 +70,9 @@ def test_the_route_follows_the_size(built_library):
     assert route((12, 2, 128), 1, 4096) == (16, 1)                # one short sequence
     assert route((12, 2, 128), 1, 16384) == (74, 0)               # one long one: split and combine over the whole GPU
     assert route((12, 2, 128), 1, LEAN_SPLIT_MAX_CONTEXT + 1) == (0, 0)
+    alone = lambda *a: choose_lean_route(FakeDispatcher(*a), False)
+    assert alone((12, 2, 128), 1, 32768) == (74, 0) and alone((32, 8, 64), 1, 32768) == (18, 0) and alone((8, 2, 256), 1, 10000)[1] == 0
+    assert route((8, 2, 256), 1, 32768) == (74, 0) and alone((8, 2, 256), 1, 32768) == alone((16, 4, 64), 1, 32768) == (0, 0)
     assert route((32, 8, 64), 64, 16384) == (0, 0)                # a batch that streams: equal shares
     assert route((32, 2, 128), 8, 4096)[1] and route((12, 2, 128), 4, 2048)[1]
     assert route((8, 8, 128), 37, 624) == (2, 2)                  # many pairs: clusters of half blocks

@@ -118,6 +118,7 @@ class LeanRoute:
 
 CLUSTER_PARTS = (2, 3, 4, 5, 6, 8, 9, 12, 16)              # more than 8 only where the device has room for such clusters
 LEAN_SPLIT_MAX_CONTEXT = 131072
+SPLIT_ALONE_BYTES = 24 << 20                               # K and V rows in a cache up to which it pays without an append
 APPEND_US = 2.0                                            # the append launch that the other routes have,
 LEAST_APPEND_US = 1.5                                      # at the least,
 SMALL_APPEND_US = 0.5                                      # in front of the one launch of a small cache
@@ -150,7 +151,11 @@ def choose_lean_route(d, append: bool) -> tuple:
     lose to the dispatcher's equal shares where a batch streams for a hundred microseconds, because a cluster's CTAs stay
     with their sequence, and to split and combine for one long sequence, whose parts fill the GPU.  Up to
     UNSPLIT_MAX_CONTEXT positions the dispatcher's layer is one launch too, and many clusters take longer to start than
-    its CTAs: 64 sequences of 32 heads on 8 of 64, room for 16 positions 4.9 us, in clusters 15.9.."""
+    its CTAs: 64 sequences of 32 heads on 8 of 64, room for 16 positions 4.9 us, in clusters 15.9.
+
+    Split and combine of one KV head a CTA, where there is no append launch to save, us / the dispatcher's: 12 heads on 2 of
+    128, 32,768 positions 9.6 / 10.3, 32 on 8 of 64 15.4 / 16.4; 8 on 2 of 256, 8,192: 8.2 / 8.7, 16,384: 12.3 / 11.9; 16 on 4
+    of 64, 16,384: 7.7 / 8.2, 32,768: 12.3 / 10.8."""
     Hq, Hkv, D, batch, context = d.num_q_heads, d.num_kv_heads, d.head_dim, d.batch_size, d.context_length
     if Hkv <= 0 or Hq % Hkv or D not in (64, 128, 256):
         return 0, 0
@@ -163,6 +168,8 @@ def choose_lean_route(d, append: bool) -> tuple:
         us = lambda kind, parts, resident: d.hip.lean_step_estimate(kind, parts, Hq, Hkv, D, batch, context, context, batch * context, resident)
         return route if us(route[1], route[0], clusters) <= MARGIN * (us(-1, 0, 0) + (SMALL_APPEND_US if append else 0.0)) else (0, 0)
     parts = d.num_sms // Hkv
+    if not append and (D == 256 or D == 64 and Hkv < 8) and context * Hkv * D * 4 > SPLIT_ALONE_BYTES:
+        return route
     if (batch == 1 and context <= LEAN_SPLIT_MAX_CONTEXT and 1 < parts <= d.max_chunks and d.hip.lean_plan(Hq, Hkv, D, parts, context, SPLIT).ok
             and d.hip.lean_estimate(SPLIT, parts, Hq, Hkv, D, 1, context, 0) < best):
         route = parts, SPLIT

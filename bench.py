@@ -627,7 +627,9 @@ def run_ours(args, rank, world, local_rank):
         achieved = split_bytes / split_s / 1e9
         layer_us = step_s * 1e6 / n_layers
         traffic = None
-        if not (args.compat or args.layers):
+        route, parts = ex.route_name or ("", 0)
+        split_route = "lean" in route                       # split and combine; the other routes are one launch of clusters
+        if not (args.compat or args.layers or route):
             traffic = NCU_TRAFFIC_BYTES.get(cubin_hash(), {}).get((args.workload, ex.dispatcher.compact))
         result = {
             "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps, "warmup": warm,
@@ -635,14 +637,19 @@ def run_ours(args, rank, world, local_rank):
             "replays_per_trial": t["replays_per_trial"], "higher_is_better": True,
             "scaling": "weak", "vs_baseline": None,
             "dtype": "f16 storage, f32 accumulate", "data": "synthetic",
-            "config": config_json(cfg, args.workload, lengths, n_layers, n_kv, ex.dispatcher.max_chunks, world,
+            "config": config_json(cfg, args.workload, lengths, n_layers, n_kv, parts or ex.dispatcher.max_chunks, world,
                                   {"input_generation": "host, seeded" if host_gen else "device fill (counter-based normal)",
                                    "programmatic_dependent_launch": not args.no_pdl,
-                                   "kv_tile_copies": "tensor-map (TMA) boxes for whole tiles, 16-byte cp.async for ragged ends" if ex.dispatcher.tensor_maps else "16-byte cp.async",
-                                   "next_layer_l2_prefetch": not args.no_prefetch and cfg.batch == 1,
-                                   "route": "%s, %d CTAs per (sequence, KV head)" % ex.route_name if ex.route_name else "the dispatcher's launches",
-                                   "combine": "inside the split launch (grid barrier)" if ex.dispatcher.fused_combine else "separate launch", "kernels": "compat" if args.compat else ("fast, compact CTAs" if ex.dispatcher.compact else "fast, full CTAs"),
-                                   "step_contents": {"off": "split + combine per layer",
+                                   "kv_tile_copies": "tensor-map (TMA) boxes for whole tiles, 16-byte cp.async for ragged ends" if ex.dispatcher.tensor_maps and not route else "16-byte cp.async",
+                                   "next_layer_l2_prefetch": not args.no_prefetch and (split_route if route else cfg.batch == 1),
+                                   "route": "%s, %d CTAs per (sequence, KV head)" % (route, parts) if route else "the dispatcher's launches",
+                                   "combine": "inside the launch (thread-block clusters)" if route and not split_route else
+                                              "inside the split launch (grid barrier)" if ex.dispatcher.fused_combine else "separate launch",
+                                   "kernels": "one work item per CTA" if route else "compat" if args.compat else ("fast, compact CTAs" if ex.dispatcher.compact else "fast, full CTAs"),
+                                   "step_contents": ("rotation launch + " if args.rope == "separate" else "") + "%s per layer%s" % (
+                                                        "split + combine" if split_route else "one launch", ", %sappend inside" % (
+                                                            "rotation and " if args.rope != "separate" else "") if args.rope != "off" else "") if route else
+                                                    {"off": "split + combine per layer",
                                                      "separate": "rotation launch + cache append + split + combine per layer",
                                                      "fused": "cache append with K rotation + split with Q rotation + combine per layer",
                                                      "fused-append": "split (with Q rotation, K rotation and the cache append) + combine per layer"}[args.rope]}),

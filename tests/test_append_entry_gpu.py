@@ -14,13 +14,14 @@ STEPS = 24
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("offsets_by_launch", [True, False], ids=["offsets-by-launch", "offsets-final"])
-@pytest.mark.parametrize("heads, start, splits, flags", [
-    ((12, 2, 128), [40], 2, ATTN_COMPACT),                       # crosses the ends of tiles of 32 and of splits
-    ((8, 2, 256), [7], 3, ATTN_COMPACT),
-    ((32, 8, 64), [1, 60, 17, 200, 31], 32, ATTN_BALANCED),
-    ((28, 4, 128), [1, 60, 17, 200, 31], 32, 0),                 # work queue, full shape
-], ids=["compact-128", "compact-256", "balanced-64", "queue-128"])
-def test_appends_then_programmatic_attention(cuda_runtime, codegen, heads, start, splits, flags, offsets_by_launch):
+@pytest.mark.parametrize("heads, start, splits, flags, n_ctas", [
+    ((12, 2, 128), [40], 2, ATTN_COMPACT, 0),                    # crosses the ends of tiles of 32 and of splits
+    ((8, 2, 256), [7], 3, ATTN_COMPACT, 0),
+    ((32, 8, 64), [1, 60, 17, 200, 31], 32, ATTN_BALANCED, 0),   # goes to clusters
+    ((32, 8, 64), [1, 60, 17, 200, 31], 32, ATTN_BALANCED, 148), # equal shares
+    ((28, 4, 128), [1, 60, 17, 200, 31], 32, 0, 0),              # work queue, full shape
+], ids=["compact-128", "compact-256", "clusters-64", "balanced-64", "queue-128"])
+def test_appends_then_programmatic_attention(cuda_runtime, codegen, heads, start, splits, flags, n_ctas, offsets_by_launch):
     """Every step appends three positions and attends, with nothing but launches between the steps.  Either a launch
     right in front of each append writes the offsets, or every append has offsets of its own.  Bound: fp32 sums of at
     most 272 probabilities of 22 bits with values N(0, 1), as in the tests of the same kernels."""
@@ -63,7 +64,7 @@ def test_appends_then_programmatic_attention(cuda_runtime, codegen, heads, start
                     off = cur
                 rt.kv_cache_append(dkn + a * row, dvn + a * row, dk, dv, off, B, Hkv, D, S * Hkv * D)
             rt.split_kv_decode(dq + step * B * Hq * D * 2, dk, dv, off, out + step * B * Hq * D * 4, True, pm, pl, po, work,
-                               B, Hq, Hkv, D, D ** -0.5, S * Hkv * D, splits, 0, flags | ATTN_PROGRAMMATIC)
+                               B, Hq, Hkv, D, D ** -0.5, S * Hkv * D, splits, 0, flags | ATTN_PROGRAMMATIC, n_ctas)
         rt.check_status(work)
         got = np.zeros((STEPS, B, Hq, D), dtype=np.float32)
         rt.safe_memcpy_device_to_host(got, ctypes.c_void_p(out), "append test output")

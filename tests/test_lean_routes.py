@@ -445,27 +445,38 @@ def test_partials_of_more_items_than_sms_each_time(cuda_runtime, codegen):
 @pytest.mark.gpu
 @pytest.mark.parametrize("rope_type,rotary", [(0, 0), (1, 0), (2, 32), (2, 64)])
 @pytest.mark.parametrize("D", [64, 128, 256])
-def test_rotation_in_the_lean_kernels_gives_the_separate_launch_s_bits(cuda_runtime, codegen, D, rope_type, rotary):
-    """The rotated row in the cache is the standalone rotation's, bit for bit, and so are the outputs of the same route."""
+@pytest.mark.parametrize("route", [(6, 1), (6, 2), (37, 0)], ids=["cluster", "half", "split"])
+def test_rotation_in_the_lean_kernels_gives_the_separate_launch_s_bits(cuda_runtime, codegen, route, D, rope_type, rotary):
+    """The rotated row in the cache is the standalone rotation's, bit for bit, and so are the outputs of the same route, which
+    are the oracle's: fp32 sums of fp16 products, 2e-5 of the result's norm."""
+    if route[1] == 2 and D == 64:
+        pytest.skip("no half blocks of 64-wide heads")
     meta = {"attention.head_count": 12, "attention.head_count_kv": 2, "attention.key_length": D, "rope_type": rope_type}
     if rotary:
         meta["rotary_dim"] = rotary
     rng = np.random.default_rng(3)
     f16 = lambda *s: rng.standard_normal(s, dtype=np.float32).astype(np.float16)
-    B, S = 2, 300
+    B, S, kw = (2, 300, {}) if route[1] else (1, 300, {"num_splits": 148})
     q, k, v, kn, vn = f16(B, 12, D), f16(B, S, 2, D), f16(B, S, 2, D), f16(B, 2, D), f16(B, 2, D)
-    off, got = np.array([250, 16], dtype=np.int32), []
+    off, got = np.array([250, 16], dtype=np.int32)[:B], []
+    cos, sin = orc.rope_tables(S, rotary or D, 1e6)
+    q_rot, k_rot = orc.rope_step(q, kn, cos, sin, off, rope_type, rotary or D)
+    ref_k, ref_v = k.copy(), v.copy()
+    orc.kv_cache_append(k_rot, vn, ref_k, ref_v, off)
+    ref = orc.decode_attention(q_rot, ref_k, ref_v, off)
     for rope in ("separate", "fused", "fused-append"):
-        ex = DecodeAttentionExecutor(cuda_runtime, codegen, meta, B, S, 1, rope=rope, lean=(6, 1))
+        ex = DecodeAttentionExecutor(cuda_runtime, codegen, meta, B, S, 1, rope=rope, lean=route, **kw)
         try:
             ex.upload_layer(0, q, k, v)
             ex.upload_new_kv(0, kn, vn)
             out = ex.execute_decode_batch(off)
+            assert ex.kernel_launches_per_step == (1 if route[1] else 2) + (rope == "separate")
             got.append((out, *ex.download_cache_rows(0, 0, 251)))
             m, l, o = ex.read_partials()                             # the split launch's, on demand
             assert np.isfinite(m).all() and l.max() > 0
         finally:
             ex.cleanup()
+    assert np.linalg.norm(got[0][0][0] - ref) <= 2e-5 * np.linalg.norm(ref) and np.array_equal(got[0][1][250], k_rot[0])
     for other in got[1:]:
         for a, b in zip(got[0], other):
             assert np.array_equal(a, b)

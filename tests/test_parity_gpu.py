@@ -211,7 +211,7 @@ def test_ragged_batch_matches_oracle(cuda_runtime, codegen):
                          ids=["d64x16", "d128x5", "d256x6", "d128g7x3", "d128mha_short", "d128skewed", "d64x200"])
 def test_balanced_partition_matches_oracle(cuda_runtime, codegen, shape):
     """Several sequences, no split count given: every CTA takes an equal share of all cached positions
-    and a sequence is cut wherever a share ends.  The output, and the partial buffers reduced by the
+    and a sequence is cut wherever a share ends (or, by default, clusters serve the step).  The output, and the partial buffers reduced by the
     oracle's combine, must match the oracle; splits past a pair's last piece must read as empty; the
     host restatement of the cuts must agree with which splits the kernel filled."""
     from vte_b200.core.split_kv_attention import balanced_pieces
@@ -222,7 +222,7 @@ def test_balanced_partition_matches_oracle(cuda_runtime, codegen, shape):
     lens = [5000, 3, 1, 40, 7, 129] if B == 6 and D == 128 else None
     q, k, v, off = make_layer_inputs(cfg, 0, lengths=lens)
     ref = orc.decode_attention(q, k, v, off)
-    for kw in ({}, {"strict_empty_splits": True}, {"num_splits": 3, "balanced": True}):
+    for kw in ({}, {"lean": (0, 0)}, {"strict_empty_splits": True}, {"num_splits": 3, "balanced": True}):
         ex = DecodeAttentionExecutor(cuda_runtime, codegen, metadata(cfg), cfg.batch, cfg.max_seq, 1, **kw)
         try:
             d = ex.dispatcher

@@ -630,7 +630,8 @@ __device__ __forceinline__ void lean_body(const LeanArgs& a)
         if (my_units == 0) return;
         if (!mbar_wait_bounded(bar_recv, 0, abort_word)) {           // nobody leaves while another CTA may still send to it
             raise_abort(abort_word, a.status, kStatusGridTimeout);
-            cluster_rejoin();
+            cluster_rejoin();                                        // every state that comes has been sent, but may not have arrived
+            mbar_wait_bounded(bar_recv, 0, nullptr, 1LL << 31);
             return;
         }
         for (int slot = warp; slot < my_units; slot += CW) {

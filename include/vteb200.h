@@ -174,7 +174,7 @@ typedef struct vteb_lean_plan_t {
 int vteb_lean_plan(int num_q_heads, int num_kv_heads, int head_dim, int n_parts, long long context, int kind,
                    vteb_lean_plan_t* plan);
 /* Estimated microseconds of one layer on a route of `kind` and `n_parts` with `resident` clusters at once (kind -1: the
- * launches of vteb_split_kv_decode), by which routes are chosen. */
+ * launches of vteb_split_kv_decode), by which routes are chosen, by room in the cache (num_q_heads has no part in it). */
 double vteb_lean_estimate(int kind, int n_parts, int num_q_heads, int num_kv_heads, int head_dim, int batch, long long context,
                           int resident, int num_sms);
 /* The same for a step whose lengths are known: `longest` positions at the most, `total` in all sequences together, in caches with

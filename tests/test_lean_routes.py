@@ -85,6 +85,17 @@ def test_the_route_follows_the_size(built_library):
             assert parts == 0 or (parts in CLUSTER_PARTS if kind else batch == 1 and parts == 37)
 
 
+def test_both_sides_of_the_rule_agree():
+    """The executors' choice is in Python, the direct entry point's in C++."""
+    import re
+    from pathlib import Path
+    from vte_b200.core import lean_route
+    csrc = Path(lean_route.__file__).resolve().parent.parent / "csrc"
+    margin = re.search(r"kLeanMargin = ([\d.]+);", (csrc / "kernels" / "lean_decode.cuh").read_text()).group(1)
+    parts = re.search(r"kParts\[\] = \{([\d, ]+)\}", (csrc / "cluster_choice.h").read_text()).group(1)
+    assert float(margin) == lean_route.MARGIN and tuple(int(x) for x in parts.split(",")) == CLUSTER_PARTS
+
+
 def test_small_caches_keep_the_one_launch_that_is_shorter(built_library):
     """Up to 128 positions the dispatcher's layer is one launch.  Timed, dispatcher / clusters, us: 64 sequences of 32 heads on
     8 of 64 3.1 / 14.1 (room for 16) and 6.4 / 16.2 (128), of 28 on 4 of 128 4.9 / 9.5, of 8 on 2 of 256 5.4 / 6.4; one

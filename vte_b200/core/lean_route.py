@@ -203,7 +203,9 @@ def unsplit_as_clusters(hip, kernels: dict, args: list, grid, block, status: int
     heads on 2 of 128, 64 positions 4.8 / 5.3, 200: 5.9 / 5.3, 600: 8.6 / 5.4, 1,500: 15.3 / 6.3, 4,000: 43 / 9.6.  So:
     caches with room for more than 256 positions (512 with two runs of query heads: 6.5 us at the least), and no more
     pairs than clusters run at once (a second wave costs more than short sequences take: 64 sequences of 200 positions
-    19 / 21, of 64 8 / 17)."""
+    19 / 21, of 64 8 / 17).  The host sees the room, not the lengths: a sequence of up to about 100 positions (150 of 256-wide
+    heads, 200 with two runs) in such a cache takes longer than its own builds, 4.9 us instead of 3.3 (one position), 4.6 (64)
+    and 4.4 (128).  One CTA alone for those gave 4.1 to 4.4, and 0.25 more to every longer one."""
     if len(args) != 13:
         return None
     value = lambda a: a if isinstance(a, int) else getattr(a, "value", None) or 0

@@ -93,7 +93,7 @@ inline double lean_estimate_us(int kind, int n_parts, int num_q_heads, int num_k
     const double walk = waves > 1.0 ? 0.84 * part + spread : part > spread ? part : spread;
     return 3.5 + 0.2 * std::log2((double)n_parts) + 2.6 * (waves - 1.0) + std::pow(std::pow(bytes / 6.1e6, 4.0) + std::pow(walk, 4.0), 0.25);
 }
-constexpr double kLeanMargin = 0.95;       // a route has to be estimated this much below kind -1
+constexpr double kLeanMargin = 0.95;       // a route has to be estimated this much below kind -1 (MARGIN in core/lean_route.py)
 
 // The same where the lengths are known: the longest sequence has `longest` positions, all together `total`, in caches with room
 // for `capacity`.  Fitted to 3,444 steps of 8 head geometries, 1 to 64 sequences, room for 16 to 65,536 positions, lengths

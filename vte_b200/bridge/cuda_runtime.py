@@ -720,7 +720,8 @@ class CudaRuntime:
     def stream_synchronize(self):
         self._require_init()
         self._check_error(self._lib.vteb_stream_synchronize(self._stream), "cudaStreamSynchronize")
-        self._check_launch_status()
+        if self._launch_status is not None and self._launch_status.value:
+            self._check_launch_status()
 
     # ------------------------------------------------------------------ peer memory
     def ipc_export(self, ptr) -> bytes:

@@ -323,11 +323,9 @@ class DecodeAttentionExecutor:
         return graph_exec, n
 
     def _pick(self, offsets: np.ndarray, newest: int):
-        """Which of the captured steps serves these offsets, the largest of which is `newest`."""
-        self._on_route = self._route is not None and (newest < self._route_pays_to or
-                                                      self._route.pays(newest + 1, int(offsets.sum(dtype=np.int64)) + self.B))
-        if self._plain_graph_exec is not None:
-            self.kernel_launches_per_step = self._launches[not self._on_route]
+        """Which of two captured steps serves these offsets, the largest of which is `newest`."""
+        self._on_route = newest < self._route_pays_to or self._route.pays(newest + 1, int(offsets.sum(dtype=np.int64)) + self.B)
+        self.kernel_launches_per_step = self._launches[not self._on_route]
 
     def build_io_graph(self):
         """One graph for a whole end-to-end step: kv offsets and every layer's Q from pinned
@@ -382,7 +380,8 @@ class DecodeAttentionExecutor:
         newest = int(off.max())
         if off.min() < 0 or newest >= self.S:
             raise CudaSafetyError(f"kv offset outside 0..{self.S - 1}")
-        self._pick(off, newest)
+        if self._plain_graph_exec is not None:
+            self._pick(off, newest)
         half, slot = divmod(self._offset_slot, OFFSET_SLOTS // 2)
         if slot == 0 and self._offset_events[half] is not None:
             self.hip.event_synchronize(self._offset_events[half])
@@ -398,9 +397,8 @@ class DecodeAttentionExecutor:
     def launch_step(self):
         """Enqueue one decode step (no host synchronisation)."""
         if self._graph_exec is not None:
-            plain = self._plain_graph_exec is not None and not self._on_route
-            self.hip.graph_launch(self._plain_graph_exec if plain else self._graph_exec)
-            self._partials_due = self._kept_names is not None and not plain
+            self.hip.graph_launch(self._graph_exec if self._on_route else self._plain_graph_exec)
+            self._partials_due = self._on_route and self._kept_names is not None
         else:
             self.hip.programmatic_launch = self.programmatic
             try:
@@ -428,10 +426,10 @@ class DecodeAttentionExecutor:
             self._wait_for_staging()
             ctypes.memmove(self._stage_offsets.value, off.ctypes.data, off.nbytes)
             ctypes.memmove(self._stage_q.value, qh.ctypes.data, qh.nbytes)
-            self._pick(off, newest)
-            plain = self._plain_io_graph_exec is not None and not self._on_route
-            self.hip.graph_launch(self._plain_io_graph_exec if plain else self._io_graph_exec)
-            self._partials_due = self._kept_names is not None and not plain
+            if self._plain_io_graph_exec is not None:
+                self._pick(off, newest)
+            self.hip.graph_launch(self._io_graph_exec if self._on_route else self._plain_io_graph_exec)
+            self._partials_due = self._on_route and self._kept_names is not None
             self.hip.stream_synchronize()
             # the status word travelled with the outputs: only a non-zero one needs the slow path
             if ctypes.c_int.from_address(self._stage_out.value + self._out_tail + 4).value != 0:

@@ -466,7 +466,6 @@ __device__ __forceinline__ void lean_body(const LeanArgs& a)
         if (i < depth) fetch(i, i);
 
     // the next layer's rows of this part
-    const bool keep = (a.flags & kLeanKeep) != 0 && part == 0;
     bool ahead = !kCluster && a.next_k_cache != nullptr && !(a.flags & kLeanKeep) && warp < 2 && end > start &&
                  (long long)total * pos_stride * 2 <= kL2PrefetchMaxBytes;
     auto fetch_ahead = [&]() {
@@ -511,13 +510,11 @@ __device__ __forceinline__ void lean_body(const LeanArgs& a)
     for (int h = threadIdx.x / CPR; h < group; h += THREADS / CPR) {
         const __half* row = a.q + ((long long)b * a.num_q_heads + (long long)kv_head * group + h) * D;
         uint4 x = *reinterpret_cast<const uint4*>(row + q_chunk * 8);
-        if (keep) *reinterpret_cast<uint4*>(const_cast<__half*>(a.next_k_cache) + (row - a.q) + q_chunk * 8) = x;
         if (rotate && rope_touches(a.rope_type, a.rotary_dim, q_chunk * 8))
             x = rope_chunk(x, row, q_chunk * 8, q_words, a.rope_type, a.rotary_dim, D);
         uint32_t* dst = q_store + ((h >> 3) * CPR + (q_chunk & ~3)) * 32 + (h & 7) * 16 + (q_chunk & 3);
         dst[0] = x.x; dst[4] = x.y; dst[8] = x.z; dst[12] = x.w;
     }
-    if (keep && kv_head == 0 && threadIdx.x == 0) reinterpret_cast<int*>(const_cast<__half*>(a.next_v_cache))[b] = total - 1;
     if (my_late && a.k_new != nullptr) {
         if (rotate && lane < CPR && rope_touches(a.rope_type, a.rotary_dim, lane * 8))
             fresh[0] = rope_chunk(fresh[0], a.k_new + new_row, lane * 8, k_words, a.rope_type, a.rotary_dim, D);
@@ -625,6 +622,12 @@ __device__ __forceinline__ void lean_body(const LeanArgs& a)
                 a.partial_l[stat] = end > start ? ll : 0.f;
             }
         }
+    }
+    if (a.flags & kLeanKeep) {                                       // behind all else: beside Q's own loads the test cost 0.1 us a launch
+        const long long from = ((long long)b * a.num_q_heads + (long long)kv_head * group) * D;
+        for (int i = threadIdx.x; part == 0 && i < group * CPR; i += THREADS)
+            reinterpret_cast<uint4*>(const_cast<__half*>(a.next_k_cache) + from)[i] = reinterpret_cast<const uint4*>(a.q + from)[i];
+        if (part == 0 && kv_head == 0 && threadIdx.x == 0) reinterpret_cast<int*>(const_cast<__half*>(a.next_v_cache))[b] = total - 1;
     }
     if constexpr (kCluster) {
         if (my_units == 0) return;

@@ -690,7 +690,7 @@ VTEB_LEAN_KERNEL(vteb_decode_cluster_d128_kernel, 128, 1, lean_warps(128), true,
 VTEB_LEAN_KERNEL(vteb_decode_cluster_d256_kernel, 256, 1, lean_warps(256), true, true, __launch_bounds__(192, 1))
 VTEB_LEAN_KERNEL(vteb_decode_cluster_2_d64_kernel, 64, 2, lean_warps(64), true, true, __launch_bounds__(256, 2))
 VTEB_LEAN_KERNEL(vteb_decode_cluster_2_d128_kernel, 128, 2, lean_warps(128), true, true, __launch_bounds__(256, 1))
-VTEB_LEAN_KERNEL(vteb_decode_cluster_half_d128_kernel, 128, 1, lean_half_warps(128), true, true, __launch_bounds__(128, 2))
+VTEB_LEAN_KERNEL(vteb_decode_cluster_half_d128_kernel, 128, 1, lean_half_warps(128), true, true, __launch_bounds__(128, 3))
 VTEB_LEAN_KERNEL(vteb_decode_cluster_half_d256_kernel, 256, 1, lean_half_warps(256), true, true, __launch_bounds__(96, 2))
 VTEB_LEAN_KERNEL(vteb_decode_cluster_half_2_d128_kernel, 128, 2, lean_half_warps(128), true, true, __launch_bounds__(128, 2))
 VTEB_LEAN_KERNEL(vteb_split_kv_lean_d64_kernel, 64, 1, lean_warps(64), false, false, __maxnreg__(160))

@@ -112,10 +112,10 @@ inline double lean_step_us(int kind, int n_parts, int num_q_heads, int num_kv_he
     const int runs = num_q_heads > 8 * num_kv_heads ? 1 : 0, d = head_dim == 64 ? 0 : head_dim == 128 ? 1 : 2;
     const double pairs = (double)batch * num_kv_heads, bytes = total * num_kv_heads * 4.0 * head_dim, g = num_q_heads / (8.0 * num_kv_heads);
     if (kind < 0 && capacity <= 128) {
-        static const double kSmall[2][3][4] = {{{2.55, .0205, .10, 0.}, {3.4, .0135, .09, .26}, {3.9, .0075, .19, 0.}},
-                                               {{3.2, .0045, .06, 0.}, {4.45, .011, .25, .3}, {4.45, .011, .25, .3}}};
+        static const double kSmall[2][3][5] = {{{2.55, .0205, .10, 0., 0.}, {3.4, .0135, .09, .26, .045}, {3.2, .0145, .30, 0., 0.}},
+                                               {{3.2, .0045, .06, 0., 0.}, {4.25, .011, .25, .3, 0.}, {4.25, .011, .25, .3, 0.}}};
         const double* c = kSmall[runs][d];
-        return c[0] + c[1] * (double)longest + c[2] * std::log2((double)batch) + c[3] * pairs / 148.0;
+        return c[0] + c[1] * (double)longest + c[2] * std::log2((double)batch) + c[3] * pairs / 148.0 + c[4] * (num_q_heads > 12 ? num_q_heads - 12 : 0);
     }
     if (kind < 0) {
         static const PlainStepFit kOne[2][3] = {{{3.52, 6.87e6, .25, .0027, 0., .25}, {4.42, 7.41e6, .01, .0557, 0., .31}, {5.44, 7.88e6, 0., 0., 0., .36}},

@@ -592,6 +592,19 @@ __device__ __forceinline__ void lean_body(const LeanArgs& a)
     }
     __syncthreads();
 
+    // What kLeanKeep asks for.  The place is by measurement: beside the load of Q the test cost every launch 0.1 us; clusters take
+    // it best behind their sends (28 layers of 1,531 positions 103.9 us, here 105.5), the split of 256-wide heads here
+    // (8 layers of 24,001 positions 112.4, at the end 115 to 117).
+    const auto keep_inputs = [&]() {
+        if (a.flags & kLeanKeep) {
+            const long long from = ((long long)b * a.num_q_heads + (long long)kv_head * group) * D;
+#pragma unroll 1
+            for (int i = threadIdx.x; part == 0 && i < group * CPR; i += THREADS)
+                reinterpret_cast<uint4*>(const_cast<__half*>(a.next_k_cache) + from)[i] = reinterpret_cast<const uint4*>(a.q + from)[i];
+            if (part == 0 && kv_head == 0 && threadIdx.x == 0) reinterpret_cast<int*>(const_cast<__half*>(a.next_v_cache))[b] = total - 1;
+        }
+    };
+    if constexpr (!kCluster) keep_inputs();
     const long long head0 = (long long)b * a.num_q_heads + (long long)kv_head * group;
     for (int idx = threadIdx.x; idx < group * (D / 4); idx += THREADS) {
         const int h = idx / (D / 4), q4 = idx - h * (D / 4);
@@ -623,12 +636,7 @@ __device__ __forceinline__ void lean_body(const LeanArgs& a)
             }
         }
     }
-    if (a.flags & kLeanKeep) {                                       // behind all else: beside Q's own loads the test cost 0.1 us a launch
-        const long long from = ((long long)b * a.num_q_heads + (long long)kv_head * group) * D;
-        for (int i = threadIdx.x; part == 0 && i < group * CPR; i += THREADS)
-            reinterpret_cast<uint4*>(const_cast<__half*>(a.next_k_cache) + from)[i] = reinterpret_cast<const uint4*>(a.q + from)[i];
-        if (part == 0 && kv_head == 0 && threadIdx.x == 0) reinterpret_cast<int*>(const_cast<__half*>(a.next_v_cache))[b] = total - 1;
-    }
+    if constexpr (kCluster) keep_inputs();
     if constexpr (kCluster) {
         if (my_units == 0) return;
         if (!mbar_wait_bounded(bar_recv, 0, abort_word)) {           // nobody leaves while another CTA may still send to it

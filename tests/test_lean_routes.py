@@ -190,6 +190,26 @@ def test_a_route_looks_no_further_than_a_pool_for_the_next_layer_s_rows(built_li
         assert ahead(without) == [0, 0]
 
 
+@pytest.mark.parametrize("forced", [False, True])
+def test_an_allocator_without_room_for_the_copy_of_q_keeps_the_dispatcher_s_launches(built_library, forced):
+    from types import SimpleNamespace
+
+    def full(size, tag, region):
+        raise CudaSafetyError("slab exhausted")
+    d, _ = real_dispatcher()
+    for name in ("lean_estimate", "lean_step_estimate", "max_active_clusters"):
+        setattr(d.hip, name, getattr(FakeHip, name))
+    ex = object.__new__(DecodeAttentionExecutor)
+    vars(ex).update(dispatcher=d, hip=d.hip, B=1, S=4096, q_bytes=3072, use_graph=True, per_layer_hook=None, launch_rewriter=None, with_append=True,
+                    _route=None, _lean=(16, 1) if forced else None, _forced_route=forced, allocator=SimpleNamespace(allocate=full))
+    if forced:
+        with pytest.raises(CudaSafetyError, match="exhausted"):
+            ex._choose_route()
+    else:
+        ex._choose_route()
+        assert ex._route is None and ex._lean == (0, 0)
+
+
 @pytest.mark.parametrize("option", ["compat", "strict_empty_splits", "emit_state", "fused_combine"])
 def test_a_forced_route_refuses_what_it_would_drop(option):
     with pytest.raises(CudaSafetyError, match="lean_route"):

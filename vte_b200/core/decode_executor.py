@@ -284,11 +284,18 @@ class DecodeAttentionExecutor:
         if self._lean is None:
             self._lean = choose_lean_route(d, append)
         if self._lean[0]:
-            self._route = LeanRoute(d, *self._lean, append)
+            route = LeanRoute(d, *self._lean, append)
+            try:
+                self._kept = self.allocator.allocate(_round_up(self.q_bytes, 256) + _round_up(4 * self.B, 256), "attn_partials_source",
+                                                     MemoryRegion.SCRATCH)
+            except CudaSafetyError:
+                if self._forced_route:
+                    raise
+                self._lean = (0, 0)                   # a caller's allocator with no room for it: the dispatcher's launches need none
+                return
+            self._route = route
             if not self._forced_route:
-                self._route_pays_to = self._route.pays_up_to()
-            self._kept = self.allocator.allocate(_round_up(self.q_bytes, 256) + _round_up(4 * self.B, 256), "attn_partials_source",
-                                                 MemoryRegion.SCRATCH)
+                self._route_pays_to = route.pays_up_to()
 
     def build_decode_graph(self):
         """Capture all layers' launches once (hip_graph_executor.py:504-725)."""

@@ -58,7 +58,7 @@ class LeanRoute:
                                                                     d.context_length, longest, total, resident)
         if self._resident is None:
             self._resident = d.hip.max_active_clusters(self.function, self.parts, self.plan.threads, self.plan.smem_bytes)
-        return us(self.kind, self.parts, self._resident) <= MARGIN * (us(-1, 0, 0) + (LEAST_APPEND_US if self.append else 0.0))
+        return us(self.kind, self.parts, self._resident) <= us(-1, 0, 0) + (LEAST_APPEND_US if self.append else 0.0)
 
     def pays_up_to(self) -> int:
         """A length up to which the route pays whatever the other sequences have."""

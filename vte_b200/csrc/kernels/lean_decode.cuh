@@ -99,8 +99,8 @@ constexpr double kLeanMargin = 0.95;       // a route has to be estimated this m
 // for `capacity`.  Fitted to 3,444 steps of 8 head geometries, 1 to 64 sequences, room for 16 to 65,536 positions, lengths
 // all the same, uniform, one or a quarter of them long and the others a fiftieth to a twentieth of it, up to 19 routes timed on
 // each: 90 % within a sixth.  Of 2,340 batches in caches above 128 positions, the clusters chosen by capacity took up to 3.3
-// times as long as kind -1 and longer than 1.03 times in 248; where every step takes the one that this finds shorter (by
-// kLeanMargin), at most 1.28 times and in 20.
+// times as long as kind -1 and longer than 1.03 times in 248; where every step takes the one that this finds shorter, at
+// most 1.37 times and in 42 (and longer than 1.03 times the clusters in 15).
 //   a cluster layer: its longest part, the starts of all clusters and the bytes overlap (a p-norm); every further wave costs as
 //   much again; merges and starts grow with the query heads of a KV head
 //   kind -1: bytes over a rate, what grows with the work items and with the longest over the mean length; up to 128 positions it

@@ -186,6 +186,42 @@ def timed_trials(rt, rdzv, launch, steps, trials=TRIALS, min_trial_ms=MIN_TRIAL_
             "trials": trials, "replays_per_trial": steps * mult}
 
 
+def one_launch_block(args, rt, rdzv, cfg, n_layers, offsets, q_all, host_layers, bytes_step):
+    """The headline step without an order among its layers (an executor's default): device and end to end."""
+    from oracle import attention_oracle as orc
+    from vte_b200.compiler import CodegenEngine
+    from vte_b200.core.decode_executor import DecodeAttentionExecutor
+    ex = DecodeAttentionExecutor(rt, CodegenEngine(), metadata(cfg), cfg.batch, cfg.max_seq, n_layers, output_f32=True)
+    try:
+        for l in range(n_layers):
+            ex.fill_cache_on_device(l, cfg.base_seed * 1000 + l, cfg.sigma_kv)
+            ex.upload_layer(l, q_all[l])
+        parity = None
+        if 0 in host_layers:
+            q, k, v, off = host_layers[0]
+            ex.upload_layer(0, q, k, v)
+            max_abs, rel = orc.parity_metrics(ex.execute_decode_batch(offsets)[0], orc.decode_attention(q, k, v, off))
+            parity = {"layer": 0, "max_abs": max_abs, "rel_l2": rel, "within_tolerance": bool(max_abs <= 2e-3 and rel <= 1e-2)}
+        ex.execute_decode_batch(offsets)
+        for _ in range(3):
+            ex.launch_step()
+        t = timed_trials(rt, rdzv, ex.launch_step, args.steps, trials=args.trials, min_trial_ms=args.min_trial_ms)
+        ex.dispatcher_check()
+        steps = max(args.steps, int(math.ceil(args.min_trial_ms / max(t["median_ms"], 1e-3))))
+        e2e = []
+        for _ in range(args.trials):
+            t0 = time.perf_counter()
+            for _ in range(steps):
+                ex.execute_decode_batch(offsets, q_host=q_all)
+            e2e.append((time.perf_counter() - t0) / steps)
+        return {"kernel": (ex.route_name or ("",))[0], "ms_per_step": t["median_ms"], "value": bytes_step / t["median_ms"] / 1e9, "unit": UNIT,
+                "e2e_ms_per_step": statistics.median(e2e) * 1e3, "e2e_value": bytes_step / statistics.median(e2e) / 1e12, "parity": parity,
+                "note": "every layer's queries are inputs of the step, so no layer waits for another; the line's own value has a launch per layer "
+                        "that follows the one in front"}
+    finally:
+        ex.cleanup()
+
+
 def cubin_hash() -> str:
     from vte_b200.compiler import CodegenEngine
     return CodegenEngine().cache_path("decode_attention", "sm_100a").stem.replace("kernel_", "")
@@ -285,7 +321,7 @@ def measure_sequences(args, rt, rdzv, rank, world, workload, n_layers, n_kv, ste
     ex = DecodeAttentionExecutor(rt, CodegenEngine(), metadata(cfg), local.batch, cfg.max_seq, n_layers,
                                  n_kv_buffers=n_kv, output_f32=True, variant=args.variant,
                                  num_splits=args.splits or None, min_chunk=None if args.min_chunk < 0 else args.min_chunk,
-                                 balanced=False if args.no_balanced else (True if args.force_balanced else None))
+                                 balanced=False if args.no_balanced else (True if args.force_balanced else None), one_launch=False)
     try:
         for buf in range(n_kv):
             _fill_sequences(rt, ex, cfg, buf, mine)
@@ -394,7 +430,7 @@ def measure_kv_range(args, rt, rdzv, rank, world, exchange, n_layers, steps, wor
         finally:
             sh.cleanup()
     if world == 1:
-        ex = DecodeAttentionExecutor(rt, CodegenEngine(), metadata(cfg), 1, total, n_layers, output_f32=True, variant=args.variant)
+        ex = DecodeAttentionExecutor(rt, CodegenEngine(), metadata(cfg), 1, total, n_layers, output_f32=True, variant=args.variant, one_launch=False)
         try:
             q_all = np.zeros((n_layers, 1, cfg.num_q_heads, cfg.head_dim), dtype=np.float16)
             for l in range(n_layers):
@@ -549,7 +585,8 @@ def run_ours(args, rank, world, local_rank):
                                  prefetch_next_layer=not args.no_prefetch,
                                  fused_combine=args.fuse, variant=args.variant, rope=args.rope,
                                  rope_theta=cfg.rope_theta or 1e6, tensor_maps=not args.no_tma,
-                                 balanced=False if args.no_balanced else (True if args.force_balanced else None))
+                                 balanced=False if args.no_balanced else (True if args.force_balanced else None),
+                                 one_launch=False)     # a model's layers depend on one another: a layer's launch follows the one in front
     # ---- inputs: seeded host generation when it is cheap, device-side fill otherwise
     host_layers = {}
     q_all = np.zeros((n_layers, cfg.batch, cfg.num_q_heads, cfg.head_dim), dtype=np.float16)
@@ -678,6 +715,10 @@ def run_ours(args, rank, world, local_rank):
             "clocks": clocks, "parity": parity,
         }
     ex.cleanup()
+
+    # ---- the same step where all layers' queries are there before it starts: one launch over all of them
+    if args.workload == "c2" and world == 1 and not args.layers and args.rope == "off" and not args.compat and not args.splits:
+        result["config"]["one_launch"] = one_launch_block(args, rt, rdzv, cfg, n_layers, offsets, q_all, host_layers, bytes_step)
 
     # ---- the workloads that shard, measured in the same run
     if args.workload == "c2" and not args.no_sharded and not args.layers and args.rope == "off" and not args.compat:

@@ -181,6 +181,21 @@ double vteb_lean_estimate(int kind, int n_parts, int num_q_heads, int num_kv_hea
  * room for `capacity` a sequence (up to 128, kind -1 is the dispatcher's one launch). */
 double vteb_lean_step_estimate(int kind, int n_parts, int num_q_heads, int num_kv_heads, int head_dim, int batch,
                                long long capacity, long long longest, long long total, int resident);
+/* What a launch of the kernels that take all layers of a step (`vteb_decode_step_*`) needs, with `n_ctas` blocks, one an SM;
+ * `hg`: KV heads a block serves at once, 0: chosen.  ok = 0: not covered (groups of more than 16 query heads, more than 8
+ * with 256-wide heads, more than 1,024 sequences). */
+typedef struct vteb_step_plan_t {
+    int ok;
+    int threads;
+    int smem_bytes;
+    int hg;
+    int state_bytes;   /* of the `boards` argument, zeroed before the first launch, as are the n_ctas counts of `launches` */
+    int max_layers;    /* a launch */
+    int hg_log2;
+    int wph;           /* warps that share a KV head */
+    int tile;          /* positions of a box of the tensor maps */
+} vteb_step_plan_t;
+int vteb_step_plan(int num_q_heads, int num_kv_heads, int head_dim, int batch, int n_ctas, int hg, vteb_step_plan_t* plan);
 /* How many clusters of `cluster` blocks of a loaded kernel the device runs at once (cuOccupancyMaxActiveClusters). */
 int vteb_max_active_clusters(void* function, int cluster, int threads, int smem_bytes, int* count);
 /* Encodes the 128-byte tensor map the fast split kernels take for a K or V cache: the cache
@@ -191,6 +206,9 @@ int vteb_max_active_clusters(void* function, int cluster, int threads, int smem_
  * counterpart: the reference's kernels read the cache with scalar loads
  * (flash_attention_split_kv_partial.hip.template:86-93). */
 int vteb_kv_tensor_map(void* out_128_bytes, const void* cache, long long n_rows, int row_halves, int box_rows);
+/* The map the whole-step kernels take: the same cache as `n_rows` rows of row_halves / 64 columns of 64 values, in boxes of
+ * `box_cols` columns x `box_rows` rows, column after column (one copy a tile). */
+int vteb_kv_tensor_map_columns(void* out_128_bytes, const void* cache, long long n_rows, int row_halves, int box_rows, int box_cols);
 /* Columns per lane of the short-list combine kernel (split counts up to 64): a warp
  * merges 32 * epl columns of one (sequence, head) row. */
 int vteb_combine_rows_epl(int rows, int head_dim);

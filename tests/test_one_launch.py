@@ -1,0 +1,297 @@
+"""A decode step as one launch over all its layers (core/step_route.py, csrc/kernels/step_decode.cuh): what may take it and
+what does, on the CPU, and the kernels against the oracle where tiles, shares and runs meet."""
+import ctypes
+from types import SimpleNamespace
+
+import numpy as np
+import pytest
+
+from oracle import attention_oracle as orc
+from vte_b200.bridge.cuda_runtime import StepArgs, StepLayer, StepPlan, load_library
+from vte_b200.bridge.errors import CudaRuntimeError, CudaSafetyError
+from vte_b200.core.decode_executor import DecodeAttentionExecutor
+from vte_b200.core.split_kv_attention import SplitKVAttentionDispatcher
+from vte_b200.core.step_route import StepRoute, one_launch_pays
+
+
+def step_plan(Hq, Hkv, D, batch, ctas=148, hg=0):
+    plan = StepPlan()
+    assert load_library().vteb_step_plan(Hq, Hkv, D, batch, ctas, hg, ctypes.byref(plan)) == 0
+    return plan
+
+
+@pytest.mark.parametrize("D", [64, 128, 256])
+@pytest.mark.parametrize("group", [1, 7, 8, 9, 16, 17])
+def test_plan_covers_what_the_kernels_do(built_library, group, D):
+    assert ctypes.sizeof(StepLayer) == 320 and ctypes.sizeof(StepArgs) == 64 * 320 + 128 < 32764
+    for Hkv in (1, 2, 3, 4, 6, 8, 12):
+        for batch in (1, 64, 1024, 1025):
+            p = step_plan(group * Hkv, Hkv, D, batch)
+            assert bool(p.ok) == (group <= (8 if D == 256 else 16) and batch <= 1024)
+            if not p.ok:
+                continue
+            warps = p.threads // 32 - 1
+            assert Hkv % p.hg == 0 and p.hg == 1 << p.hg_log2 and p.hg * p.wph == warps // (2 if D == 256 else 1) and p.tile == 16 * p.wph <= 256
+            assert (warps * 32) % (D // 8) == 0 and p.smem_bytes <= 227 * 1024
+            assert p.state_bytes == 148 * p.hg * group * (D // 2 + 1) * 16
+
+
+def a_route(layers=3, append=True, heads=(12, 2, 128), batch=2, capacity=512, f32=False, **kw):
+    """(route, mapping, offsets) over made-up addresses that do not overlap."""
+    Hq, Hkv, D = heads
+    d = object.__new__(SplitKVAttentionDispatcher)
+    vars(d).update(num_q_heads=Hq, num_kv_heads=Hkv, head_dim=D, batch_size=batch, context_length=capacity, output_f32=f32, num_sms=148,
+                   fuse_rope=False, rope_type=0, rotary_dim=D, hip=SimpleNamespace(step_plan=step_plan), **kw)
+    r = object.__new__(StepRoute)
+    vars(r).update(d=d, layers=layers, append=append, scratch=SimpleNamespace(ptr=0x1000, size=0x1000))
+    m, at = {'kv_batch_stride_elements': capacity * Hkv * D}, 0x100000
+    for l in range(layers):
+        for name, size in (('q_proj.output', batch * Hq * D * 2), ('k_proj.output', batch * Hkv * D * 2), ('v_proj.output', batch * Hkv * D * 2),
+                           ('kv_cache.k', batch * capacity * Hkv * D * 2), ('kv_cache.v', batch * capacity * Hkv * D * 2),
+                           ('attention.output', batch * Hq * D * (4 if f32 else 2))):
+            m[f'blk.{l}.{name}'] = at
+            at += size                                           # back to back: what touches does not overlap
+    return r, m, at
+
+
+def test_layers_run_side_by_side_only_where_none_reads_what_another_writes(built_library):
+    for append in (True, False):
+        r, m, free = a_route(append=append)
+        may = lambda **change: r.serves({**m, **{k.replace('__', '.'): v for k, v in change.items()}}, free, 2)
+        assert may()
+        assert not may(blk__1__q_proj__output=m['blk.0.attention.output'])                 # one layer's output is the next one's Q
+        assert not may(blk__1__q_proj__output=m['blk.0.attention.output'] + 16)
+        assert not may(blk__2__attention__output=m['blk.0.attention.output'])               # two writers
+        assert not may(blk__2__attention__output=m['blk.2.q_proj.output'])                  # in place
+        assert may(blk__2__q_proj__output=m['blk.0.q_proj.output'])                         # read twice
+        assert may(blk__2__kv_cache__k=m['blk.0.kv_cache.k']) != append                     # a shared cache: read only
+        assert not may(blk__2__kv_cache__k=m['blk.0.kv_cache.k'] + 1024) == append
+        assert not may(blk__2__attention__output=free + 0x10008) and may(blk__2__attention__output=free + 0x10010)      # 16-byte stores
+        assert may(blk__1__v_proj__output=free + 0x10008) != append
+        assert not may(blk__0__attention__output=0x1800)                                    # the route's own scratch
+        assert r.serves({**m, 'kv_batch_stride_elements': 512 * 256}, free, 2)
+        for stride in (512 * 256 + 128, 511 * 256):                                          # no whole rows; shorter than the cache
+            assert not r.serves({**m, 'kv_batch_stride_elements': stride}, free, 2)
+        assert not r.serves(m, m['blk.1.attention.output'] + 64, 2)                          # offsets under an output
+    with pytest.raises(CudaSafetyError, match="null"):
+        r, m, free = a_route()
+        r.serves({k: v for k, v in m.items() if k != 'blk.1.v_proj.output'}, free, 2)
+
+
+def test_what_goes_to_one_launch(built_library):
+    pays = lambda layers, *a: one_launch_pays(a_route(1, True, *a)[0].d, layers)
+    assert pays(28, (12, 2, 128), 1, 4096) and pays(4, (16, 1, 64), 1, 64) and pays(4, (32, 2, 128), 1, 4096)
+    assert pays(3, (8, 2, 256), 8, 4096) and not pays(3, (8, 2, 256), 1, 4096) and not pays(3, (32, 2, 128), 8, 4096)
+    assert pays(2, (32, 8, 64), 64, 16384) and not pays(2, (32, 8, 64), 8, 4096)
+    assert not pays(1, (12, 2, 128), 1, 1 << 20)                   # one layer: nothing to share out
+    assert not pays(28, (36, 2, 128), 1, 4096) and not pays(28, (18, 2, 256), 1, 4096) and not pays(28, (12, 2, 128), 1025, 64)
+
+
+@pytest.mark.parametrize("option", [dict(lean=(4, 1)), dict(compat=True), dict(strict_empty_splits=True), dict(emit_state=True), dict(num_splits=8)])
+def test_one_launch_refuses_what_it_would_drop(option):
+    with pytest.raises((CudaSafetyError, AttributeError)):
+        DecodeAttentionExecutor(None, None, {}, 1, 256, 4, one_launch=True, **option)
+
+
+HEADS = [(12, 2, 128), (32, 8, 64), (8, 2, 256), (8, 8, 128), (7, 1, 128), (6, 3, 64), (8, 1, 256), (22, 2, 128), (32, 2, 128), (16, 1, 64)]
+LENGTHS = [1, 15, 16, 17, 31, 33, 47, 48, 49, 64, 65, 95, 96, 97, 127, 128, 129, 257, 300]
+
+
+def executor(rt, codegen, heads, B, S, L, **kw):
+    meta = {"attention.head_count": heads[0], "attention.head_count_kv": heads[1], "attention.key_length": heads[2], **kw.pop("meta", {})}
+    return DecodeAttentionExecutor(rt, codegen, meta, B, S, L, **{"one_launch": True, **kw})
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("heads", HEADS)
+@pytest.mark.parametrize("append", [True, False], ids=["append", "attend"])
+@pytest.mark.parametrize("layers,lengths", [(1, LENGTHS), (3, LENGTHS), (3, [700]), (1, [5000]), (2, [1]), (5, [2049, 40])], ids=str)
+def test_one_launch_matches_the_oracle(cuda_runtime, codegen, heads, append, layers, lengths):
+    """Lengths at which a block, a warp's turn or a tile starts or ends; runs within a share and cut into 2 to 40 pieces (more
+    than eight: merged in two steps); steps in turn on the same caches.  fp32 sums of fp16 products: 2e-5 of the result's norm;
+    the newest rows are the projections' bits."""
+    Hq, Hkv, D = heads
+    B, S = len(lengths), max(lengths) + 3
+    rng = np.random.default_rng(3)
+    f16 = lambda *s: rng.standard_normal(s, dtype=np.float32).astype(np.float16)
+    ex = executor(cuda_runtime, codegen, heads, B, S, layers, with_append=append)
+    try:
+        caches = [(f16(B, S, Hkv, D), f16(B, S, Hkv, D)) for _ in range(layers)]
+        for step in range(2):
+            off = np.array([min(n + step, S) for n in lengths], dtype=np.int32) - 1
+            q, kn, vn = f16(layers, B, Hq, D), f16(layers, B, Hkv, D), f16(layers, B, Hkv, D)
+            for l, (k, v) in enumerate(caches):
+                for b in range(B):
+                    k[b, off[b] + 1:], v[b, off[b] + 1:] = np.inf, np.nan            # nothing behind the end counts
+                ex.upload_layer(l, q[l], k, v)
+                ex.upload_new_kv(l, kn[l], vn[l])
+            out = ex.execute_decode_batch(off)
+            assert ex.kernel_launches_per_step == 1 and ex.route_name[0].startswith("vteb_decode_step_")
+            for l, (k, v) in enumerate(caches):
+                if append:
+                    orc.kv_cache_append(kn[l], vn[l], k, v, off)
+                ref = orc.decode_attention(q[l], np.where(np.isfinite(k), k, 0), np.where(np.isfinite(v), v, 0), off)
+                assert np.linalg.norm(out[l] - ref) <= 2e-5 * np.linalg.norm(ref)
+                for b in (0, B - 1):
+                    got = ex.download_cache_rows(l, b, S)
+                    assert all(np.array_equal(x.view(np.uint16), y[b].view(np.uint16)) for x, y in zip(got, (k, v)))
+                for b in range(B):
+                    k[b, off[b] + 1:], v[b, off[b] + 1:] = 0.5, 0.25
+    finally:
+        ex.cleanup()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("heads,meta", [((12, 2, 128), {}), ((8, 4, 64), dict(rope_type=1)), ((8, 2, 256), dict(rope_type=2, rotary_dim=64)),
+                                        ((8, 2, 256), {}), ((16, 2, 128), dict(rope_type=2, rotary_dim=128))])
+@pytest.mark.parametrize("rope", ["fused", "fused-append"])
+def test_one_launch_rotates(cuda_runtime, codegen, heads, meta, rope):
+    """Q and the newest K row rotated on the way: the oracle's outputs, and the oracle's bits in the cache."""
+    Hq, Hkv, D = heads
+    B, S, L = 3, 600, 3
+    rng = np.random.default_rng(5)
+    f16 = lambda *s: rng.standard_normal(s, dtype=np.float32).astype(np.float16)
+    ex = executor(cuda_runtime, codegen, heads, B, S, L, rope=rope, meta=meta)
+    rope_type, width = meta.get("rope_type", 0), meta.get("rotary_dim", D)
+    cos, sin = orc.rope_tables(S, width, 1e6)
+    try:
+        off = np.array([0, 333, 599], dtype=np.int32)
+        for l in range(L):
+            q, k, v, kn, vn = f16(B, Hq, D), f16(B, S, Hkv, D), f16(B, S, Hkv, D), f16(B, Hkv, D), f16(B, Hkv, D)
+            ex.upload_layer(l, q, k, v)
+            ex.upload_new_kv(l, kn, vn)
+            if l == L - 1:
+                out = ex.execute_decode_batch(off)
+        assert ex.kernel_launches_per_step == 1
+        q, kn = orc.rope_step(q, kn, cos, sin, off, rope_type, width)
+        orc.kv_cache_append(kn, vn, k, v, off)
+        ref = orc.decode_attention(q, k, v, off)
+        assert np.linalg.norm(out[L - 1] - ref) <= 2e-5 * np.linalg.norm(ref)
+        for b in range(B):
+            got = ex.download_cache_rows(L - 1, b, S)
+            assert np.array_equal(got[0].view(np.uint16), k[b].view(np.uint16)) and np.array_equal(got[1].view(np.uint16), v[b].view(np.uint16))
+    finally:
+        ex.cleanup()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("heads,B,S", [((12, 2, 128), 1, 8192), ((32, 8, 64), 4, 2048), ((8, 2, 256), 2, 4096), ((32, 2, 128), 2, 4096)])
+def test_one_launch_is_as_exact_as_the_launches_per_layer(cuda_runtime, codegen, heads, B, S):
+    """Both against 64-bit sums: the routes it takes the place of keep fp32 sums of fp16 products, at 1.5e-7 to 2.2e-7 of the norm or
+    more; a tenth is allowed for the order of the sums."""
+    Hq, Hkv, D = heads
+    rng = np.random.default_rng(S)
+    f16 = lambda *s: rng.standard_normal(s, dtype=np.float32).astype(np.float16)
+    L, off = 2, np.full(B, S - 1, dtype=np.int32)
+    data, error = [(f16(B, Hq, D), f16(B, S, Hkv, D), f16(B, S, Hkv, D)) for _ in range(L)], []
+    ref = [orc.decode_attention(*x, off, dtype=np.float64) for x in data]
+    for one in (True, False):
+        ex = executor(cuda_runtime, codegen, heads, B, S, L, one_launch=one)
+        try:
+            for l in range(L):
+                ex.upload_layer(l, *data[l])
+            out = ex.execute_decode_batch(off)
+            error.append(max(np.linalg.norm(out[l] - ref[l]) / np.linalg.norm(ref[l]) for l in range(L)))
+        finally:
+            ex.cleanup()
+    assert error[0] <= 1.1 * error[1]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("heads", [(12, 2, 128), (32, 8, 64), (8, 2, 256), (32, 2, 128)])
+def test_infinite_values_stay_infinite(cuda_runtime, codegen, heads):
+    """An infinite V gives the infinities and NaNs of fp32 products, in columns of its own; the others are untouched."""
+    Hq, Hkv, D = heads
+    B, S, L = 2, 500, 3
+    rng = np.random.default_rng(11)
+    f16 = lambda *s: rng.standard_normal(s, dtype=np.float32).astype(np.float16)
+    ex = executor(cuda_runtime, codegen, heads, B, S, L)
+    try:
+        off = np.array([S - 1, 40], dtype=np.int32)
+        q, k, v = f16(B, Hq, D), f16(B, S, Hkv, D), f16(B, S, Hkv, D)
+        v[0, 17, 0, 3], v[0, 400, 0, 5], v[1, 40, Hkv - 1, D - 1] = np.inf, -np.inf, np.inf
+        for l in range(L):
+            ex.upload_layer(l, q, k, v)
+        out = ex.execute_decode_batch(off)
+        ref = orc.decode_attention(q, k, v, off)
+        assert np.isinf(ref).any()
+        for l in range(L):
+            assert np.array_equal(np.isposinf(out[l]), np.isposinf(ref)) and np.array_equal(np.isneginf(out[l]), np.isneginf(ref))
+            fine = np.isfinite(ref)
+            assert np.linalg.norm(out[l][fine] - ref[fine]) <= 2e-5 * np.linalg.norm(ref[fine])
+    finally:
+        ex.cleanup()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kw", [dict(with_append=True), dict(rope="fused-append"), {}], ids=str)
+def test_partials_after_one_launch_and_many_layers(cuda_runtime, codegen, kw):
+    """70 layers are two launches; the partials of the last one are those of a launch list per layer, bit for bit."""
+    heads, B, S, L = (12, 2, 128), 2, 200, 70
+    Hq, Hkv, D = heads
+    rng = np.random.default_rng(2)
+    f16 = lambda *s: rng.standard_normal(s, dtype=np.float32).astype(np.float16)
+    q, kn, vn = f16(L, B, Hq, D), f16(L, B, Hkv, D), f16(L, B, Hkv, D)
+    caches, off, got = [(f16(B, S, Hkv, D), f16(B, S, Hkv, D)) for _ in range(L)], np.array([150, 199], dtype=np.int32), []
+    for one in (True, False):
+        ex = executor(cuda_runtime, codegen, heads, B, S, L, one_launch=one, output_f32=False, **kw)
+        try:
+            for l in range(L):
+                ex.upload_layer(l, q[l], *caches[l])
+                ex.upload_new_kv(l, kn[l], vn[l])
+            out = ex.execute_decode_batch(off)
+            assert not one or ex.kernel_launches_per_step == 2
+            again = ex.execute_decode_batch(off, q)                  # from the host
+            assert np.array_equal(out, again)
+            for l in range(L):
+                ex.upload_layer(l, q[L - 1 - l])                      # the next step's
+            got.append((out, ex.read_partials()))
+        finally:
+            ex.cleanup()
+    (a, pa), (b, pb) = got
+    assert np.linalg.norm(a.astype(np.float64) - b) <= 5e-4 * np.linalg.norm(b.astype(np.float64))      # fp16 outputs, rounded once
+    used = pb[1] > 0
+    assert used.any() and np.array_equal(pa[1], pb[1]) and np.array_equal(pa[0][used], pb[0][used]) and np.array_equal(pa[2][used], pb[2][used])
+
+
+@pytest.mark.gpu
+def test_shared_caches_with_an_append_keep_their_order(cuda_runtime, codegen):
+    """Layers that append to one cache depend on one another: a launch list per layer, and `one_launch` is refused."""
+    for kw, name in ((dict(with_append=True), None), ({}, "vteb_decode_step_d128_kernel")):
+        ex = executor(cuda_runtime, codegen, (12, 2, 128), 1, 600, 4, n_kv_buffers=2, one_launch=None, **kw)
+        try:
+            ex.build_decode_graph()
+            assert (ex.route_name or ("",))[0] == name if name else not (ex.route_name or ("",))[0].startswith("vteb_decode_step")
+        finally:
+            ex.cleanup()
+    ex = executor(cuda_runtime, codegen, (12, 2, 128), 1, 600, 4, n_kv_buffers=2, with_append=True)
+    try:
+        with pytest.raises(CudaSafetyError, match="another writes"):
+            ex.build_decode_graph()
+    finally:
+        ex.cleanup()
+
+
+@pytest.mark.gpu
+def test_a_state_that_never_comes_is_reported(cuda_runtime, codegen):
+    """One CTA's count of launches is set off by five, so its state carries another number than the CTA that finishes the run
+    waits for: after 200,000 cycles the kernel gives up and says so, and the next step is right."""
+    class Short:
+        def load_kernel_safe(self, *a, **kw):
+            return codegen.load_kernel_safe(*a, vteb_wait_limit_cycles=200000, **kw)
+    ex = DecodeAttentionExecutor(cuda_runtime, Short(), {"attention.head_count": 12, "attention.head_count_kv": 2, "attention.key_length": 128},
+                                 1, 4096, 4, one_launch=True)
+    try:
+        for l in range(4):
+            ex.fill_cache_on_device(l, l + 1)
+            ex.upload_layer(l, np.ones((1, 12, 128), dtype=np.float16))
+        off = np.array([4095], dtype=np.int32)
+        good = ex.execute_decode_batch(off)
+        count = ctypes.c_void_p(ex._step.launch_counts)
+        cuda_runtime.safe_memcpy_host_to_device(count, np.array([5], dtype=np.uint32), "launch count")
+        with pytest.raises(CudaRuntimeError):
+            ex.execute_decode_batch(off)
+        cuda_runtime.safe_memcpy_host_to_device(count, np.array([2], dtype=np.uint32), "launch count")
+        assert np.array_equal(ex.execute_decode_batch(off), good)
+    finally:
+        ex.cleanup()

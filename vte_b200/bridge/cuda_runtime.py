@@ -73,6 +73,26 @@ class KvTensorMap(ctypes.Structure):
     _fields_ = [("opaque", ctypes.c_uint64 * 16)]
 
 
+class StepPlan(ctypes.Structure):
+    """Mirror of `vteb_step_plan_t` (include/vteb200.h)."""
+    _fields_ = [("ok", ctypes.c_int), ("threads", ctypes.c_int), ("smem_bytes", ctypes.c_int), ("hg", ctypes.c_int),
+                ("state_bytes", ctypes.c_int), ("max_layers", ctypes.c_int), ("hg_log2", ctypes.c_int), ("wph", ctypes.c_int), ("tile", ctypes.c_int)]
+
+
+class StepLayer(ctypes.Structure):
+    """One layer of a `vteb_decode_step_*` launch (StepLayer in csrc/kernels/step_decode.cuh)."""
+    _fields_ = ([("k_map", KvTensorMap), ("v_map", KvTensorMap)] +
+                [(name, ctypes.c_void_p) for name in ("q", "k_cache", "v_cache", "k_new", "v_new", "output")] + [("unused", ctypes.c_void_p * 2)])
+
+
+class StepArgs(ctypes.Structure):
+    """The argument of the `vteb_decode_step_*` kernels, by value (StepArgs in csrc/kernels/step_decode.cuh)."""
+    _fields_ = ([("layer", StepLayer * 64)] +
+                [(name, ctypes.c_void_p) for name in ("kv_offsets", "rope_cos", "rope_sin", "boards", "launches", "status", "keep_q", "keep_offsets")] +
+                [(name, ctypes.c_int) for name in ("keep_layer", "num_layers", "batch", "num_q_heads", "num_kv_heads", "kv_batch_stride",
+                                                   "out_kind", "rope_type", "rotary_dim", "hg", "hg_log2", "wph", "group", "groups", "group_inv")] + [("scale", ctypes.c_float)])
+
+
 class ClusterGrid(tuple):
     """Grid dimensions of a launch whose blocks form thread-block clusters of `cluster` along x."""
     def __new__(cls, dims, cluster: int):
@@ -147,8 +167,10 @@ def _declare(lib):
         "vteb_lean_plan": (i, [i, i, i, i, ll, i, ctypes.POINTER(LeanPlan)]),
         "vteb_lean_estimate": (ctypes.c_double, [i, i, i, i, i, i, ll, i, i]),
         "vteb_lean_step_estimate": (ctypes.c_double, [i, i, i, i, i, i, ll, ll, ll, i]),
+        "vteb_step_plan": (i, [i, i, i, i, i, i, ctypes.POINTER(StepPlan)]),
         "vteb_max_active_clusters": (i, [vp, i, i, i, ip]),
         "vteb_kv_tensor_map": (i, [vp, vp, ctypes.c_longlong, i, i]),
+        "vteb_kv_tensor_map_columns": (i, [vp, vp, ctypes.c_longlong, i, i, i]),
         "vteb_combine_rows_epl": (i, [i, i]),
         "vteb_split_kv_decode": (i, [vp, vp, vp, vp, vp, i, vp, vp, vp, vp, i, i, i, i, f, ll, i, i, u, i, vp]),
         "vteb_split_kv_decode_noalloc": (i, [vp, vp, vp, vp, vp, i, i, i, i, i, f, ll, i, i, u, i, vp]),
@@ -778,6 +800,12 @@ class CudaRuntime:
         """Estimated microseconds of one layer of a step with these lengths (kind -1: the dispatcher's launches)."""
         return self._lib.vteb_lean_step_estimate(kind, n_parts, num_q_heads, num_kv_heads, head_dim, batch, capacity, longest, total, resident)
 
+    def step_plan(self, num_q_heads: int, num_kv_heads: int, head_dim: int, batch: int, n_ctas: int, hg: int = 0) -> StepPlan:
+        """What a launch of the whole-step kernels needs; `hg`: KV heads a CTA serves at once, 0: chosen."""
+        plan = StepPlan()
+        self._check_error(self._lib.vteb_step_plan(num_q_heads, num_kv_heads, head_dim, batch, n_ctas, hg, ctypes.byref(plan)), "vteb_step_plan")
+        return plan
+
     def max_active_clusters(self, function, cluster: int, threads: int, smem_bytes: int) -> int:
         """Clusters of `cluster` blocks of a loaded kernel that the device runs at once."""
         key = (_ptr_value(function), cluster, threads, smem_bytes)
@@ -788,10 +816,15 @@ class CudaRuntime:
             self._active_clusters[key] = n.value
         return self._active_clusters[key]
 
-    def kv_tensor_map(self, cache_ptr: int, n_rows: int, row_halves: int, box_rows: int) -> KvTensorMap:
+    def kv_tensor_map(self, cache_ptr: int, n_rows: int, row_halves: int, box_rows: int, box_cols: int = 0) -> KvTensorMap:
         """Tensor map over a cache of `n_rows` position rows of `row_halves` fp16 values (boxes of
-        64 values x `box_rows` rows, 128-byte swizzle) for the fast split kernels."""
+        64 values x `box_rows` rows, 128-byte swizzle) for the fast split kernels; with `box_cols`, boxes of as many such
+        columns, for the whole-step kernels."""
         tm = KvTensorMap()
+        if box_cols:
+            self._check_error(self._lib.vteb_kv_tensor_map_columns(ctypes.byref(tm), ctypes.c_void_p(int(cache_ptr)), int(n_rows), int(row_halves),
+                                                                   int(box_rows), int(box_cols)), "vteb_kv_tensor_map_columns")
+            return tm
         self._check_error(self._lib.vteb_kv_tensor_map(ctypes.byref(tm), ctypes.c_void_p(int(cache_ptr)), int(n_rows),
                                                        int(row_halves), int(box_rows)), "vteb_kv_tensor_map")
         return tm

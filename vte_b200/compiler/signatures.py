@@ -60,6 +60,11 @@ KERNEL_SIGNATURES = {
     "vteb_decode_cluster_half_d128_kernel": _LEAN,                    # half the warps a block, two blocks an SM
     "vteb_decode_cluster_half_d256_kernel": _LEAN,
     "vteb_decode_cluster_half_2_d128_kernel": _LEAN,
+    "vteb_decode_step_d64_kernel": [ctypes.Structure],                # all layers of a step in one launch
+    "vteb_decode_step_d128_kernel": [ctypes.Structure],
+    "vteb_decode_step_d256_kernel": [ctypes.Structure],
+    "vteb_decode_step_2_d64_kernel": [ctypes.Structure],
+    "vteb_decode_step_2_d128_kernel": [ctypes.Structure],
     "vteb_split_kv_lean_d64_kernel": _LEAN,                           # one sequence: a part of one KV head per CTA
     "vteb_split_kv_lean_d128_kernel": _LEAN,
     "vteb_split_kv_lean_d256_kernel": _LEAN,

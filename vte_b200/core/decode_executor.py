@@ -25,6 +25,7 @@ from ..bridge.memory import MemoryRegion, SlabAllocator
 from ..config import ENV_NO_PDL, env_flag
 from .lean_route import LeanRoute, choose_lean_route
 from .split_kv_attention import FLAG_DIRECT_OUTPUT, SplitKVAttentionDispatcher
+from .step_route import StepRoute, one_launch_pays
 
 
 def _round_up(x: int, m: int) -> int:
@@ -43,6 +44,8 @@ OFFSET_SLOTS = 64
 
 
 class DecodeAttentionExecutor:
+    _step, _one_launch = None, False
+
     def __init__(self, hip, codegen, metadata: dict, batch_size: int, context_length: int, n_layers: int, *,
                  n_kv_buffers: Optional[int] = None, num_splits: Optional[int] = None, output_f32: bool = True,
                  use_graph: bool = True, programmatic: Optional[bool] = None, compat: bool = False,
@@ -51,7 +54,8 @@ class DecodeAttentionExecutor:
                  emit_state: bool = False, per_layer_hook=None, prefetch_next_layer: bool = True,
                  fused_combine: Optional[bool] = None, variant: str = "auto", rope: str = "off",
                  rope_theta: float = 1e6, tensor_maps: bool = True, fuse_append: bool = False,
-                 balanced: Optional[bool] = None, wide: Optional[bool] = None, lean: Optional[tuple] = None):
+                 balanced: Optional[bool] = None, wide: Optional[bool] = None, lean: Optional[tuple] = None,
+                 one_launch: Optional[bool] = None):
         self.hip = hip
         if lean is not None and lean[0] and (compat or strict_empty_splits or emit_state or fused_combine):
             raise CudaSafetyError("a route of lean_route.py has no compat kernels, empty-split partials, shard states or fused combine")
@@ -125,6 +129,12 @@ class DecodeAttentionExecutor:
                                                   tensor_maps and prefetch_next_layer)
         self._lean = lean if lean is not None else None if open_layout else (0, 0)
         self._route, self._forced_route = None, lean is not None
+        # one_launch: the whole step in one launch over all layers (step_route.py); None where it may and pays, False: a launch
+        # list per layer, in which a layer starts when the one in front of it is done, True: refused where it may not
+        if one_launch and (lean is not None or not open_layout):
+            raise CudaSafetyError("one launch for all layers takes no split layout, partials, shard states or shapes of the caller's")
+        self._one_launch = one_launch if one_launch is not None else None if lean is None and open_layout else False
+        self._step = None
         # where lengths can make the dispatcher's launches the shorter ones: a step of those is captured beside the route's, and
         # each step takes one by its longest and total length; up to _route_pays_to positions it is the route's in any case
         self._route_pays_to, self._on_route, self._launches = self.S, True, (0, 0)
@@ -246,12 +256,22 @@ class DecodeAttentionExecutor:
 
     @property
     def route_name(self):
-        """(kernel, CTAs per (sequence, KV head)) where the last captured step did not take the dispatcher's launches, else None."""
+        """(kernel, CTAs per (sequence, KV head)) where the last captured step did not take the dispatcher's launches, else None;
+        (kernel, 0) where it is one launch."""
+        if self._step is not None:
+            return self._step.name, 0
         return (self._route.name, self._route.parts) if self._route is not None and self._on_route else None
 
     def _record_all(self, after_copy: bool = False, plain: bool = False):
         n = 0
         programmatic = self.hip.programmatic_launch
+        if self._step is not None:
+            launches = self._step.launches(self.tensor_mapping, self.offsets.ptr, self.B,
+                                           (self._kept.ptr, self._kept.ptr + _round_up(self.q_bytes, 256)))
+            self._kept_names = dict(self.tensor_mapping)
+            for launch in launches:
+                self.hip.launch_kernel_recorded(*launch)
+            return len(launches)
         # within a captured step of nothing but the layers' own launches, offsets and older rows do not change
         self.dispatcher.offsets_final = self.use_graph and self.per_layer_hook is None and self.launch_rewriter is None
         for l in range(self.L):
@@ -276,11 +296,15 @@ class DecodeAttentionExecutor:
     def _choose_route(self):
         """Before a step is captured: whether its layers' launches are the dispatcher's own or a route of lean_route.py."""
         d = self.dispatcher
-        if (self._route is not None or self._lean == (0, 0) or not self.use_graph or self.per_layer_hook is not None or
-                self.launch_rewriter is not None or not d.enabled or not hasattr(self.hip, 'lean_plan')):
+        if (self._route is not None or self._step is not None or self._lean == (0, 0) and not self._one_launch or not self.use_graph or
+                self.per_layer_hook is not None or self.launch_rewriter is not None or not d.enabled or not hasattr(self.hip, 'lean_plan')):
+            if self._one_launch and self._step is None:
+                raise CudaSafetyError("one launch for all layers needs a captured step without a hook or a rewriter")
             return
         d._allocate_scratch()                         # and the work words
         append = self.with_append or d.fuse_append
+        if self._one_launch is not False and self._choose_one_launch(append):
+            return
         if self._lean is None:
             self._lean = choose_lean_route(d, append)
         if self._lean[0]:
@@ -296,6 +320,31 @@ class DecodeAttentionExecutor:
             self._route = route
             if not self._forced_route:
                 self._route_pays_to = route.pays_up_to()
+
+    def _choose_one_launch(self, append: bool) -> bool:
+        """Takes one launch for the step where its layers may run side by side and that pays."""
+        d, forced, blocks = self.dispatcher, bool(self._one_launch), []
+        if self.rope == "separate" or not hasattr(self.hip, 'step_plan') or (not forced and not one_launch_pays(d, self.L)):
+            if forced:
+                raise CudaSafetyError("one launch for all layers has no rotation launches")
+            return False
+        try:
+            step = StepRoute(d, self.allocator, self.L, append)
+            blocks.append(step.scratch)
+            self._kept = self.allocator.allocate(_round_up(self.q_bytes, 256) + _round_up(4 * self.B, 256), "attn_partials_source",
+                                                 MemoryRegion.SCRATCH)
+            blocks.append(self._kept)
+            if not step.serves(self.tensor_mapping, self.offsets.ptr, self.B):
+                raise CudaSafetyError("one launch for all layers: a layer reads or writes what another writes, or has pointers that are not 16-byte aligned")
+        except CudaSafetyError:
+            if forced:
+                raise
+            for block in blocks:
+                self.allocator.free(block)
+            self._kept = None
+            return False
+        self._step = step
+        return True
 
     def build_decode_graph(self):
         """Capture all layers' launches once (hip_graph_executor.py:504-725)."""

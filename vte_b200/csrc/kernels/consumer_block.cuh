@@ -251,6 +251,14 @@ __device__ __forceinline__ void mma_full(float (&c)[4], uint32_t a0, uint32_t a1
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
+// The same product on its own: the accumulator operand is the zero register, nothing has to be cleared first.
+__device__ __forceinline__ void mma_alone(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 "
+        "{%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
+}
+
 // 8x8 transpose of 16-bit elements across the warp: lane (g, t) gives row g, columns 2t, 2t+1
 // and receives row g, columns 2t, 2t+1 of the transposed matrix.
 __device__ __forceinline__ uint32_t movmatrix_trans(uint32_t x) {
@@ -405,17 +413,18 @@ __device__ __forceinline__ void softmax_pv_t(ConsumerStateT<MT>& st, const float
 // kernels give (kFresh).  An infinite V times a zero part of P is NaN where its product with the whole of P is infinite:
 // in a masked row, as the low part of a probability that fp16 holds exactly, or where the two parts differ in sign.  A
 // warp whose sums hold a NaN at the end of an item walks its blocks again, straight from the caches, and rewrites o in
-// its exchange rows (`n_rows` rows of `pitch` floats: o[D], 4 unused, m, ...); m and l stand.  `q`: the rows' queries;
-// `k`, `v`: the KV head's row 0, rows `stride` halves apart; blocks from position `first` on, `step` apart, below `end`.
+// its exchange rows (`n_rows` rows of `pitch` floats); m, `m_pitch` floats apart, and l stand.  `q`: the rows' queries;
+// `k`, `v`: the KV head's row 0, rows `stride` halves apart; blocks from position `first` on, `step` apart, below `end`;
+// column c at c ^ `swizzle` (a multiple of 8 below 32).
 // Checked once an item, eight sequences of sixteen heads per KV head, 8 layers: 163.4 -> 164.8 us; a check of every
 // block's products took 170.4.
 template <int D>
-__device__ __noinline__ void redo_rows_fp32(float* rows, int n_rows, int pitch, const __half* q, const __half* k, const __half* v,
-                                            long long stride, int first, int end, int step, float scale2) {
+__device__ __noinline__ void redo_rows_fp32(float* rows, int n_rows, int pitch, const float* maxima, int m_pitch, const __half* q,
+                                            const __half* k, const __half* v, long long stride, int first, int end, int step, float scale2, int swizzle = 0) {
     const int lane = threadIdx.x & 31;
     __syncwarp();
     for (int r = 0; r < n_rows; ++r) {
-        const float m = rows[r * pitch + D + 4];
+        const float m = maxima[r * m_pitch];
         float o[D / 32];
 #pragma unroll
         for (int c = 0; c < D / 32; ++c) o[c] = 0.f;
@@ -432,7 +441,7 @@ __device__ __noinline__ void redo_rows_fp32(float* rows, int n_rows, int pitch, 
                 for (int c = 0; c < D / 32; ++c) o[c] = fmaf(p, __half2float(v[j * stride + c * 32 + lane]), o[c]);
             }
 #pragma unroll
-        for (int c = 0; c < D / 32; ++c) rows[r * pitch + c * 32 + lane] = o[c];
+        for (int c = 0; c < D / 32; ++c) rows[r * pitch + c * 32 + (lane ^ swizzle)] = o[c];
     }
     __syncwarp();
 }

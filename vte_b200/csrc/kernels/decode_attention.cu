@@ -1364,3 +1364,4 @@ extern "C" __global__ void vteb_advance_step_kernel(int* __restrict__ step_word)
 
 #include "split_kv_fast.cuh"
 #include "lean_decode.cuh"
+#include "step_decode.cuh"

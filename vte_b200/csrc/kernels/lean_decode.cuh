@@ -230,9 +230,9 @@ __device__ __forceinline__ uint4 rope_chunk(uint4 x, const __half* row, int d0, 
 }
 
 // Scores of a 16-position block for NV runs of up to eight query heads, K fragments shared by the runs (transposed form
-// of consumer_block.cuh).  kFresh: products of one k-step start from zero and are summed in fp32 registers.
+// of consumer_block.cuh); `col_bytes` between 64 channels and the next 64 of a row.  kFresh: products of one k-step start from zero and are summed in fp32 registers.
 template <int D, int NV, bool kFresh>
-__device__ __forceinline__ void lean_scores(const uint32_t* q_frag, uint32_t kaddr, float (&s)[NV][4]) {
+__device__ __forceinline__ void lean_scores(const uint32_t* q_frag, uint32_t kaddr, float (&s)[NV][4], uint32_t col_bytes = 128) {
     constexpr int KS = D / 16, CH = kFresh ? 4 : 2;
     float acc[NV][CH][4];
 #pragma unroll
@@ -247,24 +247,25 @@ __device__ __forceinline__ void lean_scores(const uint32_t* q_frag, uint32_t kad
     for (int kc = 0; kc < KS; kc += 4) {
         uint32_t kf[4][4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) ldmatrix_x4((kaddr ^ (i << 5)) + (kc >> 2) * 128, kf[i][0], kf[i][1], kf[i][2], kf[i][3]);
+        for (int i = 0; i < 4; ++i) ldmatrix_x4((kaddr ^ (i << 5)) + (kc >> 2) * col_bytes, kf[i][0], kf[i][1], kf[i][2], kf[i][3]);
 #pragma unroll
         for (int i = 0; i < 4; i += 2)
 #pragma unroll
             for (int v = 0; v < NV; ++v) {
                 const uint4 qv = *reinterpret_cast<const uint4*>(q_frag + (v * (D / 8) + 2 * (kc + i)) * 32);    // k-steps kc + i, kc + i + 1
-                mma_full(acc[v][i % CH], kf[i][0], kf[i][2], kf[i][1], kf[i][3], qv.x, qv.y);
-                mma_full(acc[v][(i + 1) % CH], kf[i + 1][0], kf[i + 1][2], kf[i + 1][1], kf[i + 1][3], qv.z, qv.w);
+                if constexpr (kFresh) {
+                    mma_alone(acc[v][i], kf[i][0], kf[i][2], kf[i][1], kf[i][3], qv.x, qv.y);
+                    mma_alone(acc[v][i + 1], kf[i + 1][0], kf[i + 1][2], kf[i + 1][1], kf[i + 1][3], qv.z, qv.w);
+                } else {
+                    mma_full(acc[v][i % CH], kf[i][0], kf[i][2], kf[i][1], kf[i][3], qv.x, qv.y);
+                    mma_full(acc[v][(i + 1) % CH], kf[i + 1][0], kf[i + 1][2], kf[i + 1][1], kf[i + 1][3], qv.z, qv.w);
+                }
             }
         if constexpr (kFresh) {
 #pragma unroll
             for (int v = 0; v < NV; ++v)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    s[v][j] += (acc[v][0][j] + acc[v][1][j]) + (acc[v][2][j] + acc[v][3][j]);
-#pragma unroll
-                    for (int c = 0; c < CH; ++c) acc[v][c][j] = 0.f;
-                }
+                for (int j = 0; j < 4; ++j) s[v][j] += (acc[v][0][j] + acc[v][1][j]) + (acc[v][2][j] + acc[v][3][j]);
         }
     }
     if constexpr (!kFresh) {
@@ -278,46 +279,59 @@ __device__ __forceinline__ void lean_scores(const uint32_t* q_frag, uint32_t kad
 // Softmax step and O^T += V^T P^T for NV runs, V fragments shared by the runs; `st[v]` as in softmax_pv_t.
 template <int D, int NV, bool kFresh>
 __device__ __forceinline__ void lean_softmax_pv(ConsumerStateT<D / 16> (&st)[NV], const float (&sraw)[NV][4], uint32_t vaddr,
-                                                int left, float scale2, int g) {
+                                                int left, float scale2, int g, uint32_t col_bytes = 128) {
     constexpr int NVC = D / 64;                  // chunks of 64 output columns
     uint32_t vf[2][4][4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) ldmatrix_x4_trans(vaddr ^ (i << 5), vf[0][i][0], vf[0][i][1], vf[0][i][2], vf[0][i][3]);
     const bool valid[2] = {g < left, g + 8 < left};
+    constexpr float kSlack = VTEB_LAZY_MAX;
     uint32_t bh[NV][2], bl[NV][2];
+    float s[NV][4], p[NV][4], mx[NV][2];
+    bool up = false;
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
-        float s[4], p[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) s[i] = valid[i >> 1] ? sraw[v][i] * scale2 : kNeutralM;
-        const float mx[2] = {fmaxf(s[0], s[2]), fmaxf(s[1], s[3])};
-        st[v].mt[0] = fmaxf(st[v].mt[0], mx[0]);
-        st[v].mt[1] = fmaxf(st[v].mt[1], mx[1]);
-        constexpr float kSlack = VTEB_LAZY_MAX;
-        if (__any_sync(0xffffffffu, (mx[0] > st[v].m[0] + kSlack) | (mx[1] > st[v].m[1] + kSlack))) {
-            float corr[2];
+        for (int i = 0; i < 4; ++i) s[v][i] = valid[i >> 1] ? sraw[v][i] * scale2 : kNeutralM;
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const float m_up = fmaxf(st[v].m[h], max_over_g(mx[h]));
-                corr[h] = fast_exp2(st[v].m[h] - m_up);
-                st[v].l[h] *= corr[h];
-                st[v].m[h] = m_up;
-            }
-#pragma unroll
-            for (int i = 0; i < D / 16; ++i) { st[v].o[i][0] *= corr[0]; st[v].o[i][1] *= corr[1]; st[v].o[i][2] *= corr[0]; st[v].o[i][3] *= corr[1]; }
+        for (int h = 0; h < 2; ++h) {
+            mx[v][h] = fmaxf(s[v][h], s[v][2 + h]);
+            st[v].mt[h] = fmaxf(st[v].mt[h], mx[v][h]);
+            up = up || mx[v][h] > st[v].m[h] + kSlack;
         }
+    }
+    if (__any_sync(0xffffffffu, up)) {                               // one branch for all runs: their arithmetic overlaps
 #pragma unroll
-        for (int i = 0; i < 4; ++i) p[i] = valid[i >> 1] ? fast_exp2(s[i] - st[v].m[i & 1]) : 0.f;
-        st[v].l[0] += p[0] + p[2];
-        st[v].l[1] += p[1] + p[3];
+        for (int v = 0; v < NV; ++v)
+            if (NV == 1 || __any_sync(0xffffffffu, (mx[v][0] > st[v].m[0] + kSlack) | (mx[v][1] > st[v].m[1] + kSlack))) {
+                float corr[2];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const float m_up = fmaxf(st[v].m[h], max_over_g(mx[v][h]));
+                    corr[h] = fast_exp2(st[v].m[h] - m_up);
+                    st[v].l[h] *= corr[h];
+                    st[v].m[h] = m_up;
+                }
+#pragma unroll
+                for (int i = 0; i < D / 16; ++i) { st[v].o[i][0] *= corr[0]; st[v].o[i][1] *= corr[1]; st[v].o[i][2] *= corr[0]; st[v].o[i][3] *= corr[1]; }
+            }
+    }
+#pragma unroll
+    for (int v = 0; v < NV; ++v)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) p[v][i] = valid[i >> 1] ? fast_exp2(s[v][i] - st[v].m[i & 1]) : 0.f;
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+        st[v].l[0] += p[v][0] + p[v][2];
+        st[v].l[1] += p[v][1] + p[v][3];
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
-            if constexpr (kFresh) { p[2 * r] *= kFreshUp; p[2 * r + 1] *= kFreshUp; }
-            const __half2 hi = __floats2half2_rn(p[2 * r], p[2 * r + 1]);
+            if constexpr (kFresh) { p[v][2 * r] *= kFreshUp; p[v][2 * r + 1] *= kFreshUp; }
+            const __half2 hi = __floats2half2_rn(p[v][2 * r], p[v][2 * r + 1]);
             const float2 hif = __half22float2(hi);
             bh[v][r] = movmatrix_trans(*reinterpret_cast<const uint32_t*>(&hi));
-            constexpr float up = kFresh ? kFreshLoUp : 1.f;
-            bl[v][r] = movmatrix_trans(pack_half2((p[2 * r] - hif.x) * up, (p[2 * r + 1] - hif.y) * up));
+            constexpr float lo_up = kFresh ? kFreshLoUp : 1.f;
+            bl[v][r] = movmatrix_trans(pack_half2((p[v][2 * r] - hif.x) * lo_up, (p[v][2 * r + 1] - hif.y) * lo_up));
         }
     }
 #pragma unroll
@@ -325,7 +339,7 @@ __device__ __forceinline__ void lean_softmax_pv(ConsumerStateT<D / 16> (&st)[NV]
         if (ch + 1 < NVC) {
 #pragma unroll
             for (int i = 0; i < 4; ++i)
-                ldmatrix_x4_trans((vaddr ^ (i << 5)) + (ch + 1) * 128, vf[(ch + 1) & 1][i][0], vf[(ch + 1) & 1][i][1],
+                ldmatrix_x4_trans((vaddr ^ (i << 5)) + (ch + 1) * col_bytes, vf[(ch + 1) & 1][i][0], vf[(ch + 1) & 1][i][1],
                                   vf[(ch + 1) & 1][i][2], vf[(ch + 1) & 1][i][3]);
         }
 #pragma unroll
@@ -334,9 +348,9 @@ __device__ __forceinline__ void lean_softmax_pv(ConsumerStateT<D / 16> (&st)[NV]
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     const uint32_t* f = vf[ch & 1][i];
-                    float hi[4] = {0.f, 0.f, 0.f, 0.f}, lo[4] = {0.f, 0.f, 0.f, 0.f};
-                    mma_full(hi, f[0], f[2], f[1], f[3], bh[v][0], bh[v][1]);
-                    mma_full(lo, f[0], f[2], f[1], f[3], bl[v][0], bl[v][1]);
+                    float hi[4], lo[4];
+                    mma_alone(hi, f[0], f[2], f[1], f[3], bh[v][0], bh[v][1]);
+                    mma_alone(lo, f[0], f[2], f[1], f[3], bl[v][0], bl[v][1]);
 #pragma unroll
                     for (int j = 0; j < 4; ++j)
                         st[v].o[ch * 4 + i][j] = fmaf(fmaf(lo[j], kFreshLoDown, hi[j]), kFreshDown, st[v].o[ch * 4 + i][j]);
@@ -587,7 +601,7 @@ __device__ __forceinline__ void lean_body(const LeanArgs& a)
     if constexpr (kFresh) {
         const float all = (probe[0] + probe[1]) + (probe[2] + probe[3]);
         if (__any_sync(0xffffffffu, all != all) && !rotate)
-            redo_rows_fp32<D>(mine, group, PITCH, a.q + ((long long)b * a.num_q_heads + (long long)kv_head * group) * D, a.k_cache + base,
+            redo_rows_fp32<D>(mine, group, PITCH, mine + D + 4, PITCH, a.q + ((long long)b * a.num_q_heads + (long long)kv_head * group) * D, a.k_cache + base,
                               a.v_cache + base, pos_stride, start + warp * kBlockPos, end, CW * kBlockPos, scale2);
     }
     __syncthreads();

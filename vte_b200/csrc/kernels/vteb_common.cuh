@@ -254,6 +254,14 @@ __device__ __forceinline__ void tma_load_box_2d(uint32_t dst_smem, const void* t
         : "memory");
 }
 
+// The same of a map of columns (vteb_kv_tensor_map_columns): one copy brings a box of several columns of 64 halves.
+__device__ __forceinline__ void tma_load_box_columns(uint32_t dst_smem, const void* tensor_map, int col, int y, uint32_t bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+        ::"r"(dst_smem), "l"(tensor_map), "r"(0), "r"(y), "r"(col), "r"(bar)
+        : "memory");
+}
+
 constexpr long long kL2PrefetchMaxBytes = 24ll << 20;   // per tensor and launch: more than this is not asked for ahead (see split_kv_fast.cuh)
 
 // Asks L2 for `bytes` (a multiple of 16) from `base` (16-byte aligned) on: requests of 8 KB, dealt to the

@@ -144,20 +144,23 @@ bool g_fast_attr_set[kMaxDevices][7];
 
 // Tensor map over a K or V cache seen as a matrix of `n_rows` position rows of `row_halves`
 // fp16 values: boxes of 64 halves x `box_rows` rows, 128-byte swizzle.
+// `box_cols` 0: a matrix of rows, in boxes of 64 halves x `box_rows` rows.  Otherwise rows of columns of 64 halves, in boxes of
+// `box_cols` columns x `box_rows` rows, which land column after column: as many boxes of the first kind in one copy.
 int encode_kv_tensor_map(vteb::KvTensorMap* out, const void* cache, unsigned long long n_rows, int row_halves,
-                         int box_rows) {
+                         int box_rows, int box_cols = 0) {
     static_assert(sizeof(vteb::KvTensorMap) == sizeof(CUtensorMap), "tensor map size");
     int rc = driver_api();
     if (rc) return rc;
     if (!out || !cache || ((uintptr_t)cache & 15) || n_rows == 0 || n_rows > 0xffffffffULL || row_halves < 64 ||
-        row_halves % 64 || box_rows < 1 || box_rows > 256)
-        return fail(VTEB_ERR_INVALID_ARGUMENT, "tensor map: cache %p rows %llu row_halves %d box_rows %d", cache,
-                    n_rows, row_halves, box_rows);
-    const cuuint64_t dims[2] = {(cuuint64_t)row_halves, (cuuint64_t)n_rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)row_halves * 2};
-    const cuuint32_t box[2] = {64u, (cuuint32_t)box_rows};
-    const cuuint32_t elem_strides[2] = {1u, 1u};
-    return check_drv(g_drv.TensorMapEncodeTiled(reinterpret_cast<CUtensorMap*>(out), CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2,
+        row_halves % 64 || box_rows < 1 || box_rows > 256 || box_cols < 0 || box_cols * 64 > row_halves)
+        return fail(VTEB_ERR_INVALID_ARGUMENT, "tensor map: cache %p rows %llu row_halves %d box_rows %d box_cols %d", cache,
+                    n_rows, row_halves, box_rows, box_cols);
+    const cuuint64_t row = (cuuint64_t)row_halves * 2;
+    const cuuint64_t dims[3] = {box_cols ? 64u : (cuuint64_t)row_halves, (cuuint64_t)n_rows, (cuuint64_t)row_halves / 64};
+    const cuuint64_t strides[2] = {row, 128u};
+    const cuuint32_t box[3] = {64u, (cuuint32_t)box_rows, (cuuint32_t)box_cols};
+    const cuuint32_t elem_strides[3] = {1u, 1u, 1u};
+    return check_drv(g_drv.TensorMapEncodeTiled(reinterpret_cast<CUtensorMap*>(out), CU_TENSOR_MAP_DATA_TYPE_FLOAT16, box_cols ? 3 : 2,
                                                 const_cast<void*>(cache), dims, strides, box, elem_strides,
                                                 CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                                                 CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE),
@@ -617,6 +620,15 @@ double vteb_lean_step_estimate(int kind, int n_parts, int num_q_heads, int num_k
     return lean_step_us(kind, n_parts, num_q_heads, num_kv_heads, head_dim, batch, capacity, longest, (double)total, resident);
 }
 
+int vteb_step_plan(int num_q_heads, int num_kv_heads, int head_dim, int batch, int n_ctas, int hg, vteb_step_plan_t* plan) {
+    if (!plan) return fail(VTEB_ERR_INVALID_ARGUMENT, "null plan");
+    const StepPlan p = make_step_plan(num_q_heads, num_kv_heads, head_dim, batch, n_ctas, hg);
+    plan->ok = p.ok; plan->threads = p.threads; plan->smem_bytes = p.smem_bytes; plan->hg = p.hg;
+    plan->state_bytes = p.state_bytes; plan->max_layers = p.max_layers;
+    plan->hg_log2 = p.hg_log2; plan->wph = p.wph; plan->tile = p.tile;
+    return 0;
+}
+
 int vteb_max_active_clusters(void* function, int cluster, int threads, int smem_bytes, int* count) {
     REQUIRE_INIT();
     if (!function || !count || cluster < 1 || cluster > 16 || threads < 1 || smem_bytes < 0)
@@ -644,6 +656,16 @@ int vteb_kv_tensor_map(void* out_128_bytes, const void* cache, long long n_rows,
     if (n_rows <= 0) return fail(VTEB_ERR_INVALID_ARGUMENT, "tensor map: %lld rows", n_rows);
     vteb::KvTensorMap tm;
     int rc = encode_kv_tensor_map(&tm, cache, (unsigned long long)n_rows, row_halves, box_rows);
+    if (rc) return rc;
+    memcpy(out_128_bytes, &tm, sizeof(tm));
+    return 0;
+}
+
+int vteb_kv_tensor_map_columns(void* out_128_bytes, const void* cache, long long n_rows, int row_halves, int box_rows, int box_cols) {
+    REQUIRE_INIT();
+    if (n_rows <= 0 || box_cols < 1) return fail(VTEB_ERR_INVALID_ARGUMENT, "tensor map: %lld rows, %d columns a box", n_rows, box_cols);
+    vteb::KvTensorMap tm;
+    int rc = encode_kv_tensor_map(&tm, cache, (unsigned long long)n_rows, row_halves, box_rows, box_cols);
     if (rc) return rc;
     memcpy(out_128_bytes, &tm, sizeof(tm));
     return 0;

@@ -65,7 +65,7 @@ def main(argv=None) -> int:
             'attention.key_length': cfg.head_dim}
     n_kv = min(L, 28)
     ex = DecodeAttentionExecutor(rt, DefiningCodegen(defines), meta, cfg.batch, cfg.max_seq, L, n_kv_buffers=n_kv,
-                                 variant=a.variant)
+                                 variant=a.variant, one_launch=False)
     trace = rt.safe_malloc(TRACE_BYTES, "trace output")
     rt.safe_memset(trace, TRACE_BYTES, "trace output")
     ex.dispatcher._external_work_ptr = trace.value          # the work words' allocation doubles as the trace buffer

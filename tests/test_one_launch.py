@@ -23,7 +23,7 @@ def step_plan(Hq, Hkv, D, batch, ctas=148, hg=0):
 @pytest.mark.parametrize("D", [64, 128, 256])
 @pytest.mark.parametrize("group", [1, 7, 8, 9, 16, 17])
 def test_plan_covers_what_the_kernels_do(built_library, group, D):
-    assert ctypes.sizeof(StepLayer) == 320 and ctypes.sizeof(StepArgs) == 64 * 320 + 128 < 32764
+    assert ctypes.sizeof(StepLayer) == 320 and ctypes.sizeof(StepArgs) == 64 * 320 + 512 < 32764
     for Hkv in (1, 2, 3, 4, 6, 8, 12):
         for batch in (1, 64, 1024, 1025):
             p = step_plan(group * Hkv, Hkv, D, batch)
@@ -82,7 +82,8 @@ def test_what_goes_to_one_launch(built_library):
     pays = lambda layers, *a: one_launch_pays(a_route(1, True, *a)[0].d, layers)
     assert pays(28, (12, 2, 128), 1, 4096) and pays(4, (16, 1, 64), 1, 64) and pays(4, (32, 2, 128), 1, 4096)
     assert pays(3, (8, 2, 256), 8, 4096) and not pays(3, (8, 2, 256), 1, 4096) and not pays(3, (32, 2, 128), 8, 4096)
-    assert pays(2, (32, 8, 64), 64, 16384) and not pays(2, (32, 8, 64), 8, 4096)
+    assert pays(2, (8, 8, 128), 64, 16384) and pays(3, (32, 8, 64), 8, 4096)
+    assert not pays(2, (32, 8, 64), 64, 16384) and not pays(3, (32, 8, 64), 64, 16384) and not pays(2, (8, 8, 128), 8, 4096)
     assert not pays(1, (12, 2, 128), 1, 1 << 20)                   # one layer: nothing to share out
     assert not pays(28, (36, 2, 128), 1, 4096) and not pays(28, (18, 2, 256), 1, 4096) and not pays(28, (12, 2, 128), 1025, 64)
 
@@ -255,6 +256,46 @@ def test_partials_after_one_launch_and_many_layers(cuda_runtime, codegen, kw):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("heads", [(12, 2, 128), (32, 8, 64), (8, 2, 256), (32, 2, 128)])
+@pytest.mark.parametrize("f32,one", [(True, True), (False, True), (True, None), (False, None)])
+def test_a_step_from_the_host_stores_its_outputs_there(cuda_runtime, codegen, heads, f32, one):
+    """The bits of the same step on the device, in its buffers as well.  Outputs above the limit go through copy nodes, to the same bits."""
+    from vte_b200.core import decode_executor as de
+    Hq, Hkv, D = heads
+    B, S, L = 3, 500, 5 if one else 2                         # two layers: clusters, a launch each
+    rng = np.random.default_rng(8)
+    f16 = lambda *s: rng.standard_normal(s, dtype=np.float32).astype(np.float16)
+    got, caches = [], [(f16(B, S, Hkv, D), f16(B, S, Hkv, D)) for _ in range(L)]
+    new = [(f16(B, Hkv, D), f16(B, Hkv, D)) for _ in range(L)]
+    steps = [(f16(L, B, Hq, D), rng.integers(0, S, B).astype(np.int32)) for _ in range(3)]
+    limit = de.STAGE_COPY_MAX_BYTES
+    for way in ("device", "host", "copies"):
+        de.STAGE_COPY_MAX_BYTES = 0 if way == "copies" else limit
+        ex = executor(cuda_runtime, codegen, heads, B, S, L, output_f32=f32, with_append=not one, one_launch=one)
+        try:
+            for l in range(L):
+                ex.upload_new_kv(l, *new[l])
+                ex.upload_cache(l, *caches[l])
+            mine = []
+            for q, off in steps:
+                if way == "device":
+                    for l in range(L):
+                        ex.upload_layer(l, q[l])
+                mine.append(ex.execute_decode_batch(off, None if way == "device" else q))
+                assert (ex._mirror() is None) == (way == "copies" or not one)
+                left_q, left_off, left = np.empty_like(q), np.empty_like(off), np.empty_like(mine[-1])
+                for to, at in ((left_q, ex.q_all.ptr), (left_off, ex.offsets.ptr), (left, ex.out_all.ptr)):
+                    cuda_runtime.safe_memcpy_device_to_host(to, ctypes.c_void_p(at), "output")
+                assert np.array_equal(left_q, q) and np.array_equal(left_off, off) and np.array_equal(left, mine[-1])
+            got.append(mine)
+        finally:
+            ex.cleanup()
+            de.STAGE_COPY_MAX_BYTES = limit
+    for other in got[1:]:
+        assert all(np.array_equal(a, b) for a, b in zip(got[0], other))
+
+
+@pytest.mark.gpu
 def test_shared_caches_with_an_append_keep_their_order(cuda_runtime, codegen):
     """Layers that append to one cache depend on one another: a launch list per layer, and `one_launch` is refused."""
     for kw, name in ((dict(with_append=True), None), ({}, "vteb_decode_step_d128_kernel")):
@@ -291,7 +332,9 @@ def test_a_state_that_never_comes_is_reported(cuda_runtime, codegen):
         cuda_runtime.safe_memcpy_host_to_device(count, np.array([5], dtype=np.uint32), "launch count")
         with pytest.raises(CudaRuntimeError):
             ex.execute_decode_batch(off)
-        cuda_runtime.safe_memcpy_host_to_device(count, np.array([2], dtype=np.uint32), "launch count")
+        with pytest.raises(CudaRuntimeError):
+            ex.execute_decode_batch(off, np.ones((4, 1, 12, 128), dtype=np.float16))
+        cuda_runtime.safe_memcpy_host_to_device(count, np.array([3], dtype=np.uint32), "launch count")
         assert np.array_equal(ex.execute_decode_batch(off), good)
     finally:
         ex.cleanup()

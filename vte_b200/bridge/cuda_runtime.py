@@ -82,15 +82,17 @@ class StepPlan(ctypes.Structure):
 class StepLayer(ctypes.Structure):
     """One layer of a `vteb_decode_step_*` launch (StepLayer in csrc/kernels/step_decode.cuh)."""
     _fields_ = ([("k_map", KvTensorMap), ("v_map", KvTensorMap)] +
-                [(name, ctypes.c_void_p) for name in ("q", "k_cache", "v_cache", "k_new", "v_new", "output")] + [("unused", ctypes.c_void_p * 2)])
+                [(name, ctypes.c_void_p) for name in ("q", "k_cache", "v_cache", "k_new", "v_new", "output", "mirror", "unused")])
 
 
 class StepArgs(ctypes.Structure):
     """The argument of the `vteb_decode_step_*` kernels, by value (StepArgs in csrc/kernels/step_decode.cuh)."""
     _fields_ = ([("layer", StepLayer * 64)] +
-                [(name, ctypes.c_void_p) for name in ("kv_offsets", "rope_cos", "rope_sin", "boards", "launches", "status", "keep_q", "keep_offsets")] +
-                [(name, ctypes.c_int) for name in ("keep_layer", "num_layers", "batch", "num_q_heads", "num_kv_heads", "kv_batch_stride",
-                                                   "out_kind", "rope_type", "rotary_dim", "hg", "hg_log2", "wph", "group", "groups", "group_inv")] + [("scale", ctypes.c_float)])
+                [(name, ctypes.c_void_p) for name in ("kv_offsets", "rope_cos", "rope_sin", "boards", "launches", "status",
+                                                     "status_mirror", "keep_q", "keep_offsets")] + [("unused", ctypes.c_void_p * 7)] +
+                [("offsets", ctypes.c_int * 64)] + [(name, ctypes.c_int) for name in ("offsets_here", "keep_layer", "num_layers", "batch", "num_q_heads", "num_kv_heads", "kv_batch_stride",
+                                                   "out_kind", "rope_type", "rotary_dim", "hg", "hg_log2", "wph", "group", "groups", "group_inv")] +
+                [("scale", ctypes.c_float), ("unused_too", ctypes.c_int * 15)])
 
 
 class ClusterGrid(tuple):
@@ -643,6 +645,26 @@ class CudaRuntime:
         self._validate_launch(function, grid, block, shared_mem, len(args))
         self._launch(function, grid, block, args, shared_mem, LAUNCH_PROGRAMMATIC if self.programmatic_launch else 0)
         return True
+
+    def prepare_launch(self, function, args: list, grid: tuple, block: tuple, shared_mem: int = 0, programmatic: bool = False):
+        """A launch whose checks and argument list are made once: calling the result launches it on the runtime's stream, with what
+        its arguments hold by then."""
+        self._validate_launch(function, grid, block, shared_mem, len(args))
+        fval = _ptr_value(function)
+        if shared_mem > self._props["shared_mem_per_block"] and self._smem_optin_set.get(fval, 0) < shared_mem:
+            self._check_error(self._lib.vteb_func_set_max_dynamic_smem(ctypes.c_void_p(fval), int(shared_mem)), "cuFuncSetAttribute")
+            self._smem_optin_set[fval] = int(shared_mem)
+        arr, keep = self._marshal(args)
+        call, flags = self._lib.vteb_launch, LAUNCH_PROGRAMMATIC if programmatic else 0
+        rest = (ctypes.c_void_p(fval), *(ctypes.c_uint(int(x)) for x in (*grid, *block, shared_mem)), self._stream, arr, ctypes.c_uint(flags))
+
+        def launch(_keep=keep):
+            if self._panic:
+                raise CudaSafetyError("runtime is in panic state (a synchronize timed out); new launches are blocked")
+            err = call(*rest)
+            if err:
+                self._check_error(err, "cuLaunchKernel")
+        return launch
 
     # ------------------------------------------------------------------ sync, graphs, events
     def synchronize(self) -> bool:

@@ -42,9 +42,11 @@ STAGE_COPY_MAX_BYTES = 1 << 20
 # queued step of 97 (28 layers, one sequence of 1,531 positions).
 OFFSET_SLOTS = 64
 
+STEP_OFFSETS = 64       # sequences whose offsets may be among the arguments of a step of one launch (kStepOffsets in csrc/kernels/step_decode.cuh)
+
 
 class DecodeAttentionExecutor:
-    _step, _one_launch = None, False
+    _step, _one_launch, _direct = None, False, ()
 
     def __init__(self, hip, codegen, metadata: dict, batch_size: int, context_length: int, n_layers: int, *,
                  n_kv_buffers: Optional[int] = None, num_splits: Optional[int] = None, output_f32: bool = True,
@@ -134,7 +136,7 @@ class DecodeAttentionExecutor:
         if one_launch and (lean is not None or not open_layout):
             raise CudaSafetyError("one launch for all layers takes no split layout, partials, shard states or shapes of the caller's")
         self._one_launch = one_launch if one_launch is not None else None if lean is None and open_layout else False
-        self._step = None
+        self._step, self._direct = None, []
         # where lengths can make the dispatcher's launches the shorter ones: a step of those is captured beside the route's, and
         # each step takes one by its longest and total length; up to _route_pays_to positions it is the route's in any case
         self._route_pays_to, self._on_route, self._launches = self.S, True, (0, 0)
@@ -262,16 +264,11 @@ class DecodeAttentionExecutor:
             return self._step.name, 0
         return (self._route.name, self._route.parts) if self._route is not None and self._on_route else None
 
-    def _record_all(self, after_copy: bool = False, plain: bool = False):
+    def _record_all(self, after_copy: bool = False, plain: bool = False, mirror: Optional[tuple] = None):
         n = 0
         programmatic = self.hip.programmatic_launch
-        if self._step is not None:
-            launches = self._step.launches(self.tensor_mapping, self.offsets.ptr, self.B,
-                                           (self._kept.ptr, self._kept.ptr + _round_up(self.q_bytes, 256)))
-            self._kept_names = dict(self.tensor_mapping)
-            for launch in launches:
-                self.hip.launch_kernel_recorded(*launch)
-            return len(launches)
+        if self._step is not None and self.per_layer_hook is None and self.launch_rewriter is None:
+            return self._record_step(mirror)
         # within a captured step of nothing but the layers' own launches, offsets and older rows do not change
         self.dispatcher.offsets_final = self.use_graph and self.per_layer_hook is None and self.launch_rewriter is None
         for l in range(self.L):
@@ -292,6 +289,17 @@ class DecodeAttentionExecutor:
             if self.per_layer_hook is not None:
                 n += int(self.per_layer_hook(l) or 0)
         return n
+
+    def _step_launches(self, mirror: Optional[tuple] = None) -> list:
+        return self._step.launches(self.tensor_mapping, self.offsets.ptr, self.B, (self._kept.ptr, self._kept.ptr + _round_up(self.q_bytes, 256)), mirror)
+
+    def _record_step(self, mirror: Optional[tuple] = None) -> int:
+        """Record the launches of a step without an order among its layers."""
+        launches = self._step_launches(mirror)
+        self._kept_names = dict(self.tensor_mapping)
+        for launch in launches:
+            self.hip.launch_kernel_recorded(*launch)
+        return len(launches)
 
     def _choose_route(self):
         """Before a step is captured: whether its layers' launches are the dispatcher's own or a route of lean_route.py."""
@@ -359,6 +367,10 @@ class DecodeAttentionExecutor:
                 return
             self._choose_route()
             self._graph_exec, n = self._capture(self._record_all)
+            if self._step is not None and self.per_layer_hook is None and self.launch_rewriter is None and self.B <= STEP_OFFSETS:
+                for fn, args, grid, block, smem in self._step_launches():
+                    args[0].offsets_here = 1
+                    self._direct.append((args[0].offsets, self.hip.prepare_launch(fn, args, grid, block, smem, self.programmatic)))
             plain = n
             if self._route_pays_to < self.S:
                 self._plain_graph_exec, plain = self._capture(lambda: self._record_all(plain=True))
@@ -404,11 +416,23 @@ class DecodeAttentionExecutor:
         finally:
             self.hip.programmatic_launch = False
 
+    def _mirror(self):
+        """Where the one launch of a step stores outputs and status for the host, or None where a copy has to bring them: with a
+        launch list per layer, outputs large enough for a copy node, or a mapping that has them elsewhere.  28 layers of 32,768
+        positions, queries from the host, with a copy launch / without: 176 / 170 us.  (Q taken from pinned memory by the CTAs
+        that need it, without the copy in front: 186.)"""
+        own = all(self.tensor_mapping.get(f'blk.{l}.attention.output') == self.out_all.ptr + l * self.out_bytes for l in range(self.L))
+        if self._step is None or not own or self._out_tail > STAGE_COPY_MAX_BYTES or self.per_layer_hook is not None or self.launch_rewriter is not None:
+            return None
+        return self._stage_out.value, self._stage_out.value + self._out_tail + 4
+
     def _record_io(self, plain: bool = False):
         if max(self._q_tail, self._out_tail) <= STAGE_COPY_MAX_BYTES:
+            mirror = self._mirror()
             self._stage_copy(self.q_all.ptr, self._stage_q.value, self._q_tail + 4 * self.B, first=True)
-            self._record_all(after_copy=True, plain=plain)
-            self._stage_copy(self._stage_out.value, self.out_all.ptr, self._out_tail + 16)
+            self._record_all(after_copy=True, plain=plain, mirror=mirror)
+            if not mirror:
+                self._stage_copy(self._stage_out.value, self.out_all.ptr, self._out_tail + 16)
         else:
             self.hip.memcpy_h2d_async(ctypes.c_void_p(self.q_all.ptr), self._stage_q, self._q_tail + 4 * self.B,
                                       "q and kv offsets staging")
@@ -429,13 +453,27 @@ class DecodeAttentionExecutor:
         self.hip.event_record(self._stage_event)
         self._stage_in_flight = True
 
-    def _update_staging_buffers(self, kv_offsets: np.ndarray):
+    def _checked_offsets(self, kv_offsets: np.ndarray):
+        """(int32[B] offsets, the largest of them)"""
         off = np.ascontiguousarray(kv_offsets, dtype=np.int32)
         if off.shape != (self.B,):
             raise CudaSafetyError(f"kv_offsets shape {off.shape} != ({self.B},)")
         newest = int(off.max())
         if off.min() < 0 or newest >= self.S:
             raise CudaSafetyError(f"kv offset outside 0..{self.S - 1}")
+        return off, newest
+
+    def _launch_with_offsets(self, off: np.ndarray):
+        """A step of one launch, its offsets among the launch's arguments: neither a copy in front of the launch nor a graph around
+        it.  us a step, a copy and a graph / this: 28 layers of one sequence of 1,531 positions 20.5 / 16.1, of 11,003 58.4 / 55.6,
+        eight layers of 24,001 of 256-wide heads 74.7 / 71.9, of eight sequences of 32 heads on 2 55.0 / 51.7."""
+        for offsets, launch in self._direct:
+            ctypes.memmove(offsets, off.ctypes.data, off.nbytes)
+            launch()
+        self._partials_due = True
+
+    def _update_staging_buffers(self, kv_offsets: np.ndarray):
+        off, newest = self._checked_offsets(kv_offsets)
         if self._plain_graph_exec is not None:
             self._pick(off, newest)
         half, slot = divmod(self._offset_slot, OFFSET_SLOTS // 2)
@@ -482,6 +520,7 @@ class DecodeAttentionExecutor:
             self._wait_for_staging()
             ctypes.memmove(self._stage_offsets.value, off.ctypes.data, off.nbytes)
             ctypes.memmove(self._stage_q.value, qh.ctypes.data, qh.nbytes)
+            ctypes.c_int.from_address(self._stage_out.value + self._out_tail + 4).value = 0
             if self._plain_io_graph_exec is not None:
                 self._pick(off, newest)
             self.hip.graph_launch(self._io_graph_exec if self._on_route else self._plain_io_graph_exec)
@@ -492,7 +531,7 @@ class DecodeAttentionExecutor:
                 self.dispatcher_check()
             return self._output_array(nbytes)
         else:
-            self._update_staging_buffers(kv_offsets)
+            off = self._checked_offsets(kv_offsets)[0] if self._direct else self._update_staging_buffers(kv_offsets)
             if q_host is not None:
                 qh = np.ascontiguousarray(q_host, dtype=np.float16)
                 if qh.nbytes != self.L * self.q_bytes:
@@ -501,7 +540,10 @@ class DecodeAttentionExecutor:
                 ctypes.memmove(self._stage_q.value, qh.ctypes.data, qh.nbytes)
                 self.hip.memcpy_h2d_async(ctypes.c_void_p(self.q_all.ptr), self._stage_q, qh.nbytes, "q staging")
                 self._mark_staging_copied()
-            self.launch_step()
+            if self._direct:
+                self._launch_with_offsets(off)
+            else:
+                self.launch_step()
             if not read_output:
                 return None
             self.hip.memcpy_d2h_async(self._stage_out, ctypes.c_void_p(self.out_all.ptr), nbytes, "attention output")

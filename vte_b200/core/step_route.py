@@ -74,11 +74,13 @@ class StepRoute:
             end_read, end_written = max(end_read, hi), max(end_written, hi if w else 0)
         return True
 
-    def launches(self, mapping: dict, kv_offset_ptr: int, batch: int, keep: tuple):
-        """`keep`: where the last layer leaves a copy of its Q and of the offsets, from which its partials can be had."""
+    def launches(self, mapping: dict, kv_offset_ptr: int, batch: int, keep: tuple, host: tuple | None = None):
+        """`keep`: where the last layer leaves a copy of its Q and of the offsets, from which its partials can be had.  `host`:
+        pinned memory (outputs, one layer's after another's, and status word) that the kernel stores to as well."""
         d = self.d
         attention_scale = d.metadata.get('attention_scale')
         row = d.num_kv_heads * d.head_dim
+        row_out = d.num_q_heads * d.head_dim * (4 if d.output_f32 else 2)
         n_rows = int(mapping['kv_batch_stride_elements']) // row * batch
         out = []
         for first in range(0, self.layers, self.plan.max_layers):
@@ -88,7 +90,11 @@ class StepRoute:
                 q, k_cache, v_cache, k_new, v_new, output = self._layer(first + i, mapping)
                 maps = (d.hip.kv_tensor_map(p, n_rows, row, self.plan.tile, self.plan.hg * d.head_dim // 64) for p in (k_cache, v_cache))
                 a.layer[i] = StepLayer(*maps, q, k_cache, v_cache, k_new, v_new, output)
+                if host:
+                    a.layer[i].mirror = host[0] + (first + i) * batch * row_out
             a.kv_offsets, a.boards, a.launches, a.status = kv_offset_ptr, self.scratch.ptr, self.launch_counts, d.work_ptr + 4
+            if host:
+                a.status_mirror = host[1]
             a.keep_q, a.keep_offsets = keep
             a.keep_layer = n - 1 if first + n == self.layers else -1
             a.num_layers, a.batch, a.num_q_heads, a.num_kv_heads = n, batch, d.num_q_heads, d.num_kv_heads
@@ -113,10 +119,13 @@ def one_launch_pays(d, layers: int) -> bool:
     head geometries, 1 to 64 sequences of 64 to 131,072 positions: six layers 1.02 to 3.5 times as fast (32 heads on 2 of 128, 64
     sequences of 4,096: 275 / 270; one of 131,072 of 8 heads on 2 of 256: 245 / 220); three layers of a batch 0.99 to 2.2
     (groups of more than eight heads from 0.85); three layers of one sequence 0.74 to 2; two layers 0.66 to 1.8, from 600 MB on
-    1.0 to 1.1.  One layer has nothing to share out that the launches per layer do not: 0.5 to 1.06."""
+    1.0 to 1.1.  One layer has nothing to share out that the launches per layer do not: 0.5 to 1.06.  Large steps of two or three
+    layers of 64-wide heads gain nothing for sure: their arithmetic keeps up with HBM at full clocks only (64 ragged sequences of 32
+    heads on 8, two layers: 345 / 338 us on one machine, 353 / 364 on another)."""
     plan = d.hip.step_plan(d.num_q_heads, d.num_kv_heads, d.head_dim, d.batch_size, d.num_sms)
     if not plan.ok or layers < 2:
         return False
-    if layers >= 4 or layers * d.batch_size * d.context_length * d.num_kv_heads * d.head_dim * 4 * (0.72 if d.batch_size == 1 else 0.5) >= ONE_LAUNCH_BYTES:
+    if layers >= 4:
         return True
-    return layers == 3 and d.batch_size > 1 and d.num_q_heads <= 8 * d.num_kv_heads
+    large = layers * d.batch_size * d.context_length * d.num_kv_heads * d.head_dim * 4 * (0.72 if d.batch_size == 1 else 0.5) >= ONE_LAUNCH_BYTES
+    return not large and layers == 3 and d.batch_size > 1 and d.num_q_heads <= 8 * d.num_kv_heads or large and d.head_dim > 64

@@ -25,19 +25,26 @@ struct StepLayer {
     KvTensorMap k_map, v_map;                             // of the caches: boxes of `tile` positions x hg * D / 64 columns
     const __half* q; __half* k_cache; __half* v_cache;
     const __half* k_new; const __half* v_new;             // this step's projections [B, Hkv, D]; null: the newest row is in the cache
-    void* output; void* unused[2];
+    void* output;
+    void* mirror; void* unused;                           // a step whose outputs go to the host: pinned memory that they are stored to as well; else null
 };
 constexpr int kStepMaxLayers = 64;                        // a launch
+constexpr int kStepOffsets = 64;                          // sequences whose offsets may come with the launch
 struct StepArgs {
     StepLayer layer[kStepMaxLayers];
     const int* kv_offsets; const __half* rope_cos; const __half* rope_sin;
     uint4* boards; unsigned* launches; int* status;       // [CTAs][hg * group][D / 2 + 1]: the state of a cut run, two tagged words an entry; [CTAs]: launches so far
-    __half* keep_q; int* keep_offsets; int keep_layer;    // a copy of that layer's Q and of the offsets, from which partials can be had; -1: none
+    int* status_mirror;                                   // the same for what `status` says
+    __half* keep_q; int* keep_offsets; void* unused[7];
+    int offsets[kStepOffsets]; int offsets_here;          // 1: the kv offsets are these, and go to kv_offsets for whoever reads them there
+    int keep_layer;                                       // keep_q, keep_offsets: a copy of that layer's Q and of the offsets, from which partials can be had; -1: none
     int num_layers, batch, num_q_heads, num_kv_heads, kv_batch_stride, out_kind, rope_type, rotary_dim;
     int hg, hg_log2, wph, group, groups, group_inv;        // of the plan: KV heads a CTA serves at once, warps of a team, query heads of a KV
                                                           // head, runs of a sequence and layer, ceil(65536 / group)
-    float scale;
+    float scale; int unused_too[15];
 };
+
+static_assert(sizeof(StepLayer) == 320 && sizeof(StepArgs) == kStepMaxLayers * 320 + 512, "mirrored by the host");
 
 __host__ __device__ constexpr int step_warps(int D, int NV) { return D == 256 ? 6 : D == 64 && NV == 1 ? 12 : 8; }     // that compute; one more fetches
 __host__ __device__ constexpr int step_teams(int D) { return D == 256 ? 2 : 1; }           // that take tiles in turn
@@ -116,6 +123,10 @@ __device__ __forceinline__ void step_body(const StepArgs& a)
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int team = TEAMS == 1 ? 0 : warp / TB, kvh = (warp - team * TB) & (hg - 1), wt = (warp - team * TB) >> a.hg_log2;
     const int tile = 16 * wph;                                       // positions
+    const auto gave_up = [&](int code) {
+        raise_abort(abort_word, a.status, code);
+        if (lane == 0 && a.status_mirror != nullptr) *a.status_mirror = code;
+    };
 
     if (tid == 0) {
         for (int i = 0; i < TEAMS * SLOTS; ++i) mbar_init(full0 + 8 * i, 1);
@@ -124,8 +135,8 @@ __device__ __forceinline__ void step_body(const StepArgs& a)
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     for (int i = tid; i < hg * q_words / 4; i += THREADS + 32) reinterpret_cast<uint4*>(q_store)[i] = make_uint4(0u, 0u, 0u, 0u);
-    grid_launch_dependents();
-    grid_dependency_wait();
+    grid_dependency_wait();                                          // and no early release: a CTA of the launch behind has no room beside this one (17.2 / 16.1 us)
+    if (blockIdx.x == 0 && tid == 0 && a.status_mirror != nullptr && *a.status != 0) *a.status_mirror = *a.status;
     if (warp == CW) {                                                // every layer's Q, 4 KB a lane, ahead of the stream
         const int bytes = a.batch * a.num_q_heads * D * 2, pieces = (bytes + 4095) >> 12;
         for (int i = blockIdx.x * 32 + lane; i < a.num_layers * pieces; i += gridDim.x * 32) {
@@ -137,7 +148,8 @@ __device__ __forceinline__ void step_body(const StepArgs& a)
     if (warp == 0) {
         int sum = 0;
         for (int b0 = 0; b0 < a.batch; b0 += 32) {
-            const int b = b0 + lane, len = b < a.batch ? max(a.kv_offsets[b] + 1, 0) : 0;
+            const int b = b0 + lane, off = b >= a.batch ? -1 : a.offsets_here ? a.offsets[b] : a.kv_offsets[b], len = max(off + 1, 0);
+            if (a.offsets_here && blockIdx.x == 0 && b < a.batch) const_cast<int*>(a.kv_offsets)[b] = off;
             int n = b < a.batch ? max((len + tile - 1) / tile, 1) : 0;
             if (b < a.batch) lens[b] = len;
 #pragma unroll
@@ -202,7 +214,7 @@ __device__ __forceinline__ void step_body(const StepArgs& a)
 #pragma unroll 1
             for (int kv = 0; kv < 2; ++kv) {
                 if (sent >= SLOTS && !mbar_wait_bounded(empty0 + 8 * slot, phase ^ 1, abort_word)) {
-                    raise_abort(abort_word, a.status, kStatusEmptyTimeout);
+                    gave_up(kStatusEmptyTimeout);
                     ok = false;
                     break;
                 }
@@ -276,9 +288,15 @@ __device__ __forceinline__ void step_body(const StepArgs& a)
         const float inv = fmaxf(sum, 1e-20f);
         const float4 y = make_float4(acc.x / inv, acc.y / inv, acc.z / inv, acc.w / inv);
         const long long at = ((long long)r.b * a.num_q_heads + r.h * rows + j) * D + q4 * 4;
-        void* const out = a.layer[r.l].output;
-        if (a.out_kind == 2) *reinterpret_cast<float4*>(reinterpret_cast<float*>(out) + at) = y;
-        else *reinterpret_cast<uint2*>(reinterpret_cast<__half*>(out) + at) = make_uint2(pack_half2(y.x, y.y), pack_half2(y.z, y.w));
+        const StepLayer& L = a.layer[r.l];
+        if (a.out_kind == 2) {
+            *reinterpret_cast<float4*>(reinterpret_cast<float*>(L.output) + at) = y;
+            if (L.mirror != nullptr) *reinterpret_cast<float4*>(reinterpret_cast<float*>(L.mirror) + at) = y;
+        } else {
+            const uint2 h = make_uint2(pack_half2(y.x, y.y), pack_half2(y.z, y.w));
+            *reinterpret_cast<uint2*>(reinterpret_cast<__half*>(L.output) + at) = h;
+            if (L.mirror != nullptr) *reinterpret_cast<uint2*>(reinterpret_cast<__half*>(L.mirror) + at) = h;
+        }
     };
     const auto cta_of = [&](int x) {                                 // whose share the tile is in
         int c = min((int)((float)x * (float)G * __fdividef(1.f, (float)T)), G - 1);
@@ -341,7 +359,7 @@ __device__ __forceinline__ void step_body(const StepArgs& a)
             };
             const auto arrived = [&]() {
                 if (alive && !mbar_wait_bounded(full0 + 8 * (team * SLOTS + landed), phase, abort_word)) {
-                    raise_abort(abort_word, a.status, kStatusFullTimeout);
+                    gave_up(kStatusFullTimeout);
                     alive = false;                                   // walks on without waiting: nobody is left alone at a barrier
                 }
                 __syncwarp();
@@ -537,7 +555,10 @@ __device__ __forceinline__ void step_body(const StepArgs& a)
             else store_out(r, j, q4, acc, ll);
         }
     }
-    if (!in_time) atomicCAS(a.status, 0, kStatusGridTimeout);
+    if (!in_time) {
+        atomicCAS(a.status, 0, kStatusGridTimeout);
+        if (a.status_mirror != nullptr) *a.status_mirror = kStatusGridTimeout;
+    }
 }
 
 #define VTEB_STEP_KERNEL(NAME, DIM, NV)                                                                              \

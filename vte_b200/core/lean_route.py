@@ -200,7 +200,8 @@ def unsplit_as_clusters(hip, kernels: dict, args: list, grid, block, status: int
 
     Its geometry has one block walk a whole sequence; a cluster per (sequence, KV head) has as many SMs on it as the grid
     leaves and reads K and V once for the group.  us a layer, plain stream order, builds / clusters: four sequences of 12
-    heads on 2 of 128, 64 positions 4.8 / 5.3, 200: 5.9 / 5.3, 600: 8.6 / 5.4, 1,500: 15.3 / 6.3, 4,000: 43 / 9.6.  So:
+    heads on 2 of 128, 64 positions 4.8 / 5.3, 200: 5.9 / 5.3, 600: 8.6 / 5.4, 1,500: 15.3 / 6.3, 4,000: 43 / 9.6 (the clusters 0.6 less
+    since they set themselves up ahead of their wait).  So:
     caches with room for more than 256 positions (512 with two runs of query heads: 6.5 us at the least), and no more
     pairs than clusters run at once (a second wave costs more than short sequences take: 64 sequences of 200 positions
     19 / 21, of 64 8 / 17).  The host sees the room, not the lengths: a sequence of up to about 100 positions (150 of 256-wide

@@ -416,18 +416,10 @@ __device__ __forceinline__ void lean_body(const LeanArgs& a)
             return;
         }
     }
-    if (a.flags & kFlagWaitFirst) grid_dependency_wait();
-
-    const int total = a.kv_offsets[b] + 1;
-    const int chunk = vteb_round_up((total + N - 1) / N, kBlockPos);
-    const int start = (int)min((long long)part * chunk, (long long)total), end = min(start + chunk, total);
-    const int nblk = (end - start + kBlockPos - 1) / kBlockPos;
-    // The newest row may be written by the launch in front (or comes from k_new): this CTA's last block gets it after the wait.
-    const bool late = end > start && end == total && !((a.flags & kLeanRowsFinal) && a.k_new == nullptr);
-    const int load_end = late ? end - 1 : end;
-    const long long pos_stride = (long long)a.num_kv_heads * D;      // halves between positions
-    const long long base = (long long)b * a.kv_batch_stride + (long long)kv_head * D;
-
+    // With kFlagWaitFirst nothing is read before the launch in front is done; what needs no memory is set up before that (28
+    // launches of four sequences of 100 to 1,500 positions, each behind the one in front: 161.7 -> 144.1 us).
+    const bool wait_first = a.flags & kFlagWaitFirst;
+    int total = wait_first ? 0 : a.kv_offsets[b] + 1;
     const int units = group * (D / 32), my_units = kCluster && part < units ? (units - part + N - 1) / N : 0;
     if (threadIdx.x == 0) {
         mbar_init(bar_recv, 1);
@@ -436,9 +428,22 @@ __device__ __forceinline__ void lean_body(const LeanArgs& a)
         if (my_units > 0) mbar_arrive_expect_tx(bar_recv, my_units * N * kLeanUnit * 4);
     }
     for (int i = threadIdx.x; i < NV * CPR * 8; i += THREADS) reinterpret_cast<uint4*>(q_store)[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (wait_first) {
+        if constexpr (kCluster) cluster_arrive();
+        grid_dependency_wait();
+        total = a.kv_offsets[b] + 1;
+    }
     __syncthreads();
     grid_launch_dependents();
-    if constexpr (kCluster) cluster_arrive();
+    if constexpr (kCluster) { if (!wait_first) cluster_arrive(); }
+    const int chunk = vteb_round_up((total + N - 1) / N, kBlockPos);
+    const int start = (int)min((long long)part * chunk, (long long)total), end = min(start + chunk, total);
+    const int nblk = (end - start + kBlockPos - 1) / kBlockPos;
+    // The newest row may be written by the launch in front (or comes from k_new): this CTA's last block gets it after the wait.
+    const bool late = end > start && end == total && !((a.flags & kLeanRowsFinal) && a.k_new == nullptr);
+    const int load_end = late ? end - 1 : end;
+    const long long pos_stride = (long long)a.num_kv_heads * D;      // halves between positions
+    const long long base = (long long)b * a.kv_batch_stride + (long long)kv_head * D;
 
     // ---- this warp's blocks: warp, warp + CW, ...; block i in slot i % depth.  Swizzled rows: chunk c of row r at c ^ (r & 7).
     const uint32_t ring_w = smem_u32(ring) + warp * depth * BLK;

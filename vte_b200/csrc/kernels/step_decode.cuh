@@ -9,16 +9,19 @@
 // on a board, in 64-bit words that carry the number of the launch (valid exactly when they carry it, so without a fence), and
 // the last merges them, bounded, in their order; it waits for CTAs with lower numbers only.
 //
-// What bounds it: HBM, and about 13 us of start, first tile, merge and finish.  us a step, launches per layer / one launch, 12 heads
-// on 2 KV heads of 128, one sequence: 28 layers of 1,531 positions 104.4 / 20.4, of 11,003 181.4 / 58.4, four of a million 649 / 603
-// (7.1 TB/s); 8 ragged sequences of 32 heads on 8 of 64, ten layers 245.7 / 192.3.  What was measured on the way there:
+// What bounds it: HBM, and about 9 us of launch, start (2), first tile (1.3), merges (1.3 a run) and finish (2 to 2.5).  us a step,
+// launches per layer / one launch, 12 heads on 2 KV heads of 128, one sequence: 28 layers of 1,531 positions 104 / 15.5, of 11,003
+// 182 / 54, four of a million 649 / 604 (7.1 TB/s); 8 ragged sequences of 32 heads on 8 of 64, ten layers 246 / 193.  Nine to
+// sixteen query heads per KV head are bound by block arithmetic: an SM takes 40 B/ns, its share of HBM is 45.  What was measured:
 //   128 KB of tiles in flight an SM, not 192: with more, the SMs of the two largest clusters of SMs get 15 % less than the others
 //     and every share waits for them (a million positions 676 / 614, 28 layers of 32,768 174 / 164);
 //   one copy a tile in place of one per 64 channels: the warp that fetches was the limit (an SM alone, 64-wide heads 52 / 58
 //     B/ns, 256-wide 59 / 70); 16-byte asynchronous copies by every warp 5.8 TB/s on 64 ragged sequences of 64-wide heads (6.5);
 //   64-wide heads: twelve warps (8: 40 B/ns an SM, below its share of HBM), four heads a CTA (rows of 512 bytes; 128: 6.0 TB/s);
 //   256-wide heads: two teams of three warps that take tiles in turn: 24 KB a tile, five in flight (48 KB, three: 209 / 205);
-//   tagged words in place of a fence, a counter and a reload: 28.6 / 22.6 for 28 layers of 1,531.
+//   tagged words in place of a fence, a counter and a reload: 28.6 / 22.6 for 28 layers of 1,531;
+//   up to sixteen states merged at once, not eight, and the fetching warp ahead of the others: one of 24,001, 256-wide, eight layers
+//     71.9 / 71.2, 28 layers of 1,531 16.1 / 15.6.
 #pragma once
 
 struct StepLayer {
@@ -52,7 +55,8 @@ __host__ __device__ constexpr int step_tile_bytes(int D, int NV) { return step_w
 __host__ __device__ constexpr int step_slots(int D, int NV) { return (128 << 10) / step_tile_bytes(D, NV); }   // K or V tiles in flight: 128 KB
 constexpr int kStepStatePad = 4;                          // floats after o[D] in a kept state: m, l, 2 unused
 constexpr int kStepMaxBatch = 1024;
-constexpr int kStepFan = 8;                               // CTAs whose states of one run are merged at once
+constexpr int kStepFan = 16;                              // CTAs whose states of one run are merged at once
+constexpr int kStepFew = 7;                               // of a run, where more would have less than three tiles each
 constexpr int kStepCtrlBytes = 256;                       // barriers (full, empty: 24 at most), abort word
 
 // What a launch needs.  ok = 0: a geometry or batch that it does not cover.  hg 0: rows of 256 bytes and more are read in full wherever
@@ -128,28 +132,21 @@ __device__ __forceinline__ void step_body(const StepArgs& a)
         if (lane == 0 && a.status_mirror != nullptr) *a.status_mirror = code;
     };
 
-    if (tid == 0) {
-        for (int i = 0; i < TEAMS * SLOTS; ++i) mbar_init(full0 + 8 * i, 1);
-        for (int i = 0; i < SLOTS; ++i) mbar_init(empty0 + 8 * i, TB);
-        *abort_word = 0;
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    for (int i = tid; i < hg * q_words / 4; i += THREADS + 32) reinterpret_cast<uint4*>(q_store)[i] = make_uint4(0u, 0u, 0u, 0u);
-    grid_dependency_wait();                                          // and no early release: a CTA of the launch behind has no room beside this one (17.2 / 16.1 us)
-    if (blockIdx.x == 0 && tid == 0 && a.status_mirror != nullptr && *a.status != 0) *a.status_mirror = *a.status;
-    if (warp == CW) {                                                // every layer's Q, 4 KB a lane, ahead of the stream
-        const int bytes = a.batch * a.num_q_heads * D * 2, pieces = (bytes + 4095) >> 12;
-        for (int i = blockIdx.x * 32 + lane; i < a.num_layers * pieces; i += gridDim.x * 32) {
-            const int l = i / pieces, at = (i - l * pieces) << 12;
-            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(reinterpret_cast<const unsigned char*>(a.layer[l].q) + at), "r"(min(4096, bytes - at)) : "memory");
+    // The warp that fetches goes ahead: it sets up the barriers and adds up the lengths, and starts on its tiles while the others still
+    // prepare Q's fragments.
+    unsigned tag = 0;
+    if (warp == CW) {
+        if (lane == 0) {
+            for (int i = 0; i < TEAMS * SLOTS; ++i) mbar_init(full0 + 8 * i, 1);
+            for (int i = 0; i < SLOTS; ++i) mbar_init(empty0 + 8 * i, TB);
+            *abort_word = 0;
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         }
-    }
-    const unsigned tag = a.launches[blockIdx.x] + 1;                 // every CTA counts the launches: all have the same number
-    if (warp == 0) {
+        grid_dependency_wait();                                      // and no early release: a CTA of the launch behind has no room beside this one (17.2 / 16.1 us)
+        if (a.status_mirror != nullptr && blockIdx.x == 0 && lane == 0 && *a.status != 0) *a.status_mirror = *a.status;
         int sum = 0;
         for (int b0 = 0; b0 < a.batch; b0 += 32) {
-            const int b = b0 + lane, off = b >= a.batch ? -1 : a.offsets_here ? a.offsets[b] : a.kv_offsets[b], len = max(off + 1, 0);
-            if (a.offsets_here && blockIdx.x == 0 && b < a.batch) const_cast<int*>(a.kv_offsets)[b] = off;
+            const int b = b0 + lane, len = b >= a.batch ? 0 : max((a.offsets_here ? a.offsets[b] : a.kv_offsets[b]) + 1, 0);
             int n = b < a.batch ? max((len + tile - 1) / tile, 1) : 0;
             if (b < a.batch) lens[b] = len;
 #pragma unroll
@@ -161,12 +158,18 @@ __device__ __forceinline__ void step_body(const StepArgs& a)
             sum += __shfl_sync(0xffffffffu, n, 31);
         }
         if (lane == 0) pre[0] = 0;
+        __syncwarp();
+        asm volatile("bar.arrive 2, %0;" ::"n"(THREADS + 32) : "memory");
+    } else {
+        for (int i = tid; i < hg * q_words / 4; i += THREADS) reinterpret_cast<uint4*>(q_store)[i] = make_uint4(0u, 0u, 0u, 0u);
+        grid_dependency_wait();
+        tag = a.launches[blockIdx.x] + 1;                            // every CTA counts the launches: all have the same number
+        asm volatile("bar.sync 2, %0;" ::"n"(THREADS + 32) : "memory");
     }
-    __syncthreads();
 
     const int N = pre[a.batch], T = a.num_layers * groups * N, cta = blockIdx.x;
-    // One merge for a run (at most kStepFan pieces) where that costs a CTA up to three tiles: a second one takes longer.
-    const int few = a.num_layers * groups * a.batch * (kStepFan - 1), G = min(min((int)gridDim.x, T), T <= 3 * few ? few : T);
+    // Few states to merge for a run where that costs a CTA up to three tiles.
+    const int few = a.num_layers * groups * a.batch * kStepFew, G = min(min((int)gridDim.x, T), T <= 3 * few ? few : T);
     if (tid == 0) a.launches[cta] = tag;
     if (cta >= G) return;
     // CTA c's share starts at floor(c T / G).  Divisions by way of floats: quotients below 2^20 are at most one off.
@@ -233,6 +236,8 @@ __device__ __forceinline__ void step_body(const StepArgs& a)
                 if (++slot == SLOTS) { slot = 0; phase ^= 1; }
             }
         }
+        if (a.offsets_here && cta == 0)                              // for whoever reads them there; not in front: a path of one CTA's own is slow to fetch
+            for (int b = lane; b < a.batch; b += 32) const_cast<int*>(a.kv_offsets)[b] = a.offsets[b];
         if (!ok)                                                     // its own copies have to land before the CTA may end
             for (int i = 1; i <= min(sent, SLOTS); ++i) {
                 const uint32_t bar = full_of(sent - i);

@@ -106,6 +106,18 @@ int vteb_stream_begin_capture(void* stream, int mode);
 int vteb_stream_end_capture(void* stream, void** graph);
 int vteb_graph_instantiate(void** graph_exec, void* graph);
 int vteb_graph_launch(void* graph_exec, void* stream);
+/* A captured step from the host and back in one call: offsets (refused outside 0..capacity - 1) and queries into the pinned staging
+ * memory that the graph reads, the graph, a wait for the stream, and the outputs from the staging memory that it leaves
+ * them in.  VTEB_ERR_DEVICE_STATUS, without outputs, when the status word in staging memory is not zero by then. */
+typedef struct vteb_host_step_t {
+    void* stage_offsets;
+    void* stage_q;
+    const void* stage_out;
+    volatile int* status;       /* cleared before the launch */
+    size_t q_bytes, out_bytes;
+    int batch, capacity;
+} vteb_host_step_t;
+int vteb_host_step(const vteb_host_step_t* step, void* graph_exec, void* stream, const int* offsets, const void* q, void* out);
 int vteb_graph_destroy(void* graph);
 int vteb_graph_exec_destroy(void* graph_exec);
 int vteb_graph_node_count(void* graph, size_t* count);

@@ -277,6 +277,11 @@ def test_a_step_from_the_host_stores_its_outputs_there(cuda_runtime, codegen, he
                 ex.upload_new_kv(l, *new[l])
                 ex.upload_cache(l, *caches[l])
             mine = []
+            for bad in (np.array([0, S, 1], dtype=np.int32), np.array([0, -1, 1], dtype=np.int32), np.zeros(B + 1, dtype=np.int32)):
+                with pytest.raises(CudaSafetyError):
+                    ex.execute_decode_batch(bad, steps[0][0])
+                with pytest.raises(CudaSafetyError):
+                    ex.execute_decode_batch(bad)
             for q, off in steps:
                 if way == "device":
                     for l in range(L):

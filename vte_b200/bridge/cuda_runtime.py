@@ -52,6 +52,7 @@ ATTN_NO_TENSOR_MAPS = 32
 ATTN_BALANCED = 64
 ATTN_SHORT_SPLITS = 128
 
+ERR_INVALID_ARGUMENT = -1
 ERR_DEVICE_STATUS = -6
 
 
@@ -93,6 +94,12 @@ class StepArgs(ctypes.Structure):
                 [("offsets", ctypes.c_int * 64)] + [(name, ctypes.c_int) for name in ("offsets_here", "keep_layer", "num_layers", "batch", "num_q_heads", "num_kv_heads", "kv_batch_stride",
                                                    "out_kind", "rope_type", "rotary_dim", "hg", "hg_log2", "wph", "group", "groups", "group_inv")] +
                 [("scale", ctypes.c_float), ("unused_too", ctypes.c_int * 15)])
+
+
+class HostStep(ctypes.Structure):
+    """Mirror of `vteb_host_step_t` (include/vteb200.h)."""
+    _fields_ = [("stage_offsets", ctypes.c_void_p), ("stage_q", ctypes.c_void_p), ("stage_out", ctypes.c_void_p), ("status", ctypes.c_void_p),
+                ("q_bytes", ctypes.c_size_t), ("out_bytes", ctypes.c_size_t), ("batch", ctypes.c_int), ("capacity", ctypes.c_int)]
 
 
 class ClusterGrid(tuple):
@@ -147,6 +154,7 @@ def _declare(lib):
         "vteb_stream_end_capture": (i, [vp, vpp]),
         "vteb_graph_instantiate": (i, [vpp, vp]),
         "vteb_graph_launch": (i, [vp, vp]),
+        "vteb_host_step": (i, [ctypes.POINTER(HostStep), vp, vp, vp, vp, vp]),
         "vteb_graph_destroy": (i, [vp]),
         "vteb_graph_exec_destroy": (i, [vp]),
         "vteb_graph_node_count": (i, [vp, szp]),
@@ -727,6 +735,20 @@ class CudaRuntime:
         if self._panic:
             raise CudaSafetyError("runtime is in panic state; graph launch blocked")
         self._check_error(self._lib.vteb_graph_launch(graph_exec, self._stream), "cudaGraphLaunch")
+
+    def host_step(self, step: HostStep, graph_exec, offsets: int, q: int, out: int) -> bool:
+        """A captured step from host memory and back (addresses of contiguous arrays).  False, and no outputs, where a kernel gave up."""
+        self._require_init()
+        if self._panic:
+            raise CudaSafetyError("runtime is in panic state; graph launch blocked")
+        err = self._lib.vteb_host_step(ctypes.byref(step), graph_exec, self._stream, offsets, q, out)
+        if err == ERR_INVALID_ARGUMENT:
+            raise CudaSafetyError(self._last_error())
+        if err and err != ERR_DEVICE_STATUS:
+            self._check_error(err, "vteb_host_step")
+        if self._launch_status is not None and self._launch_status.value:
+            self._check_launch_status()
+        return not err
 
     def graph_node_count(self, graph) -> int:
         n = ctypes.c_size_t(0)

@@ -20,6 +20,7 @@ from typing import Optional
 
 import numpy as np
 
+from ..bridge.cuda_runtime import HostStep
 from ..bridge.errors import CudaSafetyError
 from ..bridge.memory import MemoryRegion, SlabAllocator
 from ..config import ENV_NO_PDL, env_flag
@@ -136,7 +137,7 @@ class DecodeAttentionExecutor:
         if one_launch and (lean is not None or not open_layout):
             raise CudaSafetyError("one launch for all layers takes no split layout, partials, shard states or shapes of the caller's")
         self._one_launch = one_launch if one_launch is not None else None if lean is None and open_layout else False
-        self._step, self._direct = None, []
+        self._step, self._direct, self._host_step = None, [], None
         # where lengths can make the dispatcher's launches the shorter ones: a step of those is captured beside the route's, and
         # each step takes one by its longest and total length; up to _route_pays_to positions it is the route's in any case
         self._route_pays_to, self._on_route, self._launches = self.S, True, (0, 0)
@@ -511,25 +512,27 @@ class DecodeAttentionExecutor:
             # the whole step as one graph launch
             self.build_io_graph()
             off = np.ascontiguousarray(kv_offsets, dtype=np.int32)
-            newest = int(off.max()) if off.shape == (self.B,) else self.S
-            if newest >= self.S or off.min() < 0:
+            if off.shape != (self.B,):
                 raise CudaSafetyError(f"kv_offsets must be int32[{self.B}] within 0..{self.S - 1}")
             qh = np.ascontiguousarray(q_host, dtype=np.float16)
             if qh.nbytes != self.L * self.q_bytes:
                 raise CudaSafetyError("q_host must be [L, B, Hq, D] fp16")
             self._wait_for_staging()
-            ctypes.memmove(self._stage_offsets.value, off.ctypes.data, off.nbytes)
-            ctypes.memmove(self._stage_q.value, qh.ctypes.data, qh.nbytes)
-            ctypes.c_int.from_address(self._stage_out.value + self._out_tail + 4).value = 0
             if self._plain_io_graph_exec is not None:
-                self._pick(off, newest)
-            self.hip.graph_launch(self._io_graph_exec if self._on_route else self._plain_io_graph_exec)
+                self._pick(off, int(off.max()))
+            if self._host_step is None:
+                self._host_step = HostStep(self._stage_offsets.value, self._stage_q.value, self._stage_out.value, self._stage_out.value + self._out_tail + 4,
+                                           self.L * self.q_bytes, nbytes, self.B, self.S)
+            out = np.empty((self.L, self.B, self.Hq, self.D + 2 if self.emit_state else self.D),
+                           dtype=np.float32 if (self.output_f32 or self.emit_state) else np.float16)
+            # staging, graph, wait and the copy of the outputs, in one call
+            done = self.hip.host_step(self._host_step, self._io_graph_exec if self._on_route else self._plain_io_graph_exec,
+                                      off.ctypes.data, qh.ctypes.data, out.ctypes.data)
             self._partials_due = self._on_route and self._kept_names is not None
-            self.hip.stream_synchronize()
-            # the status word travelled with the outputs: only a non-zero one needs the slow path
-            if ctypes.c_int.from_address(self._stage_out.value + self._out_tail + 4).value != 0:
+            if not done:                              # the status word travelled with the outputs
                 self.dispatcher_check()
-            return self._output_array(nbytes)
+                return self._output_array(nbytes)
+            return out
         else:
             off = self._checked_offsets(kv_offsets)[0] if self._direct else self._update_staging_buffers(kv_offsets)
             if q_host is not None:

@@ -462,6 +462,23 @@ int vteb_graph_launch(void* graph_exec, void* stream) {
     return check_rt(cudaGraphLaunch((cudaGraphExec_t)graph_exec, (cudaStream_t)stream), "cudaGraphLaunch");
 }
 
+int vteb_host_step(const vteb_host_step_t* step, void* graph_exec, void* stream, const int* offsets, const void* q, void* out) {
+    REQUIRE_INIT();
+    if (!step || !graph_exec || !offsets || !q || !out) return fail(VTEB_ERR_INVALID_ARGUMENT, "null argument");
+    for (int b = 0; b < step->batch; ++b)
+        if (offsets[b] < 0 || offsets[b] >= step->capacity)
+            return fail(VTEB_ERR_INVALID_ARGUMENT, "kv_offsets must be int32[%d] within 0..%d", step->batch, step->capacity - 1);
+    memcpy(step->stage_offsets, offsets, sizeof(int) * (size_t)step->batch);
+    memcpy(step->stage_q, q, step->q_bytes);
+    *step->status = 0;
+    int rc = check_rt(cudaGraphLaunch((cudaGraphExec_t)graph_exec, (cudaStream_t)stream), "cudaGraphLaunch");
+    if (rc) return rc;
+    if ((rc = check_rt(cudaStreamSynchronize((cudaStream_t)stream), "cudaStreamSynchronize"))) return rc;
+    if (*step->status != 0) return fail(VTEB_ERR_DEVICE_STATUS, "a kernel gave up on a bounded wait (code %d)", (int)*step->status);
+    memcpy(out, step->stage_out, step->out_bytes);
+    return 0;
+}
+
 int vteb_graph_destroy(void* graph) {
     REQUIRE_INIT();
     return check_rt(cudaGraphDestroy((cudaGraph_t)graph), "cudaGraphDestroy");

@@ -206,6 +206,7 @@ typedef struct vteb_step_plan_t {
     int hg_log2;
     int wph;           /* warps that share a KV head */
     int tile;          /* positions of a box of the tensor maps */
+    int fan;           /* blocks whose states of one run are merged at once */
 } vteb_step_plan_t;
 int vteb_step_plan(int num_q_heads, int num_kv_heads, int head_dim, int batch, int n_ctas, int hg, vteb_step_plan_t* plan);
 /* How many clusters of `cluster` blocks of a loaded kernel the device runs at once (cuOccupancyMaxActiveClusters). */

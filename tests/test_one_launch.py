@@ -33,6 +33,7 @@ def test_plan_covers_what_the_kernels_do(built_library, group, D):
             warps = p.threads // 32 - 1
             assert Hkv % p.hg == 0 and p.hg == 1 << p.hg_log2 and p.hg * p.wph == warps // (2 if D == 256 else 1) and p.tile == 16 * p.wph <= 256
             assert (warps * 32) % (D // 8) == 0 and p.smem_bytes <= 227 * 1024
+            assert 4 <= p.fan <= 16
             assert p.state_bytes == 148 * p.hg * group * (D // 2 + 1) * 16
 
 

@@ -77,7 +77,7 @@ class KvTensorMap(ctypes.Structure):
 class StepPlan(ctypes.Structure):
     """Mirror of `vteb_step_plan_t` (include/vteb200.h)."""
     _fields_ = [("ok", ctypes.c_int), ("threads", ctypes.c_int), ("smem_bytes", ctypes.c_int), ("hg", ctypes.c_int),
-                ("state_bytes", ctypes.c_int), ("max_layers", ctypes.c_int), ("hg_log2", ctypes.c_int), ("wph", ctypes.c_int), ("tile", ctypes.c_int)]
+                ("state_bytes", ctypes.c_int), ("max_layers", ctypes.c_int), ("hg_log2", ctypes.c_int), ("wph", ctypes.c_int), ("tile", ctypes.c_int), ("fan", ctypes.c_int)]
 
 
 class StepLayer(ctypes.Structure):
@@ -93,7 +93,7 @@ class StepArgs(ctypes.Structure):
                                                      "status_mirror", "keep_q", "keep_offsets")] + [("unused", ctypes.c_void_p * 7)] +
                 [("offsets", ctypes.c_int * 64)] + [(name, ctypes.c_int) for name in ("offsets_here", "keep_layer", "num_layers", "batch", "num_q_heads", "num_kv_heads", "kv_batch_stride",
                                                    "out_kind", "rope_type", "rotary_dim", "hg", "hg_log2", "wph", "group", "groups", "group_inv")] +
-                [("scale", ctypes.c_float), ("unused_too", ctypes.c_int * 15)])
+                [("scale", ctypes.c_float), ("fan", ctypes.c_int), ("unused_too", ctypes.c_int * 14)])
 
 
 class HostStep(ctypes.Structure):

@@ -99,7 +99,7 @@ class StepRoute:
             a.keep_layer = n - 1 if first + n == self.layers else -1
             a.num_layers, a.batch, a.num_q_heads, a.num_kv_heads = n, batch, d.num_q_heads, d.num_kv_heads
             a.hg, a.hg_log2, a.wph, a.group = self.plan.hg, self.plan.hg_log2, self.plan.wph, d.num_q_heads // d.num_kv_heads
-            a.groups, a.group_inv = d.num_kv_heads // a.hg, -(-65536 // a.group)
+            a.groups, a.group_inv, a.fan = d.num_kv_heads // a.hg, -(-65536 // a.group), self.plan.fan
             a.kv_batch_stride, a.out_kind = int(mapping.get('kv_batch_stride_elements', 0)), 2 if d.output_f32 else 1
             a.rope_type = -1
             if d.fuse_rope:

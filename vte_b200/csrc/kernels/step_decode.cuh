@@ -12,7 +12,7 @@
 // What bounds it: HBM, and about 9 us of launch, start (2), first tile (1.3), merges (1.3 a run) and finish (2 to 2.5).  us a step,
 // launches per layer / one launch, 12 heads on 2 KV heads of 128, one sequence: 28 layers of 1,531 positions 104 / 15.5, of 11,003
 // 182 / 54, four of a million 649 / 604 (7.1 TB/s); 8 ragged sequences of 32 heads on 8 of 64, ten layers 246 / 193.  Nine to
-// sixteen query heads per KV head are bound by block arithmetic: an SM takes 40 B/ns, its share of HBM is 45.  What was measured:
+// sixteen query heads per KV head are bound by block arithmetic: an SM takes 43 B/ns, its share of HBM is 45.  What was measured:
 //   128 KB of tiles in flight an SM, not 192: with more, the SMs of the two largest clusters of SMs get 15 % less than the others
 //     and every share waits for them (a million positions 676 / 614, 28 layers of 32,768 174 / 164);
 //   one copy a tile in place of one per 64 channels: the warp that fetches was the limit (an SM alone, 64-wide heads 52 / 58
@@ -21,7 +21,9 @@
 //   256-wide heads: two teams of three warps that take tiles in turn: 24 KB a tile, five in flight (48 KB, three: 209 / 205);
 //   tagged words in place of a fence, a counter and a reload: 28.6 / 22.6 for 28 layers of 1,531;
 //   up to sixteen states merged at once, not eight, and the fetching warp ahead of the others: one of 24,001, 256-wide, eight layers
-//     71.9 / 71.2, 28 layers of 1,531 16.1 / 15.6.
+//     71.9 / 71.2, 28 layers of 1,531 16.1 / 15.6;
+//   two runs of 128-wide heads: seven computing warps and the fetching one have 255 registers each, eight and one 168 and spill (8
+//     sequences of 32 heads on 2, eight layers: 51.2 / 47.4).
 #pragma once
 
 struct StepLayer {
@@ -44,26 +46,26 @@ struct StepArgs {
     int num_layers, batch, num_q_heads, num_kv_heads, kv_batch_stride, out_kind, rope_type, rotary_dim;
     int hg, hg_log2, wph, group, groups, group_inv;        // of the plan: KV heads a CTA serves at once, warps of a team, query heads of a KV
                                                           // head, runs of a sequence and layer, ceil(65536 / group)
-    float scale; int unused_too[15];
+    float scale; int fan; int unused_too[14];
 };
 
 static_assert(sizeof(StepLayer) == 320 && sizeof(StepArgs) == kStepMaxLayers * 320 + 512, "mirrored by the host");
 
-__host__ __device__ constexpr int step_warps(int D, int NV) { return D == 256 ? 6 : D == 64 && NV == 1 ? 12 : 8; }     // that compute; one more fetches
+__host__ __device__ constexpr int step_warps(int D, int NV) { return D == 256 ? 6 : D == 128 && NV == 2 ? 7 : D == 64 && NV == 1 ? 12 : 8; }     // that compute; one more fetches
 __host__ __device__ constexpr int step_teams(int D) { return D == 256 ? 2 : 1; }           // that take tiles in turn
 __host__ __device__ constexpr int step_tile_bytes(int D, int NV) { return step_warps(D, NV) / step_teams(D) * 32 * D; }    // a 16-position block for every warp of a team
 __host__ __device__ constexpr int step_slots(int D, int NV) { return (128 << 10) / step_tile_bytes(D, NV); }   // K or V tiles in flight: 128 KB
 constexpr int kStepStatePad = 4;                          // floats after o[D] in a kept state: m, l, 2 unused
 constexpr int kStepMaxBatch = 1024;
-constexpr int kStepFan = 16;                              // CTAs whose states of one run are merged at once
+constexpr int kStepMostFan = 16;                          // CTAs whose states of one run are merged at once, where shared memory holds as many
 constexpr int kStepFew = 7;                               // of a run, where more would have less than three tiles each
 constexpr int kStepCtrlBytes = 256;                       // barriers (full, empty: 24 at most), abort word
 
 // What a launch needs.  ok = 0: a geometry or batch that it does not cover.  hg 0: rows of 256 bytes and more are read in full wherever
 // they lie, so wider heads go one a CTA (fewer rows to merge: 12 heads on 2 of 128, two a CTA 26.6 / 22.6 us); 64-wide heads up to four.
-struct StepPlan { int ok, threads, smem_bytes, hg, state_bytes, max_layers, hg_log2, wph, tile; };
+struct StepPlan { int ok, threads, smem_bytes, hg, state_bytes, max_layers, hg_log2, wph, tile, fan; };
 __host__ __device__ inline StepPlan make_step_plan(int num_q_heads, int num_kv_heads, int head_dim, int batch, int n_ctas, int hg = 0) {
-    StepPlan p = {0, 0, 0, 0, 0, kStepMaxLayers, 0, 0, 0};
+    StepPlan p = {0, 0, 0, 0, 0, kStepMaxLayers, 0, 0, 0, 0};
     if ((head_dim != 64 && head_dim != 128 && head_dim != 256) || num_kv_heads <= 0 || num_q_heads <= 0 || num_q_heads % num_kv_heads ||
         batch < 1 || batch > kStepMaxBatch || n_ctas < 1) return p;
     const int group = num_q_heads / num_kv_heads, runs = group > 8 ? 2 : 1, warps = step_warps(head_dim, runs), team = warps / step_teams(head_dim);
@@ -82,6 +84,10 @@ __host__ __device__ inline StepPlan make_step_plan(int num_q_heads, int num_kv_h
     p.state_bytes = n_ctas * hg * group * (head_dim / 2 + 1) * 16;
     p.smem_bytes = 1024 + step_slots(head_dim, runs) * (step_tile_bytes(head_dim, runs) + hg * head_dim * 2) + hg * runs * (head_dim / 8) * 128 +
                    warps * runs * 8 * 16 + kStepCtrlBytes + hg * group * (head_dim + kStepStatePad) * 4 + vteb::vteb_round_up((2 * batch + 1) * 4, 16);
+    // states that the ring holds at once, less two for parts merged before (32 heads on 2 of 128, one of 16,384 positions, four layers,
+    // 19 CTAs a run: 63 us with sixteen, which take two goes)
+    p.fan = step_slots(head_dim, runs) * step_tile_bytes(head_dim, runs) / (hg * group * (head_dim + kStepStatePad) * 4) - 2;
+    p.fan = p.fan < 4 ? 4 : p.fan > kStepMostFan ? kStepMostFan : p.fan;
     p.ok = p.smem_bytes <= 227 * 1024;
     return p;
 }
@@ -437,7 +443,7 @@ __device__ __forceinline__ void step_body(const StepArgs& a)
         bool keep = was_begun && !goes_on;                           // the state stays here, until this CTA finishes the run or a part of it
         if (goes_on && was_begun) {
             const int k = cta - cta_of(run.start);
-            keep = (k + 1) % kStepFan == 0 && cta_of(run.end - 1) - cta + k >= kStepFan;
+            keep = (k + 1) % a.fan == 0 && cta_of(run.end - 1) - cta + k >= a.fan;
         }
         if (keep) finish = goes_on ? 2 : 1;
         for (int idx = tid; idx < rows * (D / 4); idx += THREADS) {
@@ -488,11 +494,11 @@ __device__ __forceinline__ void step_body(const StepArgs& a)
     if (!finish) return;
     step_sync<THREADS>();
     // ---- a cut run: the states of the CTAs in front, in order, then this CTA's.  Only CTAs with lower numbers are waited for: they run or
-    // are done.  Of more than kStepFan CTAs in a run, every kStepFan-th merges what lies between the one before it and itself.
+    // are done.  Of more than `fan` CTAs in a run, every fan-th merges what lies between the one before it and itself.
     const StepRun& r = finish == 2 ? run : head;
     const int c0 = cta_of(r.start), k = cta - c0;
-    const int parts = finish == 2 || k < kStepFan ? 0 : k / kStepFan, from = finish == 2 ? k + 1 - kStepFan : parts * kStepFan, sources = parts + k - from;
-    const auto source = [&](int i) { return c0 + (i < parts ? (i + 1) * kStepFan - 1 : from + i - parts); };
+    const int fan = a.fan, parts = finish == 2 || k < fan ? 0 : k / fan, from = finish == 2 ? k + 1 - fan : parts * fan, sources = parts + k - from;
+    const auto source = [&](int i) { return c0 + (i < parts ? (i + 1) * fan - 1 : from + i - parts); };
     const long long t_start = clock64();
     bool in_time = true;
     constexpr int ENTRIES = D / 2 + 1, AT_ONCE = 8;

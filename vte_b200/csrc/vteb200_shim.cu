@@ -642,7 +642,7 @@ int vteb_step_plan(int num_q_heads, int num_kv_heads, int head_dim, int batch, i
     const StepPlan p = make_step_plan(num_q_heads, num_kv_heads, head_dim, batch, n_ctas, hg);
     plan->ok = p.ok; plan->threads = p.threads; plan->smem_bytes = p.smem_bytes; plan->hg = p.hg;
     plan->state_bytes = p.state_bytes; plan->max_layers = p.max_layers;
-    plan->hg_log2 = p.hg_log2; plan->wph = p.wph; plan->tile = p.tile;
+    plan->hg_log2 = p.hg_log2; plan->wph = p.wph; plan->tile = p.tile; plan->fan = p.fan;
     return 0;
 }
 

@@ -1,6 +1,7 @@
 """A decode step as one launch over all its layers (core/step_route.py, csrc/kernels/step_decode.cuh): what may take it and
 what does, on the CPU, and the kernels against the oracle where tiles, shares and runs meet."""
 import ctypes
+import re
 from types import SimpleNamespace
 
 import numpy as np
@@ -93,6 +94,21 @@ def test_what_goes_to_one_launch(built_library):
 def test_one_launch_refuses_what_it_would_drop(option):
     with pytest.raises((CudaSafetyError, AttributeError)):
         DecodeAttentionExecutor(None, None, {}, 1, 256, 4, one_launch=True, **option)
+
+
+def kernel_source():
+    from vte_b200.compiler.codegen import KERNEL_DIR
+    return (KERNEL_DIR / "step_decode.cuh").read_text()
+
+
+def test_boards_are_written_and_read_in_whole_tagged_words():
+    """A value and the number that makes it valid are one scalar of one access on either side, ordered as relaxed ones are: the
+    elements of a vector access have no order among themselves, and a plain store beside a relaxed load is a race."""
+    src = kernel_source()
+    assert "ulonglong2* boards;" in src and len(re.findall(r"= a\.boards \+", src)) == src.count("a.boards") == 2    # written, read
+    assert "st.relaxed.gpu.global.v2.b64 [%0]" in src and "ld.relaxed.gpu.global.v2.b64 {%0, %1}" in src
+    assert len(re.findall(r"store_entry\(to ", src)) == 3 and src.count("= load_entry(from_at[u])") == 2
+    assert not re.search(r"\*to = |\bto\[[0-9D]|\*from_at|relaxed\S*\.v4", src)          # by no other access
 
 
 HEADS = [(12, 2, 128), (32, 8, 64), (8, 2, 256), (8, 8, 128), (7, 1, 128), (6, 3, 64), (8, 1, 256), (22, 2, 128), (32, 2, 128), (16, 1, 64)]

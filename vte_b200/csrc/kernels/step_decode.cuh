@@ -6,8 +6,8 @@
 // each, into a ring; `wph` warps serve a KV head, a 16-position block of every tile each (block arithmetic of lean_decode.cuh,
 // fp32 sums).  At the end of a run the warps' states meet in the tile they have just done with, while the rest of the ring keeps
 // filling.  A run that lies in one share is normalised and stored.  Of one that was cut, each CTA but the last leaves its state
-// on a board, in 64-bit words that carry the number of the launch (valid exactly when they carry it, so without a fence), and
-// the last merges them, bounded, in their order; it waits for CTAs with lower numbers only.
+// on a board, in 64-bit words that carry the number of the launch (each written and read in one relaxed access, so valid exactly
+// when it carries it, without a fence), and the last merges them, bounded, in their order; it waits for CTAs with lower numbers only.
 //
 // What bounds it: HBM, and about 9 us of launch, start (2), first tile (1.3), merges (1.3 a run) and finish (2 to 2.5).  us a step,
 // launches per layer / one launch, 12 heads on 2 KV heads of 128, one sequence: 28 layers of 1,531 positions 104 / 15.5, of 11,003
@@ -38,7 +38,7 @@ constexpr int kStepOffsets = 64;                          // sequences whose off
 struct StepArgs {
     StepLayer layer[kStepMaxLayers];
     const int* kv_offsets; const __half* rope_cos; const __half* rope_sin;
-    uint4* boards; unsigned* launches; int* status;       // [CTAs][hg * group][D / 2 + 1]: the state of a cut run, two tagged words an entry; [CTAs]: launches so far
+    ulonglong2* boards; unsigned* launches; int* status;  // [CTAs][hg * group][D / 2 + 1]: the state of a cut run, two tagged words an entry; [CTAs]: launches so far
     int* status_mirror;                                   // the same for what `status` says
     __half* keep_q; int* keep_offsets; void* unused[7];
     int offsets[kStepOffsets]; int offsets_here;          // 1: the kv offsets are these, and go to kv_offsets for whoever reads them there
@@ -105,11 +105,18 @@ struct StepRun {
     }
 };
 
-__device__ __forceinline__ uint4 ld_relaxed_16(const uint4* p) {
-    uint4 v;
-    asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+// An entry of a board: two fp32 values, each in a 64-bit word with the launch's number above it.  A vector access is as many scalar
+// ones in no order, so the elements are the words: a number seen has come with its value.
+__device__ __forceinline__ void store_entry(ulonglong2* p, float x, float y, unsigned tag) {
+    const unsigned long long up = (unsigned long long)tag << 32;
+    asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"(up | __float_as_uint(x)), "l"(up | __float_as_uint(y)) : "memory");
+}
+__device__ __forceinline__ ulonglong2 load_entry(const ulonglong2* p) {
+    ulonglong2 v;
+    asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(p) : "memory");
     return v;
 }
+__device__ __forceinline__ bool entry_of(const ulonglong2& v, unsigned tag) { return (unsigned)(v.x >> 32) == tag && (unsigned)(v.y >> 32) == tag; }
 template <int THREADS> __device__ __forceinline__ void step_sync() { asm volatile("bar.sync 1, %0;" ::"n"(THREADS) : "memory"); }   // of the warps that compute
 
 template <int D, int NV>
@@ -316,10 +323,10 @@ __device__ __forceinline__ void step_body(const StepArgs& a)
         return c;
     };
     const auto push = [&](int j, int q4, const float4& acc, float m, float l) {      // to the CTA that finishes the run or the part
-        uint4* const to = a.boards + ((long long)cta * rows + j) * (D / 2 + 1);
-        to[2 * q4] = make_uint4(__float_as_uint(acc.x), tag, __float_as_uint(acc.y), tag);
-        to[2 * q4 + 1] = make_uint4(__float_as_uint(acc.z), tag, __float_as_uint(acc.w), tag);
-        if (q4 == 0) to[D / 2] = make_uint4(__float_as_uint(m), tag, __float_as_uint(l), tag);
+        ulonglong2* const to = a.boards + ((long long)cta * rows + j) * (D / 2 + 1);
+        store_entry(to + 2 * q4, acc.x, acc.y, tag);
+        store_entry(to + 2 * q4 + 1, acc.z, acc.w, tag);
+        if (q4 == 0) store_entry(to + D / 2, m, l, tag);
     };
     const StepRun head = run;                                        // the run that was cut at the share's start, if any was
     int finish = 0;                                                  // 1: a run that CTAs in front began, 2: a part of one that goes on
@@ -518,8 +525,8 @@ __device__ __forceinline__ void step_body(const StepArgs& a)
                 settle();
 #pragma unroll 1
                 while (i < n) {
-                    uint4 w[AT_ONCE];
-                    const uint4* from_at[AT_ONCE];
+                    ulonglong2 w[AT_ONCE];
+                    const ulonglong2* from_at[AT_ONCE];
                     float* to[AT_ONCE];
 #pragma unroll
                     for (int u = 0; u < AT_ONCE; ++u) {
@@ -528,7 +535,7 @@ __device__ __forceinline__ void step_body(const StepArgs& a)
                             const int row = e / ENTRIES;
                             from_at[u] = a.boards + (long long)source(i0 + i) * entries + e;
                             to[u] = reinterpret_cast<float*>(ring) + (i * rows + row) * SP + 2 * (e - row * ENTRIES);
-                            w[u] = ld_relaxed_16(from_at[u]);
+                            w[u] = load_entry(from_at[u]);
                             e += THREADS;
                             settle();
                         }
@@ -536,11 +543,11 @@ __device__ __forceinline__ void step_body(const StepArgs& a)
 #pragma unroll
                     for (int u = 0; u < AT_ONCE; ++u)
                         if (to[u] != nullptr) {
-                            while ((w[u].y != tag || w[u].w != tag) && in_time) {
-                                w[u] = ld_relaxed_16(from_at[u]);
+                            while (!entry_of(w[u], tag) && in_time) {
+                                w[u] = load_entry(from_at[u]);
                                 if (clock64() - t_start > kWaitLimitCycles) in_time = false;
                             }
-                            *reinterpret_cast<float2*>(to[u]) = make_float2(__uint_as_float(w[u].x), __uint_as_float(w[u].z));
+                            *reinterpret_cast<float2*>(to[u]) = make_float2(__uint_as_float((unsigned)w[u].x), __uint_as_float((unsigned)w[u].y));
                         }
                 }
                 step_sync<THREADS>();

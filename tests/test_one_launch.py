@@ -8,8 +8,11 @@ import numpy as np
 import pytest
 
 from oracle import attention_oracle as orc
-from vte_b200.bridge.cuda_runtime import StepArgs, StepLayer, StepPlan, load_library
+from tests.test_host_logic import FakeCodegen, FakeRuntime
+from tests.test_lean_routes import FakeHip
+from vte_b200.bridge.cuda_runtime import KvTensorMap, StepArgs, StepLayer, StepPlan, load_library
 from vte_b200.bridge.errors import CudaRuntimeError, CudaSafetyError
+from vte_b200.bridge.memory import SlabAllocator
 from vte_b200.core.decode_executor import DecodeAttentionExecutor
 from vte_b200.core.split_kv_attention import SplitKVAttentionDispatcher
 from vte_b200.core.step_route import StepRoute, one_launch_pays
@@ -94,6 +97,78 @@ def test_what_goes_to_one_launch(built_library):
 def test_one_launch_refuses_what_it_would_drop(option):
     with pytest.raises((CudaSafetyError, AttributeError)):
         DecodeAttentionExecutor(None, None, {}, 1, 256, 4, one_launch=True, **option)
+
+
+class HostOnly(FakeRuntime, FakeHip):
+    """A runtime whose launches are names in a list: nothing is dereferenced but pinned memory."""
+    step_plan, programmatic_launch = staticmethod(step_plan), False
+
+    def __init__(self):
+        super().__init__()
+        self.log, self.recording, self.maps, self.pinned = [], None, [], []
+
+    def _names(self, launches): return [self.loaded[fn.value - 0x1001][1] for fn, *_ in launches]
+    def launched(self):
+        names, self.log = self._names(self.log), []
+        return names
+    def get_real_mem_info(self): return 180 << 30, 180 << 30
+    def host_alloc(self, n):
+        self.pinned.append(ctypes.create_string_buffer(n))
+        return ctypes.c_void_p(ctypes.addressof(self.pinned[-1]))
+    def stream_begin_capture(self): self.recording = []
+    def stream_end_capture(self):
+        graph, self.recording = self.recording, None
+        return graph
+    def launch_kernel_recorded(self, *launch): (self.log if self.recording is None else self.recording).append(launch)
+    def graph_instantiate(self, graph): return graph
+    def graph_launch(self, graph): self.log += graph
+    def prepare_launch(self, *launch): return lambda: self.log.append(launch[:5])
+    def host_step(self, step, graph, offsets, q, out):
+        self.log += graph
+        return True
+    def kv_tensor_map(self, ptr, n_rows, row_halves, box_rows, box_cols=0):
+        self.maps.append((ptr, n_rows, row_halves))
+        return KvTensorMap()
+    def event_create(self): return ctypes.c_void_p(1)
+    def _nothing(self, *a, **kw): return True
+    graph_destroy = graph_exec_destroy = host_free = stream_synchronize = check_status = event_record = event_synchronize = _nothing
+    event_destroy = memcpy_h2d_async = memcpy_d2h_async = memset_async = safe_memcpy_host_to_device = safe_memcpy_device_to_host = _nothing
+
+
+def host_only(B=1, S=4096, L=4, heads=(12, 2, 128), **kw):
+    rt = HostOnly()
+    meta = {"attention.head_count": heads[0], "attention.head_count_kv": heads[1], "attention.key_length": heads[2]}
+    return DecodeAttentionExecutor(rt, FakeCodegen(), meta, B, S, L, **kw), rt
+
+
+def test_nothing_is_launched_after_cleanup(built_library):
+    """The device memory of an executor with an allocator of its own is gone by then; the staging memory is in any case."""
+    off, q = np.array([100], dtype=np.int32), np.zeros((4, 1, 12, 128), dtype=np.float16)
+    ex, rt = host_only()
+    ex.execute_decode_batch(off, read_output=False)
+    ex.execute_decode_batch(off, q)
+    assert rt.launched() == ["vteb_decode_step_d128_kernel", "vteb_stage_copy_kernel", "vteb_decode_step_d128_kernel"]
+    ex.cleanup()
+    for call in (lambda: ex.execute_decode_batch(off, read_output=False), lambda: ex.execute_decode_batch(off), lambda: ex.execute_decode_batch(off, q),
+                 ex.launch_step, ex.build_decode_graph, ex.build_io_graph):
+        with pytest.raises(CudaSafetyError, match="cleaned up"):
+            call()
+    assert rt.launched() == []
+    rt = HostOnly()                                                    # a caller's allocator outlives the executor
+    allocator = SlabAllocator(rt, 180 << 30, requested_pool_size=1 << 30)
+    allocator.initialize()
+    meta = {"attention.head_count": 12, "attention.head_count_kv": 2, "attention.key_length": 128}
+    ex = DecodeAttentionExecutor(rt, FakeCodegen(), meta, 1, 4096, 4, allocator=allocator)
+    ex.execute_decode_batch(off, read_output=False)
+    ex.cleanup()
+    rt.launched()
+    ex.launch_step()
+    ex.build_decode_graph()
+    ex.launch_step()
+    assert rt.launched() == ["vteb_decode_step_d128_kernel"] * 2
+    with pytest.raises(CudaSafetyError, match="cleaned up"):
+        ex.execute_decode_batch(off, read_output=False)
+    assert rt.launched() == []
 
 
 def kernel_source():

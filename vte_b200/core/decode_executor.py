@@ -47,7 +47,7 @@ STEP_OFFSETS = 64       # sequences whose offsets may be among the arguments of 
 
 
 class DecodeAttentionExecutor:
-    _step, _one_launch, _direct = None, False, ()
+    _step, _one_launch, _direct, _closed = None, False, (), False
 
     def __init__(self, hip, codegen, metadata: dict, batch_size: int, context_length: int, n_layers: int, *,
                  n_kv_buffers: Optional[int] = None, num_splits: Optional[int] = None, output_f32: bool = True,
@@ -355,8 +355,14 @@ class DecodeAttentionExecutor:
         self._step = step
         return True
 
+    def _require_open(self, staging: bool = False):
+        """A cleaned-up executor has no staging memory, and device memory only where the caller's allocator holds it."""
+        if self._closed and (staging or self._owns_allocator):
+            raise CudaSafetyError("the executor has been cleaned up: its memory is gone")
+
     def build_decode_graph(self):
         """Capture all layers' launches once (hip_graph_executor.py:504-725)."""
+        self._require_open()
         if self._graph_exec is not None:
             return
         self.hip.programmatic_launch = self.programmatic
@@ -369,6 +375,7 @@ class DecodeAttentionExecutor:
             self._choose_route()
             self._graph_exec, n = self._capture(self._record_all)
             if self._step is not None and self.per_layer_hook is None and self.launch_rewriter is None and self.B <= STEP_OFFSETS:
+                self._direct = []
                 for fn, args, grid, block, smem in self._step_launches():
                     args[0].offsets_here = 1
                     self._direct.append((args[0].offsets, self.hip.prepare_launch(fn, args, grid, block, smem, self.programmatic)))
@@ -403,6 +410,7 @@ class DecodeAttentionExecutor:
         copy nodes.  A step is then one graph launch instead of three copies and a launch (the
         reference stages its offsets with a separate copy before each launch,
         vte/core/hip_graph_executor.py:772-789)."""
+        self._require_open(staging=True)
         if self._io_graph_exec is not None or not self.use_graph:
             return
         if self._copy_fn is None:                         # before the capture begins
@@ -491,6 +499,7 @@ class DecodeAttentionExecutor:
 
     def launch_step(self):
         """Enqueue one decode step (no host synchronisation)."""
+        self._require_open()
         if self._graph_exec is not None:
             self.hip.graph_launch(self._graph_exec if self._on_route else self._plain_graph_exec)
             self._partials_due = self._on_route and self._kept_names is not None
@@ -506,6 +515,7 @@ class DecodeAttentionExecutor:
         """One decode step end to end: stage offsets (and, when given, every layer's
         Q [L,B,Hq,D] fp16) host -> device, replay the graph, read every layer's
         output back.  Returns [L,B,Hq,D] (fp32 or fp16)."""
+        self._require_open(staging=True)
         self.build_decode_graph()
         nbytes = self.L * self.out_bytes
         if q_host is not None and read_output and self.use_graph:
@@ -603,6 +613,8 @@ class DecodeAttentionExecutor:
         return m, l, o
 
     def cleanup(self):
+        self._closed = True
+        self._direct, self._host_step = [], None          # launches on device memory and staging memory that go below
         if self._stage_event is not None:
             self.hip.event_destroy(self._stage_event)
             self._stage_event = None

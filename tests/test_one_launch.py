@@ -171,6 +171,22 @@ def test_nothing_is_launched_after_cleanup(built_library):
     assert rt.launched() == []
 
 
+@pytest.mark.parametrize("spare", [0, 1, 100, 4096])
+def test_tiles_end_where_the_last_sequence_s_room_does(built_library, spare):
+    """With a stride longer than the cache, the rows behind the last sequence may be anybody's: the maps end in front of them."""
+    B, S = 3, 500
+    ex, rt = host_only(B, S)
+    row = 256
+    ex.tensor_mapping['kv_batch_stride_elements'] = (S + spare) * row
+    for l in range(ex.L):                                              # K of all layers, then V, in somebody else's memory
+        for i, name in enumerate(("k", "v")):
+            ex.tensor_mapping[f'blk.{l}.kv_cache.{name}'] = 0x5000_0000_0000 + (i * ex.L + l) * B * (S + spare) * row * 2
+    ex.build_decode_graph()
+    assert ex.route_name[0] == "vteb_decode_step_d128_kernel"
+    step = [m for m in rt.maps if m[0] >= 0x5000_0000_0000]
+    assert len(step) >= 2 * ex.L and all(n_rows == (B - 1) * (S + spare) + S and halves == row for _, n_rows, halves in step)
+
+
 def kernel_source():
     from vte_b200.compiler.codegen import KERNEL_DIR
     return (KERNEL_DIR / "step_decode.cuh").read_text()

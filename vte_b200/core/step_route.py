@@ -81,7 +81,8 @@ class StepRoute:
         attention_scale = d.metadata.get('attention_scale')
         row = d.num_kv_heads * d.head_dim
         row_out = d.num_q_heads * d.head_dim * (4 if d.output_f32 else 2)
-        n_rows = int(mapping['kv_batch_stride_elements']) // row * batch
+        # as far as `serves` has looked: the last sequence's room, not its stride, ends what a tile may read
+        n_rows = int(mapping['kv_batch_stride_elements']) // row * (batch - 1) + d.context_length
         out = []
         for first in range(0, self.layers, self.plan.max_layers):
             n = min(self.plan.max_layers, self.layers - first)

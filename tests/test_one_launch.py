@@ -202,6 +202,16 @@ def test_boards_are_written_and_read_in_whole_tagged_words():
     assert not re.search(r"\*to = |\bto\[[0-9D]|\*from_at|relaxed\S*\.v4", src)          # by no other access
 
 
+def test_no_copy_outlives_its_block():
+    """The warp that fetches stops where another gave up, whose tiles may have a copy under way to them, and waits for its last copies
+    whoever it was; no row is appended that may not have come."""
+    src = kernel_source()
+    fetching = src[src.index("// ---- the tiles of the share"):src.index("// ---- Q of a run's heads")]
+    assert re.search(r"!mbar_wait_bounded\(empty0 [^)]*\) \|\| \*abort_word != 0\)", fetching)
+    assert re.search(r"\n        for \(int i = 1; i <= min\(sent, SLOTS\); \+\+i\) \{", fetching) and "if (!ok" not in fetching
+    assert "if (lane < CPR && *abort_word == 0) {" in src
+
+
 HEADS = [(12, 2, 128), (32, 8, 64), (8, 2, 256), (8, 8, 128), (7, 1, 128), (6, 3, 64), (8, 1, 256), (22, 2, 128), (32, 2, 128), (16, 1, 64)]
 LENGTHS = [1, 15, 16, 17, 31, 33, 47, 48, 49, 64, 65, 95, 96, 97, 127, 128, 129, 257, 300]
 

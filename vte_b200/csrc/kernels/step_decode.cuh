@@ -229,7 +229,8 @@ __device__ __forceinline__ void step_body(const StepArgs& a)
             const bool newest = t == run.end - 1 && L.k_new != nullptr;
 #pragma unroll 1
             for (int kv = 0; kv < 2; ++kv) {
-                if (sent >= SLOTS && !mbar_wait_bounded(empty0 + 8 * slot, phase ^ 1, abort_word)) {
+                // a tile given back by a warp that gave up may have a copy under way to it still
+                if (sent >= SLOTS && __any_sync(0xffffffffu, !mbar_wait_bounded(empty0 + 8 * slot, phase ^ 1, abort_word) || *abort_word != 0)) {
                     gave_up(kStatusEmptyTimeout);
                     ok = false;
                     break;
@@ -251,11 +252,11 @@ __device__ __forceinline__ void step_body(const StepArgs& a)
         }
         if (a.offsets_here && cta == 0)                              // for whoever reads them there; not in front: a path of one CTA's own is slow to fetch
             for (int b = lane; b < a.batch; b += 32) const_cast<int*>(a.kv_offsets)[b] = a.offsets[b];
-        if (!ok)                                                     // its own copies have to land before the CTA may end
-            for (int i = 1; i <= min(sent, SLOTS); ++i) {
-                const uint32_t bar = full_of(sent - i);
-                mbar_wait_bounded(bar & 0x7fffffffu, bar >> 31, nullptr);
-            }
+        // Every copy lands before this warp, and with it the CTA, ends: the computing warps may have given up.
+        for (int i = 1; i <= min(sent, SLOTS); ++i) {
+            const uint32_t bar = full_of(sent - i);
+            mbar_wait_bounded(bar & 0x7fffffffu, bar >> 31, nullptr);
+        }
         return;
     }
 
@@ -360,7 +361,7 @@ __device__ __forceinline__ void step_body(const StepArgs& a)
             const auto put_newest = [&](int kv, int s) {
                 const int head_at = run.h * hg + kvh;
                 __half* cache = (kv ? L.v_cache : L.k_cache) + (long long)run.b * a.kv_batch_stride + (len - 1) * pos_stride + head_at * D;
-                if (lane < CPR) {
+                if (lane < CPR && *abort_word == 0) {                // where a wait was given up the row may not be here
                     uint4 w = reinterpret_cast<const uint4*>(fresh + (s * hg + kvh) * D * 2)[lane];
                     if (!kv && rope_touches(a.rope_type, a.rotary_dim, lane * 8))
                         w = rope_chunk(w, L.k_new + (long long)run.b * pos_stride + head_at * D, lane * 8,

@@ -187,6 +187,35 @@ def test_tiles_end_where_the_last_sequence_s_room_does(built_library, spare):
     assert len(step) >= 2 * ex.L and all(n_rows == (B - 1) * (S + spare) + S and halves == row for _, n_rows, halves in step)
 
 
+@pytest.mark.parametrize("one", [None, True])
+def test_a_step_is_captured_for_the_mapping_of_its_time(built_library, one):
+    """Between the capture of a device-side step and that of a step from the host, layer 1's Q becomes layer 0's output: layers
+    that depend on one another take a launch list each, and partials are that list's own."""
+    off, q = np.array([100], dtype=np.int32), np.zeros((4, 1, 12, 128), dtype=np.float16)
+    ex, rt = host_only(output_f32=False, with_append=True, one_launch=one)
+    ex.execute_decode_batch(off, read_output=False)
+    assert rt.launched() == ["vteb_decode_step_d128_kernel"] and ex._partials_due
+    ex.tensor_mapping['blk.1.q_proj.output'] = ex.tensor_mapping['blk.0.attention.output']
+    if one:
+        with pytest.raises(CudaSafetyError, match="another writes"):
+            ex.execute_decode_batch(off, q)
+        assert rt.launched() == []
+        return
+    ex.build_io_graph()
+    assert ex._partials_due and ex.route_name is None
+    ex.execute_decode_batch(off, q)
+    names = rt.launched()
+    assert not any(n.startswith("vteb_decode_step") for n in names) and names.count("kv_cache_append_kernel") == 4 and not ex._partials_due
+    assert names[0] == names[-1] == "vteb_stage_copy_kernel"           # and the outputs are brought by a copy
+    ex.execute_decode_batch(off, read_output=False)                    # the captured one
+    assert rt.launched() == ["vteb_decode_step_d128_kernel"] and ex._partials_due
+    ex, rt = host_only(output_f32=False)                               # a hook that came in between
+    ex.execute_decode_batch(off, read_output=False)
+    hooked, ex.per_layer_hook = [], lambda layer: hooked.append(layer)
+    ex.execute_decode_batch(off, q)
+    assert hooked == [0, 1, 2, 3] and not ex._partials_due
+
+
 def kernel_source():
     from vte_b200.compiler.codegen import KERNEL_DIR
     return (KERNEL_DIR / "step_decode.cuh").read_text()

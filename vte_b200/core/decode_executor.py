@@ -44,10 +44,13 @@ STAGE_COPY_MAX_BYTES = 1 << 20
 OFFSET_SLOTS = 64
 
 STEP_OFFSETS = 64       # sequences whose offsets may be among the arguments of a step of one launch (kStepOffsets in csrc/kernels/step_decode.cuh)
+NOT_SIDE_BY_SIDE = "one launch for all layers: a layer reads or writes what another writes, or has pointers that are not 16-byte aligned"
 
 
 class DecodeAttentionExecutor:
     _step, _one_launch, _direct, _closed = None, False, (), False
+    _graph_kept = _io_kept = None
+    _recorded_step = False
 
     def __init__(self, hip, codegen, metadata: dict, batch_size: int, context_length: int, n_layers: int, *,
                  n_kv_buffers: Optional[int] = None, num_splits: Optional[int] = None, output_f32: bool = True,
@@ -143,7 +146,7 @@ class DecodeAttentionExecutor:
         self._route_pays_to, self._on_route, self._launches = self.S, True, (0, 0)
         self._plain_graph_exec = self._plain_io_graph_exec = None
         # what partials of a routed step can be had from: the last layer's Q and offsets as the step saw them, the names it
-        # was captured with, and whether the partial buffers are still to be filled
+        # was captured with (each graph's, and the last step's), and whether the partial buffers are still to be filled
         self._kept, self._kept_names, self._partials_due = None, None, False
         self.k_cache = [A(self.kv_bytes, f"kv_cache.k.{i}", MemoryRegion.KV_CACHE) for i in range(self.n_kv)]
         self.v_cache = [A(self.kv_bytes, f"kv_cache.v.{i}", MemoryRegion.KV_CACHE) for i in range(self.n_kv)]
@@ -261,14 +264,15 @@ class DecodeAttentionExecutor:
     def route_name(self):
         """(kernel, CTAs per (sequence, KV head)) where the last captured step did not take the dispatcher's launches, else None;
         (kernel, 0) where it is one launch."""
-        if self._step is not None:
+        if self._step is not None and self._recorded_step:
             return self._step.name, 0
         return (self._route.name, self._route.parts) if self._route is not None and self._on_route else None
 
-    def _record_all(self, after_copy: bool = False, plain: bool = False, mirror: Optional[tuple] = None):
+    def _record_all(self, after_copy: bool = False, plain: bool = False, one_launch: bool = False, mirror: Optional[tuple] = None):
         n = 0
         programmatic = self.hip.programmatic_launch
-        if self._step is not None and self.per_layer_hook is None and self.launch_rewriter is None:
+        self._recorded_step = one_launch
+        if one_launch:
             return self._record_step(mirror)
         # within a captured step of nothing but the layers' own launches, offsets and older rows do not change
         self.dispatcher.offsets_final = self.use_graph and self.per_layer_hook is None and self.launch_rewriter is None
@@ -302,18 +306,28 @@ class DecodeAttentionExecutor:
             self.hip.launch_kernel_recorded(*launch)
         return len(launches)
 
-    def _choose_route(self):
-        """Before a step is captured: whether its layers' launches are the dispatcher's own or a route of lean_route.py."""
+    def _serves_one_launch(self) -> bool:
+        """Whether a step that is recorded now may be the one launch: the mapping may be another than the one it was chosen with."""
+        if self._step is None or self.per_layer_hook is not None or self.launch_rewriter is not None:
+            return False
+        serves = self._step.serves(self.tensor_mapping, self.offsets.ptr, self.B)
+        if self._one_launch and not serves:
+            raise CudaSafetyError(NOT_SIDE_BY_SIDE)
+        return serves
+
+    def _choose_route(self) -> bool:
+        """Before a step is captured: whether its layers' launches are the dispatcher's own or a route of lean_route.py.  True where
+        one launch for all of them has just been found to serve."""
         d = self.dispatcher
         if (self._route is not None or self._step is not None or self._lean == (0, 0) and not self._one_launch or not self.use_graph or
                 self.per_layer_hook is not None or self.launch_rewriter is not None or not d.enabled or not hasattr(self.hip, 'lean_plan')):
             if self._one_launch and self._step is None:
                 raise CudaSafetyError("one launch for all layers needs a captured step without a hook or a rewriter")
-            return
+            return False
         d._allocate_scratch()                         # and the work words
         append = self.with_append or d.fuse_append
         if self._one_launch is not False and self._choose_one_launch(append):
-            return
+            return True
         if self._lean is None:
             self._lean = choose_lean_route(d, append)
         if self._lean[0]:
@@ -325,10 +339,11 @@ class DecodeAttentionExecutor:
                 if self._forced_route:
                     raise
                 self._lean = (0, 0)                   # a caller's allocator with no room for it: the dispatcher's launches need none
-                return
+                return False
             self._route = route
             if not self._forced_route:
                 self._route_pays_to = route.pays_up_to()
+        return False
 
     def _choose_one_launch(self, append: bool) -> bool:
         """Takes one launch for the step where its layers may run side by side and that pays."""
@@ -344,7 +359,7 @@ class DecodeAttentionExecutor:
                                                  MemoryRegion.SCRATCH)
             blocks.append(self._kept)
             if not step.serves(self.tensor_mapping, self.offsets.ptr, self.B):
-                raise CudaSafetyError("one launch for all layers: a layer reads or writes what another writes, or has pointers that are not 16-byte aligned")
+                raise CudaSafetyError(NOT_SIDE_BY_SIDE)
         except CudaSafetyError:
             if forced:
                 raise
@@ -372,31 +387,33 @@ class DecodeAttentionExecutor:
                 n += 1 if self.rope == "separate" else 0
                 self.kernel_launches_per_step = (n if (self.with_append or self.dispatcher.fuse_append) else n - 1) * self.L
                 return
-            self._choose_route()
-            self._graph_exec, n = self._capture(self._record_all)
-            if self._step is not None and self.per_layer_hook is None and self.launch_rewriter is None and self.B <= STEP_OFFSETS:
+            one = self._choose_route() or self._serves_one_launch()
+            self._graph_exec, n, self._graph_kept = self._capture(lambda: self._record_all(one_launch=one))
+            if one and self.B <= STEP_OFFSETS:
                 self._direct = []
                 for fn, args, grid, block, smem in self._step_launches():
                     args[0].offsets_here = 1
                     self._direct.append((args[0].offsets, self.hip.prepare_launch(fn, args, grid, block, smem, self.programmatic)))
             plain = n
             if self._route_pays_to < self.S:
-                self._plain_graph_exec, plain = self._capture(lambda: self._record_all(plain=True))
+                self._plain_graph_exec, plain, _ = self._capture(lambda: self._record_all(plain=True))
             self._launches = n, plain
             self.kernel_launches_per_step = n
         finally:
             self.hip.programmatic_launch = False
 
     def _capture(self, record):
-        """(executable graph, what `record` returns) of what `record` launches."""
+        """(executable graph, what `record` returns, the names that partials can be had with) of what `record` launches."""
+        last, self._kept_names = self._kept_names, None
         self.hip.stream_begin_capture()
         try:
             n = record()
         finally:
             graph = self.hip.stream_end_capture()
+            kept, self._kept_names = self._kept_names, last
         graph_exec = self.hip.graph_instantiate(graph)
         self.hip.graph_destroy(graph)
-        return graph_exec, n
+        return graph_exec, n, kept
 
     def _pick(self, offsets: np.ndarray, newest: int):
         """Which of two captured steps serves these offsets, the largest of which is `newest`."""
@@ -416,12 +433,12 @@ class DecodeAttentionExecutor:
         if self._copy_fn is None:                         # before the capture begins
             self._copy_fn = self.codegen.load_kernel_safe(self.hip, 'decode_attention', self.hip.get_gpu_architecture(),
                                                           'vteb_stage_copy_kernel')[1]
-        self._choose_route()
+        one = self._choose_route() or self._serves_one_launch()
         self.hip.programmatic_launch = self.programmatic
         try:
-            self._io_graph_exec, _ = self._capture(self._record_io)
+            self._io_graph_exec, _, self._io_kept = self._capture(lambda: self._record_io(one_launch=one))
             if self._route_pays_to < self.S:
-                self._plain_io_graph_exec, _ = self._capture(lambda: self._record_io(plain=True))
+                self._plain_io_graph_exec, _, _ = self._capture(lambda: self._record_io(plain=True))
         finally:
             self.hip.programmatic_launch = False
 
@@ -435,17 +452,17 @@ class DecodeAttentionExecutor:
             return None
         return self._stage_out.value, self._stage_out.value + self._out_tail + 4
 
-    def _record_io(self, plain: bool = False):
+    def _record_io(self, plain: bool = False, one_launch: bool = False):
         if max(self._q_tail, self._out_tail) <= STAGE_COPY_MAX_BYTES:
-            mirror = self._mirror()
+            mirror = self._mirror() if one_launch else None
             self._stage_copy(self.q_all.ptr, self._stage_q.value, self._q_tail + 4 * self.B, first=True)
-            self._record_all(after_copy=True, plain=plain, mirror=mirror)
+            self._record_all(after_copy=True, plain=plain, one_launch=one_launch, mirror=mirror)
             if not mirror:
                 self._stage_copy(self._stage_out.value, self.out_all.ptr, self._out_tail + 16)
         else:
             self.hip.memcpy_h2d_async(ctypes.c_void_p(self.q_all.ptr), self._stage_q, self._q_tail + 4 * self.B,
                                       "q and kv offsets staging")
-            self._record_all(plain=plain)
+            self._record_all(plain=plain, one_launch=one_launch)
             self.hip.memcpy_d2h_async(self._stage_out, ctypes.c_void_p(self.out_all.ptr), self._out_tail + 16,
                                       "attention output and status word")
 
@@ -472,6 +489,10 @@ class DecodeAttentionExecutor:
             raise CudaSafetyError(f"kv offset outside 0..{self.S - 1}")
         return off, newest
 
+    def _leaves(self, names: Optional[dict]):
+        """After a step: the names that its partials can be had with, None where they are in the partial buffers."""
+        self._kept_names, self._partials_due = names, names is not None
+
     def _launch_with_offsets(self, off: np.ndarray):
         """A step of one launch, its offsets among the launch's arguments: neither a copy in front of the launch nor a graph around
         it.  us a step, a copy and a graph / this: 28 layers of one sequence of 1,531 positions 20.5 / 16.1, of 11,003 58.4 / 55.6,
@@ -479,7 +500,7 @@ class DecodeAttentionExecutor:
         for offsets, launch in self._direct:
             ctypes.memmove(offsets, off.ctypes.data, off.nbytes)
             launch()
-        self._partials_due = True
+        self._leaves(self._graph_kept)
 
     def _update_staging_buffers(self, kv_offsets: np.ndarray):
         off, newest = self._checked_offsets(kv_offsets)
@@ -502,11 +523,12 @@ class DecodeAttentionExecutor:
         self._require_open()
         if self._graph_exec is not None:
             self.hip.graph_launch(self._graph_exec if self._on_route else self._plain_graph_exec)
-            self._partials_due = self._on_route and self._kept_names is not None
+            self._leaves(self._graph_kept if self._on_route else None)
         else:
-            self.hip.programmatic_launch = self.programmatic
+            self.hip.programmatic_launch, self._kept_names = self.programmatic, None
             try:
-                self._record_all()
+                self._record_all(one_launch=self._serves_one_launch())
+                self._leaves(self._kept_names)
             finally:
                 self.hip.programmatic_launch = False
 
@@ -538,7 +560,7 @@ class DecodeAttentionExecutor:
             # staging, graph, wait and the copy of the outputs, in one call
             done = self.hip.host_step(self._host_step, self._io_graph_exec if self._on_route else self._plain_io_graph_exec,
                                       off.ctypes.data, qh.ctypes.data, out.ctypes.data)
-            self._partials_due = self._on_route and self._kept_names is not None
+            self._leaves(self._io_kept if self._on_route else None)
             if not done:                              # the status word travelled with the outputs
                 self.dispatcher_check()
                 return self._output_array(nbytes)

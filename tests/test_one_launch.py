@@ -93,12 +93,6 @@ def test_what_goes_to_one_launch(built_library):
     assert not pays(28, (36, 2, 128), 1, 4096) and not pays(28, (18, 2, 256), 1, 4096) and not pays(28, (12, 2, 128), 1025, 64)
 
 
-@pytest.mark.parametrize("option", [dict(lean=(4, 1)), dict(compat=True), dict(strict_empty_splits=True), dict(emit_state=True), dict(num_splits=8)])
-def test_one_launch_refuses_what_it_would_drop(option):
-    with pytest.raises((CudaSafetyError, AttributeError)):
-        DecodeAttentionExecutor(None, None, {}, 1, 256, 4, one_launch=True, **option)
-
-
 class HostOnly(FakeRuntime, FakeHip):
     """A runtime whose launches are names in a list: nothing is dereferenced but pinned memory."""
     step_plan, programmatic_launch = staticmethod(step_plan), False
@@ -139,6 +133,26 @@ def host_only(B=1, S=4096, L=4, heads=(12, 2, 128), **kw):
     rt = HostOnly()
     meta = {"attention.head_count": heads[0], "attention.head_count_kv": heads[1], "attention.key_length": heads[2]}
     return DecodeAttentionExecutor(rt, FakeCodegen(), meta, B, S, L, **kw), rt
+
+
+@pytest.mark.parametrize("option", [dict(lean=(4, 1)), dict(lean=(0, 0)), dict(compat=True), dict(strict_empty_splits=True), dict(emit_state=True),
+                                    dict(num_splits=8), dict(use_graph=False), dict(fused_combine=True), dict(balanced=True), dict(wide=False),
+                                    dict(variant="full"), dict(min_chunk=64), dict(tensor_maps=False), dict(prefetch_next_layer=False)], ids=str)
+def test_one_launch_refuses_what_it_would_drop(built_library, option):
+    with pytest.raises(CudaSafetyError, match="one launch for all layers"):
+        host_only(one_launch=True, **option)
+    for fine in (dict(one_launch=True), option if "lean" not in option else dict(lean=(0, 0)), dict(one_launch=False, **option)):
+        ex, rt = host_only(**fine)                                     # by itself neither is
+        ex.execute_decode_batch(np.array([100], dtype=np.int32), read_output=False)
+        assert (rt.launched() == ["vteb_decode_step_d128_kernel"]) == (fine == dict(one_launch=True))
+
+
+@pytest.mark.parametrize("late", [dict(rope="separate"), dict(per_layer_hook=lambda layer: 0), dict(n_kv_buffers=2, with_append=True)], ids=str)
+def test_one_launch_refuses_what_it_cannot_keep_in_order(built_library, late):
+    ex, rt = host_only(one_launch=True, **late)
+    with pytest.raises(CudaSafetyError, match="one launch for all layers"):
+        ex.build_decode_graph()
+    assert rt.launched() == []
 
 
 def test_nothing_is_launched_after_cleanup(built_library):

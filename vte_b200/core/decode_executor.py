@@ -65,6 +65,13 @@ class DecodeAttentionExecutor:
         self.hip = hip
         if lean is not None and lean[0] and (compat or strict_empty_splits or emit_state or fused_combine):
             raise CudaSafetyError("a route of lean_route.py has no compat kernels, empty-split partials, shard states or fused combine")
+        # nothing that the caller has asked for ties the step to the dispatcher's own launches
+        open_layout = not (num_splits or compat or strict_empty_splits or emit_state or fused_combine or balanced is not None or
+                           wide is not None) and (fixed_chunk_size is None and min_chunk is None and variant == "auto" and
+                                                  tensor_maps and prefetch_next_layer)
+        if one_launch and (lean is not None or not open_layout or not use_graph):
+            raise CudaSafetyError("one launch for all layers takes no split layout, partials, shard states or shapes of the caller's, "
+                                  "and no step without a graph")
         # rope: "off" = Q and K arrive rotated; "separate" = the reference's standalone rotation
         # launch runs before the append (rotating the projections in place); "fused" = the append
         # rotates K and the split kernel rotates Q.  Either way the step includes the append.
@@ -130,15 +137,10 @@ class DecodeAttentionExecutor:
 
         # lean: (CTAs per (sequence, KV head), kind) of a route of lean_route.py; (0, 0) never, None where one pays and
         # the caller has asked for nothing that the dispatcher's own launches have and these have not.
-        open_layout = not (num_splits or compat or strict_empty_splits or emit_state or fused_combine or balanced is not None or
-                           wide is not None) and (fixed_chunk_size is None and min_chunk is None and variant == "auto" and
-                                                  tensor_maps and prefetch_next_layer)
         self._lean = lean if lean is not None else None if open_layout else (0, 0)
         self._route, self._forced_route = None, lean is not None
         # one_launch: the whole step in one launch over all layers (step_route.py); None where it may and pays, False: a launch
         # list per layer, in which a layer starts when the one in front of it is done, True: refused where it may not
-        if one_launch and (lean is not None or not open_layout):
-            raise CudaSafetyError("one launch for all layers takes no split layout, partials, shard states or shapes of the caller's")
         self._one_launch = one_launch if one_launch is not None else None if lean is None and open_layout else False
         self._step, self._direct, self._host_step = None, [], None
         # where lengths can make the dispatcher's launches the shorter ones: a step of those is captured beside the route's, and

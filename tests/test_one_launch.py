@@ -118,6 +118,8 @@ class HostOnly(FakeRuntime, FakeHip):
     def graph_launch(self, graph): self.log += graph
     def prepare_launch(self, *launch): return lambda: self.log.append(launch[:5])
     def host_step(self, step, graph, offsets, q, out):
+        if not all(0 <= x < step.capacity for x in (ctypes.c_int * step.batch).from_address(offsets)):
+            raise CudaSafetyError("kv_offsets out of range")
         self.log += graph
         return True
     def kv_tensor_map(self, ptr, n_rows, row_halves, box_rows, box_cols=0):
@@ -228,6 +230,22 @@ def test_a_step_is_captured_for_the_mapping_of_its_time(built_library, one):
     hooked, ex.per_layer_hook = [], lambda layer: hooked.append(layer)
     ex.execute_decode_batch(off, q)
     assert hooked == [0, 1, 2, 3] and not ex._partials_due
+
+
+def test_a_refused_step_picks_no_launches(built_library):
+    """A long sequence of two captured steps, route and dispatcher's launches: offsets out of range leave the choice as it was."""
+    B, S, L = 32, 32768, 2
+    ex, rt = host_only(B, S, L, one_launch=False)
+    q, none, far = np.zeros((L, B, 12, 128), dtype=np.float16), np.zeros(B, dtype=np.int32), np.array([S] + [0] * (B - 1), dtype=np.int32)
+    ex.build_decode_graph()
+    ex.build_io_graph()
+    assert ex._plain_io_graph_exec is not None
+    ex.execute_decode_batch(none, read_output=False)
+    before = ex._on_route, ex.route_name, ex.kernel_launches_per_step
+    for call in (dict(q_host=q), dict(read_output=False)):
+        with pytest.raises(CudaSafetyError):
+            ex.execute_decode_batch(far, **call)
+        assert (ex._on_route, ex.route_name, ex.kernel_launches_per_step) == before
 
 
 def kernel_source():

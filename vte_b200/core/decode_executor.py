@@ -552,8 +552,8 @@ class DecodeAttentionExecutor:
             if qh.nbytes != self.L * self.q_bytes:
                 raise CudaSafetyError("q_host must be [L, B, Hq, D] fp16")
             self._wait_for_staging()
-            if self._plain_io_graph_exec is not None:
-                self._pick(off, int(off.max()))
+            if self._plain_io_graph_exec is not None:  # refused offsets pick nothing
+                self._pick(*self._checked_offsets(off))
             if self._host_step is None:
                 self._host_step = HostStep(self._stage_offsets.value, self._stage_q.value, self._stage_out.value, self._stage_out.value + self._out_tail + 4,
                                            self.L * self.q_bytes, nbytes, self.B, self.S)

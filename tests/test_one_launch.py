@@ -404,6 +404,43 @@ def test_infinite_values_stay_infinite(cuda_runtime, codegen, heads):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("heads,meta,B,way", [
+    ((12, 2, 128), {}, 2, dict(one_launch=True)), ((8, 4, 64), dict(rope_type=1), 2, dict(one_launch=True)),
+    ((8, 2, 256), dict(rope_type=2, rotary_dim=64), 2, dict(one_launch=True)), ((16, 2, 128), dict(rope_type=2, rotary_dim=64), 2, dict(one_launch=True)),
+    ((12, 2, 128), {}, 2, dict(lean=(8, 1))), ((8, 4, 64), dict(rope_type=1), 2, dict(lean=(4, 1))), ((8, 2, 256), {}, 2, dict(lean=(5, 2))),
+    ((8, 2, 256), dict(rope_type=2, rotary_dim=64), 1, dict(lean=(20, 0)))], ids=str)
+@pytest.mark.parametrize("rope", ["fused", "fused-append"])
+def test_infinite_values_stay_infinite_under_a_rotation(cuda_runtime, codegen, heads, meta, B, way, rope):
+    """The same where the kernel rotates Q itself, the newest row's V among the infinite ones."""
+    Hq, Hkv, D = heads
+    S, L = 500, 2
+    rng = np.random.default_rng(12)
+    f16 = lambda *s: rng.standard_normal(s, dtype=np.float32).astype(np.float16)
+    ex = executor(cuda_runtime, codegen, heads, B, S, L, rope=rope, meta=meta, **{"one_launch": None, **way})
+    rope_type, width = meta.get("rope_type", 0), meta.get("rotary_dim", D)
+    try:
+        off = np.array([S - 1, 40], dtype=np.int32)[:B]
+        q, k, v, kn, vn = f16(B, Hq, D), f16(B, S, Hkv, D), f16(B, S, Hkv, D), f16(B, Hkv, D), f16(B, Hkv, D)
+        v[0, 17, 0, 3], v[0, 400, 0, 5], v[0, :400:7, Hkv - 1, 9] = np.inf, -np.inf, np.inf
+        vn[0, 0, 40], vn[B - 1, Hkv - 1, D - 1] = np.inf, -np.inf
+        for l in range(L):
+            ex.upload_layer(l, q, k, v)
+            ex.upload_new_kv(l, kn, vn)
+        out = ex.execute_decode_batch(off)
+        assert ex.route_name is not None
+        q, kn = orc.rope_step(q, kn, *orc.rope_tables(S, width, 1e6), off, rope_type, width)
+        orc.kv_cache_append(kn, vn, k, v, off)
+        ref = orc.decode_attention(q, k, v, off)
+        fine = np.isfinite(ref)
+        assert np.isposinf(ref).any() and np.isneginf(ref).any()
+        for l in range(L):
+            assert np.array_equal(np.isposinf(out[l]), np.isposinf(ref)) and np.array_equal(np.isneginf(out[l]), np.isneginf(ref))
+            assert np.linalg.norm(out[l][fine] - ref[fine]) <= 2e-5 * np.linalg.norm(ref[fine])
+    finally:
+        ex.cleanup()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("kw", [dict(with_append=True), dict(rope="fused-append"), {}], ids=str)
 def test_partials_after_one_launch_and_many_layers(cuda_runtime, codegen, kw):
     """70 layers are two launches; the partials of the last one are those of a launch list per layer, bit for bit."""

@@ -413,13 +413,26 @@ __device__ __forceinline__ void softmax_pv_t(ConsumerStateT<MT>& st, const float
 // kernels give (kFresh).  An infinite V times a zero part of P is NaN where its product with the whole of P is infinite:
 // in a masked row, as the low part of a probability that fp16 holds exactly, or where the two parts differ in sign.  A
 // warp whose sums hold a NaN at the end of an item walks its blocks again, straight from the caches, and rewrites o in
-// its exchange rows (`n_rows` rows of `pitch` floats); m, `m_pitch` floats apart, and l stand.  `q`: the rows' queries;
+// its exchange rows (`n_rows` rows of `pitch` floats); m, `m_pitch` floats apart, and l stand.  `q(r, d)`: the rows' queries;
 // `k`, `v`: the KV head's row 0, rows `stride` halves apart; blocks from position `first` on, `step` apart, below `end`;
 // column c at c ^ `swizzle` (a multiple of 8 below 32).
 // Checked once an item, eight sequences of sixteen heads per KV head, 8 layers: 163.4 -> 164.8 us; a check of every
 // block's products took 170.4.
-template <int D>
-__device__ __noinline__ void redo_rows_fp32(float* rows, int n_rows, int pitch, const float* maxima, int m_pitch, const __half* q,
+template <int D> struct QueryRows {                                   // in memory, as the products took them
+    const __half* q;
+    __device__ __forceinline__ float operator()(int r, int d) const { return __half2float(q[r * D + d]); }
+};
+template <int D> struct QueryFragments {                              // in shared memory, rotated where the kernel rotates (lean_decode.cuh)
+    uint32_t words;
+    static __device__ __forceinline__ int row(int r) { return (r >> 3) * (D * 4) + (r & 7) * 16; }
+    __device__ __forceinline__ float operator()(int r, int d) const {
+        __half_raw x;
+        asm("ld.shared.b16 %0, [%1];" : "=h"(x.x) : "r"(words + (row(r) + (d >> 5) * 128 + ((d & 7) >> 1) * 4 + ((d >> 3) & 3)) * 4 + (d & 1) * 2));
+        return __half2float(__half(x));
+    }
+};
+template <int D, class Queries>
+__device__ __noinline__ void redo_rows_fp32(float* rows, int n_rows, int pitch, const float* maxima, int m_pitch, const Queries q,
                                             const __half* k, const __half* v, long long stride, int first, int end, int step, float scale2, int swizzle = 0) {
     const int lane = threadIdx.x & 31;
     __syncwarp();
@@ -433,7 +446,7 @@ __device__ __noinline__ void redo_rows_fp32(float* rows, int n_rows, int pitch, 
                 float x = 0.f;
 #pragma unroll
                 for (int c = 0; c < D / 32; ++c)
-                    x = fmaf(__half2float(q[r * D + c * 32 + lane]), __half2float(k[j * stride + c * 32 + lane]), x);
+                    x = fmaf(q(r, c * 32 + lane), __half2float(k[j * stride + c * 32 + lane]), x);
 #pragma unroll
                 for (int off = 16; off > 0; off >>= 1) x += __shfl_xor_sync(0xffffffffu, x, off);
                 const float p = fast_exp2(x * scale2 - m);

@@ -381,6 +381,14 @@ __device__ __forceinline__ void lean_softmax_pv(ConsumerStateT<D / 16> (&st)[NV]
     }
 }
 
+// Q as redo_rows_fp32 takes it: the fragments at their place in shared memory, with no register spent on it.
+template <int D> struct LeanQueries {
+    __device__ __forceinline__ float operator()(int r, int d) const {
+        extern __shared__ __align__(128) unsigned char smem_raw[];
+        return QueryFragments<D>{smem_u32(smem_raw) + kLeanCtrlBytes}(r, d);
+    }
+};
+
 // D: head width; NV: runs of eight query heads a warp serves; CW: warps.
 template <int D, int NV, int CW, bool kFresh, bool kCluster>
 __device__ __forceinline__ void lean_body(const LeanArgs& a)
@@ -605,9 +613,9 @@ __device__ __forceinline__ void lean_body(const LeanArgs& a)
         }
     if constexpr (kFresh) {
         const float all = (probe[0] + probe[1]) + (probe[2] + probe[3]);
-        if (__any_sync(0xffffffffu, all != all) && !rotate)
-            redo_rows_fp32<D>(mine, group, PITCH, mine + D + 4, PITCH, a.q + ((long long)b * a.num_q_heads + (long long)kv_head * group) * D, a.k_cache + base,
-                              a.v_cache + base, pos_stride, start + warp * kBlockPos, end, CW * kBlockPos, scale2);
+        if (__any_sync(0xffffffffu, all != all))
+            redo_rows_fp32<D>(mine, group, PITCH, mine + D + 4, PITCH, LeanQueries<D>{}, a.k_cache + (long long)b * a.kv_batch_stride + (long long)kv_head * D,
+                              a.v_cache + (long long)b * a.kv_batch_stride + (long long)kv_head * D, pos_stride, start + warp * kBlockPos, end, CW * kBlockPos, scale2);
     }
     __syncthreads();
 

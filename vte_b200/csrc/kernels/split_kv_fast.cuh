@@ -967,7 +967,7 @@ __device__ __forceinline__ void fast_partial_body(const FastArgs& a)
                 if (!__any_sync(0xffffffffu, nan)) return false;
                 const long long kv0 = (long long)item_b * a.kv_batch_stride + (long long)(item_hgroup * plan.hg + kv_hh) * D;
                 redo_rows_fp32<D>(merge + (size_t)warp * vgroup * pitch, vgroup, pitch, merge + (size_t)warp * vgroup * pitch + D + 4, pitch,
-                                  a.q + ((long long)item_b * a.num_q_heads + (long long)(item_hgroup * vhg + hh) * vgroup) * D,
+                                  QueryRows<D>{a.q + ((long long)item_b * a.num_q_heads + (long long)(item_hgroup * vhg + hh) * vgroup) * D},
                                   a.k_cache + kv0, a.v_cache + kv0, (long long)a.num_kv_heads * D, item_first, item_end,
                                   plan.wph * kBlockPos, scale2);
                 return true;

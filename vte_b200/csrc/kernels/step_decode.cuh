@@ -436,12 +436,12 @@ __device__ __forceinline__ void step_body(const StepArgs& a)
                     }
                 }
             const float all = (probe[0] + probe[1]) + (probe[2] + probe[3]);
-            if (__any_sync(0xffffffffu, all != all) && a.rope_type < 0) {
+            if (__any_sync(0xffffffffu, all != all)) {
                 const int head_at = run.h * hg + kvh;
 #pragma unroll 1
                 for (int r = 0; r < group; ++r)
                     redo_rows_fp32<D>(state_row(own, slot_k, slot_v, r), 1, D, &stats[warp * NV * 8 + r].x, 4,
-                                      L.q + ((long long)run.b * a.num_q_heads + head_at * group + r) * D, L.k_cache + (long long)run.b * a.kv_batch_stride + head_at * D,
+                                      QueryFragments<D>{smem_u32(q_store + kvh * q_words + QueryFragments<D>::row(r))}, L.k_cache + (long long)run.b * a.kv_batch_stride + head_at * D,
                                       L.v_cache + (long long)run.b * a.kv_batch_stride + head_at * D, pos_stride, first, min((s1 - run.start) * tile, len), TEAMS * tile, scale2, ((r >> 1) & 3) << 3);
             }
         } else if (lane < group) stats[warp * NV * 8 + lane] = make_float4(kNeutralM, 0.f, kNeutralM, 0.f);

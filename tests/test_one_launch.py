@@ -322,6 +322,31 @@ def test_one_launch_matches_the_oracle(cuda_runtime, codegen, heads, append, lay
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("heads", HEADS)
+@pytest.mark.parametrize("layers,lengths", [(1, [17000]), (1, [2100]), (2, [9000])], ids=str)
+def test_cut_runs_are_merged_once_or_twice(cuda_runtime, codegen, heads, layers, lengths):
+    """Either side of eight tiles a CTA with no more states of a run than one merge takes: above it a run lies in up to 148 shares, whose
+    states are merged in two steps.  fp32 sums: 2e-5 of the result's norm."""
+    Hq, Hkv, D = heads
+    B, S = len(lengths), max(lengths)
+    rng = np.random.default_rng(21)
+    f16 = lambda *s: rng.standard_normal(s, dtype=np.float32).astype(np.float16)
+    ex = executor(cuda_runtime, codegen, heads, B, S, layers)
+    try:
+        data = [(f16(B, Hq, D), f16(B, S, Hkv, D), f16(B, S, Hkv, D)) for _ in range(layers)]
+        for l in range(layers):
+            ex.upload_layer(l, *data[l])
+        off = np.array(lengths, dtype=np.int32) - 1
+        for _ in range(2):
+            out = ex.execute_decode_batch(off)
+            for l in range(layers):
+                ref = orc.decode_attention(*data[l], off)
+                assert np.linalg.norm(out[l] - ref) <= 2e-5 * np.linalg.norm(ref)
+    finally:
+        ex.cleanup()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("heads,meta", [((12, 2, 128), {}), ((8, 4, 64), dict(rope_type=1)), ((8, 2, 256), dict(rope_type=2, rotary_dim=64)),
                                         ((8, 2, 256), {}), ((16, 2, 128), dict(rope_type=2, rotary_dim=128))])
 @pytest.mark.parametrize("rope", ["fused", "fused-append"])

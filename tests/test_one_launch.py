@@ -93,6 +93,16 @@ def test_what_goes_to_one_launch(built_library):
     assert not pays(28, (36, 2, 128), 1, 4096) and not pays(28, (18, 2, 256), 1, 4096) and not pays(28, (12, 2, 128), 1025, 64)
 
 
+def test_few_layers_go_to_one_launch_only_where_none_of_their_lengths_loses_much(built_library):
+    """Choices are made for the caches' room, before lengths are known: two or three sequences of three layers, and one of
+    256-wide heads with two, were up to a seventh slower than the launches per layer for some or all lengths."""
+    pays = lambda layers, *a: one_launch_pays(a_route(1, True, *a)[0].d, layers)
+    assert not pays(2, (8, 2, 256), 1, 262144) and pays(2, (8, 2, 256), 16, 32768) and pays(3, (8, 2, 256), 1, 262144)
+    for heads in ((8, 2, 256), (32, 8, 64), (12, 2, 128)):
+        assert not pays(3, heads, 2, 4096) and not pays(3, heads, 3, 4096) and pays(3, heads, 4, 4096)
+    assert pays(4, (32, 2, 128), 1, 8192) and pays(4, (8, 2, 256), 2, 4096)
+
+
 class HostOnly(FakeRuntime, FakeHip):
     """A runtime whose launches are names in a list: nothing is dereferenced but pinned memory."""
     step_plan, programmatic_launch = staticmethod(step_plan), False

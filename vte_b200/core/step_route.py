@@ -111,22 +111,32 @@ class StepRoute:
 
 
 ONE_LAUNCH_BYTES = 600e6            # K and V of a step from which it pays with two layers too
+# Share of a cache's room that sizes are judged by where lengths are not known yet: what the caches of the measured steps hold, one
+# sequence and a batch of unequal ones.  Only `large` below depends on it, not whether four layers and more are one launch.
+IN_USE_ALONE, IN_USE_BATCH = 0.72, 0.5
 
 
 def one_launch_pays(d, layers: int) -> bool:
     """Whether a step of `layers` layers goes to one launch rather than to a launch list per layer, by sizes that do not change.
 
-    From four layers on it always does.  us a step behind a flushed L2, append included, launches per layer / one launch, over 7
-    head geometries, 1 to 64 sequences of 64 to 131,072 positions: six layers 1.02 to 3.5 times as fast (32 heads on 2 of 128, 64
-    sequences of 4,096: 275 / 270; one of 131,072 of 8 heads on 2 of 256: 245 / 220); three layers of a batch 0.99 to 2.2
-    (groups of more than eight heads from 0.85); three layers of one sequence 0.74 to 2; two layers 0.66 to 1.8, from 600 MB on
-    1.0 to 1.1.  One layer has nothing to share out that the launches per layer do not: 0.5 to 1.06.  Large steps of two or three
-    layers of 64-wide heads gain nothing for sure: their arithmetic keeps up with HBM at full clocks only (64 ragged sequences of 32
-    heads on 8, two layers: 345 / 338 us on one machine, 353 / 364 on another)."""
+    us a step behind a flushed L2, append included, launches per layer / one launch, over 7 head geometries, 1 to 64 sequences, room for
+    300 to 262,144 positions, 1 to 100 % of it in use; 448 sizes for each count of layers (252 for six), fill by fill:
+      six 1.10 to 5.0 times as fast (mean 1.99), five 0.96 to 3.8 (1.58), four 0.96 to 3.3 (1.44): always.  Below 1 are 2 % of four and 1 % of
+        five layers: 64 sequences of 300 of 32 heads on 2 of 128 half full 51 / 53, 64 of 8,192 of 8 heads on 8 half full 484 / 501;
+      three 0.80 to 3.0 (1.26): batches of four and more with groups of up to eight, 0.91 to 3.0 (64 of 300 of 12 heads on 2 half full
+        21 / 23, 16 of 32,768 of 8 on 8 1 % full 33 / 35); two or three sequences 0.86, one 0.80, wider groups 0.80;
+      two 0.62 to 2.6 (1.07): not, but for large steps of heads wider than 64: 0.89 to 1.5 (8 heads on 8, 16 of 32,768 1 % full 24 / 26,
+        half full 273 / 260), one sequence of 256-wide heads 0.93 to 1.0 and so not.
+    One layer has nothing to share out that the launches per layer do not: 0.5 to 1.06.  Large steps of two or three layers of 64-wide
+    heads gain nothing for sure: their arithmetic keeps up with HBM at full clocks only (64 ragged sequences of 32 heads on 8, two
+    layers: 345 / 338 us on one machine, 353 / 364 on another)."""
     plan = d.hip.step_plan(d.num_q_heads, d.num_kv_heads, d.head_dim, d.batch_size, d.num_sms)
     if not plan.ok or layers < 2:
         return False
     if layers >= 4:
         return True
-    large = layers * d.batch_size * d.context_length * d.num_kv_heads * d.head_dim * 4 * (0.72 if d.batch_size == 1 else 0.5) >= ONE_LAUNCH_BYTES
-    return not large and layers == 3 and d.batch_size > 1 and d.num_q_heads <= 8 * d.num_kv_heads or large and d.head_dim > 64
+    in_use = IN_USE_ALONE if d.batch_size == 1 else IN_USE_BATCH
+    large = layers * d.batch_size * d.context_length * d.num_kv_heads * d.head_dim * 4 * in_use >= ONE_LAUNCH_BYTES
+    if large:
+        return d.head_dim > 64 and not (layers == 2 and d.batch_size == 1 and d.head_dim == 256)
+    return layers == 3 and d.batch_size >= 4 and d.num_q_heads <= 8 * d.num_kv_heads

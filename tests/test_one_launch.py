@@ -197,6 +197,34 @@ def test_nothing_is_launched_after_cleanup(built_library):
     assert rt.launched() == []
 
 
+@pytest.mark.parametrize("tag", ["attn_step_boards", "attn_partials_source"])
+@pytest.mark.parametrize("one", [None, True])
+def test_an_allocator_without_room_keeps_the_launches_per_layer(built_library, tag, one):
+    """Whichever of the two blocks of a one-launch step finds no room: what the other took is given back."""
+    rt = HostOnly()
+    allocator = SlabAllocator(rt, 180 << 30, requested_pool_size=1 << 30)
+    allocator.initialize()
+    allocate, taken, refused = allocator.allocate, [], []
+
+    def without(size, name, region):
+        if name == tag:
+            refused.append(name)
+            raise CudaSafetyError("slab exhausted")
+        taken.append(allocate(size, name, region))
+        return taken[-1]
+    allocator.allocate = without
+    meta = {"attention.head_count": 12, "attention.head_count_kv": 2, "attention.key_length": 128}
+    ex = DecodeAttentionExecutor(rt, FakeCodegen(), meta, 1, 4096, 4, allocator=allocator, one_launch=one)
+    if one:
+        with pytest.raises(CudaSafetyError, match="exhausted"):
+            ex.build_decode_graph()
+        return
+    ex.execute_decode_batch(np.array([100], dtype=np.int32), read_output=False)
+    assert refused and ex._step is None and not ex._direct
+    assert not any(n.startswith("vteb_decode_step") for n in rt.launched())
+    assert [b.tag for b in taken if not b.in_use] == ([] if tag == "attn_step_boards" else ["attn_step_boards"])
+
+
 @pytest.mark.parametrize("spare", [0, 1, 100, 4096])
 def test_tiles_end_where_the_last_sequence_s_room_does(built_library, spare):
     """With a stride longer than the cache, the rows behind the last sequence may be anybody's: the maps end in front of them."""
@@ -327,6 +355,108 @@ def test_one_launch_matches_the_oracle(cuda_runtime, codegen, heads, append, lay
                     assert all(np.array_equal(x.view(np.uint16), y[b].view(np.uint16)) for x, y in zip(got, (k, v)))
                 for b in range(B):
                     k[b, off[b] + 1:], v[b, off[b] + 1:] = 0.5, 0.25
+    finally:
+        ex.cleanup()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("heads", [(12, 2, 128), (32, 8, 64), (8, 2, 256), (22, 2, 128)])
+@pytest.mark.parametrize("B", [31, 32, 33, 64, 65, 130])
+def test_batches_of_more_sequences_than_a_warp_has_lanes(cuda_runtime, codegen, heads, B):
+    """Lengths are added up 32 at a time; up to 64 offsets come with the launch, more from memory, through the captured step.  Several
+    steps queued without a wait, each with offsets of its own and its rows to append; then the last one's outputs."""
+    Hq, Hkv, D = heads
+    S, L, rng = 150, 4, np.random.default_rng(B)
+    f16 = lambda *s: rng.standard_normal(s, dtype=np.float32).astype(np.float16)
+    ex = executor(cuda_runtime, codegen, heads, B, S, L, with_append=True)
+    try:
+        q, kn, vn = f16(L, B, Hq, D), f16(L, B, Hkv, D), f16(L, B, Hkv, D)
+        caches = [(f16(B, S, Hkv, D), f16(B, S, Hkv, D)) for _ in range(L)]
+        for l in range(L):
+            ex.upload_layer(l, q[l], *caches[l])
+            ex.upload_new_kv(l, kn[l], vn[l])
+        first = rng.integers(0, S - 12, B).astype(np.int32)
+        first[[0, B - 1]] = 0, S - 13
+        for step in range(12):
+            ex.execute_decode_batch(first + step, read_output=False)
+        out = ex.execute_decode_batch(first + 12)
+        assert len(ex._direct) == (B <= 64) and ex.route_name[1] == 0
+        for l, (k, v) in enumerate(caches):
+            for step in range(13):
+                orc.kv_cache_append(kn[l], vn[l], k, v, first + step)
+            ref = orc.decode_attention(q[l], k, v, first + 12)
+            assert np.linalg.norm(out[l] - ref) <= 2e-5 * np.linalg.norm(ref)
+            for b in {0, 1, min(32, B - 1), B - 1}:
+                got = ex.download_cache_rows(l, b, S)
+                assert all(np.array_equal(x.view(np.uint16), y[b].view(np.uint16)) for x, y in zip(got, (k, v)))
+    finally:
+        ex.cleanup()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("heads", [(12, 2, 128), (32, 8, 64), (8, 2, 256), (22, 2, 128)])
+def test_a_stride_longer_than_the_cache(cuda_runtime, codegen, heads):
+    """Rows between one sequence's room and the next one's start, and behind the last one's, belong to others: neither counted nor touched."""
+    Hq, Hkv, D = heads
+    B, S, spare, L, rt = 3, 200, 7, 4, cuda_runtime
+    rows = (B - 1) * (S + spare) + S
+    rng = np.random.default_rng(4)
+    f16 = lambda *s: rng.standard_normal(s, dtype=np.float32).astype(np.float16)
+    ex, mine = executor(rt, codegen, heads, B, S, L, with_append=True), []
+    try:
+        off = np.array([S - 1, 100, S - 1], dtype=np.int32)
+        q, kn, vn, data = f16(L, B, Hq, D), f16(L, B, Hkv, D), f16(L, B, Hkv, D), []
+        ex.tensor_mapping['kv_batch_stride_elements'] = (S + spare) * Hkv * D
+        for l in range(L):
+            ex.upload_layer(l, q[l])
+            ex.upload_new_kv(l, kn[l], vn[l])
+            for name in ("k", "v"):
+                x = f16(rows, Hkv, D)
+                for b in range(B):
+                    x[b * (S + spare) + S:(b + 1) * (S + spare)] = np.inf
+                mine.append(rt.safe_malloc(x.nbytes, "kv cache"))
+                rt.safe_memcpy_host_to_device(mine[-1], x, "kv upload")
+                ex.tensor_mapping[f'blk.{l}.kv_cache.{name}'] = mine[-1].value
+                data.append(x)
+        out = ex.execute_decode_batch(off)
+        assert ex.kernel_launches_per_step == 1
+        for l in range(L):
+            per_seq = lambda x: np.stack([x[b * (S + spare):b * (S + spare) + S] for b in range(B)])
+            k, v = per_seq(data[2 * l]), per_seq(data[2 * l + 1])
+            orc.kv_cache_append(kn[l], vn[l], k, v, off)
+            ref = orc.decode_attention(q[l], k, v, off)
+            assert np.linalg.norm(out[l] - ref) <= 2e-5 * np.linalg.norm(ref)
+            for x, new, p in ((data[2 * l], kn[l], mine[2 * l]), (data[2 * l + 1], vn[l], mine[2 * l + 1])):
+                for b in range(B):
+                    x[b * (S + spare) + off[b]] = new[b]
+                got = np.empty_like(x)
+                rt.safe_memcpy_device_to_host(got, p, "kv rows for output check")
+                assert np.array_equal(got.view(np.uint16), x.view(np.uint16))
+    finally:
+        ex.cleanup()
+        for p in mine:
+            rt.safe_free(p, "kv cache")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("heads,hg", [((32, 8, 64), 1), ((32, 8, 64), 2), ((12, 2, 128), 2), ((8, 8, 128), 4), ((16, 8, 64), 4)])
+def test_heads_a_block_serves_at_once(cuda_runtime, codegen, heads, hg):
+    """Other counts of KV heads a block than the plan chooses by itself."""
+    Hq, Hkv, D = heads
+    off, rng = np.array([0, 333, 499], dtype=np.int32), np.random.default_rng(6)
+    f16 = lambda *s: rng.standard_normal(s, dtype=np.float32).astype(np.float16)
+    q, k, v = f16(3, Hq, D), f16(3, 500, Hkv, D), f16(3, 500, Hkv, D)
+    ex = executor(cuda_runtime, codegen, heads, 3, 500, 2)
+    try:
+        plan = cuda_runtime.step_plan
+        ex.hip = ex.dispatcher.hip = type("Forced", (), {"__getattr__": lambda self, name: getattr(cuda_runtime, name),
+                                                         "step_plan": staticmethod(lambda *a: plan(*a[:5], hg))})()
+        for l in range(2):
+            ex.upload_layer(l, q, k, v)
+        out = ex.execute_decode_batch(off)
+        assert ex._step.plan.hg == hg and ex.kernel_launches_per_step == 1
+        ref = orc.decode_attention(q, k, v, off)
+        assert all(np.linalg.norm(out[l] - ref) <= 2e-5 * np.linalg.norm(ref) for l in range(2))
     finally:
         ex.cleanup()
 

@@ -10,7 +10,7 @@ import pytest
 from oracle import attention_oracle as orc
 from tests.test_host_logic import FakeCodegen, FakeRuntime
 from tests.test_lean_routes import FakeHip
-from vte_b200.bridge.cuda_runtime import KvTensorMap, StepArgs, StepLayer, StepPlan, load_library
+from vte_b200.bridge.cuda_runtime import CudaRuntime, KvTensorMap, StepArgs, StepLayer, StepPlan, load_library
 from vte_b200.bridge.errors import CudaRuntimeError, CudaSafetyError
 from vte_b200.bridge.memory import SlabAllocator
 from vte_b200.core.decode_executor import DecodeAttentionExecutor
@@ -284,6 +284,23 @@ def test_a_refused_step_picks_no_launches(built_library):
         with pytest.raises(CudaSafetyError):
             ex.execute_decode_batch(far, **call)
         assert (ex._on_route, ex.route_name, ex.kernel_launches_per_step) == before
+
+
+def test_a_prepared_launch_is_refused_when_its_runtime_is_gone():
+    """As every other launch is: its function is unloaded and its stream destroyed by then, while another runtime keeps the library going."""
+    rt, launched = object.__new__(CudaRuntime), []
+    vars(rt).update(_initialized=True, _panic=False, _props={"shared_mem_per_block": 49152}, _smem_optin_set={}, _stream=ctypes.c_void_p(1),
+                    _lib=SimpleNamespace(vteb_launch=lambda *a: launched.append(a) or 0), _validate_launch=lambda *a: None)
+    launch = rt.prepare_launch(ctypes.c_void_p(0x1001), [ctypes.c_int(1)], (1, 1, 1), (32, 1, 1))
+    launch()
+    assert len(launched) == 1
+    rt._initialized = False
+    with pytest.raises(CudaSafetyError):
+        launch()
+    rt._initialized, rt._panic = True, True
+    with pytest.raises(CudaSafetyError, match="panic"):
+        launch()
+    assert len(launched) == 1
 
 
 def kernel_source():

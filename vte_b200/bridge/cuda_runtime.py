@@ -667,6 +667,7 @@ class CudaRuntime:
         rest = (ctypes.c_void_p(fval), *(ctypes.c_uint(int(x)) for x in (*grid, *block, shared_mem)), self._stream, arr, ctypes.c_uint(flags))
 
         def launch(_keep=keep):
+            self._require_init()                  # the function and the stream go with the runtime
             if self._panic:
                 raise CudaSafetyError("runtime is in panic state (a synchronize timed out); new launches are blocked")
             err = call(*rest)

@@ -20,7 +20,7 @@ from typing import Optional
 
 import numpy as np
 
-from ..bridge.cuda_runtime import HostStep
+from ..bridge.cuda_runtime import HostStep, StepArgs
 from ..bridge.errors import CudaSafetyError
 from ..bridge.memory import MemoryRegion, SlabAllocator
 from ..config import ENV_NO_PDL, env_flag
@@ -50,7 +50,7 @@ NOT_SIDE_BY_SIDE = "one launch for all layers: a layer reads or writes what anot
 class DecodeAttentionExecutor:
     _step, _one_launch, _direct, _closed = None, False, (), False
     _graph_kept = _io_kept = None
-    _recorded_step = False
+    _recorded_step = ()
 
     def __init__(self, hip, codegen, metadata: dict, batch_size: int, context_length: int, n_layers: int, *,
                  n_kv_buffers: Optional[int] = None, num_splits: Optional[int] = None, output_f32: bool = True,
@@ -266,16 +266,17 @@ class DecodeAttentionExecutor:
     def route_name(self):
         """(kernel, CTAs per (sequence, KV head)) where the last captured step did not take the dispatcher's launches, else None;
         (kernel, 0) where it is one launch."""
-        if self._step is not None and self._recorded_step:
+        if self._recorded_step:
             return self._step.name, 0
         return (self._route.name, self._route.parts) if self._route is not None and self._on_route else None
 
-    def _record_all(self, after_copy: bool = False, plain: bool = False, one_launch: bool = False, mirror: Optional[tuple] = None):
+    def _record_all(self, after_copy: bool = False, plain: bool = False, one_launch: Optional[list] = None, mirror: Optional[tuple] = None):
+        """`one_launch`: what the one launch of all layers takes from the mapping, where it serves."""
         n = 0
         programmatic = self.hip.programmatic_launch
-        self._recorded_step = one_launch
+        self._recorded_step = self._record_step(one_launch, mirror) if one_launch else ()
         if one_launch:
-            return self._record_step(mirror)
+            return len(self._recorded_step)
         # within a captured step of nothing but the layers' own launches, offsets and older rows do not change
         self.dispatcher.offsets_final = self.use_graph and self.per_layer_hook is None and self.launch_rewriter is None
         for l in range(self.L):
@@ -297,39 +298,42 @@ class DecodeAttentionExecutor:
                 n += int(self.per_layer_hook(l) or 0)
         return n
 
-    def _step_launches(self, mirror: Optional[tuple] = None) -> list:
-        return self._step.launches(self.tensor_mapping, self.offsets.ptr, self.B, (self._kept.ptr, self._kept.ptr + _round_up(self.q_bytes, 256)), mirror)
-
-    def _record_step(self, mirror: Optional[tuple] = None) -> int:
+    def _record_step(self, layers: list, mirror: Optional[tuple] = None) -> list:
         """Record the launches of a step without an order among its layers."""
-        launches = self._step_launches(mirror)
+        launches = self._step.launches(self.tensor_mapping, self.offsets.ptr, self.B, layers,
+                                       (self._kept.ptr, self._kept.ptr + _round_up(self.q_bytes, 256)), mirror)
         self._kept_names = dict(self.tensor_mapping)
         for launch in launches:
             self.hip.launch_kernel_recorded(*launch)
-        return len(launches)
+        return launches
 
-    def _serves_one_launch(self) -> bool:
-        """Whether a step that is recorded now may be the one launch: the mapping may be another than the one it was chosen with."""
+    def _serves_one_launch(self) -> Optional[list]:
+        """What the one launch takes from the mapping of this moment, which may be another than the one it was chosen with; None where
+        a step that is recorded now may not be one launch."""
         if self._step is None or self.per_layer_hook is not None or self.launch_rewriter is not None:
-            return False
-        serves = self._step.serves(self.tensor_mapping, self.offsets.ptr, self.B)
-        if self._one_launch and not serves:
+            return None
+        layers = self._step.resolve(self.tensor_mapping)
+        if self._step.serves(self.tensor_mapping, self.offsets.ptr, self.B, layers):
+            return layers
+        if self._one_launch:
             raise CudaSafetyError(NOT_SIDE_BY_SIDE)
-        return serves
+        return None
 
-    def _choose_route(self) -> bool:
-        """Before a step is captured: whether its layers' launches are the dispatcher's own or a route of lean_route.py.  True where
-        one launch for all of them has just been found to serve."""
+    def _choose_route(self) -> Optional[list]:
+        """Before a step is captured: whether its layers' launches are the dispatcher's own or a route of lean_route.py.  Where one
+        launch for all of them has just been found to serve, what it takes from the mapping."""
         d = self.dispatcher
         if (self._route is not None or self._step is not None or self._lean == (0, 0) and not self._one_launch or not self.use_graph or
                 self.per_layer_hook is not None or self.launch_rewriter is not None or not d.enabled or not hasattr(self.hip, 'lean_plan')):
             if self._one_launch and self._step is None:
                 raise CudaSafetyError("one launch for all layers needs a captured step without a hook or a rewriter")
-            return False
+            return None
         d._allocate_scratch()                         # and the work words
         append = self.with_append or d.fuse_append
-        if self._one_launch is not False and self._choose_one_launch(append):
-            return True
+        if self._one_launch is not False:
+            layers = self._choose_one_launch(append)
+            if layers:
+                return layers
         if self._lean is None:
             self._lean = choose_lean_route(d, append)
         if self._lean[0]:
@@ -341,26 +345,27 @@ class DecodeAttentionExecutor:
                 if self._forced_route:
                     raise
                 self._lean = (0, 0)                   # a caller's allocator with no room for it: the dispatcher's launches need none
-                return False
+                return None
             self._route = route
             if not self._forced_route:
                 self._route_pays_to = route.pays_up_to()
-        return False
+        return None
 
-    def _choose_one_launch(self, append: bool) -> bool:
+    def _choose_one_launch(self, append: bool) -> Optional[list]:
         """Takes one launch for the step where its layers may run side by side and that pays."""
         d, forced, blocks = self.dispatcher, bool(self._one_launch), []
         if self.rope == "separate" or not hasattr(self.hip, 'step_plan') or (not forced and not one_launch_pays(d, self.L)):
             if forced:
                 raise CudaSafetyError("one launch for all layers has no rotation launches")
-            return False
+            return None
         try:
             step = StepRoute(d, self.allocator, self.L, append)
             blocks.append(step.scratch)
             self._kept = self.allocator.allocate(_round_up(self.q_bytes, 256) + _round_up(4 * self.B, 256), "attn_partials_source",
                                                  MemoryRegion.SCRATCH)
             blocks.append(self._kept)
-            if not step.serves(self.tensor_mapping, self.offsets.ptr, self.B):
+            layers = step.resolve(self.tensor_mapping)
+            if not step.serves(self.tensor_mapping, self.offsets.ptr, self.B, layers):
                 raise CudaSafetyError(NOT_SIDE_BY_SIDE)
         except CudaSafetyError:
             if forced:
@@ -368,9 +373,9 @@ class DecodeAttentionExecutor:
             for block in blocks:
                 self.allocator.free(block)
             self._kept = None
-            return False
+            return None
         self._step = step
-        return True
+        return layers
 
     def _require_open(self, staging: bool = False):
         """A cleaned-up executor has no staging memory, and device memory only where the caller's allocator holds it."""
@@ -379,9 +384,9 @@ class DecodeAttentionExecutor:
 
     def build_decode_graph(self):
         """Capture all layers' launches once (hip_graph_executor.py:504-725)."""
-        self._require_open()
         if self._graph_exec is not None:
             return
+        self._require_open()
         self.hip.programmatic_launch = self.programmatic
         try:
             if not self.use_graph:
@@ -391,11 +396,12 @@ class DecodeAttentionExecutor:
                 return
             one = self._choose_route() or self._serves_one_launch()
             self._graph_exec, n, self._graph_kept = self._capture(lambda: self._record_all(one_launch=one))
+            self._direct = []
             if one and self.B <= STEP_OFFSETS:
-                self._direct = []
-                for fn, args, grid, block, smem in self._step_launches():
-                    args[0].offsets_here = 1
-                    self._direct.append((args[0].offsets, self.hip.prepare_launch(fn, args, grid, block, smem, self.programmatic)))
+                for fn, (captured,), grid, block, smem in self._recorded_step:
+                    args = StepArgs.from_buffer_copy(captured)
+                    args.offsets_here = 1
+                    self._direct.append((args.offsets, self.hip.prepare_launch(fn, [args], grid, block, smem, self.programmatic)))
             plain = n
             if self._route_pays_to < self.S:
                 self._plain_graph_exec, plain, _ = self._capture(lambda: self._record_all(plain=True))
@@ -429,9 +435,9 @@ class DecodeAttentionExecutor:
         copy nodes.  A step is then one graph launch instead of three copies and a launch (the
         reference stages its offsets with a separate copy before each launch,
         vte/core/hip_graph_executor.py:772-789)."""
-        self._require_open(staging=True)
         if self._io_graph_exec is not None or not self.use_graph:
             return
+        self._require_open(staging=True)
         if self._copy_fn is None:                         # before the capture begins
             self._copy_fn = self.codegen.load_kernel_safe(self.hip, 'decode_attention', self.hip.get_gpu_architecture(),
                                                           'vteb_stage_copy_kernel')[1]
@@ -454,7 +460,7 @@ class DecodeAttentionExecutor:
             return None
         return self._stage_out.value, self._stage_out.value + self._out_tail + 4
 
-    def _record_io(self, plain: bool = False, one_launch: bool = False):
+    def _record_io(self, plain: bool = False, one_launch: Optional[list] = None):
         if max(self._q_tail, self._out_tail) <= STAGE_COPY_MAX_BYTES:
             mirror = self._mirror() if one_launch else None
             self._stage_copy(self.q_all.ptr, self._stage_q.value, self._q_tail + 4 * self.B, first=True)
@@ -522,7 +528,8 @@ class DecodeAttentionExecutor:
 
     def launch_step(self):
         """Enqueue one decode step (no host synchronisation)."""
-        self._require_open()
+        if self._closed:
+            self._require_open()
         if self._graph_exec is not None:
             self.hip.graph_launch(self._graph_exec if self._on_route else self._plain_graph_exec)
             self._leaves(self._graph_kept if self._on_route else None)
@@ -539,7 +546,8 @@ class DecodeAttentionExecutor:
         """One decode step end to end: stage offsets (and, when given, every layer's
         Q [L,B,Hq,D] fp16) host -> device, replay the graph, read every layer's
         output back.  Returns [L,B,Hq,D] (fp32 or fp16)."""
-        self._require_open(staging=True)
+        if self._closed:
+            self._require_open(staging=True)
         self.build_decode_graph()
         nbytes = self.L * self.out_bytes
         if q_host is not None and read_output and self.use_graph:

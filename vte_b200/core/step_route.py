@@ -42,7 +42,11 @@ class StepRoute:
             raise CudaSafetyError(f"layer {layer}: the new K / V rows could not be resolved (null)")
         return (ptr('q_proj.output'), *d._resolve_kv_cache_ptrs(layer, mapping), *new, ptr('attention.output'))
 
-    def serves(self, mapping: dict, kv_offset_ptr: int, batch: int) -> bool:
+    def resolve(self, mapping: dict) -> list:
+        """What every layer reads and writes."""
+        return [self._layer(layer, mapping) for layer in range(self.layers)]
+
+    def serves(self, mapping: dict, kv_offset_ptr: int, batch: int, layers: list | None = None) -> bool:
         """Whether the layers of a mapping may run side by side: pointers that 16-byte accesses can take, and nothing that
         one part of the step writes overlaps with anything else in it."""
         d = self.d
@@ -55,8 +59,7 @@ class StepRoute:
         if stride % (row // 2) or stride < d.context_length * (row // 2):     # the caches are read as whole position rows
             return False
         writes = 1
-        for layer in range(self.layers):
-            pointers = self._layer(layer, mapping)
+        for pointers in self.resolve(mapping) if layers is None else layers:
             d._validate(batch, *(pointers[i] for i in (0, 1, 2, 5)), kv_offset_ptr, stride)
             if any(p % 16 for p in pointers):
                 return False
@@ -74,8 +77,8 @@ class StepRoute:
             end_read, end_written = max(end_read, hi), max(end_written, hi if w else 0)
         return True
 
-    def launches(self, mapping: dict, kv_offset_ptr: int, batch: int, keep: tuple, host: tuple | None = None):
-        """`keep`: where the last layer leaves a copy of its Q and of the offsets, from which its partials can be had.  `host`:
+    def launches(self, mapping: dict, kv_offset_ptr: int, batch: int, layers: list, keep: tuple, host: tuple | None = None):
+        """`layers`: what `resolve` found.  `keep`: where the last layer leaves a copy of its Q and of the offsets, from which its partials can be had.  `host`:
         pinned memory (outputs, one layer's after another's, and status word) that the kernel stores to as well."""
         d = self.d
         attention_scale = d.metadata.get('attention_scale')
@@ -88,7 +91,7 @@ class StepRoute:
             n = min(self.plan.max_layers, self.layers - first)
             a = StepArgs()
             for i in range(n):
-                q, k_cache, v_cache, k_new, v_new, output = self._layer(first + i, mapping)
+                q, k_cache, v_cache, k_new, v_new, output = layers[first + i]
                 maps = (d.hip.kv_tensor_map(p, n_rows, row, self.plan.tile, self.plan.hg * d.head_dim // 64) for p in (k_cache, v_cache))
                 a.layer[i] = StepLayer(*maps, q, k_cache, v_cache, k_new, v_new, output)
                 if host:

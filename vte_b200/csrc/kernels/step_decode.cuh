@@ -10,16 +10,19 @@
 // when it carries it, without a fence), and the last merges them, bounded, in their order; it waits for CTAs with lower numbers only.
 //
 // What bounds it: HBM, and about 9 us of launch, start (2), first tile (1.3), merges (1.3 a run) and finish (2 to 2.5).  us a step,
-// launches per layer / one launch, 12 heads on 2 KV heads of 128, one sequence: 28 layers of 1,531 positions 104 / 15.5, of 11,003
-// 182 / 54, four of a million 649 / 604 (7.1 TB/s); 8 ragged sequences of 32 heads on 8 of 64, ten layers 246 / 193.  Nine to
-// sixteen query heads per KV head are bound by block arithmetic: an SM takes 43 B/ns, its share of HBM is 45.  What was measured:
+// launches per layer / one launch, in turn on one machine, 12 heads on 2 KV heads of 128, one sequence: 28 layers of 1,531 positions
+// 105 / 15.9, of 11,003 183 / 55.5, four of a million 654 / 634 (6.8 TB/s); 8 ragged sequences of 32 heads on 8 of 64, ten layers 254 / 208; eight
+// of 32 on 2 of 128, eight layers 90 / 47; one of 24,001, 256-wide, eight layers 115 / 72.  Machines differ by 5 % where HBM is the
+// bound (the million 602 to 637, the eight ragged ones 192 to 209).  Nine to sixteen query heads per KV head are bound by block
+// arithmetic: an SM takes 43 B/ns, its share of HBM is 45.  What was measured:
 //   128 KB of tiles in flight an SM, not 192: with more, the SMs of the two largest clusters of SMs get 15 % less than the others
 //     and every share waits for them (a million positions 676 / 614, 28 layers of 32,768 174 / 164);
 //   one copy a tile in place of one per 64 channels: the warp that fetches was the limit (an SM alone, 64-wide heads 52 / 58
 //     B/ns, 256-wide 59 / 70); 16-byte asynchronous copies by every warp 5.8 TB/s on 64 ragged sequences of 64-wide heads (6.5);
 //   64-wide heads: twelve warps (8: 40 B/ns an SM, below its share of HBM), four heads a CTA (rows of 512 bytes; 128: 6.0 TB/s);
 //   256-wide heads: two teams of three warps that take tiles in turn: 24 KB a tile, five in flight (48 KB, three: 209 / 205);
-//   tagged words in place of a fence, a counter and a reload: 28.6 / 22.6 for 28 layers of 1,531;
+//   tagged words in place of a fence, a counter and a reload: 28.6 / 22.6 for 28 layers of 1,531 (as relaxed 64-bit accesses, with the
+//     fetching warp's last wait: 15.6 / 15.7);
 //   up to sixteen states merged at once, not eight, and the fetching warp ahead of the others: one of 24,001, 256-wide, eight layers
 //     71.9 / 71.2, 28 layers of 1,531 16.1 / 15.6;
 //   two runs of 128-wide heads: seven computing warps and the fetching one have 255 registers each, eight and one 168 and spill (8

@@ -65,7 +65,7 @@ constexpr int kStepFew = 7;                               // of a run, where mor
 // Tiles a CTA up to which a run has no more states than are merged at once: the second merge costs more than the CTAs left idle.  One
 // sequence, 32 heads on 2 of 128, four layers, us without / with (launches per layer): 4,096 positions 34.1 / 26.4 (26.7), 8,192 36.3 / 29.3
 // (32.8), 9,000 38.0 / 31.9 (34.5).  Up to four: 36.3 / 39.0 for the second; up to sixteen: 25.2 / 31.3 for 32,768 of 16 heads on 1 of 64.
-constexpr int kStepOnce = 8;
+constexpr unsigned kStepOnce = 8;
 constexpr int kStepCtrlBytes = 256;                       // barriers (full, empty: 24 at most), abort word
 
 // What a launch needs.  ok = 0: a geometry or batch that it does not cover.  hg 0: rows of 256 bytes and more are read in full wherever
@@ -190,7 +190,7 @@ __device__ __forceinline__ void step_body(const StepArgs& a)
     const int N = pre[a.batch], T = a.num_layers * groups * N, cta = blockIdx.x;
     // Few states to merge for a run where that costs a CTA up to three tiles, and no more than one merge takes where it costs up to eight.
     const int runs = a.num_layers * groups * a.batch, few = runs * kStepFew, once = runs * a.fan;
-    const int G = min(min((int)gridDim.x, T), T <= 3 * few ? few : T <= kStepOnce * once ? once : T);
+    const int G = min(min((int)gridDim.x, T), T <= 3 * few ? few : (unsigned)T <= kStepOnce * (unsigned)once ? once : T);
     if (tid == 0) a.launches[cta] = tag;
     if (cta >= G) return;
     // CTA c's share starts at floor(c T / G).  Divisions by way of floats: quotients below 2^20 are at most one off.

@@ -44,6 +44,8 @@ extern "C" {
 #define VTEB_LAUNCH_PROGRAMMATIC 1  /* programmatic dependent launch: the kernel may start
                                        before its predecessor in the stream has finished and
                                        orders itself with griddepcontrol.wait */
+#define VTEB_LAUNCH_NOT_CAPTURED 2  /* refused while the stream is being captured (as a graph launch is): the arguments
+                                     * are this launch's own, and a replay would repeat them */
 #define VTEB_LAUNCH_CLUSTER_SHIFT 8 /* bits 8 and up: blocks per thread-block cluster along x, 0 or 1
                                        for none, at most 16; has to divide the grid */
 

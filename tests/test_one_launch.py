@@ -479,6 +479,33 @@ def test_heads_a_block_serves_at_once(cuda_runtime, codegen, heads, hg):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("one", [None, False])
+def test_a_step_with_its_own_offsets_is_not_captured(cuda_runtime, codegen, one):
+    """Its offsets would be the replays' too: refused as a graph launch in a capture is, and the next step is right."""
+    rt = cuda_runtime
+    ex = executor(rt, codegen, (12, 2, 128), 1, 512, 4, one_launch=one)
+    try:
+        for l in range(4):
+            ex.fill_cache_on_device(l, l + 1)
+            ex.upload_layer(l, np.ones((1, 12, 128), dtype=np.float16))
+        off = np.array([300], dtype=np.int32)
+        good = ex.execute_decode_batch(off)
+        rt.stream_begin_capture()
+        with pytest.raises(CudaRuntimeError, match="900"):
+            ex.execute_decode_batch(off - 1, read_output=False)
+        try:
+            graph = rt.stream_end_capture()
+        except CudaRuntimeError:
+            assert one is False                                        # a refused graph launch ends the capture
+        else:
+            assert one is None and rt.graph_node_count(graph) == 0
+            rt.graph_destroy(graph)
+        assert np.array_equal(ex.execute_decode_batch(off), good)
+    finally:
+        ex.cleanup()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("heads", HEADS)
 @pytest.mark.parametrize("layers,lengths", [(1, [17000]), (1, [2100]), (2, [9000])], ids=str)
 def test_cut_runs_are_merged_once_or_twice(cuda_runtime, codegen, heads, layers, lengths):

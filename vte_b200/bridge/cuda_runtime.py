@@ -42,6 +42,7 @@ ATTR_L2_BYTES = 6
 ATTR_CLOCK_KHZ = 7
 
 LAUNCH_PROGRAMMATIC = 1
+LAUNCH_NOT_CAPTURED = 2
 LAUNCH_CLUSTER_SHIFT = 8
 
 ATTN_COMPAT = 1
@@ -656,14 +657,14 @@ class CudaRuntime:
 
     def prepare_launch(self, function, args: list, grid: tuple, block: tuple, shared_mem: int = 0, programmatic: bool = False):
         """A launch whose checks and argument list are made once: calling the result launches it on the runtime's stream, with what
-        its arguments hold by then."""
+        its arguments hold by then.  Refused in a capture: a replay would repeat what the arguments held."""
         self._validate_launch(function, grid, block, shared_mem, len(args))
         fval = _ptr_value(function)
         if shared_mem > self._props["shared_mem_per_block"] and self._smem_optin_set.get(fval, 0) < shared_mem:
             self._check_error(self._lib.vteb_func_set_max_dynamic_smem(ctypes.c_void_p(fval), int(shared_mem)), "cuFuncSetAttribute")
             self._smem_optin_set[fval] = int(shared_mem)
         arr, keep = self._marshal(args)
-        call, flags = self._lib.vteb_launch, LAUNCH_PROGRAMMATIC if programmatic else 0
+        call, flags = self._lib.vteb_launch, LAUNCH_NOT_CAPTURED | (LAUNCH_PROGRAMMATIC if programmatic else 0)
         rest = (ctypes.c_void_p(fval), *(ctypes.c_uint(int(x)) for x in (*grid, *block, shared_mem)), self._stream, arr, ctypes.c_uint(flags))
 
         def launch(_keep=keep):

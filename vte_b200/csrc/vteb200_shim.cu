@@ -375,6 +375,13 @@ int vteb_launch(void* function, unsigned gx, unsigned gy, unsigned gz, unsigned 
     const unsigned cluster = flags >> VTEB_LAUNCH_CLUSTER_SHIFT;
     if (cluster > 16 || (cluster > 1 && gx % cluster))
         return fail(VTEB_ERR_INVALID_ARGUMENT, "clusters of %u blocks do not divide a grid of %u", cluster, gx);
+    if (flags & VTEB_LAUNCH_NOT_CAPTURED) {
+        cudaStreamCaptureStatus status;
+        const int rc = check_rt(cudaStreamIsCapturing((cudaStream_t)stream, &status), "cudaStreamIsCapturing");
+        if (rc) return rc;
+        if (status != cudaStreamCaptureStatusNone)
+            return fail(cudaErrorStreamCaptureUnsupported, "a launch with arguments of its own is not captured (%d)", (int)cudaErrorStreamCaptureUnsupported);
+    }
     if ((flags & VTEB_LAUNCH_PROGRAMMATIC) || cluster > 1) {
         CUlaunchConfig cfg;
         memset(&cfg, 0, sizeof(cfg));

@@ -1,5 +1,7 @@
 """`vteb_split_kv_decode` for one sequence whose splits hold whole tiles: tensor-map copies over a cache whose rows the
 stride gives, 16-byte copies where the stride is 0."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -46,3 +48,16 @@ def test_one_sequence_of_whole_tiles(cuda_runtime, heads, compact):
     finally:
         for p in bufs:
             rt.safe_free(p, "direct entry cleanup")
+
+
+@pytest.mark.gpu
+def test_a_failed_call_does_not_fail_the_next(cuda_runtime):
+    """A failure is reported by the call that had it; a launch that is checked by the last error reports its own only."""
+    rt, p = cuda_runtime, ctypes.c_void_p()
+    assert rt._lib.vteb_malloc(ctypes.byref(p), 1 << 50) != 0          # a petabyte: refused at once
+    x = rt.safe_malloc(4096, "last error test output")
+    try:
+        rt.fill_normal_f16(x, 2048, 1)
+        rt.stream_synchronize()
+    finally:
+        rt.safe_free(x, "last error test cleanup")

@@ -31,6 +31,7 @@ int fail(int code, const char* fmt, ...) {
 
 int check_rt(cudaError_t e, const char* what) {
     if (e == cudaSuccess) return 0;
+    cudaGetLastError();                                   // reported here: a launch that is checked by the last error must not report it again
     snprintf(g_err, sizeof(g_err), "%s: %s (%d)", what, cudaGetErrorString(e), (int)e);
     return (int)e;
 }
